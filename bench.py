@@ -7,8 +7,7 @@ D=128, S=32768, bf16 inputs N(0,1) with 5 of the 128 K channels scaled x20, diag
 MXFP8 and the rest in MXFP4 unless the online router promotes them (statistic of the MXFP4 score tile >=
 TAU x that of the row's first key tile), P re-quantised to the tile's format before P.V (V quantised along
 the sequence).  One step = quantise Q and K (both formats, one pass each), quantise V and run the fused forward
-with the router inside it (band map, the forward - a promoted tile is done again in MXFP8 at the end of its row - and
-the exact forward behind it as its conditional fallback, whose CTAs return at once).  Metric: effective attention TFLOP/s =
+with the router inside it (a promoted tile is done again in MXFP8 at the end of its row).  Metric: effective attention TFLOP/s =
 4*B*Hq*S^2*D/2 / time.  With N > 1 every rank runs the same workload on its own batch element
 (batch x head sharding, no collective; weak scaling) and the value is the sum over ranks divided by
 the slowest rank's time.
@@ -41,7 +40,7 @@ import torch  # noqa: E402
 
 HQ, HKV, D = 32, 8, 128
 OUTLIERS = 5
-LAUNCHES_PER_STEP = 6      # quant Q, quant K, quant V, band map, forward, conditional exact forward (returns at once)
+LAUNCHES_PER_STEP = 4      # quant Q, quant K, quant V, forward
 TAU = 1.1                  # online router: a tile is promoted to MXFP8 iff its statistic >= TAU x the first key tile's
 # DRAM bytes (read + written) of one launch of the fused forward at S=8192, from an ncu capture; every term of it
 # (Q, K, V codes and scales, the output) grows linearly with S

@@ -179,11 +179,10 @@ int mpsa_route_online(void* map, const void* stat, int B, int Hq, int S, int Skv
  *   fp4_kind       0: the FP4 operands of Q.K^T are MXFP4 (above).  1: NVFP4 from mpsa_quant_nvfp4_bh (q4/k4 the same
  *                  packed codes, q4_sf/k4_sf [B,H,ceil(L/128),2,512] E4M3 scale tiles); fp4_scale is then the product
  *                  of the two tensor scales, applied to the scores of the FP4 tiles.  P.V keeps the MX formats.
- *   range_flag     optional (pv_mode 1): one int32, 0 on entry, private to this call.  When given, the forward runs
- *                  with the row reference fixed after the first key tile (block-scaled P carries its magnitude in
- *                  the scale codes, so nothing has to be rescaled while scores stay within 2^64 of that reference);
- *                  a score beyond that sets the word, and the exact kernel, launched behind the first one, then
- *                  recomputes the output.  Results are the same either way.  NULL: the exact kernel only.
+ *   range_flag     optional: one int32, 0 on entry, private to this call.  The forward runs with a fixed reference per row
+ *                  (see csrc/attn.cu); query tiles with a row whose maximum lies outside what that reference serves are
+ *                  done again inside the same launch with the exact row maxima, and the word is then set to 1.  Results
+ *                  are the same with or without it.
  *   acc_in, lse_in optional, together: an earlier partial result (fp32 [B,Hq,S,D], log2 denominators [B,Hq,S]) over OTHER keys;
  *                  out (fp32) and lse then receive the merged result (buffers distinct from the inputs), which saves
  *                  the separate mpsa_attn_merge pass
@@ -208,14 +207,11 @@ int mpsa_attn_fwd(const void* q8, const void* q8_sf, const void* q4, const void*
  *                 lse), else to lse
  *   stat          optional fp32 [B,Hq,nq,nk], OUTPUT: the router statistic of every tile outside the band (the
  *                 other cells are left as they are); stat_scratch: unused, may be NULL
- *   range_flag    device int, zero on entry.  The forward runs with the row reference fixed after the first key tile; if a
- *                 score leaves its 2^64 headroom the word is set and the exact kernel, launched behind it, recomputes the
- *                 output over the final map (which does not depend on the reference) - same results either way.
- * Three launches: band map; the forward (a promoted tile's MXFP4 result is left out and the tile is done again in MXFP8 by
- * the same CTA after the row's own tiles); the conditional exact forward, whose CTAs return at once unless the word is set.
+ *   range_flag    device int, zero on entry: as in mpsa_attn_fwd
+ * One launch: every CTA writes the map rows of its query tiles itself, and a tile that is promoted has its MXFP4 result left
+ * out and is done again in MXFP8 after the row's own tiles.
  * At most 4096 key tiles (512K keys).  Skv_pad, fp8_fmt, the operand pointers: as in mpsa_attn_fwd.
- *   stages        which of these to launch, a mask of 1 (band map), 2 (forward), 8 (conditional exact forward) (4 is
- *                 accepted and ignored); 15 for the operation itself, a subset for timing one stage alone. */
+ *   stages        2 or any mask with it: the operation; 1 alone: the band map only.  4 and 8 are accepted and ignored. */
 int mpsa_attn_fwd_routed(const void* q8, const void* q8_sf, const void* q4, const void* q4_sf, const void* k8,
                          const void* k8_sf, const void* k4, const void* k4_sf, const void* vt8, const void* v8_sf,
                          const void* vt4, const void* v4_sf, void* map, int band, float tau, void* out, int out_dtype,

@@ -2,6 +2,7 @@
 // code, and leaves a message retrievable with mpsa_last_error().  No exception crosses the
 // boundary and nothing here allocates device memory.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -14,9 +15,48 @@
 namespace mpsa {
 int set_error(int code, const char* fmt, ...);
 int check_launch(const char* what);
-// launchers shared between translation units; run_if: a device word, the kernels do nothing while it is zero (may be null)
-int launch_route_stat(const void* q4, const void* q4_sf, const void* k4, const void* k4_sf, void* stat, void* scratch, int B,
-                      int Hq, int Hkv, int S, int Skv, int causal, int* status, const int* run_if, void* stream);
-int launch_route_online(void* map, const void* stat, int B, int Hq, int S, int Skv, int causal, int band, float tau,
-                        float skip_tau, int use_skip, const int* run_if, void* stream);
+int sm_count();                       // of the current device
+
+// Opt-in for more than 48 KB of dynamic shared memory: a per-device attribute of a kernel, set by the first launch on
+// each device (ID tells the kernels of one function type apart).
+template <int ID, typename F>
+bool allow_smem(F* kernel, int bytes) {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<bool> done[kMaxDevices];
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (dev >= 0 && dev < kMaxDevices && done[dev].load(std::memory_order_acquire)) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (dev >= 0 && dev < kMaxDevices) done[dev].store(true, std::memory_order_release);
+  return true;
+}
+
+// One call of the fused forward (see mpsa_attn_fwd for the operands).  map null: the band rule (band, uniform) instead.
+struct AttnCall {
+  const void *q8 = nullptr, *q8_sf = nullptr, *q4 = nullptr, *q4_sf = nullptr;
+  const void *k8 = nullptr, *k8_sf = nullptr, *k4 = nullptr, *k4_sf = nullptr;
+  const void *vt = nullptr, *vt8 = nullptr, *v8_sf = nullptr, *vt4 = nullptr, *v4_sf = nullptr;
+  int pv_mode = 0;
+  const void* map = nullptr;
+  long long map_sb = 0, map_sh = 0;
+  int band = 1, uniform = 0;            // uniform: 0 no, 1 MXFP8, 2 FP4
+  bool route = false;                   // online router inside (map_rw: the map it writes)
+  float tau = 0.0f;
+  void *map_rw = nullptr, *stat_out = nullptr;
+  void* out = nullptr;
+  int out_dtype = 0;
+  void* lse = nullptr;
+  int B = 0, Hq = 0, Hkv = 0, S = 0, Skv = 0, D = 0, Skv_pad = 0, causal = 0, fp8_fmt = 1, fp4_kind = 0;
+  bool depth64 = false;                 // the upper 64 of the 128 depth elements of Q and K are zero blocks
+  float fp4_scale = 0.0f;
+  const void *ts_q = nullptr, *ts_k = nullptr;   // NVFP4: the two tensor scales in device memory, instead of fp4_scale
+  int* range_flag = nullptr;
+  int* counter = nullptr;               // a device word, zero on entry: work items are handed out in turn (fixed schedule without it)
+  const void *acc_in = nullptr, *lse_in = nullptr;
+  int* status = nullptr;
+};
+int attn_forward(const AttnCall& c, cudaStream_t st);
 }  // namespace mpsa

@@ -7,10 +7,6 @@
 #include <cuda_runtime.h>
 #include <cuda.h>
 
-#ifndef MPSA_WAIT_MODE
-#define MPSA_WAIT_MODE 0
-#endif
-
 namespace mpsa {
 
 // ---- status word written by kernels -----------------------------------------------------
@@ -25,6 +21,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// True in one lane of a converged warp.  A single-thread role must be entered through this and not through `lane == 0`:
+// only then does the compiler know that one lane runs the region and keep descriptors and addresses in uniform registers.
+// Measured (2 MMAs, a commit and a wait per round, next to 16 busy warps): 141 cycles a round, 410 with `lane == 0`.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 // ---- mbarrier ---------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -35,25 +40,32 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {      // by shared address
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
 // One probe of the barrier phase (the hardware may hold the thread for a short, implementation
 // defined time before answering).
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-#if MPSA_WAIT_MODE == 1
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 0x989680;\n\t"
-#else
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-#endif
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(bar), "r"(parity)
       : "memory");
+  return ok != 0;
+}
+
+// The same without ever holding the thread.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
 
@@ -63,29 +75,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 constexpr long long kWaitLimitCycles = 4000000000ll;
 
 // Bounded wait.  Returns false when the limit expired (and records `code` in *status) or when
-// another role already recorded a failure, so that every role unwinds promptly.
-// BACKOFF = false is for pipelines whose phases last a few hundred cycles, where the back-off below would
-// cost more than the wait itself.  `limit` (SM clock cycles) defaults to kWaitLimitCycles.
-template <bool BACKOFF = true>
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code,
-                                          long long limit = kWaitLimitCycles) {
-  if (mbar_try_wait(bar, parity)) return true;
-#if MPSA_WAIT_MODE == 0
-  // Reading the global nanosecond timer is slow; doing it once after the first unsuccessful probe
-  // doubles as a back-off that keeps a waiting warp out of its scheduler's way.
-  if (BACKOFF) {
-    unsigned long long g0;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g0));
-    (void)g0;
-  }
-#endif
+// another role already recorded a failure, so that every role unwinds promptly.  `limit` (SM clock
+// cycles) defaults to kWaitLimitCycles.  The loop behind the first probe is kept out of line: the
+// hot loops that wait stay small (instruction fetch is a bottleneck of the attention kernels).
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int* status, int code, long long limit) {
   const long long t0 = clock64();
   uint32_t spins = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
-#if MPSA_WAIT_MODE == 2
-    __nanosleep(40);
-#endif
     if ((++spins & 0x3ff) == 0) {
       if (*(volatile int*)status != KS_OK) return false;
       if (clock64() - t0 > limit) {
@@ -94,6 +91,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
       }
     }
   }
+}
+__device__ __forceinline__ bool mbar_wait_at(uint32_t bar, uint32_t parity, int* status, int code) {   // by shared address
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
+  return mbar_wait_slow(bar, parity, status, code, kWaitLimitCycles);
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code,
+                                          long long limit = kWaitLimitCycles) {
+  const uint32_t a = smem_u32(bar);
+  if (__builtin_expect(mbar_try_wait(a, parity), 1)) return true;
+  return mbar_wait_slow(a, parity, status, code, limit);
 }
 
 // ---- TMA --------------------------------------------------------------------------------

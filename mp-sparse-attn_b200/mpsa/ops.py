@@ -558,11 +558,10 @@ def attention_forward_quantized(qq: QuantizedOperand, kq: QuantizedOperand, vt, 
     lse = torch.empty((B, Hq, S), dtype=torch.float32, device=dev) if return_lse else None
     _raise_if_failed(dev)
     st = status_word(dev)
-    # quantised P.V: a per-call word lets the library run the fixed-reference kernel with the exact one as its
-    # conditional fallback (same results, see include/mpsa.h)
+    # `lazy` is accepted for earlier callers; it only decides whether the word below is kept for inspection
     flag = torch.zeros(1, dtype=torch.int32, device=dev) if (requant and lazy) else None
     global _last_range_flag
-    _last_range_flag = flag                       # kept for inspection: non-zero after the call = the exact kernel took over
+    _last_range_flag = flag                       # non-zero after the call = some query tiles were done again (include/mpsa.h)
     with torch.cuda.device(dev):
         rc = _lib.load().mpsa_attn_fwd(
             q8.data_ptr(), q8s.data_ptr(), q4.data_ptr(), q4s.data_ptr(),
@@ -583,8 +582,7 @@ def attention_forward_routed(qq: QuantizedOperand, kq: QuantizedOperand, vq: "Qu
     """The causal forward with the online router inside it (quantised P.V, MXFP4/MXFP8 operands): no stand-alone
     statistic pass.  A tile the router promotes is done again in MXFP8 by the same CTA after the row's own tiles (its
     MXFP4 result is left out).  Same precision map as precision_map_online(router_statistic(...), tau=tau).
-    stages: mask of the launches to make (1 band map, 2 forward, 8 the conditional exact forward behind it; 4 is ignored) -
-    a subset is for timing a stage alone.  return_stat: also the router statistic of the tiles outside the band (fp32
+    stages: accepted for earlier callers; any mask with 2 in it is the operation (one launch), 1 alone only the band map.  return_stat: also the router statistic of the tiles outside the band (fp32
     [B,Hq,nq,nk], zero elsewhere)."""
     if not isinstance(vq, QuantizedV):
         raise ValueError("the routed forward needs V quantised along the sequence (quantize_v_seq)")
