@@ -131,7 +131,7 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_b);
       // batched launch (blockIdx.z): operands, scale tiles and C of the batches lie one after the other
@@ -182,7 +182,7 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     // Issuing a tcgen05 instruction costs its thread ~75 cycles; a stage is 4 MMAs and 3 (MXFP8), 6 (MXFP4) or 12
     // (NVFP4) scale-tile copies, against ~710 cycles of tensor time.  The copies therefore have a thread of their own
     // (warps 6..), which signal through sf_ready[stage].
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t idj[4];                              // instruction descriptors of the four instructions of a stage
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -239,7 +239,7 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     // ------------------------------ scale-tile copiers -------------------------
     // copier ci takes the scale tiles c with c * NCOP / NC == ci of every stage; each commits once per stage
     const int ci = warp - 6;
-    if (SPLIT && ci < NCOP && lane == 0) {
+    if (SPLIT && ci < NCOP && elect_one()) {
       const uint64_t sfdesc0 = sdesc_sf_tile(smem_u32(smem + GEMM_A_BYTES + GEMM_B_BYTES));
       constexpr uint64_t STAGE_STEP = GEMM_STAGE_BYTES >> 4, SFB_STEP = GEMM_SFA_BYTES >> 4, TILE_STEP = 512 >> 4;
       bool ok = true;
