@@ -218,6 +218,43 @@ int mpsa_attn_fwd_routed(const void* q8, const void* q8_sf, const void* q4, cons
                          void* lse, void* lse_final, void* stat, void* stat_scratch, int B, int Hq, int Hkv, int S, int Skv,
                          int D, int Skv_pad, int fp8_fmt, int stages, int* range_flag, int* status, void* stream);
 
+/* A whole attention call on bf16 / fp16 inputs: quantises Q and K, prepares V and runs the fused forward - the work of
+ * mxfp_attn_kernel (ours/mxfp_attn_kernel.py:19-74) in two launches, three with smooth_k.  Strides are in elements.
+ *   q [B,Hq,S,D], k / v [B,Hkv,Skv,D], D 64 or 128.  k null: keys and values prepared earlier (k8 .. v4_sf, Skv_pad, as in
+ *                 mpsa_attn_fwd, depth padded to 128) are used instead; formats that `uniform` leaves out may be null
+ *   band, uniform precision rule: MXFP8 within `band` tiles of the diagonal; uniform 1: every tile MXFP8, 2: MXFP4, 0: neither
+ *   route, tau    the online router inside the forward (causal, pv_mode 1), as in mpsa_attn_fwd_routed
+ *   q_scale       softmax scale * log2(e), folded into Q
+ *   workspace     mpsa_attention_workspace bytes, 256-byte aligned, private to the call until it has finished on the GPU
+ *   range_flag    optional word, set to zero by the call and then used as in mpsa_attn_fwd */
+typedef struct mpsa_attention_args {
+  const void *q, *k, *v;
+  long long q_sb, q_sh, q_sl, k_sb, k_sh, k_sl, v_sb, v_sh, v_sl;
+  const void *k8, *k8_sf, *k4, *k4_sf, *vt, *vt8, *v8_sf, *vt4, *v4_sf;
+  void* out;
+  void* workspace;
+  long long workspace_bytes;
+  int *range_flag, *status;
+  int in_dtype, out_dtype, B, Hq, Hkv, S, Skv, D, Skv_pad, causal, band, uniform, route, pv_mode, fp8_fmt, smooth_k;
+  float q_scale, tau;
+} mpsa_attention_args;
+long long mpsa_attention_workspace(const mpsa_attention_args* args);
+int mpsa_attention(const mpsa_attention_args* args, void* stream);
+
+/* Two operands (Q and K) quantised along the depth in one launch, in the reference's output format: what quant_mxfp4
+ * (ours/quant_mxint8.py:453-512; fp8_fmt 0, one E2M1 code per byte) and quant_mxfp8e5 (:223-272; fp8_fmt 1, or 2 for E4M3)
+ * return.  x[i] [B,H[i],L[i],D] bf16 / fp16, codes[i] strided, scales[i] [B,H[i],L[i],D/32]; D 64 or a multiple of 128. */
+typedef struct mpsa_quant_pair_args {
+  const void* x[2];
+  void* codes[2];
+  void* scales[2];
+  long long x_sb[2], x_sh[2], x_sl[2], c_sb[2], c_sh[2], c_sl[2];
+  int H[2], L[2];
+  float s[2];
+  int in_dtype, B, D, fp8_fmt;
+} mpsa_quant_pair_args;
+int mpsa_quant_pair(const mpsa_quant_pair_args* args, void* stream);
+
 /* Merges a partial attention result into an accumulator: acc fp32 [rows, D] and lse_acc fp32 [rows] are
  * updated in place with part [rows, D] (part_dtype 0 f32, 1 f16, 2 bf16) and lse_part, where every lse is
  * log2 of the softmax denominator of its (disjoint) key set as written by mpsa_attn_fwd; rows with

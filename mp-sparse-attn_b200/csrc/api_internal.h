@@ -50,6 +50,7 @@ struct AttnCall {
   int out_dtype = 0;
   void* lse = nullptr;
   int B = 0, Hq = 0, Hkv = 0, S = 0, Skv = 0, D = 0, Skv_pad = 0, causal = 0, fp8_fmt = 1, fp4_kind = 0;
+  bool need8 = true, need4 = true;      // operand formats the map can select; the pointers of the other may be null
   bool depth64 = false;                 // the upper 64 of the 128 depth elements of Q and K are zero blocks
   float fp4_scale = 0.0f;
   const void *ts_q = nullptr, *ts_k = nullptr;   // NVFP4: the two tensor scales in device memory, instead of fp4_scale
@@ -59,4 +60,8 @@ struct AttnCall {
   int* status = nullptr;
 };
 int attn_forward(const AttnCall& c, cudaStream_t st);
+// partial column sums of x [B,H,L,D], [B*H, nchunk, D] floats, nchunk = col_sum_chunks(L)
+int col_sum_chunks(int L);
+int col_sums(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h, long long xs_l, float* part,
+             int nchunk, cudaStream_t st);
 }  // namespace mpsa

@@ -36,6 +36,7 @@
 // on TMEM data, takes 1003 cycles a tile; with all hand-offs and MMAs 1160.
 #include "api_internal.h"
 #include "common.cuh"
+#include "prep.h"
 #include "tma_host.h"
 
 #include <cuda_bf16.h>
@@ -128,6 +129,7 @@ struct AttnParams {
   int group;                         // q-heads per KV head
   int* counter;                      // optional, zero on entry: items are handed out in turn instead of by a fixed schedule
   int n_lists, list_cap;             // item slots in use (fewer than ATT_MAX_SLOTS for very long rows) and entries of a visit list
+  bool load8, load4;                 // formats of Q in use
   bool out32;                        // every row of `out` starts on a 32-byte boundary
 };
 
@@ -514,11 +516,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         const long long qsf = ((long long)head * nq + qi) * 512;
         uint8_t* dst = smem + ATT_OFF_Q + qb * ATT_Q_BYTES;
         uint8_t* sf = smem + ATT_OFF_SFQ + qb * 1536;
-        mbar_arrive_expect_tx(&q_full[qb], ATT_Q_BYTES + 512 + SF4);
-        tma_load_2d(dst, &tm_q8, &q_full[qb], 0, q_row);
-        tma_load_2d(dst + ATT_Q8_BYTES, &tm_q4, &q_full[qb], 0, q_row);
-        bulk_load(sf, p.q8_sf + qsf, 512, &q_full[qb]);
-        bulk_load(sf + 512, p.q4_sf + (NVF4 ? 2 * qsf : qsf), SF4, &q_full[qb]);
+        mbar_arrive_expect_tx(&q_full[qb], (p.load8 ? ATT_Q8_BYTES + 512 : 0) + (p.load4 ? ATT_Q4_BYTES + SF4 : 0));
+        if (p.load8) {
+          tma_load_2d(dst, &tm_q8, &q_full[qb], 0, q_row);
+          bulk_load(sf, p.q8_sf + qsf, 512, &q_full[qb]);
+        }
+        if (p.load4) {
+          tma_load_2d(dst + ATT_Q8_BYTES, &tm_q4, &q_full[qb], 0, q_row);
+          bulk_load(sf + 512, p.q4_sf + (NVF4 ? 2 * qsf : qsf), SF4, &q_full[qb]);
+        }
         ++q_loads;
       };
       int ls = 0;
@@ -1408,6 +1414,13 @@ extern "C" int mpsa_prepare_vt(const void* v, int in_dtype, void* vt, int B, int
   if (!v || !vt || B <= 0 || H <= 0 || Skv <= 0 || D <= 0) return set_error(MPSA_ERR_BAD_ARG, "prepare_vt: bad argument");
   if (Skv_pad < Skv || Skv_pad % 8) return set_error(MPSA_ERR_BAD_ARG, "prepare_vt: Skv_pad must be >= Skv and a multiple of 8");
   if (B * H > 65535) return set_error(MPSA_ERR_UNSUPPORTED, "prepare_vt: B*H must be below 65536");
+  if (in_dtype != 2 && (D == 64 || D == 128) && Skv_pad % 128 == 0 && !((uintptr_t)v % 16) && !((uintptr_t)vt % 16) && !((vs_b * 2) % 16) &&
+      !((vs_h * 2) % 16) && !((vs_l * 2) % 16)) {
+    PrepCall c;
+    c.D = D;
+    c.v.v = v; c.v.B = B; c.v.H = H; c.v.Skv = Skv; c.v.pitch = Skv_pad; c.v.vs_b = vs_b; c.v.vs_h = vs_h; c.v.vs_l = vs_l; c.v.vt16 = vt;
+    return prep_launch(c, in_dtype, true, false, 1, (cudaStream_t)stream);
+  }
   dim3 grid((Skv_pad + 63) / 64, (D + 63) / 64, B * H);
   cudaStream_t st = (cudaStream_t)stream;
   if (in_dtype == 0) prepare_vt_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)v, (__half*)vt, H, Skv, D, Skv_pad, vs_b, vs_h, vs_l);
@@ -1446,7 +1459,12 @@ int launch_attn(int grid, size_t smem, cudaStream_t st, const AttnMaps& m, const
 }
 }  // namespace
 
-int attn_forward(const AttnCall& c, cudaStream_t st) {
+int attn_forward(const AttnCall& call, cudaStream_t st) {
+  AttnCall c = call;
+  if (c.map || c.route || !c.uniform) c.need8 = c.need4 = true;
+  // a format that is never selected is not loaded; its tensor maps need an address all the same
+  if (!c.need8) { c.q8 = c.q4; c.q8_sf = c.q4_sf; c.k8 = c.k4; c.k8_sf = c.k4_sf; c.vt8 = c.vt4; c.v8_sf = c.v4_sf; }
+  if (!c.need4) { c.q4 = c.q8; c.q4_sf = c.q8_sf; c.k4 = c.k8; c.k4_sf = c.k8_sf; c.vt4 = c.vt8; c.v4_sf = c.v8_sf; }
   if (!c.q8 || !c.q8_sf || !c.q4 || !c.q4_sf || !c.k8 || !c.k8_sf || !c.k4 || !c.k4_sf || !c.out || !c.status)
     return set_error(MPSA_ERR_BAD_ARG, "attn_fwd: null pointer");
   if (c.pv_mode != 0 && c.pv_mode != 1) return set_error(MPSA_ERR_BAD_ARG, "attn_fwd: pv_mode must be 0 (fp16 P.V) or 1 (quantised P.V)");
@@ -1503,7 +1521,7 @@ int attn_forward(const AttnCall& c, cudaStream_t st) {
   p.out = c.out; p.out_dtype = c.out_dtype; p.lse = (float*)c.lse; p.acc_in = c.acc_in; p.lse_in = (const float*)c.lse_in;
   p.tau = c.tau; p.map_rw = (uint8_t*)c.map_rw; p.stat_out = (float*)c.stat_out; p.range_flag = c.range_flag; p.status = c.status;
   p.n_items = (int)n_items; p.group = c.Hq / c.Hkv; p.counter = c.counter;
-  p.out32 = (uintptr_t)c.out % 32 == 0;
+  p.out32 = (uintptr_t)c.out % 32 == 0; p.load8 = c.need8; p.load4 = c.need4;
   p.list_cap = ((c.route ? 2 * nk : nk) + 7) & ~7;
   p.n_lists = std::min(ATT_MAX_SLOTS, (ATT_SMEM_MAX - 1024 - ATT_OFF_LIST) / (p.list_cap * 2));
   const size_t smem = ATT_OFF_LIST + (size_t)p.n_lists * p.list_cap * 2 + 1024;

@@ -2,6 +2,8 @@
 arithmetic runs in the hand-written sm_100a kernels of libmpsa.so."""
 from __future__ import annotations
 
+import ctypes
+import struct
 from dataclasses import dataclass
 from typing import Optional
 
@@ -16,12 +18,43 @@ _IN_DTYPE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 _OUT_DTYPE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2, torch.float8_e5m2: 3}
 _FP8_QUANT = {"e5m2": 1, "e4m3": 2}
 _FP8_DESC = {"e5m2": 1, "e4m3": 0}
-_status = {}
 _last_range_flag = None
 
 
 def _stream():
     return torch.cuda.current_stream().cuda_stream
+
+
+class _DeviceState:
+    """Per-device words the kernels write: the status word, and the range flag of the one-call attention path."""
+
+    def __init__(self, index):
+        self.index = index
+        self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.status_ptr = self.status.data_ptr()
+        self.word = ctypes.c_int.from_address(self.status_ptr)       # read on every call: no tensor machinery
+        with torch.cuda.device(index):
+            self.range_flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+        self.range_ptr = self.range_flag.data_ptr()
+
+
+_states = {}
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+
+
+def _state(index) -> _DeviceState:
+    st = _states.get(index)
+    if st is None:
+        st = _states[index] = _DeviceState(index)
+    return st
+
+
+def _on_device(index, fn, *args):
+    """fn(*args, stream) with `index` as the current device: the usual case costs one comparison."""
+    if torch.cuda.current_device() == index:
+        return fn(*args, _raw_stream(index))
+    with torch.cuda.device(index):
+        return fn(*args, _raw_stream(index))
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -38,10 +71,8 @@ def status_word(device) -> torch.Tensor:
     """Per-device int32 word the kernels write when one of their bounded waits expires.  It lives in pinned host memory
     (reachable from the device under unified addressing: the kernels touch it only after a wait has already failed
     1024 probes), so the host can look at it before every launch without synchronising."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32).pin_memory()
-    return _status[key]
+    index = torch.device(device).index
+    return _state(torch.cuda.current_device() if index is None else index).status
 
 
 _WAIT_NAMES = {1: "TMA bytes", 2: "tensor-core commit", 3: "pipeline hand-off"}
@@ -51,10 +82,11 @@ def _raise_if_failed(device):
     """Raise if a kernel that has already finished on `device` recorded an expired wait.  No synchronisation: called by
     the wrappers before they launch, so that a failure surfaces at the next call at the latest instead of being carried
     along silently (a kernel that finds the word set gives up its own long waits too)."""
-    w = status_word(device)
-    code = int(w[0])
+    index = torch.device(device).index
+    st = _state(torch.cuda.current_device() if index is None else index)
+    code = st.word.value
     if code != 0:
-        w.zero_()
+        st.word.value = 0
         raise _lib.MpsaError(f"a kernel gave up waiting (status {code}: {_WAIT_NAMES.get(code, '?')})")
 
 
@@ -186,6 +218,48 @@ def quantize_mx(x: torch.Tensor, scale: float = 1.0, *, want_fp8=True, want_fp4=
                                                     center.data_ptr(), _FP8_QUANT[fp8_elem], *outs)
     _lib.check(rc)
     return out
+
+
+_QUANT_PAIR_ARGS = struct.Struct("@2Q2Q2Q2q2q2q2q2q2q2i2i2f4i")     # mpsa_quant_pair_args of include/mpsa.h
+
+
+def quantize_pair(q: torch.Tensor, k: torch.Tensor, sq: float, sk: float, fmt: str, tensor_layout: str = "HND"):
+    """q and k quantised along the depth in the reference's output format: (codes, scales) of each, uint8.  fmt "mxfp4" (one
+    code per byte), "e5m2" or "e4m3".  One launch where the operands allow it (16 bits, aligned, depth 64 or a multiple of 128)."""
+    _require_cuda(q, k)
+    dt = q.dtype
+    in_dtype = 0 if dt is torch.bfloat16 else 1 if dt is torch.float16 else None
+    if in_dtype is not None and k.dtype is dt and q.dim() == 4 and k.dim() == 4 and q.shape[0] == k.shape[0] and \
+            q.shape[3] == k.shape[3] and q.get_device() == k.get_device() and (q.shape[3] == 64 or q.shape[3] % 128 == 0) and \
+            sq > 0.0 and sk > 0.0 and tensor_layout in ("HND", "NHD"):
+        qs, ks = _strides16(q), _strides16(k)
+        if qs is not None and ks is not None:
+            hnd = tensor_layout == "HND"
+            B, a1, a2, D = q.shape
+            _, b1, b2, _ = k.shape
+            (Hq, Lq), (Hk, Lk) = ((a1, a2), (b1, b2)) if hnd else ((a2, a1), (b2, b1))
+            dev = q.device
+            qc, kc = torch.empty(q.shape, dtype=torch.uint8, device=dev), torch.empty(k.shape, dtype=torch.uint8, device=dev)
+            qsc = torch.empty((B, Hq, Lq, D // 32), dtype=torch.uint8, device=dev)
+            ksc = torch.empty((B, Hk, Lk, D // 32), dtype=torch.uint8, device=dev)
+            if not hnd:
+                qs, ks = (qs[0], qs[2], qs[1]), (ks[0], ks[2], ks[1])
+            cq = (Hq * Lq * D, Lq * D, D) if hnd else (Hq * Lq * D, D, Hq * D)
+            ck = (Hk * Lk * D, Lk * D, D) if hnd else (Hk * Lk * D, D, Hk * D)
+            args = _QUANT_PAIR_ARGS.pack(q.data_ptr(), k.data_ptr(), qc.data_ptr(), kc.data_ptr(), qsc.data_ptr(), ksc.data_ptr(),
+                                         qs[0], ks[0], qs[1], ks[1], qs[2], ks[2], cq[0], ck[0], cq[1], ck[1], cq[2], ck[2],
+                                         Hq, Hk, Lq, Lk, sq, sk, in_dtype, B, D, 0 if fmt == "mxfp4" else _FP8_QUANT[fmt])
+            rc = _on_device(q.get_device(), _lib.load().mpsa_quant_pair, args)
+            if rc:
+                _lib.check(rc)
+            return qc, qsc, kc, ksc
+    fp4 = fmt == "mxfp4"
+    out = []
+    for x, s in ((q, sq), (k, sk)):
+        r = quantize_mx(x, s, want_fp8=not fp4, want_fp4=fp4, reference_format=True, kernel_format=False,
+                        fp8_elem="e5m2" if fp4 else fmt, tensor_layout=tensor_layout)
+        out += [r.fp4_unpacked, r.fp4_scales] if fp4 else [r.fp8, r.fp8_scales]
+    return tuple(out)
 
 
 def quantize_int8(x: torch.Tensor, scale: float = 1.0, tensor_layout="HND"):
@@ -397,6 +471,104 @@ def prepare_kv(k: torch.Tensor, v: torch.Tensor, *, pv_mode: str = "fp16", fp8_e
     return kq, vt
 
 
+_ATTENTION_ARGS = struct.Struct("@3Q9q9Q2Qq2Q16i2f")       # mpsa_attention_args of include/mpsa.h
+_workspace_bytes = {}                                        # problem -> workspace size (bounded)
+_UNIFORM = {None: 0, "fp8": 1, "fp4": 2}
+
+
+def _strides16(t):
+    """Strides of a 4-D 16-bit tensor if the one-call path can read it as it is, else None."""
+    a, b, c, d = t.stride()
+    if d != 1 or (a | b | c) & 7 or t.data_ptr() & 15:
+        return None
+    return a, b, c
+
+
+def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out_dtype, pv_mode, route, tau, smooth_k):
+    """attention_forward through one C call (mpsa_attention), or None where that entry does not take the operands."""
+    dt = q.dtype
+    in_dtype = 0 if dt is torch.bfloat16 else 1 if dt is torch.float16 else None
+    qs = _strides16(q)
+    if in_dtype is None or qs is None or uniform not in _UNIFORM or out_dtype not in (torch.float32, torch.float16, torch.bfloat16) \
+            or fp8_elem not in _FP8_DESC or not sq > 0.0:
+        return None
+    B, Hq, S, D = q.shape
+    index = q.get_device()
+    uni = _UNIFORM[uniform]
+    skv_pad = 0
+    if kv is None:
+        if k.dtype is not dt or v.dtype is not dt or k.shape != v.shape or k.shape[0] != B or k.shape[3] != D or \
+                k.get_device() != index or v.get_device() != index:
+            return None
+        _, Hkv, Skv, _ = k.shape
+        ks, vs = _strides16(k), _strides16(v)
+        if ks is None or vs is None:
+            return None
+        kp, vp = k.data_ptr(), v.data_ptr()
+        prepared = (0,) * 9
+    else:
+        kq, vt = kv
+        codes = kq.fp8 if kq.fp8 is not None else kq.fp4
+        Hkv, Skv = codes.shape[1], codes.shape[2]
+        requant = isinstance(vt, QuantizedV)
+        pv_mode = "requant" if requant else "fp16"
+        skv_pad = (vt.vt8 if requant else vt).shape[-1]
+        if codes.get_device() != index or not _prepared_fits(kq, vt, requant, B, Hkv, Skv, D, skv_pad, uni, fp8_elem):
+            return None
+        ks = vs = (0, 0, 0)
+        kp = vp = 0
+        prepared = (_ptr(kq.fp8) or 0, _ptr(kq.fp8_sf) or 0, _ptr(kq.fp4) or 0, _ptr(kq.fp4_sf) or 0) + (
+            (0, vt.vt8.data_ptr(), vt.v8_sf.data_ptr(), vt.vt4.data_ptr(), vt.v4_sf.data_ptr()) if requant
+            else (vt.data_ptr(), 0, 0, 0, 0))
+    if Hq % Hkv or (causal and Skv < S):
+        return None
+    st = _state(index)
+    if st.word.value:
+        _raise_if_failed(q.device)
+    pv = 1 if pv_mode == "requant" else 0
+    ints = (in_dtype, _OUT_DTYPE[out_dtype], B, Hq, Hkv, S, Skv, D, skv_pad, int(causal), band, uni, int(route), pv,
+            _FP8_DESC[fp8_elem], int(smooth_k))
+    lib = _lib.load()
+    key = (ints, kp == 0)
+    need = _workspace_bytes.get(key)
+    if need is None:
+        need = lib.mpsa_attention_workspace(_ATTENTION_ARGS.pack(1, int(kp != 0), int(vp != 0), *qs, *ks, *vs, *prepared, 0, 0, 0, 0, 0,
+                                                                *ints, sq, tau))
+        if need < 0:
+            _lib.check(need)
+        if len(_workspace_bytes) >= 1024:
+            _workspace_bytes.clear()
+        _workspace_bytes[key] = need
+    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+    out = torch.empty((B, Hq, S, D), dtype=out_dtype, device=q.device)
+    global _last_range_flag
+    _last_range_flag = st.range_flag if pv else None
+    args = _ATTENTION_ARGS.pack(q.data_ptr(), kp, vp, *qs, *ks, *vs, *prepared, out.data_ptr(), ws.data_ptr(), need, st.range_ptr,
+                                st.status_ptr, *ints, sq, tau)
+    rc = _on_device(index, lib.mpsa_attention, args)
+    if rc:
+        _lib.check(rc)
+    return out
+
+
+def _prepared_fits(kq, vt, requant, B, Hkv, Skv, D, pad, uni, fp8_elem):
+    """Whether prepared keys and values have the dense layout the kernels read (depth padded to 128)."""
+    nk = -(-Skv // 128)
+    if kq.fp4_kind != "mxfp4" or kq.fp8_elem != fp8_elem or pad % 128 or pad < nk * 128:
+        return False
+    rows = B * Hkv * Skv
+    for t, sf, row, unused in ((kq.fp8, kq.fp8_sf, 128, 2), (kq.fp4, kq.fp4_sf, 64, 1)):
+        if uni == unused:
+            continue
+        if t is None or sf is None or t.numel() != rows * row or sf.numel() != B * Hkv * nk * 512 or not t.is_contiguous() or \
+                not sf.is_contiguous():
+            return False
+    if not requant:
+        return tuple(vt.shape) == (B, Hkv, D, pad) and vt.dtype is torch.float16 and vt.is_contiguous()
+    return vt.fp8_elem == fp8_elem and tuple(vt.vt8.shape) == (B, Hkv, D, pad) and tuple(vt.vt4.shape) == (B, Hkv, D, pad // 2) and \
+        vt.v8_sf.numel() == vt.v4_sf.numel() == B * Hkv * (pad // 128) * 512 and vt.vt8.is_contiguous() and vt.vt4.is_contiguous()
+
+
 def attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool, band: int = 1,
                       prec_map: Optional[torch.Tensor] = None, uniform: Optional[str] = None,
                       sm_scale: Optional[float] = None, fp8_elem: str = "e5m2",
@@ -439,6 +611,16 @@ def attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, caus
     if D not in (64, 128):
         raise ValueError("headdim should be in [64, 128].")
     sq = q_side_scale(D, sm_scale)
+    online = router == "online"
+    requant = isinstance(kv[1], QuantizedV) if kv is not None else pv_mode == "requant"
+    if rope is None and prec_map is None and fp4_kind == "mxfp4" and skip_thresh is None and not return_sparsity and \
+            pv_mode in ("fp16", "requant") and (router == "band" or (online and uniform is None and fused_router and causal and requant)):
+        out = _attention_one_call(q, k, v, kv, causal=causal, band=band, uniform=uniform, sq=sq, fp8_elem=fp8_elem, out_dtype=out_dtype,
+                                  pv_mode=pv_mode, route=online, tau=float(tau), smooth_k=smooth_k and kv is None)
+        if out is not None:
+            if check:
+                check_status(q.device)
+            return out
     rope_q = None
     if rope is not None:
         if D != 128:
@@ -802,14 +984,15 @@ def gemm_block_scaled(a: torch.Tensor, a_scale: torch.Tensor, b: torch.Tensor, b
         b = b.contiguous()
     a_scale, b_scale = a_scale.contiguous(), b_scale.contiguous()
     c = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    _raise_if_failed(a.device)
-    st = status_word(a.device)
-    with torch.cuda.device(a.device):
-        rc = _lib.load().mpsa_gemm_block_scaled(
-            a.data_ptr(), a_scale.data_ptr(), b.data_ptr(), b_scale.data_ptr(), c.data_ptr(), M, N, K,
-            a.stride(0) * a.element_size(), b.stride(0) * b.element_size(), c.stride(0), _GEMM_MODE[mode],
-            _FP8_DESC[a_elem], _FP8_DESC[b_elem], _OUT_DTYPE[out_dtype], float(alpha), st.data_ptr(), _stream())
-    _lib.check(rc)
+    index = a.get_device()
+    st = _state(index)
+    if st.word.value:
+        _raise_if_failed(a.device)
+    rc = _on_device(index, _lib.load().mpsa_gemm_block_scaled, a.data_ptr(), a_scale.data_ptr(), b.data_ptr(), b_scale.data_ptr(),
+                    c.data_ptr(), M, N, K, a.stride(0) * a.element_size(), b.stride(0) * b.element_size(), N, _GEMM_MODE[mode],
+                    _FP8_DESC[a_elem], _FP8_DESC[b_elem], _OUT_DTYPE[out_dtype], float(alpha), st.status_ptr)
+    if rc:
+        _lib.check(rc)
     if check:
         check_status(a.device)
     return c

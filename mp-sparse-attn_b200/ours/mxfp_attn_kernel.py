@@ -27,7 +27,7 @@ def mxfp_attn_kernel(q, k, v, attn_mask=None, dropout_p=0.0,
     host = not v.is_cuda
     if host and tensor_layout != "HND":
         raise ValueError("host tensors are taken in the HND layout only")
-    if not host:
+    if not host and v.get_device() != torch.cuda.current_device():
         torch.cuda.set_device(v.device)
     if tensor_layout == "NHD":
         q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)

@@ -16,27 +16,21 @@ def _sides(q, k, sm_scale, tensor_layout):
 def quant_mxfp4(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
     """-> (q codes uint8 one E2M1 code per byte, q E8M0 scales [b,h,len,D/32], k codes, k scales)."""
     sq, sk = _sides(q, k, sm_scale, tensor_layout)
-    a = _ops.quantize_mx(q, sq, want_fp8=False, reference_format=True, kernel_format=False, tensor_layout=tensor_layout)
-    b = _ops.quantize_mx(k, sk, want_fp8=False, reference_format=True, kernel_format=False, tensor_layout=tensor_layout)
-    return a.fp4_unpacked, a.fp4_scales, b.fp4_unpacked, b.fp4_scales
+    return _ops.quantize_pair(q, k, sq, sk, "mxfp4", tensor_layout)
 
 
 def quant_mxfp8e5(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
     """-> (q float8_e5m2, q E8M0 scales, k float8_e5m2, k scales)."""
     sq, sk = _sides(q, k, sm_scale, tensor_layout)
-    a = _ops.quantize_mx(q, sq, want_fp4=False, reference_format=True, kernel_format=False, tensor_layout=tensor_layout)
-    b = _ops.quantize_mx(k, sk, want_fp4=False, reference_format=True, kernel_format=False, tensor_layout=tensor_layout)
-    return a.fp8.view(torch.float8_e5m2), a.fp8_scales, b.fp8.view(torch.float8_e5m2), b.fp8_scales
+    qc, qs, kc, ks = _ops.quantize_pair(q, k, sq, sk, "e5m2", tensor_layout)
+    return qc.view(torch.float8_e5m2), qs, kc.view(torch.float8_e5m2), ks
 
 
 def quant_mxfp8e4(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
     """E4M3 variant (emax 8, clamp 448); the reference has no such quantizer."""
     sq, sk = _sides(q, k, sm_scale, tensor_layout)
-    a = _ops.quantize_mx(q, sq, want_fp4=False, reference_format=True, kernel_format=False, fp8_elem="e4m3",
-                         tensor_layout=tensor_layout)
-    b = _ops.quantize_mx(k, sk, want_fp4=False, reference_format=True, kernel_format=False, fp8_elem="e4m3",
-                         tensor_layout=tensor_layout)
-    return a.fp8.view(torch.float8_e4m3fn), a.fp8_scales, b.fp8.view(torch.float8_e4m3fn), b.fp8_scales
+    qc, qs, kc, ks = _ops.quantize_pair(q, k, sq, sk, "e4m3", tensor_layout)
+    return qc.view(torch.float8_e4m3fn), qs, kc.view(torch.float8_e4m3fn), ks
 
 
 def quant_fpxint8(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
