@@ -57,4 +57,21 @@ inline int make_tmap_2d_b16(CUtensorMap* m, const void* base, uint64_t cols, uin
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
+// 3-D output tensor [batch, rows, cols] of 1-, 2- or 4-byte elements, boxes of 64 bytes x box_rows of one batch
+// (64-byte swizzle): the box is clipped at every edge.
+inline int make_tmap_3d_store(CUtensorMap* m, void* base, int elem_bytes, uint64_t cols, uint64_t rows, uint64_t batch,
+                              uint64_t row_bytes, uint64_t batch_bytes, uint32_t box_rows) {
+  EncodeTiledFn fn = get_encode_tiled();
+  if (!fn) return -1;
+  const CUtensorMapDataType type = elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                                   : (elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8);
+  cuuint64_t dims[3] = {cols, rows, batch};
+  cuuint64_t strides[2] = {row_bytes, batch_bytes};
+  cuuint32_t box[3] = {(cuuint32_t)(64 / elem_bytes), box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, type, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)r;
+}
+
 }  // namespace mpsa

@@ -142,3 +142,37 @@ def test_batched_reference_entry_points():
         a, sa, b, sb, cfg, (ref, _, _) = initialize_block_scaled_batched_from_tensor(a_t, b_t, a_s, b_s, kind, compute_reference=True)
         out = block_scaled_batched_matmul(a, sa, b, sb, torch.float32, B, H, M, N, K, cfg)
         torch.testing.assert_close(out, ref, atol=1e-3, rtol=1e-3)
+
+
+@pytest.mark.parametrize("mode,M,N,K,dtype", [
+    ("mxfp8", 1, 8, 128, torch.bfloat16),            # one row, one stage: nearly all of the pair's tile is padding
+    ("mxfp4", 129, 1030, 640, torch.bfloat16),       # rows of C not 16-byte aligned: element stores; K ends inside a stage
+    ("nvfp4", 2049, 4360, 320, torch.float16),       # several rounds of 256-column tiles per pair, last row tile one row high
+    ("mxfp8", 4000, 1288, 384, torch.float32),       # 128-column tiles, two accumulators in turn, fp32 boxes
+    ("mxfp8", 4096, 4096, 256, torch.float8_e5m2),   # 8-bit boxes of 256-column tiles
+    ("mxfp4", 300, 272, 256, torch.float8_e5m2),     # 8-bit boxes of 128-column tiles
+])
+def test_gemm_tiles_and_stores_against_fp32(mode, M, N, K, dtype):
+    """Every store form and tile width of the pair kernel, at sizes that leave ragged edges, against an fp32 product of the
+    dequantised operands on the GPU."""
+    import mpsa
+    g = torch.Generator().manual_seed(3)
+    sides, alpha = [], 1.0
+    for rows in (M, N):
+        x = torch.randn(rows, K, generator=g).to(torch.bfloat16)
+        if mode == "nvfp4":
+            c, sc, ts = O.quant_nvfp4(x)
+            deq, alpha = O.decode_e2m1(c).float() * O.decode_e4m3(sc).float().repeat_interleave(16, 1), alpha * float(ts)
+            dev, sf = O.pack_e2m1(c), O.swizzle_scales(sc, pad_code=0)
+        else:
+            quant, fmt = (O.quant_mxfp8_side, "fp8e5") if mode == "mxfp8" else (O.quant_mxfp4_side, "fp4")
+            c, sc = quant(x, 1.0)
+            deq = O.dequant(c, sc, fmt).float()
+            dev, sf = (c if mode == "mxfp8" else O.pack_e2m1(c)), O.swizzle_scales(sc)
+        sides.append((dev.cuda(), sf.cuda(), deq.cuda()))
+    (a, sa, da), (b, sb, db) = sides
+    out = mpsa.gemm_block_scaled(a, sa, b, sb, dtype, M, N, K, mode, alpha=alpha, check=True).float().cpu()
+    ref = (da.double() @ db.double().T).float().cpu() * alpha
+    tol = {torch.float32: 1e-5, torch.float16: 1e-3, torch.bfloat16: 8e-3, torch.float8_e5m2: 0.13}[dtype]
+    scale = float(ref.abs().max())
+    assert float(((out - ref).abs() / (ref.abs() + 1e-2 * scale)).max()) <= tol, (mode, M, N, K)
