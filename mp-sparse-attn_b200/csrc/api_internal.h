@@ -34,6 +34,23 @@ bool allow_smem(F* kernel, int bytes) {
   return true;
 }
 
+// A launch that may start while the kernel before it on the stream drains (dependent: that kernel must be one of ours and
+// this one must call grid_dependency_wait() before it touches memory that the other writes or reads).
+template <typename... P, typename... A>
+void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, bool dependent, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);     // an error is reported by check_launch
+}
+
 // One call of the fused forward (see mpsa_attn_fwd for the operands).  map null: the band rule (band, uniform) instead.
 struct AttnCall {
   const void *q8 = nullptr, *q8_sf = nullptr, *q4 = nullptr, *q4_sf = nullptr;
@@ -56,10 +73,13 @@ struct AttnCall {
   const void *ts_q = nullptr, *ts_k = nullptr;   // NVFP4: the two tensor scales in device memory, instead of fp4_scale
   int* range_flag = nullptr;
   int* counter = nullptr;               // a device word, zero on entry: work items are handed out in turn (fixed schedule without it)
+  void* partial = nullptr;              // attn_split_bytes() of device memory, 256-byte aligned: lets the forward divide an item's keys among CTAs
+  bool after_prep = false;              // the kernel before this one on the stream is prep_launch's
   const void *acc_in = nullptr, *lse_in = nullptr;
   int* status = nullptr;
 };
 int attn_forward(const AttnCall& c, cudaStream_t st);
+long long attn_split_bytes(const AttnCall& c);   // 0: this call divides no item (acc_in and lse go without a division)
 // partial column sums of x [B,H,L,D], [B*H, nchunk, D] floats, nchunk = col_sum_chunks(L)
 int col_sum_chunks(int L);
 int col_sums(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h, long long xs_l, float* part,

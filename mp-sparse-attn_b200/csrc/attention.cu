@@ -80,6 +80,8 @@ long long plan(const mpsa_attention_args& a, uint8_t* ws, PrepCall& pc, AttnCall
   ac.need8 = w8; ac.need4 = w4; ac.depth64 = a.D == 64;
   ac.out = a.out; ac.out_dtype = a.out_dtype; ac.B = a.B; ac.Hq = a.Hq; ac.Hkv = a.Hkv; ac.S = a.S; ac.Skv = a.Skv; ac.D = a.D;
   ac.Skv_pad = pitch; ac.causal = a.causal; ac.fp8_fmt = a.fp8_fmt; ac.status = a.status;
+  ac.after_prep = true;
+  if (const long long bytes = attn_split_bytes(ac)) ac.partial = cv.take(bytes);
   return cv.used;
 }
 
@@ -114,6 +116,7 @@ extern "C" int mpsa_attention(const mpsa_attention_args* a, void* stream) {
   if (pc.op[1].part)
     if (int rc = col_sums(a->k, a->in_dtype, a->B, a->Hkv, a->Skv, a->D, a->k_sb, a->k_sh, a->k_sl, (float*)pc.op[1].part, pc.op[1].nchunk, st))
       return rc;
+  pc.after_sums = pc.op[1].part != nullptr;
   if (int rc = prep_launch(pc, a->in_dtype, w8, w4, a->fp8_fmt == 0 ? 2 : 1, st)) return rc;
   return attn_forward(ac, st);
 }

@@ -96,9 +96,44 @@ constexpr uint32_t ENTRY_F8 = 0x8000, ENTRY_MASK = 0x4000, ENTRY_TILE = 0x3fff; 
 #ifndef ATT_POLY_F16
 #define ATT_POLY_F16 4                                // the same, fp16 P
 #endif
+constexpr int SPLIT_MIN_RUN = 8;                      // tiles of a run at least
+constexpr int SPLIT_GAIN = 12;                        // tiles (of 0.7 us) that dividing the keys must save on the busiest CTA
 constexpr float ATT_REF_Q = 20.0f;                    // quantised P.V: the row reference, and the window of row maxima it serves
 constexpr float ATT_WIN_LO_Q = -64.0f, ATT_WIN_HI_Q = 64.0f;
 constexpr float ATT_WIN_HI_F16 = 15.0f;               // fp16 P.V: row maximum above the reference at most
+
+// Division of the keys.  Items are numbered heaviest query tile first: item = r * heads + head, r counting query tiles
+// from the last.  The first n_whole are done by one CTA each; the tiles of the others, laid end to end, are cut into runs
+// of run_tiles, one CTA each, so that a grid with fewer items than SMs, or with a last wave that is nearly empty, still
+// fills the chip.  An item that several runs share gets its result from attn_combine_kernel.
+struct SplitPlan {
+  int heads, nq, nk, causal, c1;     // c1: visible tiles of query tile 0
+  int n_whole, run_tiles;
+  __host__ __device__ long long row_tiles(int r) const { return !causal || r == 0 ? nk : nq - 1 - r + c1; }
+  __host__ __device__ long long rows_before(int r) const {          // tiles of one head's rows 0 .. r-1
+    if (!causal || r <= 1) return (long long)r * nk;
+    return nk + (long long)(r - 1) * (nq - 1 + c1) - (long long)(r - 1) * r / 2;
+  }
+  __host__ __device__ long long start(int item) const {             // tiles of all items before this one
+    const int r = item / heads;
+    return rows_before(r) * heads + (item - r * heads) * row_tiles(r);
+  }
+  __host__ __device__ int item_at(long long pos, int n_items) const {   // the item that holds a tile position
+    int lo = n_whole, hi = n_items - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (start(mid) <= pos) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+  }
+};
+static __host__ __device__ SplitPlan split_plan(int heads, int S, int Skv, int causal, int n_whole, int run_tiles) {
+  SplitPlan s;
+  s.heads = heads; s.nq = (S + ATT_BM - 1) / ATT_BM; s.nk = (Skv + ATT_BN - 1) / ATT_BN; s.causal = causal;
+  s.c1 = (ATT_BM - 1 + Skv - S) / ATT_BN + 1;
+  s.n_whole = n_whole; s.run_tiles = run_tiles;
+  return s;
+}
 
 struct AttnParams {
   int B, Hq, Hkv, S, Skv, D;        // D = value head dim (64 or 128); Q/K depth is padded to 128
@@ -126,6 +161,9 @@ struct AttnParams {
   int* range_flag;                   // optional: set to 1 when an item had to be done again (see the file header)
   int* status;
   int n_items;                       // query tiles x heads x batches
+  int n_work, n_whole;               // units handed out: n_whole items, then runs of run_tiles tiles over the other items (SplitPlan)
+  int run_tiles;
+  float* part_o; float* part_lse;    // partial results of items that several runs share: [part][item - n_whole][128][D], [..][128]
   int group;                         // q-heads per KV head
   int* counter;                      // optional, zero on entry: items are handed out in turn instead of by a fixed schedule
   int n_lists, list_cap;             // item slots in use (fewer than ATT_MAX_SLOTS for very long rows) and entries of a visit list
@@ -425,15 +463,16 @@ struct Slot {
   int n_own;         // tiles of the map row
   int n_total;       // ROUTE: appended tiles included, valid once list_done has completed
   int redo;          // set by the softmax threads: a row maximum lies outside the reference's window
-  int pad;
+  int part;          // slice of the partial results, -1: the item is this CTA's alone
 };
 
-template <int PVQ, int NVF4, int ROUTE, int E4M3>
+template <int PVQ, int NVF4, int ROUTE, int E4M3, int SPLIT>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant__ CUtensorMap tm_q4,
                 const __grid_constant__ CUtensorMap tm_k8, const __grid_constant__ CUtensorMap tm_k4,
                 const __grid_constant__ CUtensorMap tm_vt, const __grid_constant__ CUtensorMap tm_vt8,
                 const __grid_constant__ CUtensorMap tm_vt4, const AttnParams p) {
+  static_assert(!SPLIT || !ROUTE, "routed items stay whole: their appended tiles are not known in advance");
   static_assert(!ROUTE || (PVQ && !NVF4), "the router reads MXFP4 operands and runs with quantised P.V");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -492,6 +531,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dependency_wait();                           // the set-up above ran under the kernel that prepares the operands
 
   uint8_t* sK = smem + ATT_OFF_K;
   uint8_t* sV = smem + ATT_OFF_V;
@@ -810,20 +850,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     bool ok = true;
     int emitted = 0, reclaimed = 0;                 // slots filled, and taken back
     int next_local = 0;                             // static schedule: items taken so far
-    int rq[4], rn = 0;                              // items waiting to be done again (never more than the slots)
-    int redo_item = -1;                             // item whose second pass follows
+    int rq[4], rn = 0;                              // slots' work waiting to be done again (never more than the slots)
+    int redo_item = -1;                             // work whose second pass follows
     const int heads = p.Hq * p.B;
-    int held[ATT_MAX_SLOTS];                        // item number in each slot, -1: nothing that could come back
+    int held[ATT_MAX_SLOTS];                        // work in each slot, -1: nothing that could come back
+    // Work is an item number; a share of a run's also has the run in wrun (0: the whole item).
+    [[maybe_unused]] int held_run[ATT_MAX_SLOTS], rq_run[4], redo_run = 0;
+    [[maybe_unused]] int run = 0;                   // this CTA's present run, from 1
+    [[maybe_unused]] long long run_pos = 0, run_end = 0;
+    [[maybe_unused]] const SplitPlan plan = split_plan(heads, p.S, p.Skv, p.causal, p.n_whole, p.run_tiles);
+    [[maybe_unused]] const long long run_base = SPLIT ? plan.start(p.n_whole) : 0;
     auto reclaim = [&]() {
       const int s = reclaimed % NL;
       ok = __all_sync(0xffffffffu, mbar_wait(&list_empty[s], (reclaimed / NL) & 1, p.status, KS_TIMEOUT_PIPE));
       ++reclaimed;
-      int it = -1;
+      int it = -1, rw = 0;
 #pragma unroll
-      for (int k = 0; k < ATT_MAX_SLOTS; ++k) if (k == s) it = held[k];
+      for (int k = 0; k < ATT_MAX_SLOTS; ++k) if (k == s) { it = held[k]; if (SPLIT) rw = held_run[k]; }
       if (ok && it >= 0 && slots[s].redo) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) if (k == rn) rq[k] = it;
+        for (int k = 0; k < 4; ++k) if (k == rn) { rq[k] = it; if (SPLIT) rq_run[k] = rw; }
         ++rn;
       }
     };
@@ -831,14 +877,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     // numbered heaviest query tile first; they are taken from a counter in memory where the caller gives one, else in
     // snake order over the CTAs, which evens out the sum.  false: nothing left.
     auto emit = [&]() -> bool {
-      int item, mode = 0;
-      if (redo_item >= 0) { item = redo_item; mode = 2; redo_item = -1; }
+      int item, mode = 0, wrun = 0;
+      if (redo_item >= 0) { item = redo_item; if (SPLIT) wrun = redo_run; mode = 2; redo_item = -1; }
       else if (rn > 0) {
         item = rq[0];
+        if (SPLIT) { wrun = rq_run[0]; rq_run[0] = rq_run[1]; rq_run[1] = rq_run[2]; rq_run[2] = rq_run[3]; redo_run = wrun; }
         rq[0] = rq[1]; rq[1] = rq[2]; rq[2] = rq[3];
         --rn;
         mode = 1;
         redo_item = item;
+      } else if (SPLIT && run_pos < run_end) {
+        item = plan.item_at(run_pos, p.n_items);
+        wrun = run;
+        run_pos = plan.start(item + 1);
       } else {
         if (p.counter) {
           int n = 0;
@@ -848,7 +899,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           item = next_local * (int)gridDim.x + ((next_local & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
           ++next_local;
         }
-        if (item >= p.n_items) return false;
+        if (item >= p.n_work) return false;
+        if (SPLIT && item >= p.n_whole) {
+          wrun = run = item - p.n_whole + 1;
+          run_pos = run_base + (long long)(run - 1) * p.run_tiles;
+          run_end = min(run_pos + p.run_tiles, plan.start(p.n_items));
+          item = plan.item_at(run_pos, p.n_items);
+          run_pos = plan.start(item + 1);
+        }
       }
       const int s = emitted % NL;
       const int r = item / heads, bh = item - r * heads;
@@ -859,11 +917,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       const bool from_rw = ROUTE && mode > 0;       // done again: the map as the router left it
       const uint8_t* row = from_rw ? p.map_rw + row_off : (p.map ? p.map + row_off : nullptr);
       const int last_key = min(p.S - 1, qi * ATT_BM + ATT_BM - 1) + off;    // last key any row of the tile may see
-      int base = 0;
-      _Pragma("unroll 1") for (int i0 = 0; i0 < nk; i0 += 32) {
+      int base = 0, j_lo = 0, j_hi = nk, part = -1;
+      if (SPLIT && wrun > 0) {                     // the run's share of the item
+        const long long it0 = plan.start(item), it1 = plan.start(item + 1);
+        const long long a = run_base + (long long)(wrun - 1) * p.run_tiles, e = a + p.run_tiles;
+        if (it0 < a || it1 > e) {
+          part = wrun - 1 - (int)((it0 - run_base) / p.run_tiles);
+          j_lo = (int)(max(a, it0) - it0);
+          j_hi = (int)(min(e, it1) - it0);
+        }
+      }
+      _Pragma("unroll 1") for (int i0 = j_lo; i0 < j_hi; i0 += 32) {
         const int j = i0 + lane;
         int c = TILE_SKIP;
-        if (j < nk) {
+        if (j < j_hi) {
           if (row) c = __ldcg(row + j);
           else {
             c = p.uniform ? p.uniform : (abs(qi + off / ATT_BN - j) < p.band ? TILE_FP8 : TILE_FP4);
@@ -883,10 +950,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       if (lane == 0) {
         slots[s].qi = qi; slots[s].h = h; slots[s].b = b; slots[s].mode = mode; slots[s].n_own = base; slots[s].n_total = base;
         slots[s].redo = 0;
+        if (SPLIT) slots[s].part = part;
         mbar_arrive(&list_full[s]);                 // release: entries (__syncwarp) and slot are visible to who waits
       }
 #pragma unroll
-      for (int k = 0; k < ATT_MAX_SLOTS; ++k) if (k == s) held[k] = mode == 0 ? item : -1;
+      for (int k = 0; k < ATT_MAX_SLOTS; ++k) if (k == s) { held[k] = mode == 0 ? item : -1; if (SPLIT) held_run[k] = wrun; }
       ++emitted;
       return true;
     };
@@ -1215,7 +1283,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         const int mode = slots[epi_ls].mode;
         const bool tiles = (ROUTE ? slots[epi_ls].n_total : slots[epi_ls].n_own) > 0;
         const int m_glob = slots[epi_ls].qi * ATT_BM + r_in;
-        const long long row = (long long)(slots[epi_ls].b * p.Hq + slots[epi_ls].h) * p.S + m_glob;
+        const int head = slots[epi_ls].b * p.Hq + slots[epi_ls].h;
+        const long long row = (long long)head * p.S + m_glob;
+        // a share of an item: fp32 and the log2 denominator, into its slice of the partial results
+        const int part = SPLIT ? slots[epi_ls].part : -1;
+        const int item = (nq - 1 - slots[epi_ls].qi) * p.Hq * p.B + head;
         const float ref = PVQ ? (mode == 2 ? m_redo : ATT_REF_Q) : mref;
         const bool has_o = epi_part * 32 < p.D;     // this thread's 32 columns of O
         uint32_t o[32];
@@ -1245,7 +1317,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         } else if (m_glob < p.S) {
           float inv_l = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
           float lse_row = 0.0f, w_prev = 0.0f;      // w_prev: weight of the earlier partial result (merge mode)
-          if (p.lse) lse_row = l_tot > 0.0f ? ref + log2f(l_tot) : -INFINITY;
+          if (p.lse || part >= 0) lse_row = l_tot > 0.0f ? ref + log2f(l_tot) : -INFINITY;
           if (p.acc_in) {
             // two normalised partial results over disjoint key sets combine with weights 2^(lse_i - lse),
             // lse = log2(2^lse_a + 2^lse_b); every thread of a row computes the same numbers
@@ -1259,7 +1331,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               lse_row = lm + log2f(ea + eb);
             }
           }
-          if (p.lse && epi_part == 0) p.lse[row] = lse_row;    // log2(sum_k exp2(S_k)): lets partial results be merged
+          // log2(sum_k exp2(S_k)): lets partial results be merged
+          const long long prow = ((long long)part * (p.n_items - p.n_whole) + item - p.n_whole) * ATT_BM + r_in;
+          if (part >= 0) { if (epi_part == 0) p.part_lse[prow] = lse_row; }
+          else if (p.lse && epi_part == 0) p.lse[row] = lse_row;
           if (has_o) {
             const long long o_off = row * p.D + epi_part * 32;
 #pragma unroll
@@ -1277,7 +1352,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
             }
             // a lane writes 32 columns of its own row, so that a store instruction touches 32 lines: the fewest and
             // widest stores there are (32 bytes a lane where the output is 32-byte aligned)
-            if (p.out_dtype == 0) {
+            if (part >= 0) {
+              store_row<8>(p.part_o + prow * p.D + epi_part * 32, o, true);
+            } else if (p.out_dtype == 0) {
               store_row<8>(reinterpret_cast<float*>(p.out) + o_off, o, p.out32);
             } else {
 #pragma unroll
@@ -1341,6 +1418,62 @@ __global__ void __launch_bounds__(256) attn_merge_kernel(float* acc, float* lse_
   reinterpret_cast<float4*>(acc)[i] = a;
   __syncwarp();
   if (i % per_row == 0) lse_acc[r] = lnew;
+}
+
+// Results of the items that several runs share (SplitPlan): the partial results of a row combine with weights
+// 2^(lse_i - max lse), as above.  A quarter warp per row, 16 or 8 columns a lane, so that a thread has 64 bytes of every part in
+// flight: with a warp per row the kernel waited for its loads (156 items of 2 parts: 12.7 us).
+template <int W>                                    // columns of a lane: D / 8
+__global__ void __launch_bounds__(128) attn_combine_kernel(const float* part_o, const float* part_lse, SplitPlan s, int n_items, void* out,
+                                                           int out_dtype, int S) {
+  grid_dependency_wait();
+  constexpr int D = W * 8;
+  const int n_shared = n_items - s.n_whole, k = blockIdx.x, item = s.n_whole + k;
+  const int r_in = blockIdx.y * 16 + (threadIdx.x >> 3), sub = threadIdx.x & 7;
+  const long long base = s.start(s.n_whole), it0 = s.start(item) - base;
+  const int r = item / s.heads, m = (s.nq - 1 - r) * ATT_BM + r_in;
+  const int parts = (int)((it0 + s.row_tiles(r) - 1) / s.run_tiles - it0 / s.run_tiles) + 1;
+  if (parts == 1 || m >= S) return;                 // (a single run has written the output itself)
+  const long long stride = (long long)n_shared * ATT_BM, row0 = (long long)k * ATT_BM + r_in;
+  const float* src = part_o + row0 * D + sub * 4;   // lane `sub` takes columns 32 c + 4 sub .. + 3
+  float acc[W], den = 0.0f, lm = -INFINITY;
+#pragma unroll
+  for (int c = 0; c < W; ++c) acc[c] = 0.0f;
+  for (int i = 0; i < parts; ++i) {
+    const float l = __ldcg(part_lse + i * stride + row0);
+    float4 v[W / 4];
+#pragma unroll
+    for (int c = 0; c < W / 4; ++c) v[c] = __ldcg(reinterpret_cast<const float4*>(src + i * stride * D + c * 32));
+    if (l == -INFINITY) continue;                   // no visible key in this part
+    const float nm = fmaxf(lm, l), w0 = exp2f(lm - nm), w1 = exp2f(l - nm);
+    lm = nm;
+    den = fmaf(den, w0, w1);
+#pragma unroll
+    for (int c = 0; c < W / 4; ++c) {
+      acc[4 * c] = fmaf(acc[4 * c], w0, v[c].x * w1);
+      acc[4 * c + 1] = fmaf(acc[4 * c + 1], w0, v[c].y * w1);
+      acc[4 * c + 2] = fmaf(acc[4 * c + 2], w0, v[c].z * w1);
+      acc[4 * c + 3] = fmaf(acc[4 * c + 3], w0, v[c].w * w1);
+    }
+  }
+  const float inv = den > 0.0f ? 1.0f / den : 0.0f;
+  const long long o = ((long long)(item - r * s.heads) * S + m) * D + sub * 4;
+#pragma unroll
+  for (int c = 0; c < W / 4; ++c) {
+    const float x0 = acc[4 * c] * inv, x1 = acc[4 * c + 1] * inv, x2 = acc[4 * c + 2] * inv, x3 = acc[4 * c + 3] * inv;
+    if (out_dtype == 0) {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + o + c * 32) = make_float4(x0, x1, x2, x3);
+    } else {
+      uint2 h;
+      if (out_dtype == 1) {
+        h = make_uint2(pack_f16x2(x0, x1), pack_f16x2(x2, x3));
+      } else {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(x0, x1), b = __floats2bfloat162_rn(x2, x3);
+        h = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+      }
+      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(out) + o + c * 32) = h;
+    }
+  }
 }
 
 // ---- V^T preparation: V [B,Hkv,Skv,D] (any 16-bit/32-bit float, strided) -> fp16 [B,Hkv,D,Skv_pad],
@@ -1448,16 +1581,47 @@ int sm_count() {
 namespace {
 struct AttnMaps { CUtensorMap q8, q4, k8, k4, vt, vt8, vt4; };
 
-template <int PVQ, int NVF4, int ROUTE, int E4M3>
-int launch_attn(int grid, size_t smem, cudaStream_t st, const AttnMaps& m, const AttnParams& p) {
-  auto kern = attn_fwd_kernel<PVQ, NVF4, ROUTE, E4M3>;
+template <int PVQ, int NVF4, int ROUTE, int E4M3, int SPLIT = 0>
+int launch_attn(int grid, size_t smem, cudaStream_t st, bool after_prep, const AttnMaps& m, const AttnParams& p) {
+  auto kern = attn_fwd_kernel<PVQ, NVF4, ROUTE, E4M3, SPLIT>;
   // the opt-in for more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
-  if (!allow_smem<((PVQ * 2 + NVF4) * 2 + ROUTE) * 2 + E4M3>(kern, ATT_SMEM_MAX))
+  if (!allow_smem<(((PVQ * 2 + NVF4) * 2 + ROUTE) * 2 + E4M3) * 2 + SPLIT>(kern, ATT_SMEM_MAX))
     return set_error(MPSA_ERR_LAUNCH, "attn_fwd: cannot reserve %d bytes of shared memory", ATT_SMEM_MAX);
-  kern<<<grid, ATT_THREADS, smem, st>>>(m.q8, m.q4, m.k8, m.k4, m.vt, m.vt8, m.vt4, p);
+  launch_dependent(kern, dim3(grid), ATT_THREADS, smem, st, after_prep, m.q8, m.q4, m.k8, m.k4, m.vt, m.vt8, m.vt4, p);
   return check_launch("attn_fwd");
 }
+
+// Whether to cut items into runs, from where on, and how long a run is; returns the number of partial slices (0: no cut).
+// In tiles of work per CTA: without a cut the busiest CTA of the schedule has at least `whole`, the larger of the mean and
+// k times the lightest of the (k - 1) * SMs + 1 heaviest items, for every k; with one it has the mean of what is cut.  A cut
+// costs the combination (5 us), partial results in fp32 and one more item a CTA: with 12 tiles to save it breaks even (12
+// heads of 1560 tokens, 26 tiles against 14: 29.6 us either way).  16 queries against 32768 keys, 32 heads on 148 SMs, 256
+// tiles against 56: 195 -> 58 us; 512 queries, 256 against 221: 199 -> 187 us.
+int split_choose(const AttnCall& c, int nq, int nk, int& n_whole, int& run_tiles) {
+  const int heads = c.B * c.Hq, n_items = nq * heads, sms = sm_count();
+  const SplitPlan all = split_plan(heads, c.S, c.Skv, c.causal, 0, 1);
+  const long long total = all.start(n_items);
+  long long whole = (total + sms - 1) / sms;
+  for (long long k = 1; (k - 1) * sms < n_items; ++k) whole = std::max(whole, k * all.row_tiles((int)((k - 1) * sms) / heads));
+  n_whole = n_items / sms * sms;
+  // what is left over gets runs of at least SPLIT_MIN_RUN tiles; too little for that: one more wave joins it
+  auto run_of = [&](int first) { return (total - all.start(first) + sms - 1) / sms; };
+  if (n_whole > 0 && run_of(n_whole) < SPLIT_MIN_RUN) n_whole -= sms;
+  run_tiles = (int)std::max<long long>(SPLIT_MIN_RUN, run_of(n_whole));
+  const long long cut = (all.start(n_whole) + sms - 1) / sms + run_tiles;
+  if (n_whole == n_items || whole - cut < SPLIT_GAIN) { n_whole = n_items; run_tiles = 1; return 0; }
+  return (int)((all.row_tiles(n_whole / heads) - 1) / run_tiles) + 2;
+}
 }  // namespace
+
+long long attn_split_bytes(const AttnCall& c) {
+  if (c.route || c.fp4_kind) return 0;
+  const int nq = (c.S + ATT_BM - 1) / ATT_BM, nk = (c.Skv + ATT_BN - 1) / ATT_BN;
+  if ((long long)nq * c.Hq * c.B >= (1ll << 30)) return 0;
+  int n_whole, run_tiles;
+  const int parts = split_choose(c, nq, nk, n_whole, run_tiles);
+  return (long long)parts * ((long long)nq * c.Hq * c.B - n_whole) * ATT_BM * (c.D + 1) * 4;
+}
 
 int attn_forward(const AttnCall& call, cudaStream_t st) {
   AttnCall c = call;
@@ -1525,12 +1689,28 @@ int attn_forward(const AttnCall& call, cudaStream_t st) {
   p.list_cap = ((c.route ? 2 * nk : nk) + 7) & ~7;
   p.n_lists = std::min(ATT_MAX_SLOTS, (ATT_SMEM_MAX - 1024 - ATT_OFF_LIST) / (p.list_cap * 2));
   const size_t smem = ATT_OFF_LIST + (size_t)p.n_lists * p.list_cap * 2 + 1024;
-  const int grid = (int)std::min<long long>(n_items, sm_count());      // one persistent CTA per SM
-  const bool e4 = c.fp8_fmt == 0;
-  if (c.route) return e4 ? launch_attn<1, 0, 1, 1>(grid, smem, st, m, p) : launch_attn<1, 0, 1, 0>(grid, smem, st, m, p);
-  if (c.pv_mode == 0) return c.fp4_kind ? launch_attn<0, 1, 0, 0>(grid, smem, st, m, p) : launch_attn<0, 0, 0, 0>(grid, smem, st, m, p);
-  if (c.fp4_kind) return e4 ? launch_attn<1, 1, 0, 1>(grid, smem, st, m, p) : launch_attn<1, 1, 0, 0>(grid, smem, st, m, p);
-  return e4 ? launch_attn<1, 0, 0, 1>(grid, smem, st, m, p) : launch_attn<1, 0, 0, 0>(grid, smem, st, m, p);
+  int parts = 0, n_whole = p.n_items, run_tiles = 1;
+  if (c.partial) parts = split_choose(c, nq, nk, n_whole, run_tiles);
+  const long long n_shared = p.n_items - n_whole;
+  const SplitPlan plan = split_plan(c.B * c.Hq, c.S, c.Skv, c.causal, n_whole, run_tiles);
+  p.n_whole = n_whole; p.run_tiles = run_tiles;
+  p.n_work = n_whole + (int)((plan.start(p.n_items) - plan.start(n_whole) + run_tiles - 1) / run_tiles);
+  p.part_o = (float*)c.partial;
+  p.part_lse = p.part_o + parts * n_shared * ATT_BM * c.D;
+  const int grid = std::min(p.n_work, sm_count());                     // one persistent CTA per SM
+  const bool e4 = c.fp8_fmt == 0, dep = c.after_prep;
+  int rc;
+  if (parts > 0) {
+    if (c.pv_mode == 0) rc = launch_attn<0, 0, 0, 0, 1>(grid, smem, st, dep, m, p);
+    else rc = e4 ? launch_attn<1, 0, 0, 1, 1>(grid, smem, st, dep, m, p) : launch_attn<1, 0, 0, 0, 1>(grid, smem, st, dep, m, p);
+  } else if (c.route) rc = e4 ? launch_attn<1, 0, 1, 1>(grid, smem, st, dep, m, p) : launch_attn<1, 0, 1, 0>(grid, smem, st, dep, m, p);
+  else if (c.pv_mode == 0) rc = c.fp4_kind ? launch_attn<0, 1, 0, 0>(grid, smem, st, dep, m, p) : launch_attn<0, 0, 0, 0>(grid, smem, st, dep, m, p);
+  else if (c.fp4_kind) rc = e4 ? launch_attn<1, 1, 0, 1>(grid, smem, st, dep, m, p) : launch_attn<1, 1, 0, 0>(grid, smem, st, dep, m, p);
+  else rc = e4 ? launch_attn<1, 0, 0, 1>(grid, smem, st, dep, m, p) : launch_attn<1, 0, 0, 0>(grid, smem, st, dep, m, p);
+  if (rc || parts == 0) return rc;
+  launch_dependent(c.D == 64 ? attn_combine_kernel<8> : attn_combine_kernel<16>, dim3((unsigned)n_shared, ATT_BM / 16), 128, 0, st, true,
+                   (const float*)p.part_o, (const float*)p.part_lse, plan, p.n_items, c.out, c.out_dtype, c.S);
+  return check_launch("attn_combine");
 }
 
 }  // namespace mpsa

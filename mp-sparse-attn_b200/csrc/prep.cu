@@ -10,6 +10,7 @@
 // for x > 0 the pattern is a piecewise linear logarithm, the softmax scale folded into Q only moves the class boundaries, and
 // a boundary is an integer (found on the host by trying the 128 mantissas).  5.5 instructions an element.
 #include "api_internal.h"
+#include "common.cuh"
 #include "quant_math.h"
 #include "prep.h"
 
@@ -382,6 +383,7 @@ template <typename T, bool W8, bool W4, bool E4M3, bool D64>
 __global__ void __launch_bounds__(PREP_THREADS, 4) prep_kernel(const __grid_constant__ PrepCall p) {
   extern __shared__ __align__(128) uint8_t prep_smem[];
   int cta = blockIdx.x;
+  grid_dependency_wait();
   if (cta == 0 && threadIdx.x < 2) {
     // words the launches behind this one expect to find zero
     int* z = threadIdx.x ? p.zero1 : p.zero0;
@@ -399,10 +401,10 @@ __global__ void __launch_bounds__(PREP_THREADS, 4) prep_kernel(const __grid_cons
 
 template <typename T>
 int launch_prep(const PrepCall& p, bool w8, bool w4, bool e4m3, int grid, size_t smem, cudaStream_t st) {
-#define MPSA_PREP(A, B, C)                                                                                  \
+#define MPSA_PREP(A, B, C)                                                                                                    \
   do {                                                                                                      \
-    if (p.D == 64) prep_kernel<T, A, B, C, true><<<grid, PREP_THREADS, smem, st>>>(p);                      \
-    else prep_kernel<T, A, B, C, false><<<grid, PREP_THREADS, smem, st>>>(p);                               \
+    if (p.D == 64) launch_dependent(prep_kernel<T, A, B, C, true>, dim3(grid), PREP_THREADS, smem, st, p.after_sums, p);  \
+    else launch_dependent(prep_kernel<T, A, B, C, false>, dim3(grid), PREP_THREADS, smem, st, p.after_sums, p);         \
   } while (0)
   if (w8 && w4) { if (e4m3) MPSA_PREP(true, true, true); else MPSA_PREP(true, true, false); }
   else if (w4) { if (e4m3) MPSA_PREP(false, true, true); else MPSA_PREP(false, true, false); }

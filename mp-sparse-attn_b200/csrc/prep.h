@@ -47,6 +47,7 @@ struct PrepCall {
   PrepV v;
   int D = 0;
   int *zero0 = nullptr, *zero1 = nullptr;              // words set to zero on the way
+  bool after_sums = false;                             // the kernel before this one on the stream is col_sums'
 };
 
 PrepThresholds prep_thresholds(float s);

@@ -529,11 +529,12 @@ def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out
     ints = (in_dtype, _OUT_DTYPE[out_dtype], B, Hq, Hkv, S, Skv, D, skv_pad, int(causal), band, uni, int(route), pv,
             _FP8_DESC[fp8_elem], int(smooth_k))
     lib = _lib.load()
-    key = (ints, kp == 0)
+    key = (ints, kp == 0, index)                   # the size depends on the number of SMs too
     need = _workspace_bytes.get(key)
     if need is None:
-        need = lib.mpsa_attention_workspace(_ATTENTION_ARGS.pack(1, int(kp != 0), int(vp != 0), *qs, *ks, *vs, *prepared, 0, 0, 0, 0, 0,
-                                                                *ints, sq, tau))
+        with torch.cuda.device(index):
+            need = lib.mpsa_attention_workspace(_ATTENTION_ARGS.pack(1, int(kp != 0), int(vp != 0), *qs, *ks, *vs, *prepared, 0, 0, 0, 0, 0,
+                                                                    *ints, sq, tau))
         if need < 0:
             _lib.check(need)
         if len(_workspace_bytes) >= 1024:
