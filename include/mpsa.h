@@ -225,6 +225,7 @@ int mpsa_attn_fwd_routed(const void* q8, const void* q8_sf, const void* q4, cons
  *   band, uniform precision rule: MXFP8 within `band` tiles of the diagonal; uniform 1: every tile MXFP8, 2: MXFP4, 0: neither
  *   route, tau    the online router inside the forward (causal, pv_mode 1), as in mpsa_attn_fwd_routed
  *   q_scale       softmax scale * log2(e), folded into Q
+ *   fp4_kind      0 MXFP4 score tiles; 1 NVFP4 (D 128, k given, band rule, no smooth_k): two more launches and a memset
  *   workspace     mpsa_attention_workspace bytes, 256-byte aligned, private to the call until it has finished on the GPU
  *   range_flag    optional word, set to zero by the call and then used as in mpsa_attn_fwd */
 typedef struct mpsa_attention_args {
@@ -235,7 +236,7 @@ typedef struct mpsa_attention_args {
   void* workspace;
   long long workspace_bytes;
   int *range_flag, *status;
-  int in_dtype, out_dtype, B, Hq, Hkv, S, Skv, D, Skv_pad, causal, band, uniform, route, pv_mode, fp8_fmt, smooth_k;
+  int in_dtype, out_dtype, B, Hq, Hkv, S, Skv, D, Skv_pad, causal, band, uniform, route, pv_mode, fp8_fmt, smooth_k, fp4_kind;
   float q_scale, tau;
 } mpsa_attention_args;
 long long mpsa_attention_workspace(const mpsa_attention_args* args);

@@ -84,4 +84,8 @@ long long attn_split_bytes(const AttnCall& c);   // 0: this call divides no item
 int col_sum_chunks(int L);
 int col_sums(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h, long long xs_l, float* part,
              int nchunk, cudaStream_t st);
+// NVFP4 codes and E4M3 scale tiles of x [B,H,L,D] (16-bit, D a multiple of 64), given the bits of amax |x * s| in device memory;
+// launched as a dependent of the kernel before it
+int nvfp4_quant(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h, long long xs_l, float s,
+                unsigned* amax, void* codes, void* scales, float* tensor_scale, cudaStream_t st);
 }  // namespace mpsa

@@ -25,20 +25,29 @@ long long plan(const mpsa_attention_args& a, uint8_t* ws, PrepCall& pc, AttnCall
     return set_error(MPSA_ERR_BAD_ARG, "attention: bad shape");
   if (a.in_dtype != 0 && a.in_dtype != 1) return set_error(MPSA_ERR_UNSUPPORTED, "attention: inputs must be bf16 or fp16");
   if (a.uniform < 0 || a.uniform > 2 || (a.route && a.uniform)) return set_error(MPSA_ERR_BAD_ARG, "attention: bad precision rule");
-  const bool prepared = a.k == nullptr;
+  const bool prepared = a.k == nullptr, nvfp4 = a.fp4_kind == 1;
+  if (a.fp4_kind != 0 && (!nvfp4 || a.D != 128 || prepared || a.smooth_k || a.route || a.uniform))
+    return set_error(MPSA_ERR_UNSUPPORTED, "attention: NVFP4 score tiles go with depth 128, the band rule and keys in 16 bits");
   const long long qrows = (long long)a.B * a.Hq * a.S, krows = (long long)a.B * a.Hkv * a.Skv;
   const long long nq = (a.S + 127) / 128, nk = (a.Skv + 127) / 128;
   const int pitch = prepared ? a.Skv_pad : (int)nk * 128;
   w8 = a.uniform != 2;
-  w4 = a.uniform != 1;
+  w4 = a.uniform != 1 && !nvfp4;
+  const bool q4 = w4 || nvfp4;
+  const int sf4 = nvfp4 ? 1024 : 512;                   // bytes of FP4 scales per 128 rows
   Carver cv{ws};
   int* counter = (int*)cv.take(4);
+  uint8_t* const words = nvfp4 ? cv.take(16) : nullptr; // two maxima, two tensor scales
+  if (nvfp4) {
+    pc.op[0].amax = (unsigned*)words; pc.op[1].amax = (unsigned*)words + 1;
+    ac.ts_q = (float*)words + 2; ac.ts_k = (float*)words + 3;
+  }
   PrepOperand& q = pc.op[0];
   q.x = a.q; q.B = a.B; q.H = a.Hq; q.L = a.S; q.xs_b = a.q_sb; q.xs_h = a.q_sh; q.xs_l = a.q_sl; q.s = a.q_scale;
   ac.q8 = q.fp8_codes = w8 ? cv.take(qrows * 128) : nullptr;
   ac.q8_sf = q.sf8_tiled = w8 ? cv.take((long long)a.B * a.Hq * nq * 512) : nullptr;
-  ac.q4 = q.fp4_packed = w4 ? cv.take(qrows * 64) : nullptr;
-  ac.q4_sf = q.sf4_tiled = w4 ? cv.take((long long)a.B * a.Hq * nq * 512) : nullptr;
+  ac.q4 = q.fp4_packed = q4 ? cv.take(qrows * 64) : nullptr;
+  ac.q4_sf = q.sf4_tiled = q4 ? cv.take((long long)a.B * a.Hq * nq * sf4) : nullptr;
   // rows of 128 depth elements whatever D is: with D = 64 the upper half is never multiplied (depth64)
   q.o8_l = 128; q.o8_h = 128ll * a.S; q.o8_b = q.o8_h * a.Hq; q.p4_row = 64;
   if (prepared) {
@@ -49,8 +58,8 @@ long long plan(const mpsa_attention_args& a, uint8_t* ws, PrepCall& pc, AttnCall
     k.x = a.k; k.B = a.B; k.H = a.Hkv; k.L = a.Skv; k.xs_b = a.k_sb; k.xs_h = a.k_sh; k.xs_l = a.k_sl; k.s = 1.0f;
     ac.k8 = k.fp8_codes = w8 ? cv.take(krows * 128) : nullptr;
     ac.k8_sf = k.sf8_tiled = w8 ? cv.take((long long)a.B * a.Hkv * nk * 512) : nullptr;
-    ac.k4 = k.fp4_packed = w4 ? cv.take(krows * 64) : nullptr;
-    ac.k4_sf = k.sf4_tiled = w4 ? cv.take((long long)a.B * a.Hkv * nk * 512) : nullptr;
+    ac.k4 = k.fp4_packed = q4 ? cv.take(krows * 64) : nullptr;
+    ac.k4_sf = k.sf4_tiled = q4 ? cv.take((long long)a.B * a.Hkv * nk * sf4) : nullptr;
     k.o8_l = 128; k.o8_h = 128ll * a.Skv; k.o8_b = k.o8_h * a.Hkv; k.p4_row = 64;
     if (a.smooth_k) {
       k.nchunk = col_sum_chunks(a.Skv);
@@ -65,8 +74,8 @@ long long plan(const mpsa_attention_args& a, uint8_t* ws, PrepCall& pc, AttnCall
     } else {
       ac.vt8 = v.vt8 = w8 ? cv.take(vrows * pitch) : nullptr;
       ac.v8_sf = v.v8_sf = w8 ? cv.take(vtiles) : nullptr;
-      ac.vt4 = v.vt4 = w4 ? cv.take(vrows * pitch / 2) : nullptr;
-      ac.v4_sf = v.v4_sf = w4 ? cv.take(vtiles) : nullptr;
+      ac.vt4 = v.vt4 = q4 ? cv.take(vrows * pitch / 2) : nullptr;
+      ac.v4_sf = v.v4_sf = q4 ? cv.take(vtiles) : nullptr;
     }
   }
   ac.map_sh = nq * nk;
@@ -77,7 +86,7 @@ long long plan(const mpsa_attention_args& a, uint8_t* ws, PrepCall& pc, AttnCall
   pc.zero1 = a.range_flag;
   ac.counter = counter; ac.range_flag = a.range_flag;
   ac.pv_mode = a.pv_mode; ac.band = a.band; ac.uniform = a.uniform; ac.route = a.route != 0; ac.tau = a.tau;
-  ac.need8 = w8; ac.need4 = w4; ac.depth64 = a.D == 64;
+  ac.need8 = w8; ac.need4 = q4; ac.fp4_kind = a.fp4_kind; ac.depth64 = a.D == 64;
   ac.out = a.out; ac.out_dtype = a.out_dtype; ac.B = a.B; ac.Hq = a.Hq; ac.Hkv = a.Hkv; ac.S = a.S; ac.Skv = a.Skv; ac.D = a.D;
   ac.Skv_pad = pitch; ac.causal = a.causal; ac.fp8_fmt = a.fp8_fmt; ac.status = a.status;
   ac.after_prep = true;
@@ -117,7 +126,14 @@ extern "C" int mpsa_attention(const mpsa_attention_args* a, void* stream) {
     if (int rc = col_sums(a->k, a->in_dtype, a->B, a->Hkv, a->Skv, a->D, a->k_sb, a->k_sh, a->k_sl, (float*)pc.op[1].part, pc.op[1].nchunk, st))
       return rc;
   pc.after_sums = pc.op[1].part != nullptr;
+  if (a->fp4_kind && cudaMemsetAsync(pc.op[0].amax, 0, 2 * sizeof(unsigned), st) != cudaSuccess) return check_launch("attention");
   if (int rc = prep_launch(pc, a->in_dtype, w8, w4, a->fp8_fmt == 0 ? 2 : 1, st)) return rc;
+  for (int i = 0; a->fp4_kind && i < 2; ++i) {
+    const PrepOperand& o = pc.op[i];
+    if (int rc = nvfp4_quant(o.x, a->in_dtype, o.B, o.H, o.L, a->D, o.xs_b, o.xs_h, o.xs_l, o.s, o.amax, o.fp4_packed, o.sf4_tiled,
+                             (float*)(i ? ac.ts_k : ac.ts_q), st))
+      return rc;
+  }
   return attn_forward(ac, st);
 }
 

@@ -144,6 +144,8 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
   uint8_t* o4 = W4 && p.fp4_unpacked ? p.fp4_unpacked + (long long)b * p.o4_b + (long long)h * p.o4_h + (long long)r0 * p.o4_l + c : nullptr;
   uint8_t* op = W4 && p.fp4_packed ? p.fp4_packed + row0 * p.p4_row + (c >> 1) : nullptr;
   const long long s8 = p.o8_l * RSTEP, s4 = p.o4_l * RSTEP, sp = p.p4_row * RSTEP;
+  constexpr bool AMAX = W8 && !W4;                      // NVFP4 next to MXFP8: this pass finds the tensor's maximum for it
+  [[maybe_unused]] float amax_all = 0.0f;
   const int nblk = D >> 5;
   const long long rm0 = row0 * nblk + tile_d * 4;
   // 512-byte scale tiles: row r, block k at byte (r % 32) * 16 + (r / 32) * 4 + k
@@ -173,6 +175,7 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
     m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
     // the maximum of the rounded products |x| * s is the rounded product of the maximum (s > 0)
     const float amax = __fmul_rn(pattern_to_float<T>(m), p.s);
+    if (AMAX) amax_all = fmaxf(amax_all, amax);
     uint32_t code8 = 127, code4 = 127;
     if (live) {
       if (W8) {
@@ -278,6 +281,10 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
         }
       }
     }
+  }
+  if (AMAX && p.amax) {                                 // few warps find a new maximum: the others only look at the word
+    const unsigned a = __reduce_max_sync(0xffffffffu, __float_as_uint(amax_all));
+    if ((tid & 31) == 0 && a > __ldcg(p.amax)) atomicMax(p.amax, a);
   }
 }
 

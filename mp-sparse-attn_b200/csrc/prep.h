@@ -28,6 +28,7 @@ struct PrepOperand {
   uint8_t* fp4_packed = nullptr; long long p4_row = 0; // [B,H,L] rows of p4_row bytes
   uint8_t* sc8_rows = nullptr; uint8_t* sc4_rows = nullptr;       // [B,H,L,D/32]
   uint8_t* sf8_tiled = nullptr; uint8_t* sf4_tiled = nullptr;     // [B,H,ceil(L/128),ceil(D/128),512]
+  unsigned* amax = nullptr;                            // optional word, zero before: bits of the largest |x * s|
   PrepThresholds thr;                                  // filled in by prep_launch
   int ctas = 0;
 };

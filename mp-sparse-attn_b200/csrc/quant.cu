@@ -13,12 +13,14 @@
 // The kernel is HBM-bound: algorithmic bytes per element are 2 (bf16 in) + 1 (fp8) + 1/32, or
 // 2 + 1/2 + 1/32 for packed fp4.
 #include "api_internal.h"
+#include "common.cuh"
 #include "quant_math.h"
 #include "prep.h"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <mutex>
+#include <type_traits>
 
 namespace mpsa {
 
@@ -508,91 +510,141 @@ __global__ void __launch_bounds__(256) quant_v_seq_kernel(const QuantVParams p) 
 // ---- NVFP4: 16-element blocks, E4M3 block scales, one fp32 tensor scale ------------------------------
 // The reference only has the GEMM mode string for this format (ours/block_scaled_matmul.py:321-324), no
 // quantizer.  Definition used here: ts = amax(tensor) / (6 * 448); block scale = e4m3_rne(amax(block) /
-// (6 * ts)); element = e2m1_rne(x / (scale * ts)).  Two launches: stage 1 leaves one partial amax per CTA
-// in a scratch array (no atomics, nothing to zero), stage 2 reduces the partials and quantises.
+// (6 * ts)); element = e2m1_rne(x / (scale * ts)).  Two launches: stage 1 leaves amax(tensor) in one word (the maximum of the
+// bit patterns, which for magnitudes is the maximum of the values), stage 2 quantises.  In a whole attention call the MX
+// quantizer, which reads the operand anyway, does stage 1.
 struct QuantNvParams {
   const void* x; int rows, cols; long long ld; float s;
   int H; long long xs_b, xs_h;              // batch (blockIdx.z = b * H + h): input strides in elements; 2-D: H = 1, strides 0
-  float* scratch; int n_partials;
+  unsigned* amax;                           // bits of amax |x * s| over the tensor; zero before stage 1
   uint8_t* codes; long long ldc_bytes;      // [batch, rows, cols/2]
   uint8_t* scales;                          // [batch, ceil(rows/128), cols/64, 512] E4M3 bytes
   float* tensor_scale;
 };
 
+// Stage 1.  CTA tile: 128 rows x 512 columns, 16 elements per step and thread, four steps' loads in flight.
 template <typename T>
 __global__ void __launch_bounds__(kQuantThreads) nvfp4_amax_kernel(const QuantNvParams p) {
-  __shared__ float red[kQuantThreads / 32];
   const int tid = threadIdx.x;
   const T* xb = reinterpret_cast<const T*>(p.x) + (blockIdx.z / p.H) * p.xs_b + (blockIdx.z % p.H) * p.xs_h;
   float amax = 0.0f;
-  // CTA tile: 128 rows x 512 columns, 16 elements per step and thread
-  for (int i = tid; i < 128 * 32; i += kQuantThreads) {
-    const int r = blockIdx.x * 128 + (i >> 5), c = blockIdx.y * 512 + (i & 31) * 16;
-    if (r < p.rows && c < p.cols) {
-      float v[16];
-      load16<T>(xb + (long long)r * p.ld + c, v);
+  [[maybe_unused]] uint32_t top = 0;
+  const int c = blockIdx.y * 512 + (tid & 31) * 16, r0 = blockIdx.x * 128 + (tid >> 5);
+  if (c < p.cols) {
+#pragma unroll 1
+    for (int i0 = 0; i0 < 16; i0 += 4) {
+      Raw16<T> raw[4];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(__fmul_rn(v[j], p.s)));
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + (i0 + i) * 8;
+        raw[i] = Raw16<T>{};
+        if (r < p.rows) load_raw<T>(xb + (long long)r * p.ld + c, raw[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if constexpr (sizeof(T) == 2) {               // the order of the magnitudes is the order of their patterns
+          const uint32_t w[8] = {raw[i].q[0].x, raw[i].q[0].y, raw[i].q[0].z, raw[i].q[0].w, raw[i].q[1].x, raw[i].q[1].y, raw[i].q[1].z, raw[i].q[1].w};
+#pragma unroll
+          for (int j = 0; j < 8; ++j) top = __vmaxu2(top, w[j] & 0x7fff7fffu);
+        } else {
+          float v[16];
+          unpack16(raw[i], v);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(__fmul_rn(v[j], p.s)));
+        }
+      }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((tid & 31) == 0) red[tid >> 5] = amax;
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < kQuantThreads / 32; ++w) amax = fmaxf(amax, red[w]);
-    p.scratch[(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = amax;
+  if constexpr (sizeof(T) == 2) {
+    top = max(top & 0xffffu, top >> 16);
+    amax = fabsf(__fmul_rn(std::is_same<T, __half>::value ? __half2float(__ushort_as_half((unsigned short)top)) : __uint_as_float(top << 16), p.s));
   }
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+  // few warps find a new maximum: the others only look at the word
+  if ((tid & 31) == 0 && m > __ldcg(p.amax)) atomicMax(p.amax, m);
 }
 
+// Stage 2.  A thread owns four runs of 16 elements (one scale block each) of a 128 x 128 tile; their loads go out first.  Bound by
+// instruction issue with an IEEE division per element (375 instructions a block, 183 us for 168M bf16 elements).  Now the
+// block's reciprocal r = RN(1 / scale) serves all 16 quotients: q = v r, then twice q += (v - q scale) r with fused
+// multiply-adds, which leaves the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34, 1990: the first step makes q
+// faithful, the second rounds it), and packed pairs make that 2.5 instructions an element: 105 us, 4.2 TB/s.
+__device__ __forceinline__ void nv_mul2(float& a, float& b, float c) {      // (a, b) *= c, one instruction for the pair
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(a), "+f"(b) : "f"(c));
+}
+__device__ __forceinline__ void nv_fma2(float& d0, float& d1, float a0, float a1, float c, float e0, float e1) {  // d = a * (c, c) + e
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmov.b64 z, {%5, %6};\n\tfma.rn.f32x2 x, x, y, z;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(c), "f"(e0), "f"(e1));
+}
 template <typename T>
-__global__ void __launch_bounds__(kQuantThreads) nvfp4_quant_kernel(const QuantNvParams p) {
+__global__ void __launch_bounds__(kQuantThreads, sizeof(T) == 2 ? 4 : 2) nvfp4_quant_kernel(const QuantNvParams p) {
   __shared__ __align__(16) uint8_t sf[2][512];
-  __shared__ float red[kQuantThreads / 32];
-  __shared__ float ts_s;
   const int tid = threadIdx.x;
-  // tensor amax = max of the partials
-  float amax = 0.0f;
-  for (int i = tid; i < p.n_partials; i += kQuantThreads) amax = fmaxf(amax, p.scratch[i]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((tid & 31) == 0) red[tid >> 5] = amax;
-  reinterpret_cast<uint32_t*>(&sf[0][0])[tid] = 0;   // 1024 bytes: padding rows carry scale 0
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < kQuantThreads / 32; ++w) amax = fmaxf(amax, red[w]);
-    float ts = __fdiv_rn(amax, 2688.0f);              // 6 * 448
-    if (ts == 0.0f) ts = 1.0f;
-    ts_s = ts;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) *p.tensor_scale = ts;
-  }
-  __syncthreads();
-  const float ts = ts_s;
-  const float denom = __fmul_rn(6.0f, ts);
+  grid_dependency_wait();
   const T* xb = reinterpret_cast<const T*>(p.x) + (blockIdx.z / p.H) * p.xs_b + (blockIdx.z % p.H) * p.xs_h;
   uint8_t* codes = p.codes + (long long)blockIdx.z * p.rows * p.ldc_bytes;
-  const int row0 = blockIdx.x * 128, col0 = blockIdx.y * 128;
+  const int row0 = blockIdx.x * 128, c = blockIdx.y * 128 + (tid & 7) * 16;
+  Raw16<T> raw[kRunsPerThread];
 #pragma unroll
   for (int i = 0; i < kRunsPerThread; ++i) {
-    const int g = tid + i * kQuantThreads;          // 16-element block index inside the 128x128 tile
-    const int rl = g >> 3, r = row0 + rl, c = col0 + (g & 7) * 16;
-    if (r >= p.rows || c >= p.cols) continue;
-    float v[16], bmax = 0.0f;
-    load16<T>(xb + (long long)r * p.ld + c, v);
+    const int r = row0 + (tid >> 3) + i * (kQuantThreads / 8);
+    raw[i] = Raw16<T>{};
+    if (r < p.rows && c < p.cols) load_raw<T>(xb + (long long)r * p.ld + c, raw[i]);
+  }
+  float ts = __fdiv_rn(__uint_as_float(__ldcg(p.amax)), 2688.0f);     // 6 * 448
+  if (ts == 0.0f) ts = 1.0f;
+  if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) *p.tensor_scale = ts;
+  const float denom = __fmul_rn(6.0f, ts);
+  reinterpret_cast<uint32_t*>(&sf[0][0])[tid] = 0;   // 1024 bytes: padding rows carry scale 0
+  __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      v[j] = __fmul_rn(v[j], p.s);
-      bmax = fmaxf(bmax, fabsf(v[j]));
+  for (int i = 0; i < kRunsPerThread; ++i) {
+    const int rl = (tid >> 3) + i * (kQuantThreads / 8), r = row0 + rl;
+    if (r >= p.rows || c >= p.cols) continue;
+    float v[16], bmax;
+    unpack16(raw[i], v);
+    if constexpr (sizeof(T) == 2) {
+      // the order of the magnitudes is the order of their patterns, and the largest product is that of the largest (s > 0)
+      const uint32_t w[8] = {raw[i].q[0].x, raw[i].q[0].y, raw[i].q[0].z, raw[i].q[0].w, raw[i].q[1].x, raw[i].q[1].y, raw[i].q[1].z, raw[i].q[1].w};
+      uint32_t m = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m = __vmaxu2(m, w[j] & 0x7fff7fffu);
+      m = max(m & 0xffffu, m >> 16);
+      bmax = fabsf(__fmul_rn(std::is_same<T, __half>::value ? __half2float(__ushort_as_half((unsigned short)m)) : __uint_as_float(m << 16), p.s));
+    } else {
+      bmax = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) bmax = fmaxf(bmax, fabsf(__fmul_rn(v[j], p.s)));
     }
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) nv_mul2(v[j], v[j + 1], p.s);
     const float ratio = fminf(__fdiv_rn(bmax, denom), 448.0f);
     const __nv_fp8_storage_t s8 = __nv_cvt_float_to_fp8(ratio, __NV_SATFINITE, __NV_E4M3);
     const float sdec = __half2float(__half(__nv_cvt_fp8_to_halfraw(s8, __NV_E4M3)));
     const float scf = __fmul_rn(sdec, ts);
     float y[16];
+    if (scf > 1e-25f && scf < 1e25f) {              // no step leaves the normal range where a code could change
+      const float inv = __frcp_rn(scf);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) y[j] = (scf == 0.0f) ? 0.0f : __fdiv_rn(v[j], scf);
+      for (int j = 0; j < 16; j += 2) {
+        float q0 = v[j], q1 = v[j + 1], e0, e1;
+        nv_mul2(q0, q1, inv);
+#pragma unroll
+        for (int step = 0; step < 2; ++step) {
+          nv_fma2(e0, e1, q0, q1, -scf, v[j], v[j + 1]);
+          nv_fma2(q0, q1, e0, e1, inv, q0, q1);
+        }
+        y[j] = q0;
+        y[j + 1] = q1;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) y[j] = scf == 0.0f ? 0.0f : __fdiv_rn(v[j], scf);
+    }
     *reinterpret_cast<uint2*>(codes + (long long)r * p.ldc_bytes + (c >> 1)) = make_uint2(cvt_e2m1x8(y), cvt_e2m1x8(y + 8));
-    const int blk = (g & 7);                        // block inside the tile: chunk blk / 4, column blk % 4
+    const int blk = tid & 7;                        // block inside the tile: chunk blk / 4, column blk % 4
     sf[blk >> 2][(rl & 31) * 16 + (rl >> 5) * 4 + (blk & 3)] = (uint8_t)s8;
   }
   __syncthreads();
@@ -893,13 +945,27 @@ static int launch_nvfp4(const void* x, int in_dtype, int rows, int cols, long lo
     return set_error(MPSA_ERR_UNSUPPORTED, "%s: needs %lld floats of scratch, %lld available", who, n_partials, scratch_floats);
   if (g1.y > 65535 || g2.y > 65535) return set_error(MPSA_ERR_UNSUPPORTED, "%s: too many columns", who);
   QuantNvParams p;
-  p.x = x; p.rows = rows; p.cols = cols; p.ld = ld; p.s = s; p.scratch = scratch; p.n_partials = (int)n_partials;
+  p.x = x; p.rows = rows; p.cols = cols; p.ld = ld; p.s = s; p.amax = reinterpret_cast<unsigned*>(scratch);
   p.codes = (uint8_t*)codes; p.ldc_bytes = ldc_bytes; p.scales = (uint8_t*)scales; p.tensor_scale = tensor_scale;
   p.H = H; p.xs_b = xs_b; p.xs_h = xs_h;
-  if (in_dtype == 0) { nvfp4_amax_kernel<__nv_bfloat16><<<g1, kQuantThreads, 0, st>>>(p); nvfp4_quant_kernel<__nv_bfloat16><<<g2, kQuantThreads, 0, st>>>(p); }
-  else if (in_dtype == 1) { nvfp4_amax_kernel<__half><<<g1, kQuantThreads, 0, st>>>(p); nvfp4_quant_kernel<__half><<<g2, kQuantThreads, 0, st>>>(p); }
-  else { nvfp4_amax_kernel<float><<<g1, kQuantThreads, 0, st>>>(p); nvfp4_quant_kernel<float><<<g2, kQuantThreads, 0, st>>>(p); }
+  if (cudaMemsetAsync(scratch, 0, sizeof(unsigned), st) != cudaSuccess) return check_launch(who);
+  if (in_dtype == 0) nvfp4_amax_kernel<__nv_bfloat16><<<g1, kQuantThreads, 0, st>>>(p);
+  else if (in_dtype == 1) nvfp4_amax_kernel<__half><<<g1, kQuantThreads, 0, st>>>(p);
+  else nvfp4_amax_kernel<float><<<g1, kQuantThreads, 0, st>>>(p);
+  launch_dependent(in_dtype == 0 ? nvfp4_quant_kernel<__nv_bfloat16> : (in_dtype == 1 ? nvfp4_quant_kernel<__half> : nvfp4_quant_kernel<float>),
+                   g2, kQuantThreads, 0, st, true, p);
   return check_launch(who);
+}
+
+int mpsa::nvfp4_quant(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h, long long xs_l, float s,
+                      unsigned* amax, void* codes, void* scales, float* tensor_scale, cudaStream_t st) {
+  if ((long long)B * H > 65535) return set_error(MPSA_ERR_UNSUPPORTED, "attention: batch x heads must be in [1, 65535]");
+  QuantNvParams p;
+  p.x = x; p.rows = L; p.cols = D; p.ld = xs_l; p.s = s; p.amax = amax; p.codes = (uint8_t*)codes; p.ldc_bytes = D / 2;
+  p.scales = (uint8_t*)scales; p.tensor_scale = tensor_scale; p.H = H; p.xs_b = xs_b; p.xs_h = xs_h;
+  launch_dependent(in_dtype == 0 ? nvfp4_quant_kernel<__nv_bfloat16> : nvfp4_quant_kernel<__half>, dim3((L + 127) / 128, (D + 127) / 128, B * H),
+                   kQuantThreads, 0, st, true, p);
+  return check_launch("quant_nvfp4");
 }
 
 extern "C" int mpsa_quant_nvfp4_scratch_floats(int rows, int cols) {

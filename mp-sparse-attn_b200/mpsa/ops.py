@@ -471,7 +471,7 @@ def prepare_kv(k: torch.Tensor, v: torch.Tensor, *, pv_mode: str = "fp16", fp8_e
     return kq, vt
 
 
-_ATTENTION_ARGS = struct.Struct("@3Q9q9Q2Qq2Q16i2f")       # mpsa_attention_args of include/mpsa.h
+_ATTENTION_ARGS = struct.Struct("@3Q9q9Q2Qq2Q17i2f")       # mpsa_attention_args of include/mpsa.h
 _workspace_bytes = {}                                        # problem -> workspace size (bounded)
 _UNIFORM = {None: 0, "fp8": 1, "fp4": 2}
 
@@ -484,7 +484,8 @@ def _strides16(t):
     return a, b, c
 
 
-def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out_dtype, pv_mode, route, tau, smooth_k):
+def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out_dtype, pv_mode, route, tau, smooth_k,
+                        nvfp4):
     """attention_forward through one C call (mpsa_attention), or None where that entry does not take the operands."""
     dt = q.dtype
     in_dtype = 0 if dt is torch.bfloat16 else 1 if dt is torch.float16 else None
@@ -527,7 +528,7 @@ def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out
         _raise_if_failed(q.device)
     pv = 1 if pv_mode == "requant" else 0
     ints = (in_dtype, _OUT_DTYPE[out_dtype], B, Hq, Hkv, S, Skv, D, skv_pad, int(causal), band, uni, int(route), pv,
-            _FP8_DESC[fp8_elem], int(smooth_k))
+            _FP8_DESC[fp8_elem], int(smooth_k), int(nvfp4))
     lib = _lib.load()
     key = (ints, kp == 0, index)                   # the size depends on the number of SMs too
     need = _workspace_bytes.get(key)
@@ -614,10 +615,12 @@ def attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, caus
     sq = q_side_scale(D, sm_scale)
     online = router == "online"
     requant = isinstance(kv[1], QuantizedV) if kv is not None else pv_mode == "requant"
-    if rope is None and prec_map is None and fp4_kind == "mxfp4" and skip_thresh is None and not return_sparsity and \
+    nvfp4 = fp4_kind == "nvfp4"
+    if rope is None and prec_map is None and (fp4_kind == "mxfp4" or (nvfp4 and D == 128 and kv is None and not smooth_k and
+                                                                      uniform is None and not online)) and skip_thresh is None and not return_sparsity and \
             pv_mode in ("fp16", "requant") and (router == "band" or (online and uniform is None and fused_router and causal and requant)):
         out = _attention_one_call(q, k, v, kv, causal=causal, band=band, uniform=uniform, sq=sq, fp8_elem=fp8_elem, out_dtype=out_dtype,
-                                  pv_mode=pv_mode, route=online, tau=float(tau), smooth_k=smooth_k and kv is None)
+                                  pv_mode=pv_mode, route=online, tau=float(tau), smooth_k=smooth_k and kv is None, nvfp4=nvfp4)
         if out is not None:
             if check:
                 check_status(q.device)
