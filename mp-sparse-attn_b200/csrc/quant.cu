@@ -662,9 +662,15 @@ __global__ void __launch_bounds__(kQuantThreads, sizeof(T) == 2 ? 4 : 2) nvfp4_q
 
 namespace mpsa {
 // ---- mean over the sequence per (batch, head, depth index): the vector "smooth K" subtracts ------------------
-// Two launches, fixed summation order: partial column sums of kMeanRows rows per CTA, then their sum / L rounded to
+// Two launches, fixed summation order: partial column sums of some rows per CTA, then their sum / L rounded to
 // the input dtype (torch's mean of a 16-bit tensor accumulates in fp32 and returns the input dtype).
-constexpr int kMeanRows = 512;
+// Rows per CTA: 128 to 512 so that there are some 32 CTAs for a head where it is long enough (a layer of 12 heads with 512
+// rows each left the GPU waiting for four loads in a row: 7803 tokens 21 us, now MEASURE), and not more, because the quantizer adds
+// up the partial sums.
+static __host__ __device__ inline int col_sum_rows(int L) {
+  const int r = ((L + 31) / 32 + 127) & ~127;
+  return r < 128 ? 128 : (r > 512 ? 512 : r);
+}
 // A thread owns 8 columns of every sixteenth row of the chunk and adds its rows one after the other (a fixed order), with
 // eight loads in flight: one layer's K gives a CTA or two per SM, so the bytes in flight are what counts (7803 x 12 x 128:
 // 19 -> 9 us).
@@ -681,9 +687,9 @@ __global__ void __launch_bounds__(256) col_sum_kernel(const T* x, float* part, i
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-  const int r_end = min(L, (chunk + 1) * kMeanRows);
+  const int rows = col_sum_rows(L), r_end = min(L, (chunk + 1) * rows);
   if (c < D) {
-    for (int r = chunk * kMeanRows + rg; r < r_end; r += 128) {
+    for (int r = chunk * rows + rg; r < r_end; r += 128) {
       Cols8<T> v[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
@@ -842,10 +848,10 @@ int mpsa::col_sums(const void* x, int in_dtype, int B, int H, int L, int D, long
   else col_sum_kernel<float><<<grid, 256, 0, st>>>((const float*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
   return check_launch("col_mean");
 }
-int mpsa::col_sum_chunks(int L) { return (L + kMeanRows - 1) / kMeanRows; }
+int mpsa::col_sum_chunks(int L) { return (L + col_sum_rows(L) - 1) / col_sum_rows(L); }
 
 extern "C" long long mpsa_col_mean_scratch_floats(int B, int H, int L, int D) {
-  return (long long)B * H * ((L + kMeanRows - 1) / kMeanRows) * D;
+  return (long long)B * H * mpsa::col_sum_chunks(L) * D;
 }
 
 extern "C" int mpsa_col_mean(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h,
@@ -857,7 +863,7 @@ extern "C" int mpsa_col_mean(const void* x, int in_dtype, int B, int H, int L, i
   if (((uintptr_t)x % 16) || ((xs_b * esz) % 16) || ((xs_h * esz) % 16) || ((xs_l * esz) % 16))
     return set_error(MPSA_ERR_BAD_ARG, "col_mean: input base and strides must be 16-byte aligned");
   if (scratch_floats < mpsa_col_mean_scratch_floats(B, H, L, D)) return set_error(MPSA_ERR_BAD_ARG, "col_mean: scratch too small");
-  const int nchunk = (L + kMeanRows - 1) / kMeanRows;
+  const int nchunk = mpsa::col_sum_chunks(L);
   dim3 grid(nchunk, (D + 127) / 128, B * H);
   if (grid.y > 65535 || grid.z > 65535) return set_error(MPSA_ERR_UNSUPPORTED, "col_mean: B*H and D/128 must be below 65536");
   cudaStream_t st = (cudaStream_t)stream;
