@@ -1,8 +1,6 @@
 """Block quantizers with the signatures of ours/quant_mxint8.py of the reference
 (quant_fpxint8 :61, quant_fpxint8_warp :116, quant_mxfp8e5 :223, quant_mxfp4 :453), running as one
 hand-written CUDA kernel launch per operand."""
-import torch
-
 from mpsa import ops as _ops
 
 
@@ -22,15 +20,13 @@ def quant_mxfp4(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
 def quant_mxfp8e5(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
     """-> (q float8_e5m2, q E8M0 scales, k float8_e5m2, k scales)."""
     sq, sk = _sides(q, k, sm_scale, tensor_layout)
-    qc, qs, kc, ks = _ops.quantize_pair(q, k, sq, sk, "e5m2", tensor_layout)
-    return qc.view(torch.float8_e5m2), qs, kc.view(torch.float8_e5m2), ks
+    return _ops.quantize_pair(q, k, sq, sk, "e5m2", tensor_layout)
 
 
 def quant_mxfp8e4(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
     """E4M3 variant (emax 8, clamp 448); the reference has no such quantizer."""
     sq, sk = _sides(q, k, sm_scale, tensor_layout)
-    qc, qs, kc, ks = _ops.quantize_pair(q, k, sq, sk, "e4m3", tensor_layout)
-    return qc.view(torch.float8_e4m3fn), qs, kc.view(torch.float8_e4m3fn), ks
+    return _ops.quantize_pair(q, k, sq, sk, "e4m3", tensor_layout)
 
 
 def quant_fpxint8(q, k, BLKQ=128, BLKK=64, sm_scale=None, tensor_layout="HND"):
