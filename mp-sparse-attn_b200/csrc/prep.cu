@@ -130,7 +130,6 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
       } else {
         float t = 0.0f;
         const float* part = p.part + (long long)bh * p.nchunk * D + col;
-#pragma unroll 16
         for (int ch = 0; ch < p.nchunk; ++ch) t += __ldcg(part + (long long)ch * D);
         float lo, hi;
         unpack2<T>(pack2<T>(__fdiv_rn(t, (float)p.L), 0.0f), lo, hi);

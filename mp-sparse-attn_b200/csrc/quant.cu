@@ -662,11 +662,12 @@ __global__ void __launch_bounds__(kQuantThreads, sizeof(T) == 2 ? 4 : 2) nvfp4_q
 
 namespace mpsa {
 // ---- mean over the sequence per (batch, head, depth index): the vector "smooth K" subtracts ------------------
-// Two launches, fixed summation order: partial column sums of some rows per CTA, then their sum / L rounded to
+// Two launches, fixed summation order: partial column sums of some rows per cluster of CTAs, then their sum / L rounded to
 // the input dtype (torch's mean of a 16-bit tensor accumulates in fp32 and returns the input dtype).
-// Rows per CTA: 128 to 512 so that there are some 32 CTAs for a head where it is long enough (a layer of 12 heads with 512
-// rows each left the GPU waiting for four loads in a row: 7803 tokens 21 us, now MEASURE), and not more, because the quantizer adds
-// up the partial sums.
+// Rows per CTA: 128 to 512, so that a head has some 32 CTAs where it is long enough: with 512 always, a layer of 12 heads left
+// the GPU waiting for four loads in a row (7803 tokens: 21 us, now 12).  Eight CTAs add theirs up through distributed shared
+// memory, because every CTA of the quantizer reads all partial sums of its head: 31 of them cost it 18 us.
+constexpr int kSumCluster = 8;
 static __host__ __device__ inline int col_sum_rows(int L) {
   const int r = ((L + 31) / 32 + 127) & ~127;
   return r < 128 ? 128 : (r > 512 ? 512 : r);
@@ -676,9 +677,11 @@ static __host__ __device__ inline int col_sum_rows(int L) {
 // 19 -> 9 us).
 template <typename T> struct Cols8 { uint4 q[sizeof(T) == 4 ? 2 : 1]; };
 template <typename T>
-__global__ void __launch_bounds__(256) col_sum_kernel(const T* x, float* part, int H, int L, int D, long long xs_b,
-                                                      long long xs_h, long long xs_l, int nchunk) {
+__global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(256)
+col_sum_kernel(const T* x, float* part, int H, int L, int D, long long xs_b,
+               long long xs_h, long long xs_l, int nchunk) {
   __shared__ float acc_s[16][128];
+  __shared__ float sum_s[128];
   const int chunk = blockIdx.x, col0 = blockIdx.y * 128, bh = blockIdx.z;
   const int b = bh / H, h = bh % H;
   const int c8 = threadIdx.x & 15, rg = threadIdx.x >> 4;      // 16 threads x 8 columns per row, 16 rows per pass
@@ -710,13 +713,26 @@ __global__ void __launch_bounds__(256) col_sum_kernel(const T* x, float* part, i
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc_s[rg][c8 * 8 + j] = acc[j];
   __syncthreads();
-  const int col = col0 + threadIdx.x;
-  if (threadIdx.x < 128 && col < D) {
+  if (threadIdx.x < 128) {
     float t = 0.0f;
 #pragma unroll
     for (int g = 0; g < 16; ++g) t += acc_s[g][threadIdx.x];
-    part[((long long)bh * nchunk + chunk) * D + col] = t;
+    sum_s[threadIdx.x] = t;
   }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int col = col0 + threadIdx.x;
+  if (chunk % kSumCluster == 0 && threadIdx.x < 128 && col < D) {
+    float t = 0.0f;
+#pragma unroll
+    for (int g = 0; g < kSumCluster; ++g) {
+      float v;
+      asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}"
+                   : "=f"(v) : "r"(smem_u32(&sum_s[threadIdx.x])), "r"(g) : "memory");
+      t += v;
+    }
+    part[((long long)bh * nchunk + chunk / kSumCluster) * D + col] = t;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // sum_s has been read
 }
 
 template <typename T>
@@ -842,13 +858,13 @@ extern "C" int mpsa_rope_quant_mx(const void* x, int in_dtype, int B, int H, int
 
 int mpsa::col_sums(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h, long long xs_l,
                    float* part, int nchunk, cudaStream_t st) {
-  const dim3 grid(nchunk, (D + 127) / 128, B * H);
+  const dim3 grid(nchunk * kSumCluster, (D + 127) / 128, B * H);
   if (in_dtype == 0) col_sum_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
   else if (in_dtype == 1) col_sum_kernel<__half><<<grid, 256, 0, st>>>((const __half*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
   else col_sum_kernel<float><<<grid, 256, 0, st>>>((const float*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
   return check_launch("col_mean");
 }
-int mpsa::col_sum_chunks(int L) { return (L + col_sum_rows(L) - 1) / col_sum_rows(L); }
+int mpsa::col_sum_chunks(int L) { return (L + kSumCluster * col_sum_rows(L) - 1) / (kSumCluster * col_sum_rows(L)); }
 
 extern "C" long long mpsa_col_mean_scratch_floats(int B, int H, int L, int D) {
   return (long long)B * H * mpsa::col_sum_chunks(L) * D;
