@@ -87,28 +87,86 @@ __device__ __forceinline__ float fp4_snap_fast(float y) {
   return fabsf(y) >= 1.0f ? z : h;
 }
 
+// E2M1 codes of 16 elements from their packed patterns, one code per byte in element order; kb: exponent field of the x whose scaled
+// value lies in [1, 2).  Position of |x| above y = .5 in pattern steps, bits 7.. counting binades: a class is a binade and
+// whether the position inside it reaches `upper`.  Positions up to there collapse into 0 and, where y > .125, get `upper`
+// added back: everything in (.125, 1) is one class.
+__device__ __forceinline__ void e2m1_patterns(const uint32_t* w, int kb, const PrepThresholds& thr, uint32_t* q) {
+  const int k1 = thr.k1 - (kb << 7), kn = k1 + thr.kd;
+  const uint32_t c1 = __byte_perm(k1, 0, 0x1010), cn = __byte_perm(kn, 0, 0x1010);
+  uint32_t u[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t t = w[j] & 0x7fff7fffu;
+    const uint32_t pos = __viaddmin_s16x2_relu(t, c1, thr.cmax);
+    const uint32_t n = __viaddmin_s16x2_relu(t, cn, 0x00010001u);      // 1 iff y > .125
+    const uint32_t q0 = pos * 4 + n * thr.ck;
+    u[j] = __viaddmin_u16x2(q0, thr.ca, q0 | 0x01fc01fcu);             // class in bits 8..10, never carried into the next binade
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t cd = __byte_perm(u[2 * j], u[2 * j + 1], 0x7531), sn = __byte_perm(w[2 * j], w[2 * j + 1], 0x7531);
+    q[j] = cd | ((sn >> 4) & 0x08080808u);
+  }
+}
+__device__ __forceinline__ void e2m1_no_minus_zero(const uint32_t* w, uint32_t* q) {      // -0 counts as positive
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if ((w[j] & 0xffffu) == 0x8000u) q[j >> 1] &= ~(0x08u << ((j & 1) * 16));
+    if ((w[j] >> 16) == 0x8000u) q[j >> 1] &= ~(0x0800u << ((j & 1) * 16));
+  }
+}
+template <typename T>
+__device__ __forceinline__ void e2m1_arithmetic(const uint32_t* w, float s, float inv_scale, uint32_t* q) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    float y[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float x0, x1;
+      unpack2<T>(w[4 * j + k], x0, x1);
+      y[2 * k] = fp4_snap_fast(__fmaf_rn(__fmul_rn(x0, s), inv_scale, 0.0f));
+      y[2 * k + 1] = fp4_snap_fast(__fmaf_rn(__fmul_rn(x1, s), inv_scale, 0.0f));
+    }
+    const uint32_t e = cvt_e2m1x8(y), ev = e & 0x0f0f0f0fu, od = (e >> 4) & 0x0f0f0f0fu;
+    q[2 * j] = __byte_perm(ev, od, 0x5140);
+    q[2 * j + 1] = __byte_perm(ev, od, 0x7362);
+  }
+}
+// n / d for n below the bound the host checked (see div_magic), one multiplication; magic 0: an ordinary division, d = 1 apart
+__device__ __forceinline__ int div_by(int n, int d, uint32_t magic) {
+  return d == 1 ? n : (magic ? (int)__umulhi((uint32_t)n, magic) : n / d);
+}
+
 // One tile of 128 rows (depth 128 and more) or 256 rows (depth 64) of one (batch, head).  A thread owns runs of 16 elements, two
 // neighbouring lanes one 32-element block.  All loads of the CTA go out before any arithmetic, held as they arrived;
 // scale codes are gathered with shuffles and stored a row at a time, so that no thread waits for another.  (Persistent
 // CTAs that copy their next tile to shared memory under the present one were slower: 172 against 141 us for 167M elements.)
+// What bounds it is instruction issue, so the loop over the runs is straight-line code for blocks in the middle of the
+// exponent range (24 -> 18 instructions an element with both formats, most of the difference branches; 67M elements 56.7 ->
+// 46.7 us, MXFP4 alone to one code a byte 5.7 TB/s, MXFP8 alone 6.9); a warp that meets another block - all zero, near an end
+// of the range, or whose maximum is so close below a power of two that log2 rounds up - fetches the run again after the
+// loop and takes the general code.  MXFP4 needs more registers than four CTAs an SM leave it (spills): three.
 template <typename T, bool W8, bool W4, bool E4M3, bool D64>
 __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D, float* mean) {
   constexpr bool PATTERNS = W4 && std::is_same<T, __nv_bfloat16>::value;
   constexpr int LPR = D64 ? 4 : 8;                      // 16-element runs of a row inside the tile
   constexpr int ROWS = D64 ? 256 : 128;
   constexpr int RSTEP = PREP_THREADS / LPR;             // a thread's four runs are this many rows apart
+  constexpr int EMAX8 = E4M3 ? 8 : 7, EMAX4 = 3;
   const int tid = threadIdx.x;
   const int cl = (tid & (LPR - 1)) * 16, rl0 = tid / LPR;
   const int ntd = D64 ? 1 : D >> 7;
   const int ntl = (p.L + ROWS - 1) / ROWS;
-  const int v0 = D64 ? tile : tile / ntd, tile_d = D64 ? 0 : tile - v0 * ntd;
-  const int bh = v0 / ntl, tile_l = v0 - bh * ntl;
-  const int b = bh / p.H, h = bh - b * p.H, c = tile_d * 128 + cl;
+  const int v0 = ntd == 1 ? tile : tile / ntd, tile_d = tile - v0 * ntd;
+  const int bh = div_by(v0, ntl, p.ntl_magic), tile_l = v0 - bh * ntl;
+  const int b = div_by(bh, p.H, p.h_magic), h = bh - b * p.H, c = tile_d * 128 + cl;
   const int r0 = tile_l * ROWS + rl0, n_live = p.L - r0;     // run i is inside the operand iff i * RSTEP < n_live
+  const T* const x0 = reinterpret_cast<const T*>(p.x) + (long long)b * p.xs_b + (long long)h * p.xs_h + (long long)r0 * p.xs_l + c;
+  const long long xstep = p.xs_l * RSTEP;
   uint4 raw[4][2];
   {
-    const T* x = reinterpret_cast<const T*>(p.x) + (long long)b * p.xs_b + (long long)h * p.xs_h + (long long)r0 * p.xs_l + c;
-    const long long step = p.xs_l * RSTEP;
+    const T* x = x0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       raw[i][0] = raw[i][1] = make_uint4(0, 0, 0, 0);
@@ -116,7 +174,7 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
         raw[i][0] = __ldg(reinterpret_cast<const uint4*>(x));
         raw[i][1] = __ldg(reinterpret_cast<const uint4*>(x) + 1);
       }
-      x += step;
+      x += xstep;
     }
   }
   const bool centred = p.part || p.mean;
@@ -151,135 +209,172 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
   // 512-byte scale tiles: row r, block k at byte (r % 32) * 16 + (r / 32) * 4 + k
   const int ntr = (p.L + 127) >> 7, tr0 = tile_l * (ROWS >> 7);
   const long long tl0 = (((long long)bh * ntr + tr0) * ntd + tile_d) * 512 + (rl0 & 31) * 16 + (rl0 >> 5) * 4;
+  auto centre = [&](uint32_t* w) {
+    if (centred) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float a, d;
+        unpack2<T>(w[j], a, d);
+        w[j] = pack2<T>(a - mean[cl + 2 * j], d - mean[cl + 2 * j + 1]);
+      }
+    }
+  };
+  // Block maximum on the patterns: without the sign their order as integers is the order of the magnitudes, and the maximum of
+  // the rounded products |x| * s is the rounded product of the maximum (s > 0).  The smallest pattern as a signed number is
+  // 0x8000 iff there is a -0.
+  auto block_amax = [&](const uint32_t* w, uint32_t& lowest) {
+    uint32_t m = 0;
+    lowest = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      m = __vimax3_s16x2(m, w[j] & 0x7fff7fffu, w[j + 1] & 0x7fff7fffu);
+      if (PATTERNS) lowest = __vimin3_s16x2(lowest, w[j], w[j + 1]);
+    }
+    m = max(m & 0xffffu, m >> 16);
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    return __fmul_rn(pattern_to_float<T>(m), p.s);
+  };
+  auto store_fp4 = [&](int i, const uint32_t* q) {
+    if (o4) *reinterpret_cast<uint4*>(o4 + i * s4) = make_uint4(q[0], q[1], q[2], q[3]);
+    if (op) {
+      uint32_t pk[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {                     // bytes -> nibbles
+        const uint32_t a = q[2 * k] | (q[2 * k] >> 4), d = q[2 * k + 1] | (q[2 * k + 1] >> 4);        // bytes 0 and 2 hold two codes each
+        pk[k] = __byte_perm(a, d, 0x6420);
+      }
+      *reinterpret_cast<uint2*>(op + i * sp) = make_uint2(pk[0], pk[1]);
+    }
+  };
+  // a row's scale codes in one word, one store per row and layout; rows beyond L and blocks beyond D hold 1.0
+  auto gather = [&](uint32_t code) {
+    uint32_t v = code << (((tid >> 1) & (LPR / 2 - 1)) * 8);
+    v |= __shfl_xor_sync(0xffffffffu, v, 2);
+    if (!D64) v |= __shfl_xor_sync(0xffffffffu, v, 4);
+    return v;
+  };
+  auto store_scale = [&](int i, bool live, uint8_t* st, uint8_t* rm, uint32_t v) {
+    if (st && (D64 ? tr0 + (i >> 1) : tr0) < ntr) *reinterpret_cast<uint32_t*>(st + tl0 + (D64 ? (i >> 1) * 512 + (i & 1) * 8 : i * 4)) = D64 ? v | 0x7f7f0000u : v;
+    if (rm && live) {
+      if (D64) *reinterpret_cast<uint16_t*>(rm + rm0 + i * (RSTEP * 2)) = (uint16_t)v;
+      else *reinterpret_cast<uint32_t*>(rm + rm0 + (long long)i * RSTEP * nblk) = v;
+    }
+  };
+  // With |es| <= 16 (mild) and the exponent field of the block's maximum in 48 .. 230 no scale code is clamped, s / scale and the
+  // products that matter are normal, and every code boundary is the pattern of a normal number.
+  const bool fast_operand = p.thr.mild && (!PATTERNS || p.thr.valid);
+  uint32_t todo = 0, exps[4];                           // runs that need the general code; exponent fields of a row's blocks
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const bool live = i * RSTEP < n_live;
     uint32_t w[8] = {raw[i][0].x, raw[i][0].y, raw[i][0].z, raw[i][0].w, raw[i][1].x, raw[i][1].y, raw[i][1].z, raw[i][1].w};
-    if (centred) {
+    centre(w);
+    uint32_t lowest;
+    const float amax = block_amax(w, lowest);
+    if (AMAX) amax_all = fmaxf(amax_all, live ? amax : 0.0f);
+    const uint32_t ab = __float_as_uint(amax), ef = ab >> 23;
+    const bool plain = !live || (fast_operand && ef - 48u <= 182u && (ab & 0x007fffffu) < 0x007fff00u);
+    if (!__all_sync(0xffffffffu, plain)) {
+      todo |= 1u << i;
+      exps[i] = 0;
+      continue;
+    }
+    if (W8) {
+      const float f = p.s * __uint_as_float((254u + EMAX8 - ef) << 23);      // s / scale
+      uint32_t o[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float x0, x1;
-        unpack2<T>(w[j], x0, x1);
-        w[j] = pack2<T>(x0 - mean[cl + 2 * j], x1 - mean[cl + 2 * j + 1]);
+      for (int j = 0; j < 4; ++j) {
+        float a0, a1, a2, a3;
+        unpack2<T>(w[2 * j], a0, a1);
+        unpack2<T>(w[2 * j + 1], a2, a3);
+        mul2(a0, a1, f);
+        mul2(a2, a3, f);
+        o[j] = cvt_fp8x4<E4M3>(a0, a1, a2, a3);
+      }
+      if (o8 && live) *reinterpret_cast<uint4*>(o8 + i * s8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    if (W4) {
+      uint32_t q[4];
+      if (PATTERNS) {
+        e2m1_patterns(w, (int)ef - EMAX4 - p.thr.es, p.thr, q);
+        if ((lowest & 0xffffu) == 0x8000u || (lowest >> 16) == 0x8000u) e2m1_no_minus_zero(w, q);
+      } else {
+        e2m1_arithmetic<T>(w, p.s, __uint_as_float((254u + EMAX4 - ef) << 23), q);
+      }
+      if (live) store_fp4(i, q);
+    }
+    exps[i] = gather(live ? ef : 0u);
+  }
+  // scale code = exponent field - emax: no byte borrows from the next (rows whose run is still to do are written again below)
+  if ((tid & (LPR - 1)) == 0) {
+    constexpr uint32_t ONES = D64 ? 0x0101u : 0x01010101u;
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      if (!(f ? W4 : W8)) continue;
+      uint32_t v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = i * RSTEP < n_live ? exps[i] - ONES * (f ? EMAX4 : EMAX8) : 0x7f7f7f7fu;
+      uint8_t* st = f ? p.sf4_tiled : p.sf8_tiled;
+      uint8_t* rm = f ? p.sc4_rows : p.sc8_rows;
+      if (st && !D64) *reinterpret_cast<uint4*>(st + tl0) = make_uint4(v[0], v[1], v[2], v[3]);      // rows 32 apart lie side by side
+      if (rm || D64) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) store_scale(i, i * RSTEP < n_live, D64 ? st : nullptr, rm, v[i]);
       }
     }
-    // block maximum on the patterns: their order as unsigned integers is the order of the magnitudes.  The smallest
-    // pattern as a signed number is 0x8000 iff there is a -0.
-    uint32_t m = 0, lowest = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      m = __vmaxu2(m, w[j] & 0x7fff7fffu);
-      if (PATTERNS) lowest = __vmins2(lowest, w[j]);
+  }
+#pragma unroll 1
+  for (; todo; todo &= todo - 1) {
+    const int i = __ffs(todo) - 1;
+    const bool live = i * RSTEP < n_live;
+    uint4 r[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+    if (live) {
+      r[0] = __ldg(reinterpret_cast<const uint4*>(x0 + i * xstep));
+      r[1] = __ldg(reinterpret_cast<const uint4*>(x0 + i * xstep) + 1);
     }
-    m = max(m & 0xffffu, m >> 16);
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    // the maximum of the rounded products |x| * s is the rounded product of the maximum (s > 0)
-    const float amax = __fmul_rn(pattern_to_float<T>(m), p.s);
-    if (AMAX) amax_all = fmaxf(amax_all, amax);
+    uint32_t w[8] = {r[0].x, r[0].y, r[0].z, r[0].w, r[1].x, r[1].y, r[1].z, r[1].w};
+    centre(w);
+    uint32_t lowest;
+    const float amax = block_amax(w, lowest);
     uint32_t code8 = 127, code4 = 127;
     if (live) {
       if (W8) {
-        const BlockScale b8 = mx_block_scale(amax, E4M3 ? 8 : 7);
+        const BlockScale b8 = mx_block_scale(amax, EMAX8);
         code8 = b8.code;
         uint32_t o[4];
-        if (b8.zero) {
-          o[0] = o[1] = o[2] = o[3] = 0;                // the reference stores the NaN pattern of 0/0 here
-        } else {
-          const bool one = p.thr.mild && b8.code > 20 && b8.code < 235;   // s / scale and the products that matter are normal
-          const float f = one ? p.s * b8.inv_scale : p.s;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float x0, x1, x2, x3;
-            unpack2<T>(w[2 * j], x0, x1);
-            unpack2<T>(w[2 * j + 1], x2, x3);
-            mul2(x0, x1, f);
-            mul2(x2, x3, f);
-            if (!one) { mul2(x0, x1, b8.inv_scale); mul2(x2, x3, b8.inv_scale); }
-            o[j] = cvt_fp8x4<E4M3>(x0, x1, x2, x3);
-          }
+        for (int j = 0; j < 4; ++j) {
+          float a0, a1, a2, a3;
+          unpack2<T>(w[2 * j], a0, a1);
+          unpack2<T>(w[2 * j + 1], a2, a3);
+          mul2(a0, a1, p.s);
+          mul2(a2, a3, p.s);
+          mul2(a0, a1, b8.inv_scale);
+          mul2(a2, a3, b8.inv_scale);
+          o[j] = b8.zero ? 0u : cvt_fp8x4<E4M3>(a0, a1, a2, a3);      // the reference stores the NaN pattern of 0/0 there
         }
         if (o8) *reinterpret_cast<uint4*>(o8 + i * s8) = make_uint4(o[0], o[1], o[2], o[3]);
       }
       if (W4) {
-        const BlockScale b4 = mx_block_scale(amax, 3);
+        const BlockScale b4 = mx_block_scale(amax, EMAX4);
         code4 = b4.code;
-        uint32_t q[4];                                  // one code per byte, element order
-        const int base = (int)b4.code - p.thr.es;       // exponent field of the x whose scaled value lies in [1, 2)
+        uint32_t q[4];
+        const int base = (int)b4.code - p.thr.es;
         if (b4.zero) {
           q[0] = q[1] = q[2] = q[3] = 0x08080808u;      // 0/0 in the reference: sign 1, exponent 0, mantissa 0
         } else if (PATTERNS && p.thr.valid && base >= 4 && base <= 253) {
-          // position of |x| above y = .5 in pattern steps, bits 7.. counting binades: a class is a binade and whether the
-          // position inside it reaches `upper`.  Positions up to there collapse into 0 and, where y > .125, get `upper`
-          // added back: everything in (.125, 1) is one class.
-          const int k1 = p.thr.k1 - (base << 7), kn = k1 + p.thr.kd;
-          const uint32_t c1 = __byte_perm(k1, 0, 0x1010), cn = __byte_perm(kn, 0, 0x1010);
-          uint32_t u[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint32_t t = w[j] & 0x7fff7fffu;
-            const uint32_t pos = __viaddmin_s16x2_relu(t, c1, p.thr.cmax);
-            const uint32_t n = __viaddmin_s16x2_relu(t, cn, 0x00010001u);      // 1 iff y > .125
-            const uint32_t q0 = pos * 4 + n * p.thr.ck;
-            u[j] = __viaddmin_u16x2(q0, p.thr.ca, q0 | 0x01fc01fcu);           // class in bits 8..10, never carried into the next binade
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t cd = __byte_perm(u[2 * j], u[2 * j + 1], 0x7531), sn = __byte_perm(w[2 * j], w[2 * j + 1], 0x7531);
-            q[j] = cd | ((sn >> 4) & 0x08080808u);
-          }
-          if ((lowest & 0xffffu) == 0x8000u || (lowest >> 16) == 0x8000u) {    // -0 counts as positive
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if ((w[j] & 0xffffu) == 0x8000u) q[j >> 1] &= ~(0x08u << ((j & 1) * 16));
-              if ((w[j] >> 16) == 0x8000u) q[j >> 1] &= ~(0x0800u << ((j & 1) * 16));
-            }
-          }
+          e2m1_patterns(w, base, p.thr, q);
+          e2m1_no_minus_zero(w, q);
         } else {
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            float y[8];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              float x0, x1;
-              unpack2<T>(w[4 * j + k], x0, x1);
-              y[2 * k] = fp4_snap_fast(__fmaf_rn(__fmul_rn(x0, p.s), b4.inv_scale, 0.0f));
-              y[2 * k + 1] = fp4_snap_fast(__fmaf_rn(__fmul_rn(x1, p.s), b4.inv_scale, 0.0f));
-            }
-            const uint32_t e = cvt_e2m1x8(y), ev = e & 0x0f0f0f0fu, od = (e >> 4) & 0x0f0f0f0fu;
-            q[2 * j] = __byte_perm(ev, od, 0x5140);
-            q[2 * j + 1] = __byte_perm(ev, od, 0x7362);
-          }
+          e2m1_arithmetic<T>(w, p.s, b4.inv_scale, q);
         }
-        if (o4) *reinterpret_cast<uint4*>(o4 + i * s4) = make_uint4(q[0], q[1], q[2], q[3]);
-        if (op) {
-          uint32_t pk[2];
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {                 // bytes -> nibbles
-            const uint32_t a = q[2 * k] | (q[2 * k] >> 4), d = q[2 * k + 1] | (q[2 * k + 1] >> 4);    // bytes 0 and 2 hold two codes each
-            pk[k] = __byte_perm(a, d, 0x6420);
-          }
-          *reinterpret_cast<uint2*>(op + i * sp) = make_uint2(pk[0], pk[1]);
-        }
+        store_fp4(i, q);
       }
     }
-    // a row's scale codes in one word, one store per row and layout; rows beyond L and blocks beyond D hold 1.0
-    const bool tiled_row = (D64 ? tr0 + (i >> 1) : tr0) < ntr;
-    const long long tl = tl0 + (D64 ? (i >> 1) * 512 + (i & 1) * 8 : i * 4);
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      if (!(f ? W4 : W8)) continue;
-      uint32_t v = (f ? code4 : code8) << (((tid >> 1) & (LPR / 2 - 1)) * 8);
-      v |= __shfl_xor_sync(0xffffffffu, v, 2);
-      if (!D64) v |= __shfl_xor_sync(0xffffffffu, v, 4);
-      if ((tid & (LPR - 1)) == 0) {
-        uint8_t* st = f ? p.sf4_tiled : p.sf8_tiled;
-        uint8_t* rm = f ? p.sc4_rows : p.sc8_rows;
-        if (st && tiled_row) *reinterpret_cast<uint32_t*>(st + tl) = D64 ? v | 0x7f7f0000u : v;
-        if (rm && live) {
-          if (D64) *reinterpret_cast<uint16_t*>(rm + rm0 + i * (RSTEP * 2)) = (uint16_t)v;
-          else *reinterpret_cast<uint32_t*>(rm + rm0 + (long long)i * RSTEP * nblk) = v;
-        }
-      }
+    const uint32_t v8 = W8 ? gather(code8) : 0u, v4 = W4 ? gather(code4) : 0u;
+    if ((tid & (LPR - 1)) == 0) {
+      if (W8) store_scale(i, live, p.sf8_tiled, p.sc8_rows, v8);
+      if (W4) store_scale(i, live, p.sf4_tiled, p.sc4_rows, v4);
     }
   }
   if (AMAX && p.amax) {                                 // few warps find a new maximum: the others only look at the word
@@ -387,7 +482,7 @@ __device__ __forceinline__ void v_tile(const PrepV& p, int cta, int D, uint8_t* 
 }
 
 template <typename T, bool W8, bool W4, bool E4M3, bool D64>
-__global__ void __launch_bounds__(PREP_THREADS, 4) prep_kernel(const __grid_constant__ PrepCall p) {
+__global__ void __launch_bounds__(PREP_THREADS, W4 ? 3 : 4) prep_kernel(const __grid_constant__ PrepCall p) {
   extern __shared__ __align__(128) uint8_t prep_smem[];
   int cta = blockIdx.x;
   grid_dependency_wait();
@@ -460,6 +555,12 @@ bool prep_operand_ok(const PrepOperand& p, int D) {
          (p.xs_h * 2) % 16 == 0 && (p.xs_l * 2) % 16 == 0;
 }
 
+// n / d == mulhi(n, magic) for 0 <= n < bound: magic = ceil(2^32 / d) is too large by less than d / 2^32 of a unit, which
+// does no harm while n d < 2^32 (d = 1 has no such magic); 0 otherwise
+static uint32_t div_magic(int d, long long bound) {
+  return d > 1 && bound * d < (1ll << 32) ? (uint32_t)(((1ull << 32) + d - 1) / d) : 0;
+}
+
 int prep_launch(PrepCall& p, int in_dtype, bool w8, bool w4, int fp8_fmt, cudaStream_t st) {
   long long ctas = 0;
   const int rows_cta = p.D == 64 ? 256 : 128, ntd = p.D == 64 ? 1 : p.D / 128;
@@ -467,6 +568,8 @@ int prep_launch(PrepCall& p, int in_dtype, bool w8, bool w4, int fp8_fmt, cudaSt
     o.ctas = 0;
     if (!o.x) continue;
     o.thr = prep_thresholds(o.s);
+    o.ntl_magic = div_magic((o.L + rows_cta - 1) / rows_cta, (long long)o.B * o.H * ((o.L + rows_cta - 1) / rows_cta));
+    o.h_magic = div_magic(o.H, (long long)o.B * o.H);
     const long long n = (long long)o.B * o.H * ((o.L + rows_cta - 1) / rows_cta) * ntd;
     ctas += n;
     if (ctas > 0x3fffffff) return set_error(MPSA_ERR_UNSUPPORTED, "prep: operand too large");

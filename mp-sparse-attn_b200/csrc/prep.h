@@ -29,7 +29,8 @@ struct PrepOperand {
   uint8_t* sc8_rows = nullptr; uint8_t* sc4_rows = nullptr;       // [B,H,L,D/32]
   uint8_t* sf8_tiled = nullptr; uint8_t* sf4_tiled = nullptr;     // [B,H,ceil(L/128),ceil(D/128),512]
   unsigned* amax = nullptr;                            // optional word, zero before: bits of the largest |x * s|
-  PrepThresholds thr;                                  // filled in by prep_launch
+  PrepThresholds thr;                                  // filled in by prep_launch, like what follows
+  uint32_t ntl_magic = 0, h_magic = 0;                 // division by row tiles and by heads
   int ctas = 0;
 };
 
