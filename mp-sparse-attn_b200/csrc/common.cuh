@@ -32,6 +32,9 @@ __device__ __forceinline__ bool elect_one() {
 
 // In a kernel launched as a dependent of the one before it: returns when that one is complete and its writes are visible.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets a kernel launched as a dependent of this one start as soon as every CTA of this one has got here (it still waits for this
+// one's end before it reads what this one writes).
+__device__ __forceinline__ void grid_dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- mbarrier ---------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

@@ -186,6 +186,8 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
       if (p.mean) {
         mean[tid] = p.mean[(long long)bh * D + col];
       } else {
+        // only this waits for the column sums: everything else a launch reads or writes was ready, and free, before them
+        grid_dependency_wait();
         float t = 0.0f;
         const float* part = p.part + (long long)bh * p.nchunk * D + col;
         for (int ch = 0; ch < p.nchunk; ++ch) t += __ldcg(part + (long long)ch * D);
@@ -485,7 +487,7 @@ template <typename T, bool W8, bool W4, bool E4M3, bool D64>
 __global__ void __launch_bounds__(PREP_THREADS, W4 ? 3 : 4) prep_kernel(const __grid_constant__ PrepCall p) {
   extern __shared__ __align__(128) uint8_t prep_smem[];
   int cta = blockIdx.x;
-  grid_dependency_wait();
+  grid_dependents_go();
   if (cta == 0 && threadIdx.x < 2) {
     // words the launches behind this one expect to find zero
     int* z = threadIdx.x ? p.zero1 : p.zero0;

@@ -582,6 +582,7 @@ template <typename T>
 __global__ void __launch_bounds__(kQuantThreads, sizeof(T) == 2 ? 4 : 2) nvfp4_quant_kernel(const QuantNvParams p) {
   __shared__ __align__(16) uint8_t sf[2][512];
   const int tid = threadIdx.x;
+  grid_dependents_go();
   grid_dependency_wait();
   const T* xb = reinterpret_cast<const T*>(p.x) + (blockIdx.z / p.H) * p.xs_b + (blockIdx.z % p.H) * p.xs_h;
   uint8_t* codes = p.codes + (long long)blockIdx.z * p.rows * p.ldc_bytes;
@@ -682,6 +683,7 @@ col_sum_kernel(const T* x, float* part, int H, int L, int D, long long xs_b,
                long long xs_h, long long xs_l, int nchunk) {
   __shared__ float acc_s[16][128];
   __shared__ float sum_s[128];
+  grid_dependents_go();
   const int chunk = blockIdx.x, col0 = blockIdx.y * 128, bh = blockIdx.z;
   const int b = bh / H, h = bh % H;
   const int c8 = threadIdx.x & 15, rg = threadIdx.x >> 4;      // 16 threads x 8 columns per row, 16 rows per pass
