@@ -1660,17 +1660,23 @@ int attn_forward(const AttnCall& call, cudaStream_t st) {
 
   AttnMaps m;
   const uint64_t qrows = (uint64_t)c.B * c.Hq * c.S, krows = (uint64_t)c.B * c.Hkv * c.Skv, vrows = (uint64_t)c.B * c.Hkv * c.D;
-  bool bad = make_tmap_2d_bytes(&m.q8, c.q8, ATT_DQK, qrows, ATT_DQK, 128, ATT_BM, CU_TENSOR_MAP_SWIZZLE_128B) ||
-             make_tmap_2d_bytes(&m.q4, c.q4, ATT_DQK / 2, qrows, ATT_DQK / 2, 64, ATT_BM, CU_TENSOR_MAP_SWIZZLE_64B) ||
-             make_tmap_2d_bytes(&m.k8, c.k8, ATT_DQK, krows, ATT_DQK, 128, ATT_BN, CU_TENSOR_MAP_SWIZZLE_128B) ||
-             make_tmap_2d_bytes(&m.k4, c.k4, ATT_DQK / 2, krows, ATT_DQK / 2, 64, ATT_BN, CU_TENSOR_MAP_SWIZZLE_64B);
+  // an absent format's maps are copies of the other's (they are not dereferenced): encoding takes 0.4 us of the host's time each
+  bool bad = false;
+  if (c.need8) bad = make_tmap_2d_bytes(&m.q8, c.q8, ATT_DQK, qrows, ATT_DQK, 128, ATT_BM, CU_TENSOR_MAP_SWIZZLE_128B) ||
+                     make_tmap_2d_bytes(&m.k8, c.k8, ATT_DQK, krows, ATT_DQK, 128, ATT_BN, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (c.need4) bad = bad || make_tmap_2d_bytes(&m.q4, c.q4, ATT_DQK / 2, qrows, ATT_DQK / 2, 64, ATT_BM, CU_TENSOR_MAP_SWIZZLE_64B) ||
+                     make_tmap_2d_bytes(&m.k4, c.k4, ATT_DQK / 2, krows, ATT_DQK / 2, 64, ATT_BN, CU_TENSOR_MAP_SWIZZLE_64B);
+  if (!c.need8) { m.q8 = m.q4; m.k8 = m.k4; }
+  if (!c.need4) { m.q4 = m.q8; m.k4 = m.k8; }
   if (c.pv_mode == 0) {
     bad = bad || make_tmap_2d_b16(&m.vt, c.vt, c.Skv_pad, vrows, (uint64_t)c.Skv_pad * 2, 64, c.D, CU_TENSOR_MAP_SWIZZLE_128B);
-    m.vt8 = m.vt4 = m.vt;        // not dereferenced in this mode
+    m.vt8 = m.vt4 = m.vt;
   } else {
-    bad = bad || make_tmap_2d_bytes(&m.vt8, c.vt8, c.Skv_pad, vrows, c.Skv_pad, 128, c.D, CU_TENSOR_MAP_SWIZZLE_128B) ||
-          make_tmap_2d_bytes(&m.vt4, c.vt4, c.Skv_pad / 2, vrows, c.Skv_pad / 2, 64, c.D, CU_TENSOR_MAP_SWIZZLE_64B);
-    m.vt = m.vt8;                // not dereferenced in this mode
+    if (c.need8) bad = bad || make_tmap_2d_bytes(&m.vt8, c.vt8, c.Skv_pad, vrows, c.Skv_pad, 128, c.D, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (c.need4) bad = bad || make_tmap_2d_bytes(&m.vt4, c.vt4, c.Skv_pad / 2, vrows, c.Skv_pad / 2, 64, c.D, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (!c.need8) m.vt8 = m.vt4;
+    if (!c.need4) m.vt4 = m.vt8;
+    m.vt = m.vt8;
   }
   if (bad) return set_error(MPSA_ERR_LAUNCH, "attn_fwd: cuTensorMapEncodeTiled failed");
 
