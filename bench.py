@@ -6,7 +6,7 @@ Workload (N=1): causal prefill attention shaped like a Llama-3-8B layer - B=1, H
 D=128, S=32768, bf16 inputs N(0,1) with 5 of the 128 K channels scaled x20, diagonal tiles in
 MXFP8 and the rest in MXFP4 unless the online router promotes them (statistic of the MXFP4 score tile >=
 TAU x that of the row's first key tile), P re-quantised to the tile's format before P.V (V quantised along
-the sequence).  One step = quantise Q and K (both formats, one pass each), quantise V and run the fused forward
+the sequence).  One step = quantise Q, K (both formats) and V in one launch and run the fused forward
 with the router inside it (a promoted tile is done again in MXFP8 at the end of its row).  Metric: effective attention TFLOP/s =
 4*B*Hq*S^2*D/2 / time.  With N > 1 every rank runs the same workload on its own batch element
 (batch x head sharding, no collective; weak scaling) and the value is the sum over ranks divided by
@@ -40,7 +40,7 @@ import torch  # noqa: E402
 
 HQ, HKV, D = 32, 8, 128
 OUTLIERS = 5
-LAUNCHES_PER_STEP = 4      # quant Q, quant K, quant V, forward
+LAUNCHES_PER_STEP = 2      # operand preparation (Q, K, V in one launch), forward
 TAU = 1.1                  # online router: a tile is promoted to MXFP8 iff its statistic >= TAU x the first key tile's
 # DRAM bytes (read + written) of one launch of the fused forward at S=8192, from an ncu capture; every term of it
 # (Q, K, V codes and scales, the output) grows linearly with S
@@ -203,8 +203,7 @@ def run_ours(args):
 
     vt = mpsa.quantize_v_seq(v)
     plain_ms = time_forward(vt)                  # one launch over the final map (no router inside)
-    # the dominant kernel of the step: the routed forward (router inside; the band-map launch before it
-    # takes a few microseconds and is inside the bracket), and the whole routed forward
+    # the dominant kernel of the step: the routed forward (router inside, one launch)
     attn_ms = timed(lambda: mpsa.attention_forward_routed(qq, kq, vt, 1, HQ, HKV, S, S, D, band=1, tau=TAU, stages=3))
     routed_ms = timed(lambda: mpsa.attention_forward_routed(qq, kq, vt, 1, HQ, HKV, S, S, D, band=1, tau=TAU))
     band = mpsa.precision_map_band(S, S, True, 1, 128, dev)
