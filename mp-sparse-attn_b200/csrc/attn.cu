@@ -22,9 +22,9 @@
 // anything before the end of the item.  Quantised P.V: block-scaled P carries its magnitude in E8M0 codes, and with
 // an integral reference the element codes do not depend on it at all; m = 20 serves every row whose maximum M lies in
 // [-44, 84] (P, O and the row sums then stay within 2^-64 .. 2^64).  fp16 P.V: m is the row maximum of the item's first
-// tile, good while M - m is in [0, 15] (P at most 2^15; fp16 keeps its relative precision over that range).  An item with
-// a row outside its window is done again a little later, in two passes: the first finds the exact row maxima, the second
-// uses them as references.
+// tile, or what its scores let expect of the item where that is higher, good while M - m is in [-6, 15] (P at most 2^15;
+// fp16 keeps its relative precision down to 2^-8 of the largest P at least).  An item with a row outside its window is
+// done again a little later, with the row maxima that the first pass found as references.
 //
 // Roles: warp 0 TMA loads, warp 1 Q.K^T issuer, warp 2 P.V issuer, warp 3 hands out work items, builds their visit lists
 // (the non-skipped cells of the map row) and routes, warps 4.. softmax and epilogue (a warp reaches the TMEM lane
@@ -57,6 +57,7 @@ constexpr int ATT_Q8_BYTES = ATT_BM * 128, ATT_Q4_BYTES = ATT_BM * 64;
 constexpr int ATT_Q_BYTES = ATT_Q8_BYTES + ATT_Q4_BYTES;
 constexpr int ATT_K_BYTES = ATT_BN * 128;             // slot sized for the FP8 tile; FP4 uses half
 constexpr int ATT_V_BYTES = 128 * ATT_BN * 2;         // V^T tile, up to D=128 rows of 128 fp16
+constexpr int ATT_MAX_SLOTS = 3;                                          // work items whose visit lists are in shared memory at a time
 constexpr int ATT_OFF_Q = 0;                                              // [2] Q8 tile, Q4 tile
 constexpr int ATT_OFF_K = ATT_OFF_Q + 2 * ATT_Q_BYTES;
 constexpr int ATT_OFF_V = ATT_OFF_K + ATT_KSTAGES * ATT_K_BYTES;
@@ -66,14 +67,14 @@ constexpr int ATT_OFF_SFP = ATT_OFF_SFK + ATT_KSTAGES * 1024;             // P s
 constexpr int ATT_OFF_XROW = ATT_OFF_SFP + (2 + ATT_VSLOTS_MAX) * 512;    // float [2][2][4][128]: row sums and row maxima of the four threads of a row
 constexpr int ATT_OFF_RMAX = ATT_OFF_XROW + 2 * 2 * 4 * 128 * 4;          // float [2 buffers][2][128]: slice maxima for the router; fp16 P.V: first-tile maxima
 constexpr int ATT_OFF_MROW = ATT_OFF_RMAX + 2 * 2 * 128 * 4;              // float [128]: row reference (fp16 P.V)
-constexpr int ATT_OFF_BAR = ATT_OFF_MROW + 128 * 4;
-constexpr int ATT_MAX_SLOTS = 3;                                          // work items whose visit lists are in shared memory at a time
+constexpr int ATT_OFF_MSLOT = ATT_OFF_MROW + 128 * 4;                     // float [MAX_SLOTS][128]: row maxima of the item that was in the slot
+constexpr int ATT_OFF_BAR = ATT_OFF_MSLOT + ATT_MAX_SLOTS * 128 * 4;
 // barriers the softmax threads use in their tile loop, by number
 constexpr int ATT_B_SFULL = 4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX;
 constexpr int ATT_B_SFREE = ATT_B_SFULL + 2, ATT_B_PREADY = ATT_B_SFULL + 4, ATT_B_PVDONE = ATT_B_SFULL + 8, ATT_B_ST = ATT_B_SFULL + 14;
 constexpr int ATT_NUM_BARS = 4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX + 4 + 8 + 2 + 2 + 12;
 constexpr int ATT_BAR_BYTES = 1024;                                       // barriers, TMEM slot, router words, item slots
-static_assert(ATT_NUM_BARS * 8 + 32 + ATT_MAX_SLOTS * 32 <= ATT_BAR_BYTES, "the barrier block does not fit its share of shared memory");
+static_assert(ATT_NUM_BARS * 8 + 32 + ATT_MAX_SLOTS * 36 <= ATT_BAR_BYTES, "the barrier block does not fit its share of shared memory");
 constexpr int ATT_OFF_LIST = ATT_OFF_BAR + ATT_BAR_BYTES;                 // visit lists: n_lists x list_cap uint16
 constexpr int ATT_MAX_KTILES = 8192;                                      // longest row of the precision map (1M keys)
 constexpr int ATT_SMEM_MAX = 232448;
@@ -100,7 +101,7 @@ constexpr int SPLIT_MIN_RUN = 8;                      // tiles of a run at least
 constexpr int SPLIT_GAIN = 12;                        // tiles (of 0.7 us) that dividing the keys must save on the busiest CTA
 constexpr float ATT_REF_Q = 20.0f;                    // quantised P.V: the row reference, and the window of row maxima it serves
 constexpr float ATT_WIN_LO_Q = -64.0f, ATT_WIN_HI_Q = 64.0f;
-constexpr float ATT_WIN_HI_F16 = 15.0f;               // fp16 P.V: row maximum above the reference at most
+constexpr float ATT_WIN_LO_F16 = -6.0f, ATT_WIN_HI_F16 = 15.0f;   // fp16 P.V: the same window (P at most 2^15; normal numbers down to 2^-8 of the largest)
 
 // Division of the keys.  Items are numbered heaviest query tile first: item = r * heads + head, r counting query tiles
 // from the last.  The first n_whole are done by one CTA each; the tiles of the others, laid end to end, are cut into runs
@@ -459,7 +460,8 @@ __device__ __forceinline__ void softmax_block_f16(const uint32_t* sc, float mref
 // One slot of the visit-list ring: a work item and its tiles.
 struct Slot {
   int qi, h, b;
-  int mode;          // 0 an item's ordinary pass; 1, 2 the two passes of an item that is done again; -1 no more items
+  int mode;          // 0 an item's ordinary pass; 1 it is done again; -1 no more items
+  int from;          // mode 1: slot of the first pass, which left the row maxima
   int n_own;         // tiles of the map row
   int n_total;       // ROUTE: appended tiles included, valid once list_done has completed
   int redo;          // set by the softmax threads: a row maximum lies outside the reference's window
@@ -850,12 +852,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     bool ok = true;
     int emitted = 0, reclaimed = 0;                 // slots filled, and taken back
     int next_local = 0;                             // static schedule: items taken so far
-    int rq[4], rn = 0;                              // slots' work waiting to be done again (never more than the slots)
-    int redo_item = -1;                             // work whose second pass follows
+    int redo_item = -1, redo_from = 0;              // work to be done again: it is the next to be handed out
     const int heads = p.Hq * p.B;
     int held[ATT_MAX_SLOTS];                        // work in each slot, -1: nothing that could come back
     // Work is an item number; a share of a run's also has the run in wrun (0: the whole item).
-    [[maybe_unused]] int held_run[ATT_MAX_SLOTS], rq_run[4], redo_run = 0;
+    [[maybe_unused]] int held_run[ATT_MAX_SLOTS], redo_run = 0;
     [[maybe_unused]] int run = 0;                   // this CTA's present run, from 1
     [[maybe_unused]] long long run_pos = 0, run_end = 0;
     [[maybe_unused]] const SplitPlan plan = split_plan(heads, p.S, p.Skv, p.causal, p.n_whole, p.run_tiles);
@@ -867,25 +868,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       int it = -1, rw = 0;
 #pragma unroll
       for (int k = 0; k < ATT_MAX_SLOTS; ++k) if (k == s) { it = held[k]; if (SPLIT) rw = held_run[k]; }
-      if (ok && it >= 0 && slots[s].redo) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) if (k == rn) { rq[k] = it; if (SPLIT) rq_run[k] = rw; }
-        ++rn;
-      }
+      if (ok && it >= 0 && slots[s].redo) { redo_item = it; redo_run = rw; redo_from = s; }
     };
     // The next item into the next slot, which is free: first what has to be done again, then the schedule.  Items are
     // numbered heaviest query tile first; they are taken from a counter in memory where the caller gives one, else in
     // snake order over the CTAs, which evens out the sum.  false: nothing left.
     auto emit = [&]() -> bool {
       int item, mode = 0, wrun = 0;
-      if (redo_item >= 0) { item = redo_item; if (SPLIT) wrun = redo_run; mode = 2; redo_item = -1; }
-      else if (rn > 0) {
-        item = rq[0];
-        if (SPLIT) { wrun = rq_run[0]; rq_run[0] = rq_run[1]; rq_run[1] = rq_run[2]; rq_run[2] = rq_run[3]; redo_run = wrun; }
-        rq[0] = rq[1]; rq[1] = rq[2]; rq[2] = rq[3];
-        --rn;
+      if (redo_item >= 0) {
+        item = redo_item;
+        if (SPLIT) wrun = redo_run;
         mode = 1;
-        redo_item = item;
+        redo_item = -1;
       } else if (SPLIT && run_pos < run_end) {
         item = plan.item_at(run_pos, p.n_items);
         wrun = run;
@@ -948,7 +942,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       }
       __syncwarp();
       if (lane == 0) {
-        slots[s].qi = qi; slots[s].h = h; slots[s].b = b; slots[s].mode = mode; slots[s].n_own = base; slots[s].n_total = base;
+        slots[s].qi = qi; slots[s].h = h; slots[s].b = b; slots[s].mode = mode; slots[s].from = redo_from; slots[s].n_own = base; slots[s].n_total = base;
         slots[s].redo = 0;
         if (SPLIT) slots[s].part = part;
         mbar_arrive(&list_full[s]);                 // release: entries (__syncwarp) and slot are visible to who waits
@@ -1025,7 +1019,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       const bool want = !exhausted && emitted - seq < ahead;
       if (want ? emitted - reclaimed >= NL : (seq == emitted && reclaimed < emitted)) {
         reclaim();
-        if (rn > 0) exhausted = false;
+        if (redo_item >= 0) exhausted = false;
       } else if (want) {
         exhausted = !emit();
       } else if (seq < emitted) {
@@ -1054,6 +1048,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     float* xrow = reinterpret_cast<float*>(smem + ATT_OFF_XROW);
     float* rmax = reinterpret_cast<float*>(smem + ATT_OFF_RMAX);
     float* mrow = reinterpret_cast<float*>(smem + ATT_OFF_MROW);
+    float* mslot = reinterpret_cast<float*>(smem + ATT_OFF_MSLOT);
     uint8_t* psf_dst = sSFP + wg * 512 + lane * 16 + q * 4 + g * 2;
     const float nvmul = NVF4 ? (p.ts_q ? *p.ts_q * *p.ts_k : p.fp4_scale) : 1.0f;   // scores of NVFP4 tiles lack the tensor scales
     // An item's epilogue is put off until this thread has done its first tile of the next item, so that neither the last
@@ -1069,7 +1064,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     const uint32_t pv16_flip = (g == 1 && wg == 1) ? 0 : 1;
     uint32_t kp = 0;                                // parity of this warpgroup's tile count
     float* rmax_w = rmax + (wg * 2 + g) * 128 + r_in;
-    float m_redo = 0.0f;                            // row maximum found by the first pass of an item that is done again
+    float m_redo = 0.0f;                            // row reference of an item that is done again: the maximum its first pass found
     float mref = 0.0f, l_run = 0.0f, m_run = -INFINITY;   // row reference; partial row sum and maximum over this thread's keys
     [[maybe_unused]] float pend_l = 0.0f;           // ROUTE: row sum of the last MXFP4 tile, until its decision is looked up
     [[maybe_unused]] int pend_t = -1;
@@ -1215,7 +1210,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           ok = __all_sync(0xffffffffu, mbar_wait(&list_full[ls], l_par, p.status, KS_TIMEOUT_PIPE));
           if (!ok) break;
           mode = slots[ls].mode;
-          do_epi = epi && mode == 2;                // its row maxima are needed now
+          do_epi = epi && mode == 1;                // m_redo may still be in use
         }
         if (do_epi) {
         } else if (mode < 0) {
@@ -1229,7 +1224,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           lim = p.causal ? min(p.Skv - 1, m_glob + off) : (p.Skv - 1);   // last visible key of this row
           l_run = 0.0f;
           m_run = -INFINITY;
-          mref = mode == 2 ? m_redo : ((PVQ && mode == 0) ? ATT_REF_Q : 0.0f);
+          if (mode == 1) m_redo = mslot[slots[ls].from * 128 + r_in];
+          mref = mode == 1 ? m_redo : (PVQ ? ATT_REF_Q : 0.0f);
           i = (t0 & 1) ^ wg;                        // first tile of the list this warpgroup owns
           if (PVQ == 0 && mode == 0 && n_tiles > 0) {
             // the row's reference: the maximum of the item's first tile, found by its owners
@@ -1239,7 +1235,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               tc_fence_after();
               const uint32_t e = lists[ls * p.list_cap];
               const int last = lim - ((int)(e & ENTRY_TILE) * ATT_BN + g * 64);
-              float mx = -INFINITY;
+              float mx = -INFINITY, s0 = 0.0f, s1 = 0.0f, q0 = 0.0f, q1 = 0.0f;
 #pragma unroll
               for (int c = 0; c < 2; ++c) {
                 uint32_t sc[32];
@@ -1247,15 +1243,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
                 tmem_ld_wait();
                 if (e & ENTRY_MASK) mask32(sc, last - c * 32);
                 mx = fmaxf(mx, block_max32(sc));
+#pragma unroll
+                for (int k = 0; k < 32; k += 2) {
+                  const float a = __uint_as_float(sc[k]), c2 = __uint_as_float(sc[k + 1]);
+                  add2(s0, s1, a, c2);
+                  q0 = fmaf(a, a, q0);
+                  q1 = fmaf(c2, c2, q1);
+                }
               }
-              if (NVF4 && !(e & ENTRY_F8)) mx *= nvmul;
+              if (NVF4 && !(e & ENTRY_F8)) { mx *= nvmul; s0 *= nvmul; s1 *= nvmul; q0 *= nvmul * nvmul; q1 *= nvmul * nvmul; }
               rmax[g * 128 + r_in] = mx;
+              // expected maximum of the item's scores, from this thread's 64: mean + z(n) sigma, z(n) = 2.59 + .2 log2(n / 128) that
+              // of n normal variables
+              const float mean = (s0 + s1) * (1.0f / 64.0f), var = fmaxf((q0 + q1) * (1.0f / 64.0f) - mean * mean, 0.0f);
+              rmax[(2 + g) * 128 + r_in] = (e & ENTRY_MASK) ? -INFINITY : mean + sqrtf(var) * (2.59f + 0.2f * __log2f((float)n_tiles));
               __syncwarp();
               if (lane == 0) mbar_arrive(&x_bar[q]);
               ok = __all_sync(0xffffffffu, mbar_wait(&x_bar[q], n_ref & 1, p.status, KS_TIMEOUT_PIPE));
               if (!ok) break;
               mref = fmaxf(rmax[r_in], rmax[128 + r_in]);
               if (mref == -INFINITY) mref = 0.0f;
+              // The reference follows the expected maximum where that is higher: with outlier channels in the keys most items
+              // of 32768 keys left the window above the first tile's maximum (16.4 ms, against 8.1 now).
+              mref = fmaxf(mref, 0.5f * (rmax[256 + r_in] + rmax[384 + r_in]) - 1.0f);
               if (g == 0) {
                 mrow[r_in] = mref;
                 __syncwarp();
@@ -1288,7 +1298,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         // a share of an item: fp32 and the log2 denominator, into its slice of the partial results
         const int part = SPLIT ? slots[epi_ls].part : -1;
         const int item = (nq - 1 - slots[epi_ls].qi) * p.Hq * p.B + head;
-        const float ref = PVQ ? (mode == 2 ? m_redo : ATT_REF_Q) : mref;
+        const float ref = PVQ ? (mode == 1 ? m_redo : ATT_REF_Q) : mref;
         const bool has_o = epi_part * 32 < p.D;     // this thread's 32 columns of O
         uint32_t o[32];
         if (tiles) {
@@ -1303,18 +1313,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         if (mode == 0) {
           const float over = m_tot - ref;           // rows of the ragged tail hold no data
           const bool out_of_window = m_glob < p.S && m_tot != -INFINITY &&
-                                     (PVQ ? (over < ATT_WIN_LO_Q || over > ATT_WIN_HI_Q) : (over < 0.0f || over > ATT_WIN_HI_F16));
+                                     (PVQ ? (over < ATT_WIN_LO_Q || over > ATT_WIN_HI_Q) : (over < ATT_WIN_LO_F16 || over > ATT_WIN_HI_F16));
           if (out_of_window) {
             slots[epi_ls].redo = 1;
             if (p.range_flag) *p.range_flag = 1;
           }
+          if (epi_part == 0) mslot[epi_ls * 128 + r_in] = m_tot == -INFINITY ? 0.0f : (PVQ ? ceilf(m_tot) : m_tot);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&list_empty[epi_ls]);
         epi = false;
-        if (mode == 1) {
-          m_redo = (m_tot == -INFINITY) ? 0.0f : (PVQ ? ceilf(m_tot) : m_tot);
-        } else if (m_glob < p.S) {
+        if (m_glob < p.S) {
           float inv_l = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
           float lse_row = 0.0f, w_prev = 0.0f;      // w_prev: weight of the earlier partial result (merge mode)
           if (p.lse || part >= 0) lse_row = l_tot > 0.0f ? ref + log2f(l_tot) : -INFINITY;
