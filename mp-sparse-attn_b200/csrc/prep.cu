@@ -527,10 +527,16 @@ PrepThresholds prep_thresholds(float s) {
   t.es = e - 1;
   t.mild = t.es >= -16 && t.es <= 16;
   // y = fl(x * s): the first of the 128 mantissas whose product reaches the next binade
-  int first = 128;
-  for (int m = 0; m < 128; ++m) {
-    if ((1.0f + (float)m / 128.0f) * ms >= 2.0f) { first = m; break; }
-  }
+  // (products of neighbouring mantissas differ by ms / 128, far more than a rounding: everything here is strictly monotone)
+  auto lowest = [](int n, auto reached) {               // smallest i in [0, n] with reached(i), n if none
+    int lo = 0, hi = n;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (reached(mid)) hi = mid; else lo = mid + 1;
+    }
+    return lo;
+  };
+  const int first = lowest(128, [&](int m) { return (1.0f + (float)m / 128.0f) * ms >= 2.0f; });
   // y's mantissa at position k = 0 .. 127 of its own binade
   auto mant = [&](int k) {
     const int m = first + k;                            // x mantissas first .. 127, then 0 .. first - 1 of the next binade
@@ -538,8 +544,7 @@ PrepThresholds prep_thresholds(float s) {
   };
   const int shift = 128 - first;                        // added to a pattern, bits 7.. count the binades of y
   const int strict = mant(0) == 1.0f;                   // position 0 of a binade is a power of two exactly
-  t.upper = 0;
-  while (t.upper < 128 && !(mant(t.upper) > 1.25f)) ++t.upper;
+  t.upper = lowest(128, [&](int k) { return mant(k) > 1.25f; });
   t.valid = t.upper <= 64;
   t.k1 = shift + 0x80 - t.upper;
   t.kd = t.upper - 0x80 + 0x180 - strict + 1;
@@ -547,7 +552,6 @@ PrepThresholds prep_thresholds(float s) {
   t.cmax = lanes(0x1ff - t.upper);
   t.ca = lanes((0x40 - t.upper) * 4);
   t.ck = (uint32_t)t.upper * 4;
-  for (int k = 0; k < 128; ++k) t.valid = t.valid && mant(k) >= 1.0f && mant(k) < 2.0f && (k == 0 || mant(k) > mant(k - 1));
   return t;
 }
 
