@@ -99,6 +99,7 @@ constexpr uint32_t ENTRY_F8 = 0x8000, ENTRY_MASK = 0x4000, ENTRY_TILE = 0x3fff; 
 #endif
 constexpr int SPLIT_MIN_RUN = 8;                      // tiles of a run at least
 constexpr int SPLIT_GAIN = 12;                        // tiles (of 0.7 us) that dividing the keys must save on the busiest CTA
+constexpr int SPLIT_MIN_OWN = 4, SPLIT_GAIN_OWN = 7;  // the same two where every part has a CTA to itself
 constexpr float ATT_REF_Q = 20.0f;                    // quantised P.V: the row reference, and the window of row maxima it serves
 constexpr float ATT_WIN_LO_Q = -64.0f, ATT_WIN_HI_Q = 64.0f;
 constexpr float ATT_WIN_LO_F16 = -6.0f, ATT_WIN_HI_F16 = 15.0f;   // fp16 P.V: the same window (P at most 2^15; normal numbers down to 2^-8 of the largest)
@@ -110,12 +111,14 @@ constexpr float ATT_WIN_LO_F16 = -6.0f, ATT_WIN_HI_F16 = 15.0f;   // fp16 P.V: t
 struct SplitPlan {
   int heads, nq, nk, causal, c1;     // c1: visible tiles of query tile 0
   int n_whole, run_tiles;
+  int pad;                           // 0, or the places every item takes: a multiple of run_tiles, so that no run holds two items
   __host__ __device__ long long row_tiles(int r) const { return !causal || r == 0 ? nk : nq - 1 - r + c1; }
   __host__ __device__ long long rows_before(int r) const {          // tiles of one head's rows 0 .. r-1
     if (!causal || r <= 1) return (long long)r * nk;
     return nk + (long long)(r - 1) * (nq - 1 + c1) - (long long)(r - 1) * r / 2;
   }
   __host__ __device__ long long start(int item) const {             // tiles of all items before this one
+    if (pad) return (long long)item * pad;
     const int r = item / heads;
     return rows_before(r) * heads + (item - r * heads) * row_tiles(r);
   }
@@ -128,11 +131,11 @@ struct SplitPlan {
     return lo;
   }
 };
-static __host__ __device__ SplitPlan split_plan(int heads, int S, int Skv, int causal, int n_whole, int run_tiles) {
+static __host__ __device__ SplitPlan split_plan(int heads, int S, int Skv, int causal, int n_whole, int run_tiles, int pad) {
   SplitPlan s;
   s.heads = heads; s.nq = (S + ATT_BM - 1) / ATT_BM; s.nk = (Skv + ATT_BN - 1) / ATT_BN; s.causal = causal;
   s.c1 = (ATT_BM - 1 + Skv - S) / ATT_BN + 1;
-  s.n_whole = n_whole; s.run_tiles = run_tiles;
+  s.n_whole = n_whole; s.run_tiles = run_tiles; s.pad = pad;
   return s;
 }
 
@@ -163,7 +166,7 @@ struct AttnParams {
   int* status;
   int n_items;                       // query tiles x heads x batches
   int n_work, n_whole;               // units handed out: n_whole items, then runs of run_tiles tiles over the other items (SplitPlan)
-  int run_tiles;
+  int run_tiles, run_pad;
   float* part_o; float* part_lse;    // partial results of items that several runs share: [part][item - n_whole][128][D], [..][128]
   int group;                         // q-heads per KV head
   int* counter;                      // optional, zero on entry: items are handed out in turn instead of by a fixed schedule
@@ -843,7 +846,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     [[maybe_unused]] int held_run[ATT_MAX_SLOTS], redo_run = 0;
     [[maybe_unused]] int run = 0;                   // this CTA's present run, from 1
     [[maybe_unused]] long long run_pos = 0, run_end = 0;
-    [[maybe_unused]] const SplitPlan plan = split_plan(heads, p.S, p.Skv, p.causal, p.n_whole, p.run_tiles);
+    [[maybe_unused]] const SplitPlan plan = split_plan(heads, p.S, p.Skv, p.causal, p.n_whole, p.run_tiles, p.run_pad);
     [[maybe_unused]] const long long run_base = SPLIT ? plan.start(p.n_whole) : 0;
     auto reclaim = [&]() {
       const int s = reclaimed % NL;
@@ -897,12 +900,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       const int last_key = min(p.S - 1, qi * ATT_BM + ATT_BM - 1) + off;    // last key any row of the tile may see
       int base = 0, j_lo = 0, j_hi = nk, part = -1;
       if (SPLIT && wrun > 0) {                     // the run's share of the item
-        const long long it0 = plan.start(item), it1 = plan.start(item + 1);
+        const long long it0 = plan.start(item), it1 = it0 + plan.row_tiles(r);
         const long long a = run_base + (long long)(wrun - 1) * p.run_tiles, e = a + p.run_tiles;
         if (it0 < a || it1 > e) {
           part = wrun - 1 - (int)((it0 - run_base) / p.run_tiles);
           j_lo = (int)(max(a, it0) - it0);
-          j_hi = (int)(min(e, it1) - it0);
+          j_hi = (int)(min(e, it1) - it0);          // (padded places at the end: no tile)
         }
       }
       _Pragma("unroll 1") for (int i0 = j_lo; i0 < j_hi; i0 += 32) {
@@ -1589,10 +1592,13 @@ int launch_attn(int grid, size_t smem, cudaStream_t st, bool after_prep, const A
 // k times the lightest of the (k - 1) * SMs + 1 heaviest items, for every k; with one it has the mean of what is cut.  A cut
 // costs the combination (5 us), partial results in fp32 and one more item a CTA: with 12 tiles to save it breaks even (12
 // heads of 1560 tokens, 26 tiles against 14: 29.6 us either way).  16 queries against 32768 keys, 32 heads on 148 SMs, 256
-// tiles against 56: 195 -> 58 us; 512 queries, 256 against 221: 199 -> 187 us.
-int split_choose(const AttnCall& c, int nq, int nk, int& n_whole, int& run_tiles) {
+// tiles against 56: 195 -> 58 us; 512 queries, 256 against 221: 199 -> 187 us.  Short runs over light items lose (8 heads of
+// 2500 tokens, causal, runs of 12 tiles in up to 12 items: 28 -> 48 us), parts with a CTA to themselves gain from 7 tiles on
+// (16 queries of 2048 keys, 16 tiles against 4: 20.2 -> 16.4 us).
+int split_choose(const AttnCall& c, int nq, int nk, int& n_whole, int& run_tiles, int& pad) {
+  pad = 0;
   const int heads = c.B * c.Hq, n_items = nq * heads, sms = sm_count();
-  const SplitPlan all = split_plan(heads, c.S, c.Skv, c.causal, 0, 1);
+  const SplitPlan all = split_plan(heads, c.S, c.Skv, c.causal, 0, 1, 0);
   const long long total = all.start(n_items);
   long long whole = (total + sms - 1) / sms;
   for (long long k = 1; (k - 1) * sms < n_items; ++k) whole = std::max(whole, k * all.row_tiles((int)((k - 1) * sms) / heads));
@@ -1602,6 +1608,14 @@ int split_choose(const AttnCall& c, int nq, int nk, int& n_whole, int& run_tiles
   if (n_whole > 0 && run_of(n_whole) < SPLIT_MIN_RUN) n_whole -= sms;
   run_tiles = (int)std::max<long long>(SPLIT_MIN_RUN, run_of(n_whole));
   const long long cut = (all.start(n_whole) + sms - 1) / sms + run_tiles;
+  if (n_items * 2 <= sms) {
+    // so few items that each gets CTAs of its own: equal parts, one a CTA, which saves the second item a CTA
+    const int n = (int)all.row_tiles(0), k = std::min(sms / n_items, (n + SPLIT_MIN_OWN - 1) / SPLIT_MIN_OWN), run = (n + k - 1) / k;
+    if (k > 1 && whole - run >= SPLIT_GAIN_OWN && run <= cut + SPLIT_GAIN - SPLIT_GAIN_OWN) {
+      n_whole = 0; run_tiles = run; pad = (n + run - 1) / run * run;
+      return pad / run + 1;
+    }
+  }
   if (n_whole == n_items || whole - cut < SPLIT_GAIN) { n_whole = n_items; run_tiles = 1; return 0; }
   return (int)((all.row_tiles(n_whole / heads) - 1) / run_tiles) + 2;
 }
@@ -1611,8 +1625,8 @@ long long attn_split_bytes(const AttnCall& c) {
   if (c.route || c.fp4_kind) return 0;
   const int nq = (c.S + ATT_BM - 1) / ATT_BM, nk = (c.Skv + ATT_BN - 1) / ATT_BN;
   if ((long long)nq * c.Hq * c.B >= (1ll << 30)) return 0;
-  int n_whole, run_tiles;
-  const int parts = split_choose(c, nq, nk, n_whole, run_tiles);
+  int n_whole, run_tiles, pad;
+  const int parts = split_choose(c, nq, nk, n_whole, run_tiles, pad);
   return (long long)parts * ((long long)nq * c.Hq * c.B - n_whole) * ATT_BM * (c.D + 1) * 4;
 }
 
@@ -1688,11 +1702,11 @@ int attn_forward(const AttnCall& call, cudaStream_t st) {
   p.list_cap = ((c.route ? 2 * nk : nk) + 7) & ~7;
   p.n_lists = std::min(ATT_MAX_SLOTS, (ATT_SMEM_MAX - 1024 - ATT_OFF_LIST) / (p.list_cap * 2));
   const size_t smem = ATT_OFF_LIST + (size_t)p.n_lists * p.list_cap * 2 + 1024;
-  int parts = 0, n_whole = p.n_items, run_tiles = 1;
-  if (c.partial) parts = split_choose(c, nq, nk, n_whole, run_tiles);
+  int parts = 0, n_whole = p.n_items, run_tiles = 1, pad = 0;
+  if (c.partial) parts = split_choose(c, nq, nk, n_whole, run_tiles, pad);
   const long long n_shared = p.n_items - n_whole;
-  const SplitPlan plan = split_plan(c.B * c.Hq, c.S, c.Skv, c.causal, n_whole, run_tiles);
-  p.n_whole = n_whole; p.run_tiles = run_tiles;
+  const SplitPlan plan = split_plan(c.B * c.Hq, c.S, c.Skv, c.causal, n_whole, run_tiles, pad);
+  p.n_whole = n_whole; p.run_tiles = run_tiles; p.run_pad = pad;
   p.n_work = n_whole + (int)((plan.start(p.n_items) - plan.start(n_whole) + run_tiles - 1) / run_tiles);
   p.part_o = (float*)c.partial;
   p.part_lse = p.part_o + parts * n_shared * ATT_BM * c.D;

@@ -9,6 +9,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("S,Skv,Hq,Hkv,D,causal,pv_mode,gain", [
     (16, 2048, 32, 8, 128, True, "requant", 1.0),       # two runs of a row, 16 rows of a tile in use
     (1, 16300, 3, 1, 128, True, "requant", 1.0),        # one row, a ragged last key tile, most runs inside one item
+    (900, 1300, 4, 2, 128, True, "fp16", 1.0),          # three parts with a CTA each, the last one empty for the shorter rows
     (130, 20000, 8, 2, 64, True, "fp16", 1.0),          # two query tiles of different length, depth 64
     (1560, 1560, 12, 12, 128, False, "requant", 1.0),   # 156 items on 148 SMs
     (700, 9000, 16, 4, 128, False, "fp16", 1.0),
