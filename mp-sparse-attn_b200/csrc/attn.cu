@@ -1252,7 +1252,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               if (mref == -INFINITY) mref = 0.0f;
               // The reference follows the expected maximum where that is higher: with outlier channels in the keys most items
               // of 32768 keys left the window above the first tile's maximum (16.4 ms, against 8.1 now).
-              mref = fmaxf(mref, 0.5f * (rmax[256 + r_in] + rmax[384 + r_in]) - 1.0f);
+              // (By whole octaves, which leave P's mantissas and so its rounding as they are.)
+              mref += floorf(fmaxf(0.5f * (rmax[256 + r_in] + rmax[384 + r_in]) - 1.0f - mref, 0.0f));
               if (g == 0) {
                 mrow[r_in] = mref;
                 __syncwarp();
