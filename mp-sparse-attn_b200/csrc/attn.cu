@@ -22,8 +22,8 @@
 // anything before the end of the item.  Quantised P.V: block-scaled P carries its magnitude in E8M0 codes, and with
 // an integral reference the element codes do not depend on it at all; m = 20 serves every row whose maximum M lies in
 // [-44, 84] (P, O and the row sums then stay within 2^-64 .. 2^64).  fp16 P.V: m is the row maximum of the item's first
-// tile, or what its scores let expect of the item where that is higher, good while M - m is in [-6, 15] (P at most 2^15;
-// fp16 keeps its relative precision down to 2^-8 of the largest P at least).  An item with a row outside its window is
+// tile, or what its scores let expect of the item where that is higher, good while M - m is in [-8, 15] (P at most 2^15;
+// fp16 keeps its relative precision down to 2^-6 of the largest P at least, and 2^-16 of it beyond).  An item with a row outside its window is
 // done again a little later, with the row maxima that the first pass found as references.
 //
 // Roles: warp 0 TMA loads, warp 1 Q.K^T issuer, warp 2 P.V issuer, warp 3 hands out work items, builds their visit lists
@@ -102,7 +102,7 @@ constexpr int SPLIT_GAIN = 12;                        // tiles (of 0.7 us) that 
 constexpr int SPLIT_MIN_OWN = 4, SPLIT_GAIN_OWN = 7;  // the same two where every part has a CTA to itself
 constexpr float ATT_REF_Q = 20.0f;                    // quantised P.V: the row reference, and the window of row maxima it serves
 constexpr float ATT_WIN_LO_Q = -64.0f, ATT_WIN_HI_Q = 64.0f;
-constexpr float ATT_WIN_LO_F16 = -6.0f, ATT_WIN_HI_F16 = 15.0f;   // fp16 P.V: the same window (P at most 2^15; normal numbers down to 2^-8 of the largest)
+constexpr float ATT_WIN_LO_F16 = -8.0f, ATT_WIN_HI_F16 = 15.0f;   // fp16 P.V: the same window (P at most 2^15; normal numbers down to 2^-6 of the largest)
 
 // Division of the keys.  Items are numbered heaviest query tile first: item = r * heads + head, r counting query tiles
 // from the last.  The first n_whole are done by one CTA each; the tiles of the others, laid end to end, are cut into runs
@@ -1251,9 +1251,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               mref = fmaxf(rmax[r_in], rmax[128 + r_in]);
               if (mref == -INFINITY) mref = 0.0f;
               // The reference follows the expected maximum where that is higher: with outlier channels in the keys most items
-              // of 32768 keys left the window above the first tile's maximum (16.4 ms, against 8.1 now).
+              // of 32768 keys left the window above the first tile's maximum (16.4 ms, against 7.1 now).
               // (By whole octaves, which leave P's mantissas and so its rounding as they are.)
-              mref += floorf(fmaxf(0.5f * (rmax[256 + r_in] + rmax[384 + r_in]) - 1.0f - mref, 0.0f));
+              mref += floorf(fmaxf(0.5f * (rmax[256 + r_in] + rmax[384 + r_in]) + 1.0f - mref, 0.0f));
               if (g == 0) {
                 mrow[r_in] = mref;
                 __syncwarp();
