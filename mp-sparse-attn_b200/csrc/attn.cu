@@ -32,7 +32,7 @@
 // across items, so an item's Q, K and V loads and its first tiles happen under the previous item's last ones.
 //
 // What bounds it: the exponentials.  ex2 runs at 16 per clock and SM (measured), i.e. 1024 cycles for the 16384 scores of
-// a tile; four of every 32 are computed on the FMA pipe instead.  A loop of the tile's softmax arithmetic alone, 16 warps
+// a tile; on MXFP4 tiles with quantised P.V two of every 32 are computed on the FMA pipe instead.  A loop of the tile's softmax arithmetic alone, 16 warps
 // on TMEM data, takes 1003 cycles a tile; with all hand-offs and MMAs 1160.
 #include "api_internal.h"
 #include "common.cuh"
@@ -91,12 +91,7 @@ constexpr uint32_t ATT_COL_P16 = 416;                             // fp16 P: 3 b
 constexpr int TILE_SKIP = 0, TILE_FP8 = 1, TILE_FP4 = 2;
 constexpr uint32_t ENTRY_F8 = 0x8000, ENTRY_MASK = 0x4000, ENTRY_TILE = 0x3fff;   // visit list entries
 
-#ifndef ATT_POLY_PER_BLOCK
-#define ATT_POLY_PER_BLOCK 2                          // of the 32 exponentials of a block (MXFP4 tiles)
-#endif
-#ifndef ATT_POLY_F16
-#define ATT_POLY_F16 4                                // the same, fp16 P
-#endif
+constexpr int ATT_POLY_FP4 = 2;                       // exponentials of a 32-key block on the FMA pipe, MXFP4 tiles (ex2_poly2)
 constexpr int SPLIT_MIN_RUN = 8;                      // tiles of a run at least
 constexpr int SPLIT_GAIN = 12;                        // tiles (of 0.7 us) that dividing the keys must save on the busiest CTA
 constexpr int SPLIT_MIN_OWN = 4, SPLIT_GAIN_OWN = 7;  // the same two where every part has a CTA to itself
@@ -293,8 +288,8 @@ __device__ __forceinline__ void sub2(float& a, float& b, float c, float d, float
 
 // 2^x for a pair of values on the FMA pipe, for the share of the exponentials taken off the special-function unit:
 // x = n + f with n = round(x) (adding 1.5 * 2^23 leaves n in the low mantissa bits), 2^f on [-0.5, 0.5] by a degree-4
-// polynomial (relative error 8e-6, far below half a step of any P format), 2^n by adding n to the exponent field.
-// x is clamped at -125: anything smaller is zero in every P format.
+// polynomial (relative error 8e-6, far below half a step of MXFP4), 2^n by adding n to the exponent field.
+// x is clamped at -125: anything smaller is zero in MXFP4.
 __device__ __forceinline__ void fma2(float& a, float& b, float c, float d, float e) {   // (a, b) = (a, b) * (c, d) + (e, e)
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmov.b64 z, {%4, %4};\n\t"
       "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
@@ -396,7 +391,7 @@ __device__ __forceinline__ uint32_t softmax_block_q(const uint32_t* sc, float mr
     if (NVF4) { y[i] = __uint_as_float(sc[i]); y[i + 1] = __uint_as_float(sc[i + 1]); fma2s(y[i], y[i + 1], mul, ncb); }
     else sub2(y[i], y[i + 1], __uint_as_float(sc[i]), __uint_as_float(sc[i + 1]), ncb);
   }
-  constexpr int NPOLY = (PMODE == 3) ? ATT_POLY_PER_BLOCK : 0;
+  constexpr int NPOLY = (PMODE == 3) ? ATT_POLY_FP4 : 0;
 #pragma unroll
   for (int i = 0; i < 32 - NPOLY; ++i) y[i] = ex2(y[i]);
 #pragma unroll
@@ -422,7 +417,8 @@ __device__ __forceinline__ uint32_t softmax_block_q(const uint32_t* sc, float mr
   return (uint32_t)(sh + 127);
 }
 
-// The same for fp16 P: 16 words of fp16 pairs.
+// The same for fp16 P: 16 words of fp16 pairs.  Every exponential comes from the special-function unit: the polynomial's 8e-6
+// would reach the fp32 row sums.
 template <int NVF4>
 __device__ __forceinline__ void softmax_block_f16(const uint32_t* sc, float mref, [[maybe_unused]] float mul, uint32_t* pk,
                                                   float& lsum0, float& lsum1) {
@@ -434,9 +430,7 @@ __device__ __forceinline__ void softmax_block_f16(const uint32_t* sc, float mref
     else sub2(y[i], y[i + 1], __uint_as_float(sc[i]), __uint_as_float(sc[i + 1]), nm);
   }
 #pragma unroll
-  for (int i = 0; i < 32 - ATT_POLY_F16; ++i) y[i] = ex2(y[i]);
-#pragma unroll
-  for (int i = 32 - ATT_POLY_F16; i < 32; i += 2) ex2_poly2(y[i], y[i + 1], y[i], y[i + 1]);
+  for (int i = 0; i < 32; ++i) y[i] = ex2(y[i]);
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     add2(lsum0, lsum1, y[2 * i], y[2 * i + 1]);
