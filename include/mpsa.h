@@ -179,10 +179,10 @@ int mpsa_route_online(void* map, const void* stat, int B, int Hq, int S, int Skv
  *   fp4_kind       0: the FP4 operands of Q.K^T are MXFP4 (above).  1: NVFP4 from mpsa_quant_nvfp4_bh (q4/k4 the same
  *                  packed codes, q4_sf/k4_sf [B,H,ceil(L/128),2,512] E4M3 scale tiles); fp4_scale is then the product
  *                  of the two tensor scales, applied to the scores of the FP4 tiles.  P.V keeps the MX formats.
- *   range_flag     optional: one int32, 0 on entry, private to this call.  The forward runs with a fixed reference per row
+ *   range_flag     optional: one int32, 0 on entry, private to this call.  pv_mode 1 runs with a fixed reference per row
  *                  (see csrc/attn.cu); query tiles with a row whose maximum lies outside what that reference serves are
  *                  done again inside the same launch with the exact row maxima, and the word is then set to 1.  Results
- *                  are the same with or without it.
+ *                  are the same with or without it.  pv_mode 0 moves its references as it goes and leaves the word alone.
  *   acc_in, lse_in optional, together: an earlier partial result (fp32 [B,Hq,S,D], log2 denominators [B,Hq,S]) over OTHER keys;
  *                  out (fp32) and lse then receive the merged result (buffers distinct from the inputs), which saves
  *                  the separate mpsa_attn_merge pass

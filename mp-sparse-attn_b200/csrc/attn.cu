@@ -18,13 +18,16 @@
 //               re-quantised to the tile's format (one E8M0 scale per 32 keys) and multiplied with V quantised along
 //               the sequence.  P comes from TMEM columns of its own, so that Q.K^T of tile t + 2 never waits for P.V.
 //
-// The row reference.  Nothing in a tile depends on the running maximum, so no two threads of a row have to agree on
-// anything before the end of the item.  Quantised P.V: block-scaled P carries its magnitude in E8M0 codes, and with
-// an integral reference the element codes do not depend on it at all; m = 20 serves every row whose maximum M lies in
-// [-44, 84] (P, O and the row sums then stay within 2^-64 .. 2^64).  fp16 P.V: m is the row maximum of the item's first
-// tile, or what its scores let expect of the item where that is higher, good while M - m is in [-8, 15] (P at most 2^15;
-// fp16 keeps its relative precision down to 2^-6 of the largest P at least, and 2^-16 of it beyond).  An item with a row outside its window is
-// done again a little later, with the row maxima that the first pass found as references.
+// The row reference.  Quantised P.V: block-scaled P carries its magnitude in E8M0 codes, and with an integral reference
+// the element codes do not depend on it at all; m = 20 serves every row whose maximum M lies in [-44, 84] (P, O and the row
+// sums then stay within 2^-64 .. 2^64).  Nothing in a tile depends on the running maximum, and no two threads of a row
+// have to agree on anything before the end of the item.  An item with a row outside the window is done again a little
+// later, with the row maxima that the first pass found as references.
+// fp16 P.V: m starts as the row maximum of the item's first tile, rounded down, so that it is never above the row's maximum
+// and P keeps its 11 bits down to 2^-14 of the largest at least.  It serves scores up to m + 15 (P at most 2^15).  A
+// half tile that goes beyond raises m to its own maximum, by whole octaves, and scales O and the sums by that power of
+// two, which changes no mantissa.  The half tiles of a row decide in their order, each before it hands over its P, so P.V,
+// which takes them in the same order, finds P and O at one reference.
 //
 // Roles: warp 0 TMA loads, warp 1 Q.K^T issuer, warp 2 P.V issuer, warp 3 hands out work items, builds their visit lists
 // (the non-skipped cells of the map row) and routes, warps 4.. softmax and epilogue (a warp reaches the TMEM lane
@@ -66,19 +69,23 @@ constexpr int ATT_OFF_SFK = ATT_OFF_SFQ + 2 * 1536;                       // [KS
 constexpr int ATT_OFF_SFP = ATT_OFF_SFK + ATT_KSTAGES * 1024;             // P scale tiles [2], V scale tiles [VSLOTS_MAX]
 constexpr int ATT_OFF_XROW = ATT_OFF_SFP + (2 + ATT_VSLOTS_MAX) * 512;    // float [2][2][4][128]: row sums and row maxima of the four threads of a row
 constexpr int ATT_OFF_RMAX = ATT_OFF_XROW + 2 * 2 * 4 * 128 * 4;          // float [2 buffers][2][128]: slice maxima for the router; fp16 P.V: first-tile maxima
-constexpr int ATT_OFF_MROW = ATT_OFF_RMAX + 2 * 2 * 128 * 4;              // float [128]: row reference (fp16 P.V)
+constexpr int ATT_OFF_MROW = ATT_OFF_RMAX + 2 * 2 * 128 * 4;              // float [128]: present row reference (fp16 P.V)
 constexpr int ATT_OFF_MSLOT = ATT_OFF_MROW + 128 * 4;                     // float [MAX_SLOTS][128]: row maxima of the item that was in the slot
 constexpr int ATT_OFF_BAR = ATT_OFF_MSLOT + ATT_MAX_SLOTS * 128 * 4;
 // barriers the softmax threads use in their tile loop, by number
-constexpr int ATT_B_SFULL = 4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX;
+constexpr int ATT_B_SFULL = 32;                       // (groups of four at multiples of 32 bytes: neighbours by exclusive or)
 constexpr int ATT_B_SFREE = ATT_B_SFULL + 2, ATT_B_PREADY = ATT_B_SFULL + 4, ATT_B_PVDONE = ATT_B_SFULL + 8, ATT_B_ST = ATT_B_SFULL + 14;
-constexpr int ATT_NUM_BARS = 4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX + 4 + 8 + 2 + 2 + 12;
+constexpr int ATT_B_RBAR = ATT_B_SFULL + 28;
+constexpr int ATT_NUM_BARS = ATT_B_RBAR + 16;
+static_assert(4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX <= ATT_B_SFULL, "barrier numbers overlap");
 constexpr int ATT_BAR_BYTES = 1024;                                       // barriers, TMEM slot, router words, item slots
 static_assert(ATT_NUM_BARS * 8 + 32 + ATT_MAX_SLOTS * 36 <= ATT_BAR_BYTES, "the barrier block does not fit its share of shared memory");
-constexpr int ATT_OFF_LIST = ATT_OFF_BAR + ATT_BAR_BYTES;                 // visit lists: n_lists x list_cap uint16
+constexpr int ATT_OFF_F16 = ATT_OFF_BAR + ATT_BAR_BYTES;                  // fp16 P.V: float [2][4][128], the references of XROW's sums
+constexpr int ATT_F16_BYTES = 2 * 4 * 128 * 4;
+constexpr int ATT_OFF_LIST = ATT_OFF_BAR + ATT_BAR_BYTES;                 // visit lists: n_lists x list_cap uint16 (fp16 P.V: ATT_F16_BYTES further on)
 constexpr int ATT_MAX_KTILES = 8192;                                      // longest row of the precision map (1M keys)
 constexpr int ATT_SMEM_MAX = 232448;
-static_assert(ATT_OFF_LIST + ATT_MAX_KTILES * 2 + 1024 <= ATT_SMEM_MAX, "more shared memory than a CTA can have");
+static_assert(ATT_OFF_LIST + ATT_F16_BYTES + ATT_MAX_KTILES * 2 + 1024 <= ATT_SMEM_MAX, "more shared memory than a CTA can have");
 // TMEM columns: S0 [0,128) S1 [128,256) O [256,384), scale tiles from 384, P up to 512
 constexpr uint32_t ATT_TMEM_COLS = 512;
 constexpr uint32_t ATT_COL_S = 0, ATT_COL_O = 256;
@@ -91,13 +98,16 @@ constexpr uint32_t ATT_COL_P16 = 416;                             // fp16 P: 3 b
 constexpr int TILE_SKIP = 0, TILE_FP8 = 1, TILE_FP4 = 2;
 constexpr uint32_t ENTRY_F8 = 0x8000, ENTRY_MASK = 0x4000, ENTRY_TILE = 0x3fff;   // visit list entries
 
-constexpr int ATT_POLY_FP4 = 2;                       // exponentials of a 32-key block on the FMA pipe, MXFP4 tiles (ex2_poly2)
+constexpr int ATT_POLY_FP4 = 2;                       // exponentials of a 32-key block on the FMA pipe: MXFP4 tiles (ex2_poly2<4>)
+constexpr int ATT_POLY_F16 = 2;                       // the same, fp16 P, at full precision (ex2_poly2<5>): NVFP4 video back to back 18.5 ms with 0, 17.6 with 2, 18.3 with 4
+constexpr int ATT_F16_EARLY = 4;                      // fp16 P.V: exponentials of the second block that hide the vote on the reference
 constexpr int SPLIT_MIN_RUN = 8;                      // tiles of a run at least
 constexpr int SPLIT_GAIN = 12;                        // tiles (of 0.7 us) that dividing the keys must save on the busiest CTA
 constexpr int SPLIT_MIN_OWN = 4, SPLIT_GAIN_OWN = 7;  // the same two where every part has a CTA to itself
 constexpr float ATT_REF_Q = 20.0f;                    // quantised P.V: the row reference, and the window of row maxima it serves
 constexpr float ATT_WIN_LO_Q = -64.0f, ATT_WIN_HI_Q = 64.0f;
-constexpr float ATT_WIN_LO_F16 = -8.0f, ATT_WIN_HI_F16 = 15.0f;   // fp16 P.V: the same window (P at most 2^15; normal numbers down to 2^-6 of the largest)
+constexpr float ATT_TOP_F16 = 15.0f;                  // fp16 P.V: scores up to this far above the row reference need no new one (P at most 2^15)
+constexpr float ATT_NO_REF = -3e38f;                  // fp16 P.V: reference of a row that has seen no key yet
 
 // Division of the keys.  Items are numbered heaviest query tile first: item = r * heads + head, r counting query tiles
 // from the last.  The first n_whole are done by one CTA each; the tiles of the others, laid end to end, are cut into runs
@@ -188,6 +198,17 @@ __device__ __forceinline__ void tmem_st16p(uint32_t taddr, const uint32_t* r) {
       "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st32p(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
 __device__ __forceinline__ float ex2(float x) {
@@ -287,28 +308,40 @@ __device__ __forceinline__ void sub2(float& a, float& b, float c, float d, float
 }
 
 // 2^x for a pair of values on the FMA pipe, for the share of the exponentials taken off the special-function unit:
-// x = n + f with n = round(x) (adding 1.5 * 2^23 leaves n in the low mantissa bits), 2^f on [-0.5, 0.5] by a degree-4
-// polynomial (relative error 8e-6, far below half a step of MXFP4), 2^n by adding n to the exponent field.
-// x is clamped at -125: anything smaller is zero in MXFP4.
+// x = n + f with n = round(x) (adding 1.5 * 2^23 leaves n in the low mantissa bits), 2^f on [-0.5, 0.5] by a polynomial, 2^n by
+// adding n to the exponent field.  Degree 4: relative error 8e-6, far below half a step of MXFP4; x is clamped at -125, anything
+// smaller is zero there.  Degree 5: least largest relative error among those with value 1 at 0 (found by reweighted least
+// squares), 1.6e-7 with fp32 rounding, against the 2^-22 = 2.4e-7 that ex2.approx is specified with; zero below 2^-126 like it.
 __device__ __forceinline__ void fma2(float& a, float& b, float c, float d, float e) {   // (a, b) = (a, b) * (c, d) + (e, e)
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmov.b64 z, {%4, %4};\n\t"
       "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
       : "+f"(a), "+f"(b) : "f"(c), "f"(d), "f"(e));
 }
+template <int DEGREE>
 __device__ __forceinline__ void ex2_poly2(float& y0, float& y1, float x0, float x1) {
-  x0 = fmaxf(x0, -125.0f);
-  x1 = fmaxf(x1, -125.0f);
+  x0 = fmaxf(x0, DEGREE == 4 ? -125.0f : -200.0f);
+  x1 = fmaxf(x1, DEGREE == 4 ? -125.0f : -200.0f);
   float t0, t1, n0, n1;
   sub2(t0, t1, x0, x1, 12582912.0f);              // t = x + 1.5 * 2^23
   sub2(n0, n1, t0, t1, -12582912.0f);             // n = round(x), as a float
   float f0 = x0 - n0, f1 = x1 - n1;
-  float p0 = 0.009278289f, p1 = 0.009278289f;
-  fma2(p0, p1, f0, f1, 0.055865023f);
-  fma2(p0, p1, f0, f1, 0.240308955f);
-  fma2(p0, p1, f0, f1, 0.693129539f);
-  fma2(p0, p1, f0, f1, 0.999997854f);
-  y0 = __int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23));
-  y1 = __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23));
+  float p0 = DEGREE == 4 ? 0.009278289f : 0.00132647285f, p1 = p0;
+  if (DEGREE == 4) {
+    fma2(p0, p1, f0, f1, 0.055865023f);
+    fma2(p0, p1, f0, f1, 0.240308955f);
+    fma2(p0, p1, f0, f1, 0.693129539f);
+    fma2(p0, p1, f0, f1, 0.999997854f);
+  } else {
+    fma2(p0, p1, f0, f1, 0.00967151299f);
+    fma2(p0, p1, f0, f1, 0.0555073358f);
+    fma2(p0, p1, f0, f1, 0.240222454f);
+    fma2(p0, p1, f0, f1, 0.693147004f);
+    fma2(p0, p1, f0, f1, 1.0f);
+  }
+  int i0 = __float_as_int(p0) + (__float_as_int(t0) << 23), i1 = __float_as_int(p1) + (__float_as_int(t1) << 23);
+  if (DEGREE != 4) { i0 = max(i0, 0); i1 = max(i1, 0); }      // an exponent below the smallest: the sign bit is set
+  y0 = __int_as_float(i0);
+  y1 = __int_as_float(i1);
 }
 
 // Bounded wait for a tagged word in shared memory: returns the word once its tag (bits 1..) equals `tag`, or -1 after
@@ -331,6 +364,9 @@ __device__ __forceinline__ int poll_tag(volatile int* word, int tag, int* status
   if (__builtin_expect((w >> 1) == tag, 1)) return w;
   return poll_slow(word, tag, status);
 }
+
+// 2^d for an integral d <= 127; 0 below 2^-126
+__device__ __forceinline__ float pow2i(float d) { return __int_as_float(((int)fmaxf(d, -127.0f) + 127) << 23); }
 
 // floor(d) - emax as an integer and as a float, without conversion instructions (which share the exponential's
 // pipe): d + 1.5 * 2^23 rounded DOWN holds floor(d) in its low mantissa bits (|d| < 2^22).
@@ -395,7 +431,7 @@ __device__ __forceinline__ uint32_t softmax_block_q(const uint32_t* sc, float mr
 #pragma unroll
   for (int i = 0; i < 32 - NPOLY; ++i) y[i] = ex2(y[i]);
 #pragma unroll
-  for (int i = 32 - NPOLY; i < 32; i += 2) ex2_poly2(y[i], y[i + 1], y[i], y[i + 1]);
+  for (int i = 32 - NPOLY; i < 32; i += 2) ex2_poly2<4>(y[i], y[i + 1], y[i], y[i + 1]);
   float a0 = 0.0f, a1 = 0.0f, b0 = 0.0f, b1 = 0.0f;
 #pragma unroll
   for (int i = 0; i < 32; i += 4) {
@@ -417,25 +453,62 @@ __device__ __forceinline__ uint32_t softmax_block_q(const uint32_t* sc, float mr
   return (uint32_t)(sh + 127);
 }
 
-// The same for fp16 P: 16 words of fp16 pairs.  Every exponential comes from the special-function unit: the polynomial's 8e-6
-// would reach the fp32 row sums.
-template <int NVF4>
-__device__ __forceinline__ void softmax_block_f16(const uint32_t* sc, float mref, [[maybe_unused]] float mul, uint32_t* pk,
-                                                  float& lsum0, float& lsum1) {
-  const float nm = -mref;
-  float y[32];
+// The same for fp16 P, in two steps: y = exp2(S - m) in place for the elements FROM .. TO - 1 of a block, then 16 words of fp16
+// pairs and the sums.
+template <int NVF4, int FROM, int TO>
+__device__ __forceinline__ void exp_block_f16(uint32_t* sc, float mref, [[maybe_unused]] float mul) {
+  float* y = reinterpret_cast<float*>(sc);
 #pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    if (NVF4) { y[i] = __uint_as_float(sc[i]); y[i + 1] = __uint_as_float(sc[i + 1]); fma2s(y[i], y[i + 1], mul, nm); }
-    else sub2(y[i], y[i + 1], __uint_as_float(sc[i]), __uint_as_float(sc[i + 1]), nm);
+  for (int i = FROM; i < TO; i += 2) {
+    if (NVF4) fma2s(y[i], y[i + 1], mul, -mref);
+    else sub2(y[i], y[i + 1], y[i], y[i + 1], -mref);
   }
 #pragma unroll
-  for (int i = 0; i < 32; ++i) y[i] = ex2(y[i]);
+  for (int i = FROM; i < TO; i += 2) {
+    if (i < 32 - ATT_POLY_F16) { y[i] = ex2(y[i]); y[i + 1] = ex2(y[i + 1]); }
+    else ex2_poly2<5>(y[i], y[i + 1], y[i], y[i + 1]);
+  }
+}
+__device__ __forceinline__ void pack_block_f16(const uint32_t* sc, uint32_t* pk, float& lsum0, float& lsum1) {
+  const float* y = reinterpret_cast<const float*>(sc);
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     add2(lsum0, lsum1, y[2 * i], y[2 * i + 1]);
     pk[i] = pack_f16x2(y[2 * i], y[2 * i + 1]);
   }
+}
+
+// A warp's 32 lanes of n fp32 columns of TMEM, each lane times its own factor.  Rare, and out of the way of the loop that needs it.
+static __device__ __noinline__ void scale_f32_columns(uint32_t taddr, int n, float f) {
+  uint32_t r[32];
+  tc_fence_after();
+  _Pragma("unroll 1") for (int c = 0; c < n; c += 32) {
+    tmem_ld32p(taddr + c, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * f);
+    tmem_st32p(taddr + c, r);
+  }
+  tmem_st_wait();
+}
+
+// The same for columns of fp16 pairs, 32 of them.
+static __device__ __noinline__ void scale_f16_columns(uint32_t taddr, float f) {
+  uint32_t r[32];
+  tmem_ld32p(taddr, r);
+  tmem_ld_wait();
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&r[k]));
+    r[k] = pack_f16x2(v.x * f, v.y * f);
+  }
+  tmem_st32p(taddr, r);
+  tmem_st_wait();
+}
+
+// x = *word (shared memory) if `ready`; ordered behind what `ready` was found out with, which a load beside it would not be.
+__device__ __forceinline__ void load_if(float& x, uint32_t word, bool ready) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.f32 %0, [%1];\n\t}" : "+f"(x) : "r"(word), "r"((uint32_t)ready) : "memory");
 }
 
 // One slot of the visit-list ring: a work item and its tiles.
@@ -470,7 +543,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   uint64_t* k_empty = k_full + ATT_KSTAGES;        // [KSTAGES]
   uint64_t* v_full = k_empty + ATT_KSTAGES;        // [VSLOTS_MAX]
   uint64_t* v_empty = v_full + ATT_VSLOTS_MAX;     // [VSLOTS_MAX]
-  uint64_t* s_full = v_empty + ATT_VSLOTS_MAX;     // [2]
+  uint64_t* s_full = bars + ATT_B_SFULL;           // [2]
   uint64_t* s_free = s_full + 2;                   // [2] every owner has read the S buffer
   uint64_t* p_ready = s_free + 2;                  // [4] quantised P: tile t & 1; fp16 P: (tile t & 1, 64-key half)
   uint64_t* pv_done = p_ready + 4;                 // [4] likewise
@@ -480,10 +553,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   uint64_t* x_bar = st_bar + 2;                    // [4] fp16 P.V: first-tile maxima of the two halves of a row
   uint64_t* m_bar = x_bar + 4;                     // [4] fp16 P.V: row references for the other warpgroup
   uint64_t* l_bar = m_bar + 4;                     // [4] partial sums and maxima of a row quarter
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(l_bar + 4);
+  uint64_t* r_bar = l_bar + 4;                     // [4 row quarters][tile & 1][half] fp16 P.V: this half tile has decided on the reference
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(r_bar + 16);
   volatile int* dec = reinterpret_cast<volatile int*>(tmem_slot + 4);   // [4], slot tile & 3: (tile << 1 | keep) once the router has decided on the tile
   volatile Slot* slots = reinterpret_cast<volatile Slot*>(tmem_slot + 8);   // [MAX_SLOTS]
-  uint16_t* lists = reinterpret_cast<uint16_t*>(smem + ATT_OFF_LIST);
+  uint16_t* lists = reinterpret_cast<uint16_t*>(smem + ATT_OFF_LIST + (PVQ ? 0 : ATT_F16_BYTES));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = (p.S + ATT_BM - 1) / ATT_BM, nk = (p.Skv + ATT_BN - 1) / ATT_BN;
@@ -506,6 +580,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     mbar_init(o_full, 1);
     mbar_init(o_free, 512);
     for (int s = 0; s < 4; ++s) { mbar_init(&x_bar[s], 2); mbar_init(&m_bar[s], 1); mbar_init(&l_bar[s], 4); }
+    for (int s = 0; s < 16; ++s) mbar_init(&r_bar[s], 1);
     fence_mbar_init();
     for (int s = 0; s < 4; ++s) dec[s] = -1;        // no tile decided yet
   }
@@ -1038,12 +1113,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     constexpr bool DEFER = PVQ != 0;
     bool ok = true;
     int t0 = 0;                                     // tiles of the items before this one
-    int n_ref = 0;                                  // fp16 P.V: first-tile exchanges so far
     int pb16 = (2 * wg + g) % 3;                    // fp16 P.V: P buffer of the next tile's half
     const uint32_t a_wg = smem_u32(bars) + wg * 8;  // shared address of barrier 0 of this warpgroup's pairs
-    const uint32_t a_pr16 = smem_u32(&p_ready[wg * 2 + g]), a_pv16 = smem_u32(&pv_done[g == 0 ? wg * 2 + 1 : (wg ^ 1) * 2]);
-    const uint32_t pv16_flip = (g == 1 && wg == 1) ? 0 : 1;
-    uint32_t kp = 0;                                // parity of this warpgroup's tile count
+    // fp16 P.V.  The four warps of a row quarter are numbered 2 wg + g, in the order of their half tiles.  r_bar of the warp before
+    // this one - the same tile's first half, or the second one of the other warpgroup's tile - is its turn to decide on the row
+    // reference.
+    const uint32_t a_pr16 = smem_u32(&p_ready[wg * 2 + g]), a_pv16 = smem_u32(&pv_done[(wg * 2 + g + 1) & 3]);
+    const uint32_t a_turn = (a_pv16 ^ 16) + (ATT_B_RBAR - ATT_B_PVDONE) * 8 + (r_in & 96), a_decided = a_pr16 + (ATT_B_RBAR - ATT_B_PREADY) * 8 + (r_in & 96);
+    // phase parities to wait for, as bits: 1 this warpgroup's tile count; fp16 P.V: 2 P.V of the half tile three before, 4 the half
+    // tile before (turn and P.V)
+    uint32_t par = PVQ ? 0 : ((g == 1 && wg == 1) ? 0u : 2u) | ((g == 0 && wg == 0) ? 4u : 0u);
+    float* lref = reinterpret_cast<float*>(smem + ATT_OFF_F16);
     float* rmax_w = rmax + (wg * 2 + g) * 128 + r_in;
     float m_redo = 0.0f;                            // row reference of an item that is done again: the maximum its first pass found
     float mref = 0.0f, l_run = 0.0f, m_run = -INFINITY;   // row reference; partial row sum and maximum over this thread's keys
@@ -1054,6 +1134,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     bool in_item = false, second = false, routing = false;   // second: ROUTE, the appended tiles
     bool epi = false;                               // an epilogue is outstanding: item seq - 1, in slot epi_ls
     int epi_ls = 0, epi_part = 0;
+    auto last_key = [&]() { return p.causal ? min(p.Skv - 1, slots[ls].qi * ATT_BM + r_in + off) : p.Skv - 1; };
     auto settle = [&]() {
       if (ROUTE && pend_t >= 0) {
         const int d = poll_tag(&dec[pend_t & 3], pend_t, p.status);
@@ -1078,7 +1159,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           const int last = lim - ((int)(ec & ENTRY_TILE) * ATT_BN + g * 64);   // last visible key of the slice
           float lsum0 = 0.0f, lsum1 = 0.0f;
           uint32_t sc[32];
-          ok &= mbar_wait_at(a_wg + ATT_B_SFULL * 8, kp, p.status, KS_TIMEOUT_MMA);
+          ok &= mbar_wait_at(a_wg + ATT_B_SFULL * 8, par & 1, p.status, KS_TIMEOUT_MMA);
           __syncwarp();
           tc_fence_after();
           tmem_ld32p(slice_addr, sc);
@@ -1108,7 +1189,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               }
               psc |= softmax_block_q<PM, NV>(sc, mref, b1, nvmul, pk + PW, lsum0, lsum1) << 8;
               // the P buffer and its scale tile: P.V of tile t - 2 has read them (a fresh barrier satisfies the first wait)
-              ok &= mbar_wait_at(a_wg + ATT_B_PVDONE * 8, kp ^ 1, p.status, KS_TIMEOUT_MMA);
+              ok &= mbar_wait_at(a_wg + ATT_B_PVDONE * 8, (par & 1) ^ 1, p.status, KS_TIMEOUT_MMA);
               __syncwarp();
               tc_fence_after();
               if (PM == 3) tmem_st8p(p_addr + g * 8, pk);
@@ -1123,27 +1204,78 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           } else {
             uint32_t pk[32];
             const float mul = (NVF4 && !(ec & ENTRY_F8)) ? nvmul : 1.0f;
-            tmem_ld_wait();
-            if (ec & ENTRY_MASK) mask32(sc, last);
-            const float b0 = block_max32(sc);
-            softmax_block_f16<NVF4>(sc, mref, mul, pk, lsum0, lsum1);
-            tmem_ld32p(slice_addr + 32, sc);
-            tmem_ld_wait();
+            bool dead = false;
+            _Pragma("unroll 1") while (true) {
+              tmem_ld_wait();
+              if (ec & ENTRY_MASK) mask32(sc, last);
+              m_run = fmaxf(m_run, block_max32(sc) * mul);
+              exp_block_f16<NVF4, 0, 32>(sc, mref, mul);
+              pack_block_f16(sc, pk, lsum0, lsum1);
+              tmem_ld32p(slice_addr + 32, sc);
+              tmem_ld_wait();
+              if (ec & ENTRY_MASK) mask32(sc, last - 32);
+              m_run = fmaxf(m_run, block_max32(sc) * mul);      // (no earlier score goes beyond: it would have raised the reference)
+              const bool stays = __all_sync(0xffffffffu, ok && !(m_run - mref > ATT_TOP_F16));
+              exp_block_f16<NVF4, 0, ATT_F16_EARLY>(sc, mref, mul);    // (under the vote)
+              if (__builtin_expect(stays, 1)) break;
+              if (!__all_sync(0xffffffffu, ok)) { dead = true; break; }
+              // A row goes beyond its reference: this half raises it in its turn, once the half before it has decided, and hands
+              // the turn on where every half does.
+              ok &= mbar_wait_at(a_turn, (par >> 2) & 1, p.status, KS_TIMEOUT_PIPE);
+              __syncwarp();
+              const float mc = mrow[r_in], m_new = m_run - mc > ATT_TOP_F16 ? floorf(m_run) : mc;
+              if (__any_sync(0xffffffffu, m_new != mc)) {
+                // O is at mc: it is scaled once P.V of the half before this one is done.  (That of the half two before it comes first:
+                // the wait for a phase has to know that the one before is over.)
+                ok &= mbar_wait_at(a_pv16, (par >> 1) & 1, p.status, KS_TIMEOUT_MMA);
+                ok &= mbar_wait_at(a_pv16 ^ 16, (par >> 2) & 1, p.status, KS_TIMEOUT_MMA);
+                __syncwarp();
+                scale_f32_columns(lane_base + ATT_COL_O, p.D, pow2i(mc - m_new));
+                mrow[r_in] = m_new;
+                __syncwarp();
+              }
+              l_run *= pow2i(mref - m_new);
+              mref = m_new;
+              lsum0 = lsum1 = 0.0f;
+              tmem_ld32p(slice_addr, sc);           // the tile again
+            }
+            if (dead) { ok = false; break; }
             tc_fence_before();
             mbar_arrive_at(a_wg + ATT_B_SFREE * 8);
-            if (ec & ENTRY_MASK) mask32(sc, last - 32);
-            m_run = fmaxf(m_run, fmaxf(b0, block_max32(sc)) * mul);
-            softmax_block_f16<NVF4>(sc, mref, mul, pk + 16, lsum0, lsum1);
-            // P buffer of this half, number h = 2t + g over all items: h mod 3.  P.V of half h - 3 has read it: the other
-            // half of this warpgroup's previous tile (g = 0), or the first half of the other warpgroup's (g = 1).
-            ok &= mbar_wait_at(a_pv16, kp ^ pv16_flip, p.status, KS_TIMEOUT_MMA);
-            __syncwarp();
+            exp_block_f16<NVF4, ATT_F16_EARLY, 32>(sc, mref, mul);
+            // What has to be there before P is stored, asked for in one vote: this half's turn (the half before it has decided), the
+            // reference as it was, and the P buffer of this half, number h = 2t + g over all items: h mod 3.  P.V of half h - 3 has
+            // read it: the other half of this warpgroup's previous tile (g = 0), or the first half of the other warpgroup's (g = 1).
+            const bool turn = mbar_try_wait(a_turn, (par >> 2) & 1);
+            float m_now = __int_as_float(0x7fffffff);
+            const bool room = mbar_try_wait(a_pv16, (par >> 1) & 1);
+            pack_block_f16(sc, pk + 16, lsum0, lsum1);
+            load_if(m_now, smem_u32(mrow + r_in), turn);
+            bool moved = false;
+            if (!__all_sync(0xffffffffu, turn && room && m_now == mref)) {
+              ok &= mbar_wait_at(a_turn, (par >> 2) & 1, p.status, KS_TIMEOUT_PIPE);
+              __syncwarp();
+              m_now = mrow[r_in];
+              moved = __any_sync(0xffffffffu, m_now != mref);
+              ok &= mbar_wait_at(a_pv16, (par >> 1) & 1, p.status, KS_TIMEOUT_MMA);
+              __syncwarp();
+            }
+            mbar_arrive_lane0(a_decided, lane);
             tc_fence_after();
             tmem_st16p(p_addr + pb16 * 32, pk);
             tmem_st16p(p_addr + pb16 * 32 + 16, pk + 16);
+            if (__builtin_expect(moved, 0)) {       // a half before this one has raised the reference meanwhile
+              const float f = pow2i(mref - m_now);
+              tmem_st_wait();
+              scale_f16_columns(p_addr + pb16 * 32, f);
+              l_run *= f;
+              lsum0 *= f;
+              lsum1 *= f;
+              mref = m_now;
+            }
             pb16 = pb16 == 2 ? 0 : pb16 + 1;        // four halves further on
           }
-          kp ^= 1;
+          par ^= PVQ ? 1 : 7;
           tmem_st_wait();
           tc_fence_before();
           mbar_arrive_at(PVQ ? a_wg + ATT_B_PREADY * 8 : a_pr16);
@@ -1153,8 +1285,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           } else {
             l_run += lsum0 + lsum1;
           }
-          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          if (PVQ && !__all_sync(0xffffffffu, ok)) { ok = false; break; }
         } while (more);
+        if (PVQ == 0) ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         do_epi = DEFER && epi;
       } else if (in_item) {
@@ -1171,7 +1304,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           epi_part = (((t0 & 1) ^ wg) << 1) | g;    // the same order of summation whichever warpgroup owned the first tile
           float* xl = xrow + (seq & 1) * 1024 + epi_part * 128 + r_in;
           xl[0] = l_run;
-          xl[512] = m_run;
+          if (PVQ) {
+            xl[512] = m_run;
+          } else {
+            // what rounding to fp16 makes of this thread's largest P
+            const float p_max = ex2(m_run - mref);
+            xl[512] = __half2float(__float2half_rn(p_max)) - p_max;
+            lref[(seq & 1) * 512 + epi_part * 128 + r_in] = mref;
+          }
           __syncwarp();
           if (lane == 0) mbar_arrive(&l_bar[q]);
           t0 += n_tiles;
@@ -1191,7 +1331,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           ok = __all_sync(0xffffffffu, mbar_wait(&list_full[ls], l_par, p.status, KS_TIMEOUT_PIPE));
           if (!ok) break;
           mode = slots[ls].mode;
-          do_epi = epi && mode == 1;                // m_redo may still be in use
+          do_epi = PVQ && epi && mode == 1;         // m_redo may still be in use
         }
         if (do_epi) {
         } else if (mode < 0) {
@@ -1202,21 +1342,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           routing = ROUTE && mode == 0;
           n_tiles = slots[ls].n_own;
           const int m_glob = slots[ls].qi * ATT_BM + r_in;
-          lim = p.causal ? min(p.Skv - 1, m_glob + off) : (p.Skv - 1);   // last visible key of this row
+          lim = last_key();                         // last visible key of this row
           l_run = 0.0f;
           m_run = -INFINITY;
-          if (mode == 1) m_redo = mslot[slots[ls].from * 128 + r_in];
-          mref = mode == 1 ? m_redo : (PVQ ? ATT_REF_Q : 0.0f);
+          if (PVQ && mode == 1) m_redo = mslot[slots[ls].from * 128 + r_in];
+          mref = PVQ ? (mode == 1 ? m_redo : ATT_REF_Q) : ATT_NO_REF;
           i = (t0 & 1) ^ wg;                        // first tile of the list this warpgroup owns
-          if (PVQ == 0 && mode == 0 && n_tiles > 0) {
-            // the row's reference: the maximum of the item's first tile, found by its owners
+          if (PVQ == 0 && n_tiles == 0 && i == 0 && lane == 0) {   // no exchange, but the barriers' phases follow the items
+            mbar_arrive(&x_bar[q]);
+            if (g == 0) mbar_arrive(&m_bar[q]);
+          }
+          if (PVQ == 0 && n_tiles > 0) {
+            // the row's first reference: the maximum of the item's first tile, found by its owners.  (Every thread of the row is
+            // through with the item before: its epilogue has waited for all of them.)
             if (i == 0) {
-              ok = __all_sync(0xffffffffu, mbar_wait(&s_full[wg], kp, p.status, KS_TIMEOUT_MMA));
+              ok = __all_sync(0xffffffffu, mbar_wait(&s_full[wg], par & 1, p.status, KS_TIMEOUT_MMA));
               if (!ok) break;
               tc_fence_after();
               const uint32_t e = lists[ls * p.list_cap];
-              const int last = lim - ((int)(e & ENTRY_TILE) * ATT_BN + g * 64);
-              float mx = -INFINITY, s0 = 0.0f, s1 = 0.0f, q0 = 0.0f, q1 = 0.0f;
+              const int last = last_key() - ((int)(e & ENTRY_TILE) * ATT_BN + g * 64);
+              float mx = -INFINITY;
 #pragma unroll
               for (int c = 0; c < 2; ++c) {
                 uint32_t sc[32];
@@ -1224,41 +1369,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
                 tmem_ld_wait();
                 if (e & ENTRY_MASK) mask32(sc, last - c * 32);
                 mx = fmaxf(mx, block_max32(sc));
-#pragma unroll
-                for (int k = 0; k < 32; k += 2) {
-                  const float a = __uint_as_float(sc[k]), c2 = __uint_as_float(sc[k + 1]);
-                  add2(s0, s1, a, c2);
-                  q0 = fmaf(a, a, q0);
-                  q1 = fmaf(c2, c2, q1);
-                }
               }
-              if (NVF4 && !(e & ENTRY_F8)) { mx *= nvmul; s0 *= nvmul; s1 *= nvmul; q0 *= nvmul * nvmul; q1 *= nvmul * nvmul; }
               rmax[g * 128 + r_in] = mx;
-              // expected maximum of the item's scores, from this thread's 64: mean + z(n) sigma, z(n) = 2.59 + .2 log2(n / 128) that
-              // of n normal variables
-              const float mean = (s0 + s1) * (1.0f / 64.0f), var = fmaxf((q0 + q1) * (1.0f / 64.0f) - mean * mean, 0.0f);
-              rmax[(2 + g) * 128 + r_in] = (e & ENTRY_MASK) ? -INFINITY : mean + sqrtf(var) * (2.59f + 0.2f * __log2f((float)n_tiles));
               __syncwarp();
               if (lane == 0) mbar_arrive(&x_bar[q]);
-              ok = __all_sync(0xffffffffu, mbar_wait(&x_bar[q], n_ref & 1, p.status, KS_TIMEOUT_PIPE));
+              ok = __all_sync(0xffffffffu, mbar_wait(&x_bar[q], seq & 1, p.status, KS_TIMEOUT_PIPE));
               if (!ok) break;
-              mref = fmaxf(rmax[r_in], rmax[128 + r_in]);
-              if (mref == -INFINITY) mref = 0.0f;
-              // The reference follows the expected maximum where that is higher: with outlier channels in the keys most items
-              // of 32768 keys left the window above the first tile's maximum (16.4 ms, against 7.1 now).
-              // (By whole octaves, which leave P's mantissas and so its rounding as they are.)
-              mref += floorf(fmaxf(0.5f * (rmax[256 + r_in] + rmax[384 + r_in]) + 1.0f - mref, 0.0f));
+              mref = floorf(fmaxf(rmax[r_in], rmax[128 + r_in]) * (NVF4 && !(e & ENTRY_F8) ? nvmul : 1.0f));
+              if (!(mref > ATT_NO_REF)) mref = ATT_NO_REF;   // no visible key, or only NaN
+              // rows of the ragged tail hold no data, and their scales belong to none: they never ask for another reference
+              if (m_glob >= p.S) mref = -ATT_NO_REF;
               if (g == 0) {
                 mrow[r_in] = mref;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&m_bar[q]);
               }
             } else {
-              ok = __all_sync(0xffffffffu, mbar_wait(&m_bar[q], n_ref & 1, p.status, KS_TIMEOUT_PIPE));
+              ok = __all_sync(0xffffffffu, mbar_wait(&m_bar[q], seq & 1, p.status, KS_TIMEOUT_PIPE));
               if (!ok) break;
               mref = mrow[r_in];
             }
-            ++n_ref;
           }
         }
       }
@@ -1270,8 +1400,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(o_full, seq_e & 1, p.status, KS_TIMEOUT_MMA));
         if (!ok) break;
         tc_fence_after();
-        const float l_tot = ((xl[0] + xl[128]) + xl[256]) + xl[384];
-        const float m_tot = fmaxf(fmaxf(xl[512], xl[640]), fmaxf(xl[768], xl[896]));
+        float l_tot = ((xl[0] + xl[128]) + xl[256]) + xl[384];      // sum of the row
+        float m_tot = 0.0f, ref_last = 0.0f, l_div = l_tot;         // quantised P.V: its maximum; fp16 P.V: the reference that O is at; what O is divided by
+        if (PVQ) {
+          m_tot = fmaxf(fmaxf(xl[512], xl[640]), fmaxf(xl[768], xl[896]));
+        } else {
+          // O is divided by a sum that has the largest P of each thread as fp16 has it: where one P carries the row, its rounding
+          // cancels.  (The log2 denominator is that of the unrounded sum.)
+          const float* rl = lref + (seq_e & 1) * 512 + r_in;
+          l_div += ((xl[512] + xl[640]) + xl[768]) + xl[896];
+          ref_last = fmaxf(fmaxf(rl[0], rl[128]), fmaxf(rl[256], rl[384]));
+          const float ref_first = fminf(fminf(rl[0], rl[128]), fminf(rl[256], rl[384]));
+          if (__builtin_expect(__any_sync(0xffffffffu, ref_first != ref_last), 0)) {     // some sums are at an earlier reference
+            l_tot = l_div = 0.0f;
+            _Pragma("unroll 1") for (int k = 0; k < 512; k += 128) {
+              const float f = pow2i(rl[k] - ref_last);
+              l_tot += xl[k] * f;
+              l_div += xl[512 + k] * f;
+            }
+            l_div += l_tot;
+          }
+        }
         const int mode = slots[epi_ls].mode;
         const bool tiles = (ROUTE ? slots[epi_ls].n_total : slots[epi_ls].n_own) > 0;
         const int m_glob = slots[epi_ls].qi * ATT_BM + r_in;
@@ -1280,7 +1429,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         // a share of an item: fp32 and the log2 denominator, into its slice of the partial results
         const int part = SPLIT ? slots[epi_ls].part : -1;
         const int item = (nq - 1 - slots[epi_ls].qi) * p.Hq * p.B + head;
-        const float ref = PVQ ? (mode == 1 ? m_redo : ATT_REF_Q) : mref;
+        const float ref = PVQ ? (mode == 1 ? m_redo : ATT_REF_Q) : ref_last;
         const bool has_o = epi_part * 32 < p.D;     // this thread's 32 columns of O
         uint32_t o[32];
         if (tiles) {
@@ -1292,21 +1441,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         }
         tc_fence_before();
         mbar_arrive(o_free);
-        if (mode == 0) {
+        if (PVQ && mode == 0) {
           const float over = m_tot - ref;           // rows of the ragged tail hold no data
-          const bool out_of_window = m_glob < p.S && m_tot != -INFINITY &&
-                                     (PVQ ? (over < ATT_WIN_LO_Q || over > ATT_WIN_HI_Q) : (over < ATT_WIN_LO_F16 || over > ATT_WIN_HI_F16));
-          if (out_of_window) {
+          if (m_glob < p.S && m_tot != -INFINITY && (over < ATT_WIN_LO_Q || over > ATT_WIN_HI_Q)) {
             slots[epi_ls].redo = 1;
             if (p.range_flag) *p.range_flag = 1;
           }
-          if (epi_part == 0) mslot[epi_ls * 128 + r_in] = m_tot == -INFINITY ? 0.0f : (PVQ ? ceilf(m_tot) : m_tot);
+          if (epi_part == 0) mslot[epi_ls * 128 + r_in] = m_tot == -INFINITY ? 0.0f : ceilf(m_tot);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&list_empty[epi_ls]);
         epi = false;
         if (m_glob < p.S) {
-          float inv_l = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
+          float inv_l = l_tot > 0.0f ? 1.0f / l_div : 0.0f;
           float lse_row = 0.0f, w_prev = 0.0f;      // w_prev: weight of the earlier partial result (merge mode)
           if (p.lse || part >= 0) lse_row = l_tot > 0.0f ? ref + log2f(l_tot) : -INFINITY;
           if (p.acc_in) {
@@ -1695,8 +1842,9 @@ int attn_forward(const AttnCall& call, cudaStream_t st) {
   p.n_items = (int)n_items; p.group = c.Hq / c.Hkv; p.counter = c.counter;
   p.out32 = (uintptr_t)c.out % 32 == 0; p.load8 = c.need8; p.load4 = c.need4;
   p.list_cap = ((c.route ? 2 * nk : nk) + 7) & ~7;
-  p.n_lists = std::min(ATT_MAX_SLOTS, (ATT_SMEM_MAX - 1024 - ATT_OFF_LIST) / (p.list_cap * 2));
-  const size_t smem = ATT_OFF_LIST + (size_t)p.n_lists * p.list_cap * 2 + 1024;
+  const int off_list = ATT_OFF_LIST + (c.pv_mode == 0 ? ATT_F16_BYTES : 0);
+  p.n_lists = std::min(ATT_MAX_SLOTS, (ATT_SMEM_MAX - 1024 - off_list) / (p.list_cap * 2));
+  const size_t smem = off_list + (size_t)p.n_lists * p.list_cap * 2 + 1024;
   int parts = 0, n_whole = p.n_items, run_tiles = 1, pad = 0;
   if (c.partial) parts = split_choose(c, nq, nk, n_whole, run_tiles, pad);
   const long long n_shared = p.n_items - n_whole;
