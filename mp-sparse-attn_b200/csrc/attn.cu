@@ -23,11 +23,11 @@
 // sums then stay within 2^-64 .. 2^64).  Nothing in a tile depends on the running maximum, and no two threads of a row
 // have to agree on anything before the end of the item.  An item with a row outside the window is done again a little
 // later, with the row maxima that the first pass found as references.
-// fp16 P.V: m starts as the row maximum of the item's first tile, rounded down, so that it is never above the row's maximum
-// and P keeps its 11 bits down to 2^-14 of the largest at least.  It serves scores up to m + 15 (P at most 2^15).  A
-// half tile that goes beyond raises m to its own maximum, by whole octaves, and scales O and the sums by that power of
-// two, which changes no mantissa.  The half tiles of a row decide in their order, each before it hands over its P, so P.V,
-// which takes them in the same order, finds P and O at one reference.
+// fp16 P.V: m starts as the row maximum of the item's first tile, so that it is never above the row's maximum and P keeps
+// its 11 bits down to 2^-14 of the largest at least.  It serves scores up to m + 15 (P at most 2^15).  A half tile that goes
+// beyond raises m to its own maximum and scales O and the sums, all of it 2^-15 or less from then on.  The half tiles of a row
+// decide in their order, each before it hands over its P, so P.V, which takes them in the same order, finds P and O at one
+// reference.  (With references rounded down to whole octaves no largest P was exactly 1: 5 % more error with N(0,1) keys.)
 //
 // Roles: warp 0 TMA loads, warp 1 Q.K^T issuer, warp 2 P.V issuer, warp 3 hands out work items, builds their visit lists
 // (the non-skipped cells of the map row) and routes, warps 4.. softmax and epilogue (a warp reaches the TMEM lane
@@ -364,9 +364,6 @@ __device__ __forceinline__ int poll_tag(volatile int* word, int tag, int* status
   if (__builtin_expect((w >> 1) == tag, 1)) return w;
   return poll_slow(word, tag, status);
 }
-
-// 2^d for an integral d <= 127; 0 below 2^-126
-__device__ __forceinline__ float pow2i(float d) { return __int_as_float(((int)fmaxf(d, -127.0f) + 127) << 23); }
 
 // floor(d) - emax as an integer and as a float, without conversion instructions (which share the exponential's
 // pipe): d + 1.5 * 2^23 rounded DOWN holds floor(d) in its low mantissa bits (|d| < 2^22).
@@ -1223,18 +1220,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               // the turn on where every half does.
               ok &= mbar_wait_at(a_turn, (par >> 2) & 1, p.status, KS_TIMEOUT_PIPE);
               __syncwarp();
-              const float mc = mrow[r_in], m_new = m_run - mc > ATT_TOP_F16 ? floorf(m_run) : mc;
+              const float mc = mrow[r_in], m_new = m_run - mc > ATT_TOP_F16 ? m_run : mc;
               if (__any_sync(0xffffffffu, m_new != mc)) {
                 // O is at mc: it is scaled once P.V of the half before this one is done.  (That of the half two before it comes first:
                 // the wait for a phase has to know that the one before is over.)
                 ok &= mbar_wait_at(a_pv16, (par >> 1) & 1, p.status, KS_TIMEOUT_MMA);
                 ok &= mbar_wait_at(a_pv16 ^ 16, (par >> 2) & 1, p.status, KS_TIMEOUT_MMA);
                 __syncwarp();
-                scale_f32_columns(lane_base + ATT_COL_O, p.D, pow2i(mc - m_new));
+                scale_f32_columns(lane_base + ATT_COL_O, p.D, ex2(mc - m_new));
                 mrow[r_in] = m_new;
                 __syncwarp();
               }
-              l_run *= pow2i(mref - m_new);
+              l_run *= ex2(mref - m_new);
               mref = m_new;
               lsum0 = lsum1 = 0.0f;
               tmem_ld32p(slice_addr, sc);           // the tile again
@@ -1265,7 +1262,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
             tmem_st16p(p_addr + pb16 * 32, pk);
             tmem_st16p(p_addr + pb16 * 32 + 16, pk + 16);
             if (__builtin_expect(moved, 0)) {       // a half before this one has raised the reference meanwhile
-              const float f = pow2i(mref - m_now);
+              const float f = ex2(mref - m_now);
               tmem_st_wait();
               scale_f16_columns(p_addr + pb16 * 32, f);
               l_run *= f;
@@ -1375,7 +1372,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               if (lane == 0) mbar_arrive(&x_bar[q]);
               ok = __all_sync(0xffffffffu, mbar_wait(&x_bar[q], seq & 1, p.status, KS_TIMEOUT_PIPE));
               if (!ok) break;
-              mref = floorf(fmaxf(rmax[r_in], rmax[128 + r_in]) * (NVF4 && !(e & ENTRY_F8) ? nvmul : 1.0f));
+              mref = fmaxf(rmax[r_in], rmax[128 + r_in]) * (NVF4 && !(e & ENTRY_F8) ? nvmul : 1.0f);
               if (!(mref > ATT_NO_REF)) mref = ATT_NO_REF;   // no visible key, or only NaN
               // rows of the ragged tail hold no data, and their scales belong to none: they never ask for another reference
               if (m_glob >= p.S) mref = -ATT_NO_REF;
@@ -1414,7 +1411,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           if (__builtin_expect(__any_sync(0xffffffffu, ref_first != ref_last), 0)) {     // some sums are at an earlier reference
             l_tot = l_div = 0.0f;
             _Pragma("unroll 1") for (int k = 0; k < 512; k += 128) {
-              const float f = pow2i(rl[k] - ref_last);
+              const float f = ex2(rl[k] - ref_last);
               l_tot += xl[k] * f;
               l_div += xl[512 + k] * f;
             }

@@ -134,3 +134,21 @@ def test_rows_without_a_visible_key_and_maps_that_skip():
         empty = ~visible.any(-1)
         assert bool((out[:, :, empty] == 0).all()) and bool((lse[:, :, empty] == float("-inf")).all())
         assert float((lse.double() - lse_ref)[:, :, ~empty].abs().max()) <= s_err
+
+
+@pytest.mark.parametrize("S,D", [(333, 128), (1024, 64), (4096, 128)])
+@pytest.mark.parametrize("outliers", [0, 5])
+def test_error_is_that_of_rounding_p(S, D, outliers):
+    """The error against 64 bits over whole outputs is that of rounding each P to 11 bits: with steps of 2^-10 / m for mantissas m that
+    are spread over the logarithm, the root mean square of step / sqrt(12) is 2^-10 sqrt(0.541 / 12) = 2.07e-4; it comes out smaller
+    where few keys carry a row.  Bound: 2^-12, 1.18 times that."""
+    import mpsa
+    from mpsa import ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(1, 2, S, D, generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    if outliers:
+        k[..., torch.randperm(D, generator=g, device="cuda")[:outliers]] *= 20.0
+    out = mpsa.attention_forward(q, k, v, causal=False, uniform="fp8", out_dtype=torch.float32, check=True)
+    qr, kr = (mpsa.quantize_mx(ops._pad_depth_128(x), s, reference_format=True) for x, s in ((q, ops.q_side_scale(D)), (k, 1.0)))
+    ref = _reference(_mx8(qr), _mx8(kr), v, torch.ones(S, S, dtype=torch.bool, device="cuda"))[0]
+    assert float((out.double() - ref).norm() / ref.norm()) <= 2.0 ** -12
