@@ -76,7 +76,7 @@ constexpr int ATT_OFF_BAR = ATT_OFF_MSLOT + ATT_MAX_SLOTS * 128 * 4;
 constexpr int ATT_B_SFULL = 32;                       // (groups of four at multiples of 32 bytes: neighbours by exclusive or)
 constexpr int ATT_B_SFREE = ATT_B_SFULL + 2, ATT_B_PREADY = ATT_B_SFULL + 4, ATT_B_PVDONE = ATT_B_SFULL + 8, ATT_B_ST = ATT_B_SFULL + 14;
 constexpr int ATT_B_RBAR = ATT_B_SFULL + 28;
-constexpr int ATT_NUM_BARS = ATT_B_RBAR + 16;
+constexpr int ATT_NUM_BARS = ATT_B_RBAR + 16 + 2;
 static_assert(4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX <= ATT_B_SFULL, "barrier numbers overlap");
 constexpr int ATT_BAR_BYTES = 1024;                                       // barriers, TMEM slot, router words, item slots
 static_assert(ATT_NUM_BARS * 8 + 32 + ATT_MAX_SLOTS * 36 <= ATT_BAR_BYTES, "the barrier block does not fit its share of shared memory");
@@ -551,7 +551,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   uint64_t* m_bar = x_bar + 4;                     // [4] fp16 P.V: row references for the other warpgroup
   uint64_t* l_bar = m_bar + 4;                     // [4] partial sums and maxima of a row quarter
   uint64_t* r_bar = l_bar + 4;                     // [4 row quarters][tile & 1][half] fp16 P.V: this half tile has decided on the reference
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(r_bar + 16);
+  uint64_t* drained = r_bar + 16;                  // [2] an issuer that unwinds: its last tensor operations are done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 2);
   volatile int* dec = reinterpret_cast<volatile int*>(tmem_slot + 4);   // [4], slot tile & 3: (tile << 1 | keep) once the router has decided on the tile
   volatile Slot* slots = reinterpret_cast<volatile Slot*>(tmem_slot + 8);   // [MAX_SLOTS]
   uint16_t* lists = reinterpret_cast<uint16_t*>(smem + ATT_OFF_LIST + (PVQ ? 0 : ATT_F16_BYTES));
@@ -578,6 +579,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     mbar_init(o_free, 512);
     for (int s = 0; s < 4; ++s) { mbar_init(&x_bar[s], 2); mbar_init(&m_bar[s], 1); mbar_init(&l_bar[s], 4); }
     for (int s = 0; s < 16; ++s) mbar_init(&r_bar[s], 1);
+    for (int s = 0; s < 2; ++s) mbar_init(&drained[s], 1);
     fence_mbar_init();
     for (int s = 0; s < 4; ++s) dec[s] = -1;        // no tile decided yet
   }
@@ -692,12 +694,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         if (++ls == NL) { ls = 0; l_par ^= 1; }
       }
       if (!ok) {
-        // unwind: give copies in flight a chance to land before shared memory is released
-        _Pragma("unroll 1") for (int u = max(0, q_loads - 2); u < q_loads; ++u) mbar_wait(&q_full[u & 1], (u >> 1) & 1, p.status, KS_TIMEOUT_TMA);
-        _Pragma("unroll 1") for (int u = max(0, tk - ATT_KSTAGES); u < tk; ++u)
-          mbar_wait(&k_full[u % ATT_KSTAGES], (u / ATT_KSTAGES) & 1, p.status, KS_TIMEOUT_TMA);
-        _Pragma("unroll 1") for (int u = max(0, tv - VSTAGES); u < tv; ++u)
-          mbar_wait(&v_full[u % VSTAGES], (u / VSTAGES) & 1, p.status, KS_TIMEOUT_TMA);
+        // unwind: copies in flight land before shared memory is released
+        _Pragma("unroll 1") for (int u = max(0, q_loads - 2); u < q_loads; ++u) mbar_drain(&q_full[u & 1], (u >> 1) & 1);
+        _Pragma("unroll 1") for (int u = max(0, tk - ATT_KSTAGES); u < tk; ++u) mbar_drain(&k_full[u % ATT_KSTAGES], (u / ATT_KSTAGES) & 1);
+        _Pragma("unroll 1") for (int u = max(0, tv - VSTAGES); u < tv; ++u) mbar_drain(&v_full[u % VSTAGES], (u / VSTAGES) & 1);
       }
     }
   } else if (warp == 1) {
@@ -793,6 +793,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         mbar_arrive(&list_empty[ls]);
         if (++ls == NL) { ls = 0; l_par ^= 1; }
       }
+      if (!ok) { tc_commit(&drained[0]); mbar_drain(&drained[0], 0); }   // unwind: operands and accumulators are in use until then
     }
   } else if (warp == 2) {
     // ------------------------------ P.V issuer --------------------------------
@@ -899,6 +900,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         mbar_arrive(&list_empty[ls]);
         if (++ls == NL) { ls = 0; l_par ^= 1; }
       }
+      if (!ok) { tc_commit(&drained[1]); mbar_drain(&drained[1], 0); }
     }
   } else if (warp == 3) {
     // ------------------------------ work items, visit lists and router ----------

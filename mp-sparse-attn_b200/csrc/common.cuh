@@ -114,6 +114,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return mbar_wait_slow(a, parity, status, code, limit);
 }
 
+// Wait of a role that unwinds, for what it has started itself: copies into shared memory, tensor operations.  They end by
+// themselves, so the status word, which is set by then, is not looked at; the limit only keeps the wait bounded.  Also acquires what
+// a thread of another CTA of the cluster wrote before it arrived.
+static __device__ __noinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const uint32_t a = smem_u32(bar);
+  const long long t0 = clock64();
+  for (uint32_t spins = 0;;) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(a), "r"(parity) : "memory");
+    if (done) return;
+    if ((++spins & 0x3ff) == 0 && clock64() - t0 > kWaitLimitCycles) return;
+  }
+}
+
 // ---- TMA --------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");

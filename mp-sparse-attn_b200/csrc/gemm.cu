@@ -18,13 +18,16 @@
 //   warps 2, 3   of the first CTA: the scale copies of NVFP4, which has twelve per stage
 //   warps 4-11   epilogue: a warp takes its 32 lanes and half of the columns into registers, hands the accumulator back,
 //                and only then scales, converts and writes through shared memory with TMA stores, under the next tile's MMAs
-// The ring runs on across tiles.  All hand-offs go through mbarriers with bounded waits.
+// The ring runs on across tiles.  All hand-offs go through mbarriers with bounded waits.  When one expires the roles leave their
+// loops; then, as at the ordinary end, the first CTA's producer waits for every copy that either producer has requested (drain.h), and
+// every issuing thread for its own tensor operations, before a CTA gives up its memory.
 //
 //   mode 0  MXFP8  kind::mxf8f6f4  K=32 per instruction, one E8M0 scale per 32 elements
 //   mode 1  MXFP4  kind::mxf4      K=64 per instruction, two E8M0 scales
 //   mode 2  NVFP4  kind::mxf4nvf4  K=64 per instruction, four E4M3 scales (16-element blocks)
 #include "api_internal.h"
 #include "common.cuh"
+#include "drain.h"
 #include "tma_host.h"
 
 #include <cuda_bf16.h>
@@ -39,7 +42,7 @@ constexpr int GEMM_SLAB = 128;                       // bytes of K per stage and
 constexpr int GEMM_EPI_WARPS = 8;
 constexpr int GEMM_THREADS = 128 + 32 * GEMM_EPI_WARPS;
 constexpr int GEMM_STAGING = GEMM_EPI_WARPS * 2048;  // a 32-row, 64-byte box per epilogue warp
-constexpr int GEMM_BARS = 256;                       // mbarriers and the TMEM slot
+constexpr int GEMM_BARS = 320;                       // mbarriers, the TMEM slot and the peer's count
 constexpr int GEMM_SMEM_MAX = 232448;
 constexpr uint32_t GEMM_TMEM_COLS = 512;
 
@@ -96,6 +99,9 @@ __device__ __forceinline__ void cluster_sync() {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {      // counts bytes off as an arriving copy does
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 // a TMA load into this CTA's shared memory that reports to a barrier of the pair (no multicast)
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t bar, int x, int y) {
@@ -187,7 +193,10 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   uint64_t* sf_ready = empty + ST;                       // [ST] SPLIT: the stage's scale tiles are in TMEM
   uint64_t* acc_full = sf_ready + ST;                    // [2]
   uint64_t* acc_free = acc_full + 2;                     // [2] first CTA: every epilogue warp of both CTAs has read the accumulator
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
+  uint64_t* drained = acc_free + 2;                      // [3] the issuing threads' last operations are done
+  uint64_t* peer_left = drained + 3;                     // first CTA: the other one's producer has left its count
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(peer_left + 1);
+  int* peer_issued = reinterpret_cast<int*>(tmem_slot + 1);   // first CTA: stages that the other one has requested
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
@@ -197,6 +206,8 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   if (threadIdx.x == 0) {
     for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&sf_ready[s], 2); }
     for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_free[s], 2 * GEMM_EPI_WARPS); }
+    for (int s = 0; s < 3; ++s) mbar_init(&drained[s], 1);
+    mbar_init(peer_left, 1);
     fence_mbar_init();
   }
   if (warp == 1) tmem_alloc_pair(tmem_slot, GEMM_TMEM_COLS);
@@ -211,7 +222,7 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     if (elect_one()) {
       tma_prefetch_desc(&tmap_a); tma_prefetch_desc(&tmap_b); tma_prefetch_desc(&tmap_sfa); tma_prefetch_desc(&tmap_sfb);
       bool ok = true;
-      int s = 0;
+      int s = 0, issued = 0;
       uint32_t e_par = 1;                                // parity that a never-used barrier already satisfies
       _Pragma("unroll 1") for (int tile = pair; tile < p.n_tiles && ok; tile += n_pairs) {
         int mi, ni, z;
@@ -234,14 +245,24 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           tma_load_2d_pair(st + G::A_BYTES, &tmap_b, bar, kt * GEMM_SLAB, yb);
           sfa_y += NC * 4;
           sfb_y += NC * 4;
+          ++issued;
           if (++s == ST) { s = 0; e_par ^= 1; }
         }
       }
-      if (!ok) {
-        // unwind: time for the copies in flight to land before shared memory is released (a load takes microseconds; the
-        // barrier they report to may be the other CTA's)
-        const long long t0 = clock64();
-        while (clock64() - t0 < 1000000) {}
+      // Neither CTA's shared memory is released while copies into it are in flight, whoever has given up: the first CTA, where they
+      // all report, sees every requested stage land (at the ordinary end they have), and the other one leaves with it.
+      if (rank == 1) {
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(leader_addr(peer_issued)), "r"(issued) : "memory");
+        mbar_arrive_cluster(leader_addr(peer_left));
+      } else {
+        mbar_drain(peer_left, 0);
+        const int other = *(volatile int*)peer_issued;
+        _Pragma("unroll 1") for (int u = drain_first(issued, other, ST); u < drain_end(issued, other); ++u) {
+          const DrainStep step = drain_step(u, issued, other);
+          if (step == DRAIN_ARM) mbar_arrive_expect_tx(&full[u % ST], G::LOADED);
+          else if (step == DRAIN_FILL) mbar_complete_tx(&full[u % ST], G::LOADED);
+          mbar_drain(&full[u % ST], (u / ST) & 1);
+        }
       }
     }
   } else if (warp == 1) {
@@ -296,6 +317,8 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         tc_commit_pair(&acc_full[acc]);
         if (++acc == G::NACC) { acc = 0; a_par ^= 1; }
       }
+      tc_commit_pair_local(&drained[0]);                 // the operands and the accumulators are in use until then
+      mbar_drain(&drained[0], 0);
     }
   } else if (warp < 4) {
     // ------------------------------ scale copies (NVFP4) -----------------------
@@ -325,6 +348,8 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           if (++s == ST) { s = 0; f_par ^= 1; }
         }
       }
+      tc_commit_pair_local(&drained[warp - 1]);
+      mbar_drain(&drained[warp - 1], 0);
     }
   } else {
     // ------------------------------ epilogue ----------------------------------

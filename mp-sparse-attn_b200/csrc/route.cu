@@ -58,7 +58,8 @@ route_stat_kernel(const __grid_constant__ CUtensorMap tm_q4, const __grid_consta
   uint64_t* k_empty = k_full + RT_KSTAGES;
   uint64_t* s_full = k_empty + RT_KSTAGES;       // RT_SBUF: the unit's MMAs are complete
   uint64_t* s_free = s_full + RT_SBUF;           // RT_SBUF: the four warps of the group have read the accumulator
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_free + RT_SBUF);
+  uint64_t* drained = s_free + RT_SBUF;          // RT_MAXH: the issuing threads' last operations are done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + RT_MAXH);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = (p.S + RT_BM - 1) / RT_BM, nk = (p.Skv + RT_BN - 1) / RT_BN;
@@ -75,6 +76,7 @@ route_stat_kernel(const __grid_constant__ CUtensorMap tm_q4, const __grid_consta
     mbar_init(q_full, 1);
     for (int s = 0; s < RT_KSTAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], nh); }
     for (int s = 0; s < RT_SBUF; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_free[s], 4); }
+    for (int s = 0; s < RT_MAXH; ++s) mbar_init(&drained[s], 1);
     fence_mbar_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, RT_TMEM_COLS);
@@ -108,11 +110,9 @@ route_stat_kernel(const __grid_constant__ CUtensorMap tm_q4, const __grid_consta
         issued = t + 1;
         if (++s == RT_KSTAGES) { s = 0; if (t >= RT_KSTAGES) par ^= 1; }
       }
-      if (!ok) {                                 // unwind: let the copies in flight land before the CTA exits
-        mbar_wait(q_full, 0, p.status, KS_TIMEOUT_TMA);
-        for (int t = max(0, issued - RT_KSTAGES); t < issued; ++t)
-          mbar_wait(&k_full[t % RT_KSTAGES], (t / RT_KSTAGES) & 1, p.status, KS_TIMEOUT_TMA);
-      }
+      // the CTA keeps its memory until every copy has landed, whoever has given up (at the ordinary end they have)
+      mbar_drain(q_full, 0);
+      for (int t = max(0, issued - RT_KSTAGES); t < issued; ++t) mbar_drain(&k_full[t % RT_KSTAGES], (t / RT_KSTAGES) & 1);
     }
   } else if (warp == 1 || (warp == 2 && nh == 2)) {
     // MMA issuer of head j (one thread)
@@ -147,6 +147,8 @@ route_stat_kernel(const __grid_constant__ CUtensorMap tm_q4, const __grid_consta
         tc_commit(&k_empty[s]);
         if (++s == RT_KSTAGES) { s = 0; k_par ^= 1; }
       }
+      tc_commit(&drained[j]);                    // the operands and the accumulators are in use until then
+      mbar_drain(&drained[j], 0);
     }
   } else if (warp >= 4) {
     const int q = warp & 3, g = (warp - 4) >> 2;           // TMEM lane quarter; warpgroup = accumulator it owns
