@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import ctypes
 import struct
+import threading
 from dataclasses import dataclass
 from typing import Optional
 
@@ -18,7 +19,13 @@ _IN_DTYPE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 _OUT_DTYPE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2, torch.float8_e5m2: 3}
 _FP8_QUANT = {"e5m2": 1, "e4m3": 2}
 _FP8_DESC = {"e5m2": 1, "e4m3": 0}
-_last_range_flag = None
+_last = threading.local()            # range_flag: the word of this thread's last forward that was given one
+
+
+def __getattr__(name):
+    if name == "_last_range_flag":   # non-zero: query tiles were done again (range_flag of include/mpsa.h); None: the call had no such word
+        return getattr(_last, "range_flag", None)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def _stream():
@@ -26,16 +33,13 @@ def _stream():
 
 
 class _DeviceState:
-    """Per-device words the kernels write: the status word, and the range flag of the one-call attention path."""
+    """The status word of a device, which the kernels write when a bounded wait expires."""
 
     def __init__(self, index):
         self.index = index
         self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.status_ptr = self.status.data_ptr()
         self.word = ctypes.c_int.from_address(self.status_ptr)       # read on every call: no tensor machinery
-        with torch.cuda.device(index):
-            self.range_flag = torch.zeros(1, dtype=torch.int32, device="cuda")
-        self.range_ptr = self.range_flag.data_ptr()
 
 
 _states = {}
@@ -493,8 +497,9 @@ def _strides16(t):
 
 
 def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out_dtype, pv_mode, route, tau, smooth_k,
-                        nvfp4):
-    """attention_forward through one C call (mpsa_attention), or None where that entry does not take the operands."""
+                        nvfp4, want_flag):
+    """attention_forward through one C call (mpsa_attention), or None where that entry does not take the operands.
+    want_flag: keep a range flag of this call's own (quantised P.V)."""
     dt = q.dtype
     in_dtype = 0 if dt is torch.bfloat16 else 1 if dt is torch.float16 else None
     qs = _strides16(q)
@@ -552,9 +557,8 @@ def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out
     dev = q.device
     ws = _empty((need,), (1,), torch.uint8, dev)
     out = _empty((B, Hq, S, D), (Hq * S * D, S * D, D, 1), out_dtype, dev)
-    global _last_range_flag
-    _last_range_flag = st.range_flag if pv else None
-    args = _ATTENTION_ARGS.pack(q.data_ptr(), kp, vp, *qs, *ks, *vs, *prepared, out.data_ptr(), ws.data_ptr(), need, st.range_ptr,
+    flag = _last.range_flag = _empty((1,), (1,), torch.int32, dev) if want_flag and pv else None
+    args = _ATTENTION_ARGS.pack(q.data_ptr(), kp, vp, *qs, *ks, *vs, *prepared, out.data_ptr(), ws.data_ptr(), need, _ptr(flag) or 0,
                                 st.status_ptr, *ints, sq, tau)
     rc = _on_device(index, lib.mpsa_attention, args)
     if rc:
@@ -629,7 +633,8 @@ def attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, caus
                                                                       uniform is None and not online)) and skip_thresh is None and not return_sparsity and \
             pv_mode in ("fp16", "requant") and (router == "band" or (online and uniform is None and fused_router and causal and requant)):
         out = _attention_one_call(q, k, v, kv, causal=causal, band=band, uniform=uniform, sq=sq, fp8_elem=fp8_elem, out_dtype=out_dtype,
-                                  pv_mode=pv_mode, route=online, tau=float(tau), smooth_k=smooth_k and kv is None, nvfp4=nvfp4)
+                                  pv_mode=pv_mode, route=online, tau=float(tau), smooth_k=smooth_k and kv is None, nvfp4=nvfp4,
+                                  want_flag=check)
         if out is not None:
             if check:
                 check_status(q.device)
@@ -675,7 +680,7 @@ def attention_forward_quantized(qq: QuantizedOperand, kq: QuantizedOperand, vt, 
                                 lazy: bool = True, merge_with=None):
     """The fused forward on operands that are already quantised (depth padded to 128) and a V^T from
     prepare_vt (fp16 P.V) or a QuantizedV from quantize_v_seq (quantised P.V).  Both formats of Q and K
-    must be present unless `uniform` restricts the map to one."""
+    must be present unless `uniform` restricts the map to one.  lazy: accepted for earlier callers, selects nothing."""
     requant = isinstance(vt, QuantizedV)
     dev = vt.vt8.device if requant else vt.device
     nq, nk = -(-S // 128), -(-Skv // 128)
@@ -753,10 +758,7 @@ def attention_forward_quantized(qq: QuantizedOperand, kq: QuantizedOperand, vt, 
     lse = torch.empty((B, Hq, S), dtype=torch.float32, device=dev) if return_lse else None
     _raise_if_failed(dev)
     st = status_word(dev)
-    # `lazy` is accepted for earlier callers; it only decides whether the word below is kept for inspection
-    flag = torch.zeros(1, dtype=torch.int32, device=dev) if (requant and lazy) else None
-    global _last_range_flag
-    _last_range_flag = flag                       # non-zero after the call = some query tiles were done again (include/mpsa.h)
+    flag = _last.range_flag = torch.zeros(1, dtype=torch.int32, device=dev) if requant else None
     with torch.cuda.device(dev):
         rc = _lib.load().mpsa_attn_fwd(
             q8.data_ptr(), q8s.data_ptr(), q4.data_ptr(), q4s.data_ptr(),
@@ -800,9 +802,7 @@ def attention_forward_routed(qq: QuantizedOperand, kq: QuantizedOperand, vq: "Qu
     lse = torch.empty((B, Hq, S), dtype=torch.float32, device=dev)
     lse_final = torch.empty((B, Hq, S), dtype=torch.float32, device=dev) if return_lse else None
     stat = torch.zeros((B, Hq, nq, nk), dtype=torch.float32, device=dev) if return_stat else None
-    flag = torch.zeros(1, dtype=torch.int32, device=dev)
-    global _last_range_flag
-    _last_range_flag = flag
+    flag = _last.range_flag = torch.zeros(1, dtype=torch.int32, device=dev)
     _raise_if_failed(dev)
     st = status_word(dev)
     with torch.cuda.device(dev):
