@@ -211,36 +211,42 @@ def test_block_scale_type_names_are_checked():
     _check(o.cpu(), ref, "nvfp4 by name")
 
 
-def test_fixed_reference_kernel_and_its_fallback():
-    """Quantised P.V runs with the row reference fixed after the first key tile; the exact kernel is its conditional
-    fallback.  (1) On ordinary data both give the same output.  (2) When later keys push the scores more than 2^64
-    above the first tile's maximum, the fallback must take over: the result still matches the oracle."""
+@pytest.mark.parametrize("shift,again", [(0.0, 0), (-40.0, 0), (-48.0, 1), (80.0, 0), (96.0, 1)])
+def test_fixed_reference_and_the_items_outside_its_window(shift, again):
+    """Quantised P.V runs against one row reference, good for row maxima of -44 .. 84 octaves; an item with a row outside is done again
+    with the maxima that the first pass found, and the range flag says so.  Either way the result matches the oracle."""
+    import mpsa
+    from mpsa import ops
+    g = torch.Generator().manual_seed(4)
+    q, k, v = (torch.randn(1, 2, n, 128, generator=g) * x for n, x in ((200, 0.5), (300, 0.2), (300, 1.0)))
+    q[..., 0] = 1.0 / ops.q_side_scale(128)       # every score: `shift` octaves and noise of a seventh of one
+    k[..., 0] = shift
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    qq, kq = mpsa.quantize_mx(q.cuda(), ops.q_side_scale(128)), mpsa.quantize_mx(k.cuda(), 1.0)
+    out = ops.attention_forward_quantized(qq, kq, mpsa.quantize_v_seq(v.cuda()), 1, 2, 2, 200, 300, 128, causal=False, uniform="fp8",
+                                          out_dtype=torch.float32, check=True).cpu()
+    assert int(ops._last_range_flag.item()) == again
+    _check(out, O.attention_mxfp(q, k, v, causal=False, uniform="fp8", pv_mode="requant"), (shift, "window"))
+
+
+def test_items_done_again_in_a_causal_problem():
+    """Later keys whose scores dwarf the first tile's: the items that see them are done again, the others are not."""
     import mpsa
     from mpsa import ops
     q, k, v = O.make_qkv(9, 1, 4, 2, 1024, 128, outliers=3)
-
-    def run(q, k, v, lazy):
-        sq = ops.q_side_scale(128)
-        qq, kq = mpsa.quantize_mx(q.cuda(), sq), mpsa.quantize_mx(k.cuda(), 1.0)
-        vq = mpsa.quantize_v_seq(v.cuda())
-        return ops.attention_forward_quantized(qq, kq, vq, 1, 4, 2, 1024, 1024, 128, causal=True, out_dtype=torch.float32,
-                                               check=True, lazy=lazy).cpu()
-
-    a, b = run(q, k, v, True), run(q, k, v, False)
-    assert torch.allclose(a, b, rtol=1e-5, atol=1e-6), (a - b).abs().max()
-    _check(a, O.attention_mxfp(q, k, v, causal=True, pv_mode="requant"), "fixed reference")
-    k2 = k.clone().float()
-    k2[:, :, 128:] *= 60.0                       # scores of every later tile dwarf the first tile's
-    k2 = k2.to(torch.bfloat16)
-    ref = O.attention_mxfp(q, k2, v, causal=True, pv_mode="requant")
-    out = run(q, k2, v, True)
-    assert torch.isfinite(out).all()
-    _check(out, ref, "fallback")
-    assert torch.allclose(out, run(q, k2, v, False), rtol=1e-5, atol=1e-6)
+    k = k.float()
+    k[:, :, 128:] *= 60.0
+    k = k.to(torch.bfloat16)
+    sq = ops.q_side_scale(128)
+    qq, kq = mpsa.quantize_mx(q.cuda(), sq), mpsa.quantize_mx(k.cuda(), 1.0)
+    out = ops.attention_forward_quantized(qq, kq, mpsa.quantize_v_seq(v.cuda()), 1, 4, 2, 1024, 1024, 128, causal=True,
+                                          out_dtype=torch.float32, check=True).cpu()
+    assert int(ops._last_range_flag.item()) == 1 and torch.isfinite(out).all()
+    _check(out, O.attention_mxfp(q, k, v, causal=True, pv_mode="requant"), "done again")
 
 
 def test_fixed_reference_is_not_abandoned_on_ragged_shapes():
-    """The padding rows of a ragged last query tile hold no data: they must not trigger the exact-kernel fallback."""
+    """The padding rows of a ragged last query tile hold no data: no item may be done again because of them."""
     import mpsa
     from mpsa import ops
     for S, causal in ((1560, False), (300, True)):

@@ -63,15 +63,14 @@ def test_one_call_form_uses_the_router_inside_and_matches_the_stand_alone_form()
     assert m["rel_l2"] <= 4e-3, m          # bf16 outputs of two different accumulation orders
 
 
-def test_fallback_when_scores_leave_the_fixed_reference():
-    """Later keys 2^64 and more above the first tile's maximum: the forward flags it, and the exact kernel launched behind
-    it recomputes the whole output over the final map; the result still matches the oracle,
-    and the map is the one the stand-alone router gives."""
+def test_items_done_again_when_scores_leave_the_fixed_reference():
+    """Row maxima beyond the window of the row reference: the forward does those items again over the map that its first pass left, and
+    says so; the result still matches the oracle, and the map is the one the stand-alone router gives."""
     import mpsa
     from mpsa import ops
     q, k, v = O.make_qkv(9, 1, 4, 2, 1024, 128, outliers=3)
     k2 = k.clone().float()
-    k2[:, :, 128:] *= 60.0                        # scores of every later tile dwarf the first tile's
+    k2[:, :, 128:] *= 60.0
     k2 = k2.to(torch.bfloat16)
     qq, kq, vq = _operands(q, k2, v)
     out, pm = ops.attention_forward_routed(qq, kq, vq, 1, 4, 2, 1024, 1024, 128, band=1, tau=1.1, out_dtype=torch.float32,
