@@ -35,7 +35,7 @@
 // across items, so an item's Q, K and V loads and its first tiles happen under the previous item's last ones.
 //
 // What bounds it: the exponentials.  ex2 runs at 16 per clock and SM (measured), i.e. 1024 cycles for the 16384 scores of
-// a tile; on MXFP4 tiles with quantised P.V two of every 32 are computed on the FMA pipe instead.  A loop of the tile's softmax arithmetic alone, 16 warps
+// a tile; two of every 32 are computed on the FMA pipe instead (MXFP4 tiles with quantised P.V, and fp16 P).  A loop of the tile's softmax arithmetic alone, 16 warps
 // on TMEM data, takes 1003 cycles a tile; with all hand-offs and MMAs 1160.
 #include "api_internal.h"
 #include "common.cuh"

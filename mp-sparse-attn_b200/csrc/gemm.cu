@@ -8,7 +8,7 @@
 // its own 128 rows and, in shared memory, its 128 rows of A and HALF of the tile's rows of B, which the tensor cores of both
 // SMs read.  With one CTA per 128 x 256 tile an MMA of 32 bytes of K reads 12 KB of shared memory in its 128 cycles while TMA
 // writes another 12 KB: 190 bytes per clock where an SM has 128, a ceiling of 0.67 of the tensor rate.  A pair needs 128.
-// Measured, 8192^3 to bf16: MXFP8 504 -> 381 us (2.9 PFLOP/s), MXFP4 271 -> 235, NVFP4 300 -> 237.  A 256-column MXFP8 stage
+// Measured, 8192^3 to bf16, 20 launches: MXFP8 489 -> 384 - 391 us (2.8 PFLOP/s), MXFP4 272 -> 195 - 200, NVFP4 300 -> 222 - 227.  A 256-column MXFP8 stage
 // takes 600 cycles for 512 of tensor work at the 1.4 - 1.6 GHz that the power limit leaves; the FP4 modes also load a stage's
 // 35 - 39 KB per SM in what would be 512 cycles.  1500 x 4096 x 4096 NVFP4: 27 -> 18 us; 180 x 6256 x 512: 9 -> 6 us, launch
 // and first loads.

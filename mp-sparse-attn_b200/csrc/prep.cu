@@ -582,7 +582,6 @@ int prep_launch(PrepCall& p, int in_dtype, bool w8, bool w4, int fp8_fmt, cudaSt
     o.ctas = (int)n;
   }
   p.v.ctas = 0;
-  p.v.ctas = 0;
   size_t smem = 512;
   if (p.v.v) {
     const long long n = (long long)p.v.B * p.v.H * (p.v.pitch >> 7);
