@@ -35,8 +35,8 @@
 // across items, so an item's Q, K and V loads and its first tiles happen under the previous item's last ones.
 //
 // What bounds it: the exponentials.  ex2 runs at 16 per clock and SM (measured), i.e. 1024 cycles for the 16384 scores of
-// a tile; two of every 32 are computed on the FMA pipe instead (MXFP4 tiles with quantised P.V, and fp16 P).  A loop of the tile's softmax arithmetic alone, 16 warps
-// on TMEM data, takes 1003 cycles a tile; with all hand-offs and MMAs 1160.
+// a tile; two of every 32 are computed on the FMA pipe instead (MXFP4 tiles with quantised P.V, and fp16 P).  A loop of the
+// tile's softmax arithmetic alone, 16 warps on TMEM data, takes 1003 cycles a tile; with all hand-offs and MMAs 1160.
 #include "api_internal.h"
 #include "common.cuh"
 #include "prep.h"
@@ -73,10 +73,11 @@ constexpr int ATT_OFF_MROW = ATT_OFF_RMAX + 2 * 2 * 128 * 4;              // flo
 constexpr int ATT_OFF_MSLOT = ATT_OFF_MROW + 128 * 4;                     // float [MAX_SLOTS][128]: row maxima of the item that was in the slot
 constexpr int ATT_OFF_BAR = ATT_OFF_MSLOT + ATT_MAX_SLOTS * 128 * 4;
 // barriers the softmax threads use in their tile loop, by number
-constexpr int ATT_B_SFULL = 32;                       // (groups of four at multiples of 32 bytes: neighbours by exclusive or)
+constexpr int ATT_B_SFULL = 32;
 constexpr int ATT_B_SFREE = ATT_B_SFULL + 2, ATT_B_PREADY = ATT_B_SFULL + 4, ATT_B_PVDONE = ATT_B_SFULL + 8, ATT_B_ST = ATT_B_SFULL + 14;
 constexpr int ATT_B_RBAR = ATT_B_SFULL + 28;
 constexpr int ATT_NUM_BARS = ATT_B_RBAR + 16 + 2;
+static_assert(ATT_B_PVDONE % 4 == 0, "the four are one another's neighbours by exclusive or of their addresses");
 static_assert(4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX <= ATT_B_SFULL, "barrier numbers overlap");
 constexpr int ATT_BAR_BYTES = 1024;                                       // barriers, TMEM slot, router words, item slots
 static_assert(ATT_NUM_BARS * 8 + 32 + ATT_MAX_SLOTS * 36 <= ATT_BAR_BYTES, "the barrier block does not fit its share of shared memory");
