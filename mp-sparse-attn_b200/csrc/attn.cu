@@ -29,14 +29,19 @@
 // decide in their order, each before it hands over its P, so P.V, which takes them in the same order, finds P and O at one
 // reference.  (With references rounded down to whole octaves no largest P was exactly 1: 5 % more error with N(0,1) keys.)
 //
-// Roles: warp 0 TMA loads, warp 1 Q.K^T issuer, warp 2 P.V issuer, warp 3 hands out work items, builds their visit lists
-// (the non-skipped cells of the map row) and routes, warps 4.. softmax and epilogue (a warp reaches the TMEM lane
+// Roles: warp 0 loads Q and V, warp 1 loads K and issues Q.K^T, warp 2 issues P.V, warp 3 hands out work items, builds their visit
+// lists (the non-skipped cells of the map row) and routes, warps 4.. softmax and epilogue (a warp reaches the TMEM lane
 // quarter warp % 4).  Items reach the other roles through a ring of slots, an item ahead; rings and their phases run on
 // across items, so an item's Q, K and V loads and its first tiles happen under the previous item's last ones.
 //
-// What bounds it: the exponentials.  ex2 runs at 16 per clock and SM (measured), i.e. 1024 cycles for the 16384 scores of
-// a tile; two of every 32 are computed on the FMA pipe instead (MXFP4 tiles with quantised P.V, and fp16 P).  A loop of the
-// tile's softmax arithmetic alone, 16 warps on TMEM data, takes 1003 cycles a tile; with all hand-offs and MMAs 1160.
+// What bounds it: instruction issue and latency together, then the exponentials.  A tile takes about 1200 - 1450 cycles; without any
+// exponential (timing only) it would still take 0.88 of that, without all of the softmax arithmetic 0.7.  ex2 runs at 16 per clock
+// and SM, 1024 cycles for the 16384 scores of a tile; the four softmax warps of a quarter issue some 700 instructions a tile and
+// the service warp beside them 130 - 180 more, on a scheduler that has four or five warps to choose from.  Hence:
+//  - no branch inside a tile's arithmetic: the instructions on its two sides are scheduled apart, and one that is never taken costs
+//    2 %.  Masks and shifts are applied to S in tensor memory beforehand (adjust_scores).
+//  - service threads of few instructions, on warps of their own: one thread that requested K and V was busy for 1000 - 1100 of
+//    every 1400 cycles and held the kernel up (12 heads of 7803 tokens 231 -> 224 us with K moved to the Q.K^T issuer).
 #include "api_internal.h"
 #include "common.cuh"
 #include "prep.h"
@@ -52,8 +57,8 @@ namespace mpsa {
 // ---- organisation of a CTA ------------------------------------------------------------------------------
 constexpr int ATT_BM = 128, ATT_BN = 128, ATT_DQK = 128;
 constexpr int ATT_KSTAGES = 4;                        // K ring
-constexpr int ATT_VSLOTS_MAX = 4;                     // V ring: 2 slots of 32 KB (fp16 V^T) or 4 of 16 KB (quantised V^T)
-constexpr int ATT_SERVICE_WARPS = 4;                  // 0 TMA loads, 1 Q.K^T issuer, 2 P.V issuer, 3 visit lists and router
+constexpr int ATT_VSLOTS = 4;                         // V ring, slots of 16 KB: a quantised V^T tile or a 64-key half of an fp16 one
+constexpr int ATT_SERVICE_WARPS = 4;                  // 0 loads of Q and V, 1 loads of K and Q.K^T, 2 P.V, 3 visit lists and router
 constexpr int ATT_SM_WARPS = 16;                      // softmax: 2 warpgroups (tiles in turn) x 2 column halves x 4 row quarters
 constexpr int ATT_THREADS = 32 * (ATT_SERVICE_WARPS + ATT_SM_WARPS);
 constexpr int ATT_Q8_BYTES = ATT_BM * 128, ATT_Q4_BYTES = ATT_BM * 64;
@@ -66,27 +71,27 @@ constexpr int ATT_OFF_K = ATT_OFF_Q + 2 * ATT_Q_BYTES;
 constexpr int ATT_OFF_V = ATT_OFF_K + ATT_KSTAGES * ATT_K_BYTES;
 constexpr int ATT_OFF_SFQ = ATT_OFF_V + 2 * ATT_V_BYTES;                  // [2] Q8 scale tile (512 B), Q4 scale tiles (1024 B: NVFP4 has two)
 constexpr int ATT_OFF_SFK = ATT_OFF_SFQ + 2 * 1536;                       // [KSTAGES] 1024 B
-constexpr int ATT_OFF_SFP = ATT_OFF_SFK + ATT_KSTAGES * 1024;             // P scale tiles [2], V scale tiles [VSLOTS_MAX]
-constexpr int ATT_OFF_XROW = ATT_OFF_SFP + (2 + ATT_VSLOTS_MAX) * 512;    // float [2][2][4][128]: row sums and row maxima of the four threads of a row
-constexpr int ATT_OFF_RMAX = ATT_OFF_XROW + 2 * 2 * 4 * 128 * 4;          // float [2 buffers][2][128]: slice maxima for the router; fp16 P.V: first-tile maxima
-constexpr int ATT_OFF_MROW = ATT_OFF_RMAX + 2 * 2 * 128 * 4;              // float [128]: present row reference (fp16 P.V)
+constexpr int ATT_OFF_SFP = ATT_OFF_SFK + ATT_KSTAGES * 1024;             // P scale tiles [2], V scale tiles [VSLOTS]
+constexpr int ATT_OFF_XROW = ATT_OFF_SFP + (2 + ATT_VSLOTS) * 512;    // float [2][2][4][128]: row sums and row maxima of the four threads of a row
+constexpr int ATT_OFF_RMAX = ATT_OFF_XROW + 2 * 2 * 4 * 128 * 4;          // fp16 P.V: float [2][128], first-tile maxima
+constexpr int ATT_OFF_MROW = ATT_OFF_RMAX + 2 * 128 * 4;                  // float [128]: present row reference (fp16 P.V)
 constexpr int ATT_OFF_MSLOT = ATT_OFF_MROW + 128 * 4;                     // float [MAX_SLOTS][128]: row maxima of the item that was in the slot
 constexpr int ATT_OFF_BAR = ATT_OFF_MSLOT + ATT_MAX_SLOTS * 128 * 4;
 // barriers the softmax threads use in their tile loop, by number
 constexpr int ATT_B_SFULL = 32;
 constexpr int ATT_B_SFREE = ATT_B_SFULL + 2, ATT_B_PREADY = ATT_B_SFULL + 4, ATT_B_PVDONE = ATT_B_SFULL + 8, ATT_B_ST = ATT_B_SFULL + 14;
-constexpr int ATT_B_RBAR = ATT_B_SFULL + 28;
+constexpr int ATT_B_RBAR = ATT_B_SFULL + 30;
 constexpr int ATT_NUM_BARS = ATT_B_RBAR + 16 + 2;
 static_assert(ATT_B_PVDONE % 4 == 0, "the four are one another's neighbours by exclusive or of their addresses");
-static_assert(4 + 3 * ATT_MAX_SLOTS + 2 * ATT_KSTAGES + 2 * ATT_VSLOTS_MAX <= ATT_B_SFULL, "barrier numbers overlap");
+static_assert(4 + 3 * ATT_MAX_SLOTS + ATT_KSTAGES + 2 * ATT_VSLOTS <= ATT_B_SFULL, "barrier numbers overlap");
 constexpr int ATT_BAR_BYTES = 1024;                                       // barriers, TMEM slot, router words, item slots
 static_assert(ATT_NUM_BARS * 8 + 32 + ATT_MAX_SLOTS * 36 <= ATT_BAR_BYTES, "the barrier block does not fit its share of shared memory");
-constexpr int ATT_OFF_F16 = ATT_OFF_BAR + ATT_BAR_BYTES;                  // fp16 P.V: float [2][4][128], the references of XROW's sums
-constexpr int ATT_F16_BYTES = 2 * 4 * 128 * 4;
-constexpr int ATT_OFF_LIST = ATT_OFF_BAR + ATT_BAR_BYTES;                 // visit lists: n_lists x list_cap uint16 (fp16 P.V: ATT_F16_BYTES further on)
+constexpr int ATT_OFF_EXTRA = ATT_OFF_BAR + ATT_BAR_BYTES;                // fp16 P.V: float [2][4][128], the references of XROW's sums;
+constexpr int ATT_EXTRA_BYTES = 2 * 4 * 128 * 4;                          // router: float [4 tiles][2][128], slice maxima
+constexpr int ATT_OFF_LIST = ATT_OFF_BAR + ATT_BAR_BYTES;                 // visit lists: n_lists x list_cap uint16 (ATT_EXTRA_BYTES further on where they are used)
 constexpr int ATT_MAX_KTILES = 8192;                                      // longest row of the precision map (1M keys)
 constexpr int ATT_SMEM_MAX = 232448;
-static_assert(ATT_OFF_LIST + ATT_F16_BYTES + ATT_MAX_KTILES * 2 + 1024 <= ATT_SMEM_MAX, "more shared memory than a CTA can have");
+static_assert(ATT_OFF_LIST + ATT_EXTRA_BYTES + ATT_MAX_KTILES * 2 + 1024 <= ATT_SMEM_MAX, "more shared memory than a CTA can have");
 // TMEM columns: S0 [0,128) S1 [128,256) O [256,384), scale tiles from 384, P up to 512
 constexpr uint32_t ATT_TMEM_COLS = 512;
 constexpr uint32_t ATT_COL_S = 0, ATT_COL_O = 256;
@@ -99,8 +104,10 @@ constexpr uint32_t ATT_COL_P16 = 416;                             // fp16 P: 3 b
 constexpr int TILE_SKIP = 0, TILE_FP8 = 1, TILE_FP4 = 2;
 constexpr uint32_t ENTRY_F8 = 0x8000, ENTRY_MASK = 0x4000, ENTRY_TILE = 0x3fff;   // visit list entries
 
-constexpr int ATT_POLY_FP4 = 2;                       // exponentials of a 32-key block on the FMA pipe: MXFP4 tiles (ex2_poly2<4>)
-constexpr int ATT_POLY_F16 = 2;                       // the same, fp16 P, at full precision (ex2_poly2<5>): NVFP4 video back to back 18.5 ms with 0, 17.6 with 2, 18.3 with 4
+// Exponentials of a 32-key block that run on the FMA pipe (ex2_poly2).  MXFP4 tiles with quantised P.V, exponentials before the
+// block's maximum (LATE): 512 queries of 32K 179 us with 0, 173 with 2, 164 with 4, 170 with 6.  Where they wait for the maximum:
+// routed causal 8K 400 us with 0, 397 with 2, 401 with 4.  fp16 P: NVFP4 video back to back 18.5 ms with 0, 17.6 with 2, 18.3 with 4.
+constexpr int ATT_POLY_LATE = 4, ATT_POLY_EARLY = 2, ATT_POLY_F16 = 2;
 constexpr int ATT_F16_EARLY = 4;                      // fp16 P.V: exponentials of the second block that hide the vote on the reference
 constexpr int SPLIT_MIN_RUN = 8;                      // tiles of a run at least
 constexpr int SPLIT_GAIN = 12;                        // tiles (of 0.7 us) that dividing the keys must save on the busiest CTA
@@ -309,41 +316,33 @@ __device__ __forceinline__ void sub2(float& a, float& b, float c, float d, float
 }
 
 // 2^x for a pair of values on the FMA pipe, for the share of the exponentials taken off the special-function unit:
-// x = n + f with n = round(x) (adding 1.5 * 2^23 leaves n in the low mantissa bits), 2^f on [-0.5, 0.5] by a polynomial, 2^n by
-// adding n to the exponent field.  Degree 4: relative error 8e-6, far below half a step of MXFP4; x is clamped at -125, anything
-// smaller is zero there.  Degree 5: least largest relative error among those with value 1 at 0 (found by reweighted least
-// squares), 1.6e-7 with fp32 rounding, against the 2^-22 = 2.4e-7 that ex2.approx is specified with; zero below 2^-126 like it.
+// x = n + f with n = round(x) (adding 1.5 * 2^23 leaves n in the low mantissa bits), 2^f on [-0.5, 0.5] by a polynomial of degree 5,
+// 2^n by adding n to the exponent field.  Least largest relative error among the polynomials with value 1 at 0 (found by reweighted
+// least squares), 1.6e-7 with fp32 rounding, against the 2^-22 = 2.4e-7 that ex2.approx is specified with; zero below 2^-126 like it.
 __device__ __forceinline__ void fma2(float& a, float& b, float c, float d, float e) {   // (a, b) = (a, b) * (c, d) + (e, e)
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmov.b64 z, {%4, %4};\n\t"
       "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
       : "+f"(a), "+f"(b) : "f"(c), "f"(d), "f"(e));
 }
-template <int DEGREE>
 __device__ __forceinline__ void ex2_poly2(float& y0, float& y1, float x0, float x1) {
-  x0 = fmaxf(x0, DEGREE == 4 ? -125.0f : -200.0f);
-  x1 = fmaxf(x1, DEGREE == 4 ? -125.0f : -200.0f);
+  x0 = fmaxf(x0, -200.0f);
+  x1 = fmaxf(x1, -200.0f);
   float t0, t1, n0, n1;
   sub2(t0, t1, x0, x1, 12582912.0f);              // t = x + 1.5 * 2^23
   sub2(n0, n1, t0, t1, -12582912.0f);             // n = round(x), as a float
-  float f0 = x0 - n0, f1 = x1 - n1;
-  float p0 = DEGREE == 4 ? 0.009278289f : 0.00132647285f, p1 = p0;
-  if (DEGREE == 4) {
-    fma2(p0, p1, f0, f1, 0.055865023f);
-    fma2(p0, p1, f0, f1, 0.240308955f);
-    fma2(p0, p1, f0, f1, 0.693129539f);
-    fma2(p0, p1, f0, f1, 0.999997854f);
-  } else {
-    fma2(p0, p1, f0, f1, 0.00967151299f);
-    fma2(p0, p1, f0, f1, 0.0555073358f);
-    fma2(p0, p1, f0, f1, 0.240222454f);
-    fma2(p0, p1, f0, f1, 0.693147004f);
-    fma2(p0, p1, f0, f1, 1.0f);
-  }
-  int i0 = __float_as_int(p0) + (__float_as_int(t0) << 23), i1 = __float_as_int(p1) + (__float_as_int(t1) << 23);
-  if (DEGREE != 4) { i0 = max(i0, 0); i1 = max(i1, 0); }      // an exponent below the smallest: the sign bit is set
-  y0 = __int_as_float(i0);
-  y1 = __int_as_float(i1);
+  const float f0 = x0 - n0, f1 = x1 - n1;
+  float p0 = 0.00132647285f, p1 = p0;
+  fma2(p0, p1, f0, f1, 0.00967151299f);
+  fma2(p0, p1, f0, f1, 0.0555073358f);
+  fma2(p0, p1, f0, f1, 0.240222454f);
+  fma2(p0, p1, f0, f1, 0.693147004f);
+  fma2(p0, p1, f0, f1, 1.0f);
+  // (an exponent below the smallest: the sign bit is set)
+  y0 = __int_as_float(max(__float_as_int(p0) + (__float_as_int(t0) << 23), 0));
+  y1 = __int_as_float(max(__float_as_int(p1) + (__float_as_int(t1) << 23), 0));
 }
+
+__host__ __device__ constexpr float exp2_of(int n) { return n < 0 ? 0.5f * exp2_of(n + 1) : n > 0 ? 2.0f * exp2_of(n - 1) : 1.0f; }
 
 // Bounded wait for a tagged word in shared memory: returns the word once its tag (bits 1..) equals `tag`, or -1 after
 // the limit (status set) or when another role has already recorded a failure.  The status word and the clock are looked
@@ -366,12 +365,12 @@ __device__ __forceinline__ int poll_tag(volatile int* word, int tag, int* status
   return poll_slow(word, tag, status);
 }
 
-// floor(d) - emax as an integer and as a float, without conversion instructions (which share the exponential's
+// floor(d) - emax, `least` at least, as an integer and as a float, without conversion instructions (which share the exponential's
 // pipe): d + 1.5 * 2^23 rounded DOWN holds floor(d) in its low mantissa bits (|d| < 2^22).
-__device__ __forceinline__ int block_shift(float d, int emax, float& sh_f) {
+__device__ __forceinline__ int block_shift(float d, int emax, int least, float& sh_f) {
   const float t = __fadd_rd(fmaxf(d, -1024.0f), 12582912.0f);
-  const int sh = max(__float_as_int(t) - 0x4b400000 - emax, -126);
-  sh_f = fmaxf(t - 12582912.0f - (float)emax, -126.0f);
+  const int sh = max(__float_as_int(t) - 0x4b400000 - emax, least);
+  sh_f = fmaxf(t - 12582912.0f - (float)emax, (float)least);
   return sh;
 }
 
@@ -391,13 +390,10 @@ __device__ __forceinline__ void store_row(void* dst, const uint32_t* w, bool wid
   }
 }
 
-// keys beyond `last` (an index into the 32 of this block) are masked
-__device__ __forceinline__ void mask32(uint32_t* sc, int last) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i)
-    if (i > last) sc[i] = 0xff800000u;                // -inf
+__device__ __forceinline__ void mul2(float& a, float& b, float s) {                // (a, b) *= (s, s)
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(a), "+f"(b) : "f"(s));
 }
-
 __device__ __forceinline__ void fma2s(float& a, float& b, float s, float t) {   // (a, b) = (a, b) * (s, s) + (t, t)
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmov.b64 z, {%3, %3};\n\t"
       "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
@@ -405,31 +401,36 @@ __device__ __forceinline__ void fma2s(float& a, float& b, float s, float t) {   
 }
 
 // One 32-key block of a query row for the quantised P.V: codes of P = exp2(S - m) in the tile's format and the block's E8M0
-// scale code - shared exponent floor(log2(amax P)) - emax = floor(bmax - m) - emax, folded into the exponent so that
-// exp2 delivers P / scale directly (power-of-two scaling is exact).  lsum accumulates the unrounded P (the reference sums
-// P before rounding it, ours/mxfp_attn_kernel.py:325).  A block without a visible key (bmax = -inf) comes out as zeros.
+// scale code - shared exponent floor(log2(amax P)) - emax = floor(bmax - m) - emax.  lsum accumulates the unrounded P (the reference
+// sums P before rounding it, ours/mxfp_attn_kernel.py:325).  A block without a visible key (bmax = -inf) comes out as zeros.
+//   LATE 1: the exponentials are taken of S as it is, and power-of-two scaling, which is exact, brings them into the block's range
+//           afterwards: they wait for S alone and not for the block's maximum too.  m = ATT_REF_Q enters the scale code only, and
+//           lsum lacks it.  (512 queries of 32K 175 -> 172 us, with more of them on the FMA pipe 164.)
+//   LATE 0: reference and block exponent are subtracted first.  NVFP4 launches, whose scores need a multiplication there anyway;
+//           routed ones, where the block's maximum is wanted early (routed causal 8K 393 us, LATE 407).
 //   PMODE 1 / 2: MXFP8 E5M2 / E4M3 (8 words); 3: MXFP4 (4 words)
-template <int PMODE, int NVF4>
-__device__ __forceinline__ uint32_t softmax_block_q(const uint32_t* sc, float mref, float bmax, [[maybe_unused]] float mul,
+template <int PMODE, int LATE, int NVF4>
+__device__ __forceinline__ uint32_t softmax_block_q(uint32_t* sc, [[maybe_unused]] float mref, float bmax, [[maybe_unused]] float mul,
                                                     uint32_t* pk, float& lsum0, float& lsum1) {
   constexpr int EMAX = (PMODE == 3) ? 2 : ((PMODE == 2) ? 8 : 7);
   constexpr int NW = (PMODE == 3) ? 4 : 8;
+  float* y = reinterpret_cast<float*>(sc);
   float sh_f;
-  const int sh = block_shift(bmax - mref, EMAX, sh_f);
-  const float ncb = -(mref + sh_f);               // exact: mref is integral in this mode
-  // Passes of independent instructions (the values are rewritten in place): all subtractions, then all exponentials
-  // back to back, then the sums and the packing.
-  float y[32];
+  const int sh = block_shift(LATE ? bmax : bmax - mref, EMAX, LATE ? (int)ATT_REF_Q - 126 : -126, sh_f);
+  // Passes of independent instructions (the values are rewritten in place)
+  if (!LATE) {
+    const float ncb = -(mref + sh_f);             // exact: mref is integral in this mode
 #pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    if (NVF4) { y[i] = __uint_as_float(sc[i]); y[i + 1] = __uint_as_float(sc[i + 1]); fma2s(y[i], y[i + 1], mul, ncb); }
-    else sub2(y[i], y[i + 1], __uint_as_float(sc[i]), __uint_as_float(sc[i + 1]), ncb);
+    for (int i = 0; i < 32; i += 2) {
+      if (NVF4) fma2s(y[i], y[i + 1], mul, ncb);
+      else sub2(y[i], y[i + 1], y[i], y[i + 1], ncb);
+    }
   }
-  constexpr int NPOLY = (PMODE == 3) ? ATT_POLY_FP4 : 0;
+  constexpr int NPOLY = (PMODE == 3) ? (LATE ? ATT_POLY_LATE : ATT_POLY_EARLY) : 0;
 #pragma unroll
   for (int i = 0; i < 32 - NPOLY; ++i) y[i] = ex2(y[i]);
 #pragma unroll
-  for (int i = 32 - NPOLY; i < 32; i += 2) ex2_poly2<4>(y[i], y[i + 1], y[i], y[i + 1]);
+  for (int i = 32 - NPOLY; i < 32; i += 2) ex2_poly2(y[i], y[i + 1], y[i], y[i + 1]);
   float a0 = 0.0f, a1 = 0.0f, b0 = 0.0f, b1 = 0.0f;
 #pragma unroll
   for (int i = 0; i < 32; i += 4) {
@@ -438,6 +439,17 @@ __device__ __forceinline__ uint32_t softmax_block_q(const uint32_t* sc, float mr
   }
   a0 += b0;
   a1 += b1;
+  if (LATE) {
+    const float down = __uint_as_float((uint32_t)(127 - sh) << 23);
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) mul2(y[i], y[i + 1], down);
+    lsum0 += a0;
+    lsum1 += a1;
+  } else {
+    const float two_sh = __uint_as_float((uint32_t)(sh + 127) << 23);
+    lsum0 = fmaf(a0, two_sh, lsum0);
+    lsum1 = fmaf(a1, two_sh, lsum1);
+  }
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
     constexpr int E = 32 / NW;                    // elements per word
@@ -445,10 +457,7 @@ __device__ __forceinline__ uint32_t softmax_block_q(const uint32_t* sc, float mr
                                         y[w * E + (E > 4 ? 6 : 2)], y[w * E + (E > 4 ? 7 : 3)]);
     else pk[w] = pack_fp8x4<PMODE == 2>(y[w * E], y[w * E + 1], y[w * E + 2], y[w * E + 3]);
   }
-  const float two_sh = __uint_as_float((uint32_t)(sh + 127) << 23);
-  lsum0 = fmaf(a0, two_sh, lsum0);
-  lsum1 = fmaf(a1, two_sh, lsum1);
-  return (uint32_t)(sh + 127);
+  return (uint32_t)(sh + (LATE ? 127 - (int)ATT_REF_Q : 127));
 }
 
 // The same for fp16 P, in two steps: y = exp2(S - m) in place for the elements FROM .. TO - 1 of a block, then 16 words of fp16
@@ -464,7 +473,7 @@ __device__ __forceinline__ void exp_block_f16(uint32_t* sc, float mref, [[maybe_
 #pragma unroll
   for (int i = FROM; i < TO; i += 2) {
     if (i < 32 - ATT_POLY_F16) { y[i] = ex2(y[i]); y[i + 1] = ex2(y[i + 1]); }
-    else ex2_poly2<5>(y[i], y[i + 1], y[i], y[i + 1]);
+    else ex2_poly2(y[i], y[i + 1], y[i], y[i + 1]);
   }
 }
 __device__ __forceinline__ void pack_block_f16(const uint32_t* sc, uint32_t* pk, float& lsum0, float& lsum1) {
@@ -490,7 +499,22 @@ static __device__ __noinline__ void scale_f32_columns(uint32_t taddr, int n, flo
   tmem_st_wait();
 }
 
-// The same for columns of fp16 pairs, 32 of them.
+// A warp's 64 columns of S: each lane's `shift` is subtracted, and keys beyond `last` (an index into the columns, by lane) become
+// -inf.  The few tiles that need it have their S rewritten before it is read, so that the loop over the tiles has no branch for
+// them (two in its body, never taken, cost 4 %: the instructions on the two sides of a branch are scheduled apart).
+static __device__ __noinline__ void adjust_scores(uint32_t taddr, int last, float shift) {
+  uint32_t r[32];
+  _Pragma("unroll 1") for (int c = 0; c < 64; c += 32) {
+    tmem_ld32p(taddr + c, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int k = 0; k < 32; ++k) r[k] = c + k > last ? 0xff800000u : __float_as_uint(__uint_as_float(r[k]) - shift);
+    tmem_st32p(taddr + c, r);
+  }
+  tmem_st_wait();
+}
+
+// As scale_f32_columns, for 32 columns of fp16 pairs.
 static __device__ __noinline__ void scale_f16_columns(uint32_t taddr, float f) {
   uint32_t r[32];
   tmem_ld32p(taddr, r);
@@ -538,17 +562,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   uint64_t* list_empty = list_full + ATT_MAX_SLOTS;   // [MAX_SLOTS] every reader is through with the item
   uint64_t* list_done = list_empty + ATT_MAX_SLOTS;   // [MAX_SLOTS] ROUTE: the router has been through the row, the list is final
   uint64_t* k_full = list_done + ATT_MAX_SLOTS;    // [KSTAGES]
-  uint64_t* k_empty = k_full + ATT_KSTAGES;        // [KSTAGES]
-  uint64_t* v_full = k_empty + ATT_KSTAGES;        // [VSLOTS_MAX]
-  uint64_t* v_empty = v_full + ATT_VSLOTS_MAX;     // [VSLOTS_MAX]
+  uint64_t* v_full = k_full + ATT_KSTAGES;         // [VSLOTS]
+  uint64_t* v_empty = v_full + ATT_VSLOTS;         // [VSLOTS] quantised P.V (fp16 P.V: pv_done says it)
   uint64_t* s_full = bars + ATT_B_SFULL;           // [2]
   uint64_t* s_free = s_full + 2;                   // [2] every owner has read the S buffer
   uint64_t* p_ready = s_free + 2;                  // [4] quantised P: tile t & 1; fp16 P: (tile t & 1, 64-key half)
   uint64_t* pv_done = p_ready + 4;                 // [4] likewise
   uint64_t* o_full = pv_done + 4;                  // the item's last P.V is done
   uint64_t* o_free = o_full + 1;                   // the epilogue has read O
-  uint64_t* st_bar = o_free + 1;                   // [2] ROUTE: the owners of the tile have published their slice maxima
-  uint64_t* x_bar = st_bar + 2;                    // [4] fp16 P.V: first-tile maxima of the two halves of a row
+  uint64_t* st_bar = o_free + 1;                   // [4] ROUTE, tile t & 3: its owners have published their slice maxima
+  uint64_t* x_bar = st_bar + 4;                    // [4] fp16 P.V: first-tile maxima of the two halves of a row
   uint64_t* m_bar = x_bar + 4;                     // [4] fp16 P.V: row references for the other warpgroup
   uint64_t* l_bar = m_bar + 4;                     // [4] partial sums and maxima of a row quarter
   uint64_t* r_bar = l_bar + 4;                     // [4 row quarters][tile & 1][half] fp16 P.V: this half tile has decided on the reference
@@ -556,29 +579,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 2);
   volatile int* dec = reinterpret_cast<volatile int*>(tmem_slot + 4);   // [4], slot tile & 3: (tile << 1 | keep) once the router has decided on the tile
   volatile Slot* slots = reinterpret_cast<volatile Slot*>(tmem_slot + 8);   // [MAX_SLOTS]
-  uint16_t* lists = reinterpret_cast<uint16_t*>(smem + ATT_OFF_LIST + (PVQ ? 0 : ATT_F16_BYTES));
+  uint16_t* lists = reinterpret_cast<uint16_t*>(smem + ATT_OFF_LIST + (PVQ && !ROUTE ? 0 : ATT_EXTRA_BYTES));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = (p.S + ATT_BM - 1) / ATT_BM, nk = (p.Skv + ATT_BN - 1) / ATT_BN;
   const int off = p.Skv - p.S;                      // queries are aligned to the end of the keys
   const int NL = p.n_lists;
-  constexpr int VSTAGES = PVQ ? 4 : 2;              // V ring depth, and the bytes of one slot
-  constexpr int VSLOT = PVQ ? ATT_V_BYTES / 2 : ATT_V_BYTES;
+  constexpr int VSTAGES = ATT_VSLOTS;               // V ring: a slot holds a quantised tile, or a 64-key half of an fp16 one
+  constexpr int VSLOT = ATT_V_BYTES / 2;
   constexpr int SF4 = NVF4 ? 1024 : 512;            // bytes of FP4 scales per 128 rows
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1);
       mbar_init(&s_full[s], 1); mbar_init(&s_free[s], 256);
-      mbar_init(&st_bar[s], 256);
     }
     for (int s = 0; s < ATT_MAX_SLOTS; ++s) { mbar_init(&list_full[s], 1); mbar_init(&list_empty[s], 3 + ATT_SM_WARPS); mbar_init(&list_done[s], 1); }
-    for (int s = 0; s < ATT_KSTAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
-    for (int s = 0; s < ATT_VSLOTS_MAX; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+    for (int s = 0; s < ATT_KSTAGES; ++s) mbar_init(&k_full[s], 1);
+    for (int s = 0; s < ATT_VSLOTS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
     for (int s = 0; s < 4; ++s) { mbar_init(&p_ready[s], PVQ ? 256 : 128); mbar_init(&pv_done[s], 1); }
     mbar_init(o_full, 1);
     mbar_init(o_free, 512);
-    for (int s = 0; s < 4; ++s) { mbar_init(&x_bar[s], 2); mbar_init(&m_bar[s], 1); mbar_init(&l_bar[s], 4); }
+    for (int s = 0; s < 4; ++s) { mbar_init(&x_bar[s], 2); mbar_init(&st_bar[s], 256); mbar_init(&m_bar[s], 1); mbar_init(&l_bar[s], 4); }
     for (int s = 0; s < 16; ++s) mbar_init(&r_bar[s], 1);
     for (int s = 0; s < 2; ++s) mbar_init(&drained[s], 1);
     fence_mbar_init();
@@ -597,13 +619,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   const int v_half_bytes = p.D * 128;               // one 64-key half of a V^T tile
 
   if (warp == 0) {
-    // ------------------------------ Q, K and V loads ---------------------------
+    // ------------------------------ Q and V loads ------------------------------
     if (elect_one()) {
-      tma_prefetch_desc(&tm_q8); tma_prefetch_desc(&tm_q4); tma_prefetch_desc(&tm_k8); tma_prefetch_desc(&tm_k4);
+      tma_prefetch_desc(&tm_q8); tma_prefetch_desc(&tm_q4);
       if (PVQ) { tma_prefetch_desc(&tm_vt8); tma_prefetch_desc(&tm_vt4); } else tma_prefetch_desc(&tm_vt);
       bool ok = true;
-      int sk = 0, sv = 0, tk = 0, tv = 0;           // ring slots; tiles requested so far on each ring (over all items)
-      uint32_t k_par = 1, v_par = 1;                // parity of the `empty` phase to wait for; a fresh barrier satisfies 1
+      int sv = 0, tv = 0;                           // ring slot; pieces requested so far (over all items)
+      uint32_t v_par = 1;                           // parity of the phase that frees the slot; a fresh barrier satisfies 1
       int q_loads = 0;
       auto load_q = [&](int slot) {                 // the slot's item, into set q_loads & 1
         const int qb = q_loads & 1;
@@ -625,6 +647,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         }
         ++q_loads;
       };
+      const uint32_t v_s0 = smem_u32(sV), vsf_s0 = smem_u32(sSFP + 2 * 512);
+      const uint32_t vf0 = smem_u32(v_full), ve0 = smem_u32(PVQ ? v_empty : pv_done);
       int ls = 0;
       uint32_t l_par = 0;                           // list slot and its phase parity
       _Pragma("unroll 1") for (int seq = 0; ok; ++seq) {
@@ -634,60 +658,46 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         if (!ok) break;
         const uint16_t* vl = lists + ls * p.list_cap;
         const int hk = slots[ls].b * p.Hkv + slots[ls].h / p.group;
-        const int k_row0 = hk * p.Skv;
-        const uint8_t* k8sf = p.k8_sf + (long long)hk * nk * 512;
-        const uint8_t* k4sf = p.k4_sf + (long long)hk * nk * SF4;
-        const long long vsf0 = (long long)hk * p.v_tiles * 512;
+        const uint8_t* v8sf = p.v8_sf + (long long)hk * p.v_tiles * 512;
+        const uint8_t* v4sf = p.v4_sf + (long long)hk * p.v_tiles * 512;
         const int v_row = hk * p.D;
-        auto issue_k = [&](uint32_t e) {
-          const int j = e & ENTRY_TILE;
-          const bool f8 = (e & ENTRY_F8) != 0;
-          ok = mbar_wait(&k_empty[sk], k_par, p.status, KS_TIMEOUT_PIPE);
-          if (!ok) return;
-          uint8_t* sf = smem + ATT_OFF_SFK + sk * 1024;
-          mbar_arrive_expect_tx(&k_full[sk], (f8 ? ATT_K_BYTES + 512 : ATT_K_BYTES / 2 + SF4));
-          tma_load_2d(sK + sk * ATT_K_BYTES, f8 ? &tm_k8 : &tm_k4, &k_full[sk], 0, k_row0 + j * ATT_BN);
-          if (f8) bulk_load(sf, k8sf + (long long)j * 512, 512, &k_full[sk]);
-          else bulk_load(sf, k4sf + (long long)j * SF4, SF4, &k_full[sk]);
-          ++tk;
-          if (++sk == ATT_KSTAGES) { sk = 0; k_par ^= 1; }
-        };
-        auto issue_v = [&](uint32_t e) {
-          const int j = e & ENTRY_TILE;
-          ok = mbar_wait(&v_empty[sv], v_par, p.status, KS_TIMEOUT_PIPE);
-          if (!ok) return;
-          if (PVQ == 0) {
-            mbar_arrive_expect_tx(&v_full[sv], 2 * v_half_bytes);
-            tma_load_2d(sV + sv * VSLOT, &tm_vt, &v_full[sv], j * ATT_BN, v_row);
-            tma_load_2d(sV + sv * VSLOT + v_half_bytes, &tm_vt, &v_full[sv], j * ATT_BN + 64, v_row);
-          } else {
-            // V^T tile in the tile's format: D rows of 128 (MXFP8) or 64 (MXFP4) bytes, and its scale tile
-            const bool f8 = (e & ENTRY_F8) != 0;
-            mbar_arrive_expect_tx(&v_full[sv], (f8 ? v_half_bytes : v_half_bytes / 2) + 512);
-            tma_load_2d(sV + sv * VSLOT, f8 ? &tm_vt8 : &tm_vt4, &v_full[sv], f8 ? j * ATT_BN : j * (ATT_BN / 2), v_row);
-            bulk_load(sSFP + (2 + sv) * 512, (f8 ? p.v8_sf : p.v4_sf) + vsf0 + (long long)j * 512, 512, &v_full[sv]);
-          }
-          ++tv;
-          if (++sv == VSTAGES) { sv = 0; v_par ^= 1; }
-        };
-        // K runs LEAD tiles ahead of V: the V ring is the shorter one (fp16 V^T: two slots) and must not hold K up
-        constexpr int LEAD = ATT_KSTAGES - 1;
-        int ik = 0, iv = 0;
+        const int ns = ls + 1 == NL ? 0 : ls + 1;
+        int iv = 0;
         _Pragma("unroll 1") for (int ph = 0; ph <= ROUTE && ok; ++ph) {
-          int hi;
-          if (ph == 0) {
-            hi = slots[ls].n_own;
-          } else {
-            // the next item's Q does not wait for what the router still has to decide on this one
-            const int ns = ls + 1 == NL ? 0 : ls + 1;
-            if (NL > 1 && mbar_test_wait(&list_full[ns], ns == 0 ? l_par ^ 1 : l_par) && slots[ns].mode >= 0) load_q(ns);
-            if (ok) ok = mbar_wait(&list_done[ls], l_par, p.status, KS_TIMEOUT_PIPE);
+          if (ph == 1) ok = mbar_wait(&list_done[ls], l_par, p.status, KS_TIMEOUT_PIPE);
+          if (!ok) break;
+          const int hi = ph == 0 ? slots[ls].n_own : slots[ls].n_total;
+          const int q_at = ph == 0 ? max(0, hi - 4) : -1;
+          uint32_t e = iv < hi ? vl[iv] : 0;
+          _Pragma("unroll 1") for (; iv < hi; ++iv) {
+            const uint32_t e_next = iv + 1 < hi ? vl[iv + 1] : 0;  // fetched a tile ahead of its use
+            // the next item's Q under this one's last tiles, where the item is known and the set free by then
+            if (iv == q_at && NL > 1 && q_loads == seq + 1 && mbar_test_wait(&list_full[ns], ns == 0 ? l_par ^ 1 : l_par) && slots[ns].mode >= 0 &&
+                mbar_test_wait(&q_empty[q_loads & 1], ((q_loads >> 1) & 1) ^ 1)) load_q(ns);
+            const int j = e & ENTRY_TILE;
+            if (PVQ == 0) {
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf) {      // 64-key halves; P.V of the half four before has to be done
+                if (ok) ok = mbar_wait_at(ve0 + sv * 8, v_par, p.status, KS_TIMEOUT_PIPE);
+                if (!ok) break;
+                mbar_arrive_expect_tx_at(vf0 + sv * 8, v_half_bytes);
+                tma_load_2d_at(v_s0 + sv * VSLOT, &tm_vt, vf0 + sv * 8, j * ATT_BN + 64 * hf, v_row);
+                ++tv;
+                if (++sv == VSTAGES) { sv = 0; v_par ^= 1; }
+              }
+            } else {
+              // V^T tile in the tile's format: D rows of 128 (MXFP8) or 64 (MXFP4) bytes, and its scale tile
+              ok = mbar_wait_at(ve0 + sv * 8, v_par, p.status, KS_TIMEOUT_PIPE);
+              if (!ok) break;
+              const bool f8 = (e & ENTRY_F8) != 0;
+              mbar_arrive_expect_tx_at(vf0 + sv * 8, (f8 ? v_half_bytes : v_half_bytes / 2) + 512);
+              tma_load_2d_at(v_s0 + sv * VSLOT, f8 ? &tm_vt8 : &tm_vt4, vf0 + sv * 8, f8 ? j * ATT_BN : j * (ATT_BN / 2), v_row);
+              bulk_load_at(vsf_s0 + sv * 512, (f8 ? v8sf : v4sf) + (long long)j * 512, 512, vf0 + sv * 8);
+              ++tv;
+              if (++sv == VSTAGES) { sv = 0; v_par ^= 1; }
+            }
             if (!ok) break;
-            hi = slots[ls].n_total;
-          }
-          _Pragma("unroll 1") while (ok && iv < hi) {
-            if (ik < hi && ik <= iv + LEAD) issue_k(vl[ik++]);
-            else issue_v(vl[iv++]);
+            e = e_next;
           }
         }
         if (!ok) break;
@@ -697,15 +707,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       if (!ok) {
         // unwind: copies in flight land before shared memory is released
         _Pragma("unroll 1") for (int u = max(0, q_loads - 2); u < q_loads; ++u) mbar_drain(&q_full[u & 1], (u >> 1) & 1);
-        _Pragma("unroll 1") for (int u = max(0, tk - ATT_KSTAGES); u < tk; ++u) mbar_drain(&k_full[u % ATT_KSTAGES], (u / ATT_KSTAGES) & 1);
         _Pragma("unroll 1") for (int u = max(0, tv - VSTAGES); u < tv; ++u) mbar_drain(&v_full[u % VSTAGES], (u / VSTAGES) & 1);
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ Q.K^T issuer ------------------------------
-    // S(t) goes to accumulator t & 1 as soon as its K tile has landed and the softmax threads have read S(t - 2).
-    // One thread issues; its loop holds nothing but the waits, the scale copies, the MMAs and two commits.
+    // ------------------------------ K loads and Q.K^T -------------------------
+    // S(t) goes to accumulator t & 1 as soon as its K tile has landed and the softmax threads have read S(t - 2).  The same
+    // thread requests the K tiles: when S(t - 2) has been read its MMAs are over, so the slot of tile t - 2 takes tile t + 2.
     if (elect_one()) {
+      tma_prefetch_desc(&tm_k8); tma_prefetch_desc(&tm_k4);
       uint32_t id8[4], id4[2];
 #pragma unroll
       for (int j = 0; j < 4; ++j) id8[j] = idesc_with_sf_id(idesc_block_scaled(p.fp8_fmt, p.fp8_fmt, ATT_BM, ATT_BN, 1), j, j);
@@ -718,27 +728,60 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       const uint32_t sfq8 = tmem + ATT_COL_SFQ8, sfq4 = tmem + ATT_COL_SFQ4;
       const bool half8 = p.qk_steps8 == 2, half4 = p.qk_steps4 == 1;
       bool ok = true;
-      int sk = 0, t = 0;                            // K ring slot; tile counter over all items
-      uint32_t k_par = 0, f_par = 1;                // phase parities: k_full[sk]; s_free[t & 1] (release of tile t - 2)
+      int t = 0;                                    // tile counter over all items: K ring slot t mod 4, S buffer t mod 2
+      const uint32_t sfree0 = smem_u32(s_free);
       int ls = 0;
       uint32_t l_par = 0;
+      // The request side, some tiles ahead: item (its slot and phase parity), position in its list (the end: its list is to be
+      // opened, or extended by the appended tiles, or left).
+      const uint32_t k_s0 = smem_u32(sK), ksf_s0 = smem_u32(smem + ATT_OFF_SFK), kf0 = smem_u32(k_full);
+      int rk = 0, rs = 0, ri = 0, r_hi = 0, r_row = 0, r_state = 0;      // r_state: 0 not open, 1 own tiles, 2 all of them
+      uint32_t rq_par = 0;
+      const uint8_t *r8sf = nullptr, *r4sf = nullptr;
+      // tile number rk; false: what comes next is not known yet (or there is nothing more).  May wait where the tile is needed now.
+      auto request_k = [&](bool wait) -> bool {
+        _Pragma("unroll 1") while (ri == r_hi) {
+          if (r_state == 0) {
+            if (wait) { ok = mbar_wait(&list_full[rs], rq_par, p.status, KS_TIMEOUT_PIPE); if (!ok) return false; }
+            else if (!mbar_test_wait(&list_full[rs], rq_par)) return false;
+            if (slots[rs].mode < 0) return false;
+            const int hk = slots[rs].b * p.Hkv + slots[rs].h / p.group;
+            r_row = hk * p.Skv;
+            r8sf = p.k8_sf + (long long)hk * nk * 512;
+            r4sf = p.k4_sf + (long long)hk * nk * SF4;
+            ri = 0;
+            r_hi = slots[rs].n_own;
+            r_state = ROUTE ? 1 : 2;
+          } else if (r_state == 1) {
+            if (wait) { ok = mbar_wait(&list_done[rs], rq_par, p.status, KS_TIMEOUT_PIPE); if (!ok) return false; }
+            else if (!mbar_test_wait(&list_done[rs], rq_par)) return false;
+            r_hi = slots[rs].n_total;
+            r_state = 2;
+          } else {
+            ri = r_hi = r_state = 0;
+            if (++rs == NL) { rs = 0; rq_par ^= 1; }
+          }
+        }
+        const uint32_t e = lists[rs * p.list_cap + ri++];
+        const int j = e & ENTRY_TILE, s = rk & (ATT_KSTAGES - 1);
+        const bool f8 = (e & ENTRY_F8) != 0;
+        const uint32_t bar = kf0 + s * 8, sf = ksf_s0 + s * 1024;
+        mbar_arrive_expect_tx_at(bar, f8 ? ATT_K_BYTES + 512 : ATT_K_BYTES / 2 + SF4);
+        tma_load_2d_at(k_s0 + s * ATT_K_BYTES, f8 ? &tm_k8 : &tm_k4, bar, 0, r_row + j * ATT_BN);
+        bulk_load_at(sf, f8 ? r8sf + j * 512u : r4sf + j * (uint32_t)SF4, f8 ? 512 : SF4, bar);
+        ++rk;
+        return true;
+      };
       _Pragma("unroll 1") for (int seq = 0; ok; ++seq) {
         const int qb = seq & 1;
         ok = mbar_wait(&list_full[ls], l_par, p.status, KS_TIMEOUT_PIPE);
         if (!ok || slots[ls].mode < 0) break;
-        ok = mbar_wait(&q_full[qb], (seq >> 1) & 1, p.status, KS_TIMEOUT_TMA);
-        // the Q scale columns are overwritten: the previous item's last Q.K^T has to be done with them
-        if (ok && t > 0) ok = mbar_wait(&s_full[(t - 1) & 1], ((t - 1) >> 1) & 1, p.status, KS_TIMEOUT_MMA);
-        if (!ok) break;
         const uint16_t* vl = lists + ls * p.list_cap;
         const uint64_t q8d = sdesc_kmajor_sw128(smem_u32(smem + ATT_OFF_Q + qb * ATT_Q_BYTES));
         const uint64_t q4d = sdesc_kmajor_sw64(smem_u32(smem + ATT_OFF_Q + qb * ATT_Q_BYTES + ATT_Q8_BYTES));
         const uint64_t sfq = sdesc_sf_tile(smem_u32(smem + ATT_OFF_SFQ + qb * 1536));
-        tc_fence_after();
-        tc_cp_32x128b_warpx4(sfq8, sfq);
-        tc_cp_32x128b_warpx4(sfq4, sfq + (512 >> 4));
-        if (NVF4) tc_cp_32x128b_warpx4(sfq4 + 4, sfq + (1024 >> 4));
         int i = 0;
+        bool q_there = false;
         _Pragma("unroll 1") for (int ph = 0; ph <= ROUTE && ok; ++ph) {
           int hi;
           if (ph == 0) {
@@ -748,53 +791,73 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
             if (!ok) break;
             hi = slots[ls].n_total;
           }
+          if (!ok) break;
           uint32_t e = i < hi ? vl[i] : 0;
-          _Pragma("unroll 1") for (; i < hi; ++i) {
-            const uint32_t e_next = i + 1 < hi ? vl[i + 1] : 0;    // fetched a tile ahead of its use
-            const int bsel = t & 1;
-            ok = mbar_wait(&s_free[bsel], f_par, p.status, KS_TIMEOUT_PIPE);
-            if (ok) ok = mbar_wait(&k_full[sk], k_par, p.status, KS_TIMEOUT_TMA);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t d = tmem + ATT_COL_S + bsel * 128;
-            const uint32_t sfk = tmem + ATT_COL_SFK + bsel * 8;
-            const uint64_t ksf = sfk0 + (uint64_t)(sk * (1024 >> 4));
-            tc_cp_32x128b_warpx4(sfk, ksf);
-            if (e & ENTRY_F8) {
-              const uint64_t kd = k8d0 + (uint64_t)(sk * (ATT_K_BYTES >> 4));
-              mma_mxf8f6f4(d, q8d, kd, id8[0], sfq8, sfk, 0);
-              mma_mxf8f6f4(d, q8d + 2, kd + 2, id8[1], sfq8, sfk, 1);
-              if (!half8) {
-                mma_mxf8f6f4(d, q8d + 4, kd + 4, id8[2], sfq8, sfk, 1);
-                mma_mxf8f6f4(d, q8d + 6, kd + 6, id8[3], sfq8, sfk, 1);
+          _Pragma("unroll 1") do {
+            if (i < hi && rk > t) {                 // (else its K has to be requested first)
+              if (!q_there) {                       // the item's first tile: K has been asked for before Q is waited for
+                ok = mbar_wait(&q_full[qb], (seq >> 1) & 1, p.status, KS_TIMEOUT_TMA);
+                // the Q scale columns are overwritten: the previous item's last Q.K^T has to be done with them
+                if (ok && t > 0) ok = mbar_wait(&s_full[(t - 1) & 1], ((t - 1) >> 1) & 1, p.status, KS_TIMEOUT_MMA);
+                if (!ok) break;
+                tc_fence_after();
+                tc_cp_32x128b_warpx4(sfq8, sfq);
+                tc_cp_32x128b_warpx4(sfq4, sfq + (512 >> 4));
+                if (NVF4) tc_cp_32x128b_warpx4(sfq4 + 4, sfq + (1024 >> 4));
+                q_there = true;
               }
-            } else {
-              const uint64_t kd = k4d0 + (uint64_t)(sk * (ATT_K_BYTES >> 4));
-              if (NVF4) {
-                mma_nvf4(d, q4d, kd, idn, sfq4, sfk, 0);
-                if (!half4) {
-                  tc_cp_32x128b_warpx4(sfk + 4, ksf + (512 >> 4));
-                  mma_nvf4(d, q4d + 2, kd + 2, idn, sfq4 + 4, sfk + 4, 1);
+              const uint32_t e_next = vl[min(i + 1, hi - 1)];      // fetched a tile ahead of its use
+              const int bsel = t & 1, sk = t & (ATT_KSTAGES - 1);
+              // (K first, so that only one wait lies between the release of S and the MMAs)
+              ok = mbar_wait_at(kf0 + sk * 8, (t >> 2) & 1, p.status, KS_TIMEOUT_TMA) &&
+                   mbar_wait_at(sfree0 + bsel * 8, ((t >> 1) & 1) ^ 1, p.status, KS_TIMEOUT_PIPE);
+              if (!ok) break;
+              tc_fence_after();
+              const uint32_t d = tmem + ATT_COL_S + bsel * 128;
+              const uint32_t sfk = tmem + ATT_COL_SFK + bsel * 8;
+              const uint64_t ksf = sfk0 + (uint32_t)(sk * (1024 >> 4));
+              tc_cp_32x128b_warpx4(sfk, ksf);
+              if (e & ENTRY_F8) {
+                const uint64_t kd = k8d0 + (uint32_t)(sk * (ATT_K_BYTES >> 4));
+                mma_mxf8f6f4(d, q8d, kd, id8[0], sfq8, sfk, 0);
+                mma_mxf8f6f4(d, q8d + 2, kd + 2, id8[1], sfq8, sfk, 1);
+                if (!half8) {
+                  mma_mxf8f6f4(d, q8d + 4, kd + 4, id8[2], sfq8, sfk, 1);
+                  mma_mxf8f6f4(d, q8d + 6, kd + 6, id8[3], sfq8, sfk, 1);
                 }
               } else {
-                mma_mxf4(d, q4d, kd, id4[0], sfq4, sfk, 0);
-                if (!half4) mma_mxf4(d, q4d + 2, kd + 2, id4[1], sfq4, sfk, 1);
+                const uint64_t kd = k4d0 + (uint32_t)(sk * (ATT_K_BYTES >> 4));
+                if (NVF4) {
+                  mma_nvf4(d, q4d, kd, idn, sfq4, sfk, 0);
+                  if (!half4) {
+                    tc_cp_32x128b_warpx4(sfk + 4, ksf + (512 >> 4));
+                    mma_nvf4(d, q4d + 2, kd + 2, idn, sfq4 + 4, sfk + 4, 1);
+                  }
+                } else {
+                  mma_mxf4(d, q4d, kd, id4[0], sfq4, sfk, 0);
+                  if (!half4) mma_mxf4(d, q4d + 2, kd + 2, id4[1], sfq4, sfk, 1);
+                }
               }
+              tc_commit(&s_full[bsel]);
+              ++i;
+              ++t;
+              e = e_next;
             }
-            tc_commit(&s_full[bsel]);
-            tc_commit(&k_empty[sk]);
-            if (++sk == ATT_KSTAGES) { sk = 0; k_par ^= 1; }
-            ++t;
-            if (!(t & 1)) f_par ^= 1;
-            e = e_next;
-          }
+            // S(t - 3) has been read, so the slot of tile t - 3 is free for tile t + 1 (at the start all slots are)
+            _Pragma("unroll 1") while (rk < max(t + 2, ATT_KSTAGES) && request_k(rk <= t && i < hi)) {}
+          } while (ok && i < hi);
         }
+        if (ok && !q_there) ok = mbar_wait(&q_full[qb], (seq >> 1) & 1, p.status, KS_TIMEOUT_TMA);    // (an item without tiles: its set is free once it has landed)
         if (!ok) break;
         tc_commit(&q_empty[qb]);
         mbar_arrive(&list_empty[ls]);
         if (++ls == NL) { ls = 0; l_par ^= 1; }
       }
-      if (!ok) { tc_commit(&drained[0]); mbar_drain(&drained[0], 0); }   // unwind: operands and accumulators are in use until then
+      if (!ok) {                                    // unwind: operands and accumulators are in use until then
+        tc_commit(&drained[0]);
+        mbar_drain(&drained[0], 0);
+        _Pragma("unroll 1") for (int u = max(0, rk - ATT_KSTAGES); u < rk; ++u) mbar_drain(&k_full[u % ATT_KSTAGES], (u / ATT_KSTAGES) & 1);
+      }
     }
   } else if (warp == 2) {
     // ------------------------------ P.V issuer --------------------------------
@@ -805,7 +868,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       const uint64_t vd0 = sdesc_kmajor_sw128(smem_u32(sV));        // + slot * (VSLOT >> 4)
       const uint64_t v4d0 = sdesc_kmajor_sw64(smem_u32(sV));        // MXFP4 V^T tile (64-byte rows)
       const uint64_t sfp0 = sdesc_sf_tile(smem_u32(sSFP));          // P scale tiles [2], then V scale tiles per stage
-      const uint32_t v_half16 = (uint32_t)v_half_bytes >> 4;
       const uint32_t idesc_pv = idesc_f16(0, 0, ATT_BM, p.D);
       uint32_t idp8[4], idp4[2];                                    // P.V block-scaled: M=128, N=D
 #pragma unroll
@@ -823,7 +885,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         ok = mbar_wait(o_free, (seq & 1) ^ 1, p.status, KS_TIMEOUT_PIPE);    // the previous item's O has been read
         if (!ok) break;
         const uint16_t* vl = lists + ls * p.list_cap;
-        const bool routing = ROUTE && slots[ls].mode == 0;
         uint32_t acc = 0;                           // 1 once an MMA has written O
         int i = 0;
         _Pragma("unroll 1") for (int ph = 0; ph <= ROUTE && ok; ++ph) {
@@ -838,36 +899,38 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           uint32_t e = i < hi ? vl[i] : 0;
           _Pragma("unroll 1") for (; i < hi; ++i) {
             const uint32_t e_next = i + 1 < hi ? vl[i + 1] : 0;
-            ok = mbar_wait(&v_full[sv], v_par, p.status, KS_TIMEOUT_TMA);
-            if (!ok) break;
             if (PVQ == 0) {
-              const uint64_t vd = vd0 + (uint64_t)(sv * (VSLOT >> 4));
 #pragma unroll
               for (int hf = 0; hf < 2; ++hf) {
-                ok = mbar_wait(&p_ready[(t & 1) * 2 + hf], r_par, p.status, KS_TIMEOUT_PIPE);
+                ok = mbar_wait(&v_full[sv], v_par, p.status, KS_TIMEOUT_TMA);
+                if (ok) ok = mbar_wait(&p_ready[(t & 1) * 2 + hf], r_par, p.status, KS_TIMEOUT_PIPE);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t ptm = tmem + ATT_COL_P16 + pb * 32;
-                const uint64_t vh = vd + (uint64_t)(hf * v_half16);
+                const uint64_t vh = vd0 + (uint64_t)(sv * (VSLOT >> 4));
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)      // 16 keys per instruction, 8 TMEM columns of P
                   mma_f16_ts(tmem + ATT_COL_O, ptm + ks * 8, vh + (uint64_t)(2 * ks), idesc_pv, (hf > 0 || ks > 0) ? 1u : acc);
-                tc_commit(&pv_done[(t & 1) * 2 + hf]);
+                tc_commit(&pv_done[(t & 1) * 2 + hf]);    // (frees the V slot too: slot and barrier both follow the half's number)
                 if (++pb == 3) pb = 0;
+                if (++sv == VSTAGES) { sv = 0; v_par ^= 1; }
               }
               if (!ok) break;
               acc = 1;
             } else {
+              ok = mbar_wait(&v_full[sv], v_par, p.status, KS_TIMEOUT_TMA);
+              if (!ok) break;
               const int bsel = t & 1;
+              ok = mbar_wait(&p_ready[bsel], r_par, p.status, KS_TIMEOUT_PIPE);
+              if (!ok) break;
               bool keep = true;
-              if (routing && !(e & ENTRY_F8)) {
-                // the router's word for this tile (it was written while P was being stored, as a rule)
+              if (ROUTE && !(e & ENTRY_F8)) {
+                // the router's word for this tile: written while P was being stored, as a rule (asked for first, this thread would
+                // poll for a third of its time)
                 const int d = poll_tag(&dec[t & 3], t, p.status);
                 if (d < 0) { ok = false; break; }
                 keep = (d & 1) != 0;
               }
-              ok = mbar_wait(&p_ready[bsel], r_par, p.status, KS_TIMEOUT_PIPE);
-              if (!ok) break;
               if (keep) {
                 tc_fence_after();
                 const uint32_t ptm = tmem + ATT_COL_P + bsel * 32;
@@ -888,10 +951,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
                 acc = 1;
               }
               tc_commit(&pv_done[bsel]);
+              tc_commit(&v_empty[sv]);
+              if (++sv == VSTAGES) { sv = 0; v_par ^= 1; }
             }
-            tc_commit(&v_empty[sv]);
             if (t & 1) r_par ^= 1;
-            if (++sv == VSTAGES) { sv = 0; v_par ^= 1; }
             ++t;
             e = e_next;
           }
@@ -1011,14 +1074,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     // Router: statistic of every MXFP4 tile = mean over the query rows of the row maximum.  Lane l takes rows l, 32 + l,
     // 64 + l, 96 + l of the published slice maxima; the four 32-row sums are formed by the same butterfly and added in the
     // same order as in route_stat_kernel / route_stat_finish_kernel, so the statistic is the same bit for bit.
-    [[maybe_unused]] uint32_t st_par0 = 0, st_par1 = 0;   // phase parity of st_bar[0], st_bar[1]
+    [[maybe_unused]] uint32_t st_par = 0;                 // phase parities of st_bar, as bits
     [[maybe_unused]] int t = 0;
     auto route = [&](int seq) {
       const int s = seq % NL;
       uint16_t* vl = lists + s * p.list_cap;
       const int nv = slots[s].n_own;
       int appended = 0;
-      if (slots[s].mode == 0) {
+      {
+        const bool decided = slots[s].mode != 0;    // done again: its list has the decisions of the first pass
         const int qi = slots[s].qi, h = slots[s].h, b = slots[s].b;
         const long long row_off = (long long)b * p.map_sb + (long long)h * p.map_sh + (long long)qi * nk;
         const float inv_rows = 1.0f / (float)min(ATT_BM, p.S - qi * ATT_BM);
@@ -1026,11 +1090,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         _Pragma("unroll 1") for (int i = 0; i < nv; ++i) {
           const uint32_t e = vl[i];
           if (e & ENTRY_F8) continue;               // MXFP8 by the band rule: nothing to decide
-          const int tt = t + i, bsel = tt & 1;
-          ok = __all_sync(0xffffffffu, mbar_wait(&st_bar[bsel], bsel ? st_par1 : st_par0, p.status, KS_TIMEOUT_PIPE));
-          if (bsel) st_par1 ^= 1; else st_par0 ^= 1;
+          const int tt = t + i, buf = tt & 3;
+          ok = __all_sync(0xffffffffu, mbar_wait(&st_bar[buf], (st_par >> buf) & 1, p.status, KS_TIMEOUT_PIPE));
+          st_par ^= 1u << buf;
           if (!ok) break;
-          const float* rm = reinterpret_cast<const float*>(smem + ATT_OFF_RMAX) + bsel * 2 * 128;
+          const float* rm = reinterpret_cast<const float*>(smem + ATT_OFF_EXTRA) + buf * 2 * 128;
           float pq[4];
 #pragma unroll
           for (int qq = 0; qq < 4; ++qq) {
@@ -1038,15 +1102,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
             const float mxr = fmaxf(rm[r], rm[128 + r]);
             pq[qq] = (qi * ATT_BM + r < p.S && mxr != -INFINITY) ? mxr * inv_rows : 0.0f;
           }
+          const bool up = (lane & 16) != 0, up8 = (lane & 8) != 0;
+          const float r0 = __shfl_xor_sync(0xffffffffu, up ? pq[0] : pq[2], 16), r1 = __shfl_xor_sync(0xffffffffu, up ? pq[1] : pq[3], 16);
+          const float u0 = (up ? pq[2] : pq[0]) + r0, u1 = (up ? pq[3] : pq[1]) + r1;
+          float w = (up8 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, up8 ? u0 : u1, 8);
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {        // four independent butterflies
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) pq[qq] += __shfl_xor_sync(0xffffffffu, pq[qq], o);
-          }
-          const float stat = ((pq[0] + pq[1]) + pq[2]) + pq[3];
+          for (int o = 4; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+          const float s0 = __shfl_sync(0xffffffffu, w, 0), s1 = __shfl_sync(0xffffffffu, w, 8), s2 = __shfl_sync(0xffffffffu, w, 16), s3 = __shfl_sync(0xffffffffu, w, 24);
+          const float stat = ((s0 + s1) + s2) + s3;
           const int j = e & ENTRY_TILE;
           if (j == 0) sink = stat;
-          const bool keep = !(stat >= sink * p.tau);
+          const bool keep = decided || !(stat >= sink * p.tau);
           if (lane == 0) {
             dec[tt & 3] = (tt << 1) | (keep ? 1 : 0);     // one word: readers poll it, nothing else to publish
             if (!keep) {
@@ -1054,7 +1120,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               p.map_rw[row_off + j] = TILE_FP8;
               vl[nv + appended] = (uint16_t)(e | ENTRY_F8);
             }
-            if (p.stat_out) p.stat_out[(((long long)b * p.Hq + h) * nq + qi) * nk + j] = stat;
+            if (p.stat_out && !decided) p.stat_out[(((long long)b * p.Hq + h) * nq + qi) * nk + j] = stat;
           }
           if (!keep) ++appended;
           __syncwarp();
@@ -1111,6 +1177,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     // P.V nor the warpgroup that had the last tile is waited for.  (Not with fp16 P.V: there a P buffer of the next
     // item's second tile is free only once O has been read.)
     constexpr bool DEFER = PVQ != 0;
+    constexpr bool LATE = PVQ && !NVF4 && !ROUTE;   // softmax_block_q; row sums lack the reference, an item done again has its S shifted first
+    [[maybe_unused]] bool again = false;            // the item is done again, with references of its own
     bool ok = true;
     int t0 = 0;                                     // tiles of the items before this one
     int pb16 = (2 * wg + g) % 3;                    // fp16 P.V: P buffer of the next tile's half
@@ -1123,24 +1191,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     // phase parities to wait for, as bits: 1 this warpgroup's tile count; fp16 P.V: 2 P.V of the half tile three before, 4 the half
     // tile before (turn and P.V)
     uint32_t par = PVQ ? 0 : ((g == 1 && wg == 1) ? 0u : 2u) | ((g == 0 && wg == 0) ? 4u : 0u);
-    float* lref = reinterpret_cast<float*>(smem + ATT_OFF_F16);
-    float* rmax_w = rmax + (wg * 2 + g) * 128 + r_in;
+    float* lref = reinterpret_cast<float*>(smem + ATT_OFF_EXTRA);
+    [[maybe_unused]] float* rmax_w = reinterpret_cast<float*>(smem + ATT_OFF_EXTRA) + (wg * 2 + g) * 128 + r_in;   // + 512 floats for tiles 2, 3 of 4
     float m_redo = 0.0f;                            // row reference of an item that is done again: the maximum its first pass found
     float mref = 0.0f, l_run = 0.0f, m_run = -INFINITY;   // row reference; partial row sum and maximum over this thread's keys
-    [[maybe_unused]] float pend_l = 0.0f;           // ROUTE: row sum of the last MXFP4 tile, until its decision is looked up
-    [[maybe_unused]] int pend_t = -1;
+    [[maybe_unused]] float pend_l = 0.0f;           // ROUTE: row sum of this warpgroup's last tile, if it was MXFP4, until the decision on it is looked up
+    [[maybe_unused]] int pend_t = 0;
     int ls = 0, seq = 0, n_tiles = 0, i = 0, lim = 0;
     uint32_t l_par = 0;
-    bool in_item = false, second = false, routing = false;   // second: ROUTE, the appended tiles
+    bool in_item = false, second = false;           // second: ROUTE, the appended tiles
     bool epi = false;                               // an epilogue is outstanding: item seq - 1, in slot epi_ls
     int epi_ls = 0, epi_part = 0;
     auto last_key = [&]() { return p.causal ? min(p.Skv - 1, slots[ls].qi * ATT_BM + r_in + off) : p.Skv - 1; };
-    auto settle = [&]() {
-      if (ROUTE && pend_t >= 0) {
+    auto settle = [&]() {                           // the last of the item's own tiles
+      if (pend_l != 0.0f) {
         const int d = poll_tag(&dec[pend_t & 3], pend_t, p.status);
         if (d < 0) ok = false;
-        else if (d & 1) l_run += pend_l;
-        pend_t = -1;
+        l_run += (d & 1) ? pend_l : 0.0f;
+        pend_l = 0.0f;
       }
     };
     _Pragma("unroll 1") while (ok) {
@@ -1156,12 +1224,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           i += 2;
           more = i < n_tiles && !epi;
           if (more) e = vl[i];
-          const int last = lim - ((int)(ec & ENTRY_TILE) * ATT_BN + g * 64);   // last visible key of the slice
           float lsum0 = 0.0f, lsum1 = 0.0f;
           uint32_t sc[32];
           ok &= mbar_wait_at(a_wg + ATT_B_SFULL * 8, par & 1, p.status, KS_TIMEOUT_MMA);
           __syncwarp();
           tc_fence_after();
+          if (__builtin_expect((ec & ENTRY_MASK) || (LATE && again), 0))
+            adjust_scores(slice_addr, ec & ENTRY_MASK ? lim - ((int)(ec & ENTRY_TILE) * ATT_BN + g * 64) : 64, LATE && again ? m_redo : 0.0f);
           tmem_ld32p(slice_addr, sc);
           if (PVQ) {
             uint32_t pk[16];
@@ -1171,27 +1240,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               constexpr int PW = PM == 3 ? 4 : 8;   // words of codes per block
               constexpr int NV = (NVF4 && PM == 3) ? 1 : 0;
               tmem_ld_wait();
-              if (ec & ENTRY_MASK) mask32(sc, last);
               const float b0 = NV ? block_max32(sc) * nvmul : block_max32(sc);
-              psc = softmax_block_q<PM, NV>(sc, mref, b0, nvmul, pk, lsum0, lsum1);
+              psc = softmax_block_q<PM, LATE, NV>(sc, mref, b0, nvmul, pk, lsum0, lsum1);
               tmem_ld32p(slice_addr + 32, sc);
               tmem_ld_wait();
               tc_fence_before();
               mbar_arrive_at(a_wg + ATT_B_SFREE * 8);   // S has been read: Q.K^T of tile t + 2 may overwrite it
-              if (ec & ENTRY_MASK) mask32(sc, last - 32);
-              const float b1 = NV ? block_max32(sc) * nvmul : block_max32(sc);
-              const float bm = fmaxf(b0, b1);
+              const bool p_free = mbar_test_wait_at(a_wg + ATT_B_PVDONE * 8, (par & 1) ^ 1);   // (its answer is used after the arithmetic)
+              const float b1 = NV ? block_max32(sc) * nvmul : block_max32(sc), bm = fmaxf(b0, b1);
               m_run = fmaxf(m_run, bm);
-              if (PM == 3 && routing) {             // published before the block's arithmetic, so that the router decides under it;
-                settle();                           // the previous tile of this warpgroup has been decided on, i.e. its maxima read
-                rmax_w[0] = bm;
-                mbar_arrive_at(a_wg + ATT_B_ST * 8);
+              if (ROUTE && PM == 3) {               // published before the block's arithmetic, so that the router decides under it
+                rmax_w[(par & 1) * 512] = bm;
+                mbar_arrive_at(a_wg + (ATT_B_ST + (par & 1) * 2) * 8);
               }
-              psc |= softmax_block_q<PM, NV>(sc, mref, b1, nvmul, pk + PW, lsum0, lsum1) << 8;
+              psc |= softmax_block_q<PM, LATE, NV>(sc, mref, b1, nvmul, pk + PW, lsum0, lsum1) << 8;
               // the P buffer and its scale tile: P.V of tile t - 2 has read them (a fresh barrier satisfies the first wait)
-              ok &= mbar_wait_at(a_wg + ATT_B_PVDONE * 8, (par & 1) ^ 1, p.status, KS_TIMEOUT_MMA);
+              if (!__all_sync(0xffffffffu, p_free)) ok &= mbar_wait_at(a_wg + ATT_B_PVDONE * 8, (par & 1) ^ 1, p.status, KS_TIMEOUT_MMA);
               __syncwarp();
               tc_fence_after();
+              // P.V of the tile before, which has been waited for, came after the decision on that tile: its share of the row sum
+              if (ROUTE) l_run += (dec[(t & 3) ^ 2] & 1) ? pend_l : 0.0f;
               if (PM == 3) tmem_st8p(p_addr + g * 8, pk);
               else tmem_st16p(p_addr + g * 16, pk);
             };
@@ -1207,13 +1275,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
             bool dead = false;
             _Pragma("unroll 1") while (true) {
               tmem_ld_wait();
-              if (ec & ENTRY_MASK) mask32(sc, last);
               m_run = fmaxf(m_run, block_max32(sc) * mul);
               exp_block_f16<NVF4, 0, 32>(sc, mref, mul);
-              pack_block_f16(sc, pk, lsum0, lsum1);
-              tmem_ld32p(slice_addr + 32, sc);
+              uint32_t sn[32];                      // (read before the first block is packed, whose arithmetic then fills the gaps of this one's)
+              tmem_ld32p(slice_addr + 32, sn);
               tmem_ld_wait();
-              if (ec & ENTRY_MASK) mask32(sc, last - 32);
+              pack_block_f16(sc, pk, lsum0, lsum1);
+#pragma unroll
+              for (int k = 0; k < 32; ++k) sc[k] = sn[k];
               m_run = fmaxf(m_run, block_max32(sc) * mul);      // (no earlier score goes beyond: it would have raised the reference)
               const bool stays = __all_sync(0xffffffffu, ok && !(m_run - mref > ATT_TOP_F16));
               exp_block_f16<NVF4, 0, ATT_F16_EARLY>(sc, mref, mul);    // (under the vote)
@@ -1279,9 +1348,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           tmem_st_wait();
           tc_fence_before();
           mbar_arrive_at(PVQ ? a_wg + ATT_B_PREADY * 8 : a_pr16);
-          if (routing && !(ec & ENTRY_F8)) {
-            pend_l = lsum0 + lsum1;                 // counts only if the router keeps the tile
+          if (ROUTE) {
+            pend_l = ec & ENTRY_F8 ? 0.0f : lsum0 + lsum1;     // counts only if the router keeps the tile
             pend_t = t;
+            if (ec & ENTRY_F8) l_run += lsum0 + lsum1;
           } else {
             l_run += lsum0 + lsum1;
           }
@@ -1303,7 +1373,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
           // the item's tiles are done: publish the partial results
           epi_part = (((t0 & 1) ^ wg) << 1) | g;    // the same order of summation whichever warpgroup owned the first tile
           float* xl = xrow + (seq & 1) * 1024 + epi_part * 128 + r_in;
-          xl[0] = l_run;
+          xl[0] = LATE ? l_run * exp2_of(-(int)ATT_REF_Q) : l_run;
           if (PVQ) {
             xl[512] = m_run;
           } else {
@@ -1339,7 +1409,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         } else {
           in_item = true;
           second = false;
-          routing = ROUTE && mode == 0;
+          again = mode == 1;
           n_tiles = slots[ls].n_own;
           const int m_glob = slots[ls].qi * ATT_BM + r_in;
           lim = last_key();                         // last visible key of this row
@@ -1360,14 +1430,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
               if (!ok) break;
               tc_fence_after();
               const uint32_t e = lists[ls * p.list_cap];
-              const int last = last_key() - ((int)(e & ENTRY_TILE) * ATT_BN + g * 64);
+              if (e & ENTRY_MASK) adjust_scores(slice_addr, lim - ((int)(e & ENTRY_TILE) * ATT_BN + g * 64), 0.0f);
               float mx = -INFINITY;
 #pragma unroll
               for (int c = 0; c < 2; ++c) {
                 uint32_t sc[32];
                 tmem_ld32p(slice_addr + c * 32, sc);
                 tmem_ld_wait();
-                if (e & ENTRY_MASK) mask32(sc, last - c * 32);
                 mx = fmaxf(mx, block_max32(sc));
               }
               rmax[g * 128 + r_in] = mx;
@@ -1429,7 +1498,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         // a share of an item: fp32 and the log2 denominator, into its slice of the partial results
         const int part = SPLIT ? slots[epi_ls].part : -1;
         const int item = (nq - 1 - slots[epi_ls].qi) * p.Hq * p.B + head;
-        const float ref = PVQ ? (mode == 1 ? m_redo : ATT_REF_Q) : ref_last;
+        const float ref = PVQ ? (mode == 1 ? m_redo + (LATE ? ATT_REF_Q : 0.0f) : ATT_REF_Q) : ref_last;
         const bool has_o = epi_part * 32 < p.D;     // this thread's 32 columns of O
         uint32_t o[32];
         if (tiles) {
@@ -1842,7 +1911,7 @@ int attn_forward(const AttnCall& call, cudaStream_t st) {
   p.n_items = (int)n_items; p.group = c.Hq / c.Hkv; p.counter = c.counter;
   p.out32 = (uintptr_t)c.out % 32 == 0; p.load8 = c.need8; p.load4 = c.need4;
   p.list_cap = ((c.route ? 2 * nk : nk) + 7) & ~7;
-  const int off_list = ATT_OFF_LIST + (c.pv_mode == 0 ? ATT_F16_BYTES : 0);
+  const int off_list = ATT_OFF_LIST + (c.pv_mode == 0 || c.route ? ATT_EXTRA_BYTES : 0);
   p.n_lists = std::min(ATT_MAX_SLOTS, (ATT_SMEM_MAX - 1024 - off_list) / (p.list_cap * 2));
   const size_t smem = off_list + (size_t)p.n_lists * p.list_cap * 2 + 1024;
   int parts = 0, n_whole = p.n_items, run_tiles = 1, pad = 0;
