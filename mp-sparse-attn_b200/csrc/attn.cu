@@ -117,14 +117,20 @@ constexpr float ATT_WIN_LO_Q = -64.0f, ATT_WIN_HI_Q = 64.0f;
 constexpr float ATT_TOP_F16 = 15.0f;                  // fp16 P.V: scores up to this far above the row reference need no new one (P at most 2^15)
 constexpr float ATT_NO_REF = -3e38f;                  // fp16 P.V: reference of a row that has seen no key yet
 
-// Division of the keys.  Items are numbered heaviest query tile first: item = r * heads + head, r counting query tiles
-// from the last.  The first n_whole are done by one CTA each; the tiles of the others, laid end to end, are cut into runs
+// Numbering of the items, r counting query tiles from the last.  Causal: heaviest query tile first, item = r * heads + head.
+// Otherwise all tiles weigh the same and one head comes after the other: the 148 items that run at a time then share the keys and
+// values of a few heads, which stay in L2 (32 heads of 8192 keys: 1.43 -> 0.14 GB from HBM for 0.1 GB of operands,
+// and under the power limit 1010 -> 883 us; NVFP4 video 17.7 -> 15.0 ms).
+// Division of the keys.  The first n_whole are done by one CTA each; the tiles of the others, laid end to end, are cut into runs
 // of run_tiles, one CTA each, so that a grid with fewer items than SMs, or with a last wave that is nearly empty, still
 // fills the chip.  An item that several runs share gets its result from attn_combine_kernel.
 struct SplitPlan {
   int heads, nq, nk, causal, c1;     // c1: visible tiles of query tile 0
   int n_whole, run_tiles;
   int pad;                           // 0, or the places every item takes: a multiple of run_tiles, so that no run holds two items
+  __host__ __device__ int item_of(int r, int head) const { return causal ? r * heads + head : head * nq + r; }
+  __host__ __device__ int row_of(int item) const { return causal ? item / heads : item % nq; }
+  __host__ __device__ int head_of(int item) const { return causal ? item % heads : item / nq; }
   __host__ __device__ long long row_tiles(int r) const { return !causal || r == 0 ? nk : nq - 1 - r + c1; }
   __host__ __device__ long long rows_before(int r) const {          // tiles of one head's rows 0 .. r-1
     if (!causal || r <= 1) return (long long)r * nk;
@@ -132,6 +138,7 @@ struct SplitPlan {
   }
   __host__ __device__ long long start(int item) const {             // tiles of all items before this one
     if (pad) return (long long)item * pad;
+    if (!causal) return (long long)item * nk;
     const int r = item / heads;
     return rows_before(r) * heads + (item - r * heads) * row_tiles(r);
   }
@@ -978,7 +985,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     [[maybe_unused]] int held_run[ATT_MAX_SLOTS], redo_run = 0;
     [[maybe_unused]] int run = 0;                   // this CTA's present run, from 1
     [[maybe_unused]] long long run_pos = 0, run_end = 0;
-    [[maybe_unused]] const SplitPlan plan = split_plan(heads, p.S, p.Skv, p.causal, p.n_whole, p.run_tiles, p.run_pad);
+    const SplitPlan plan = split_plan(heads, p.S, p.Skv, p.causal, p.n_whole, p.run_tiles, p.run_pad);
     [[maybe_unused]] const long long run_base = SPLIT ? plan.start(p.n_whole) : 0;
     auto reclaim = [&]() {
       const int s = reclaimed % NL;
@@ -1022,7 +1029,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         }
       }
       const int s = emitted % NL;
-      const int r = item / heads, bh = item - r * heads;
+      const int r = plan.row_of(item), bh = plan.head_of(item);
       const int qi = nq - 1 - r, b = bh / p.Hq, h = bh - b * p.Hq;
       // ordered compaction of the item's map row, 32 cells at a time; the map comes from memory, or from the band rule
       uint16_t* vl = lists + s * p.list_cap;
@@ -1497,7 +1504,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         const long long row = (long long)head * p.S + m_glob;
         // a share of an item: fp32 and the log2 denominator, into its slice of the partial results
         const int part = SPLIT ? slots[epi_ls].part : -1;
-        const int item = (nq - 1 - slots[epi_ls].qi) * p.Hq * p.B + head;
+        [[maybe_unused]] const int r = nq - 1 - slots[epi_ls].qi;
+        const int item = SPLIT ? (p.causal ? r * p.Hq * p.B + head : head * nq + r) : 0;
         const float ref = PVQ ? (mode == 1 ? m_redo + (LATE ? ATT_REF_Q : 0.0f) : ATT_REF_Q) : ref_last;
         const bool has_o = epi_part * 32 < p.D;     // this thread's 32 columns of O
         uint32_t o[32];
@@ -1638,7 +1646,7 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const float* part_o, 
   const int n_shared = n_items - s.n_whole, k = blockIdx.x, item = s.n_whole + k;
   const int r_in = blockIdx.y * 16 + (threadIdx.x >> 3), sub = threadIdx.x & 7;
   const long long base = s.start(s.n_whole), it0 = s.start(item) - base;
-  const int r = item / s.heads, m = (s.nq - 1 - r) * ATT_BM + r_in;
+  const int r = s.row_of(item), m = (s.nq - 1 - r) * ATT_BM + r_in;
   const int parts = (int)((it0 + s.row_tiles(r) - 1) / s.run_tiles - it0 / s.run_tiles) + 1;
   if (parts == 1 || m >= S) return;                 // (a single run has written the output itself)
   const long long stride = (long long)n_shared * ATT_BM, row0 = (long long)k * ATT_BM + r_in;
@@ -1664,7 +1672,7 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const float* part_o, 
     }
   }
   const float inv = den > 0.0f ? 1.0f / den : 0.0f;
-  const long long o = ((long long)(item - r * s.heads) * S + m) * D + sub * 4;
+  const long long o = ((long long)s.head_of(item) * S + m) * D + sub * 4;
 #pragma unroll
   for (int c = 0; c < W / 4; ++c) {
     const float x0 = acc[4 * c] * inv, x1 = acc[4 * c + 1] * inv, x2 = acc[4 * c + 2] * inv, x3 = acc[4 * c + 3] * inv;
