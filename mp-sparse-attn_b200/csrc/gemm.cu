@@ -216,6 +216,8 @@ gemm_block_scaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   cluster_sync();                                        // the peer's barriers are initialised
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dependency_wait();                                // the set-up above ran under the previous kernel on the stream
+  grid_dependents_go();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -464,7 +466,7 @@ int launch_gemm_shape(const GemmMaps& m, GemmParams& p, cudaStream_t st) {
   if (!allow_smem<MODE * 2 + (BN == 256)>(kernel, G::SMEM))
     return set_error(MPSA_ERR_LAUNCH, "gemm_block_scaled: cannot reserve %d bytes of shared memory", G::SMEM);
   const int pairs = std::min(p.n_tiles, std::max(1, sm_count() / 2));
-  kernel<<<2 * pairs, GEMM_THREADS, G::SMEM, st>>>(m.a, m.b, m.sfa, m.sfb, m.c, p);
+  launch_dependent(kernel, dim3(2 * pairs), GEMM_THREADS, G::SMEM, st, overlaps_previous(st), m.a, m.b, m.sfa, m.sfb, m.c, p);
   return check_launch("gemm_block_scaled");
 }
 }  // namespace

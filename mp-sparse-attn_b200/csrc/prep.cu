@@ -487,6 +487,7 @@ template <typename T, bool W8, bool W4, bool E4M3, bool D64>
 __global__ void __launch_bounds__(PREP_THREADS, W4 ? 3 : 4) prep_kernel(const __grid_constant__ PrepCall p) {
   extern __shared__ __align__(128) uint8_t prep_smem[];
   int cta = blockIdx.x;
+  if (!p.after_sums) grid_dependency_wait();            // (behind the column sums: where they are read)
   grid_dependents_go();
   if (cta == 0 && threadIdx.x < 2) {
     // words the launches behind this one expect to find zero
@@ -505,10 +506,11 @@ __global__ void __launch_bounds__(PREP_THREADS, W4 ? 3 : 4) prep_kernel(const __
 
 template <typename T>
 int launch_prep(const PrepCall& p, bool w8, bool w4, bool e4m3, int grid, size_t smem, cudaStream_t st) {
+  const bool dep = p.after_sums || overlaps_previous(st);
 #define MPSA_PREP(A, B, C)                                                                                                    \
   do {                                                                                                      \
-    if (p.D == 64) launch_dependent(prep_kernel<T, A, B, C, true>, dim3(grid), PREP_THREADS, smem, st, p.after_sums, p);  \
-    else launch_dependent(prep_kernel<T, A, B, C, false>, dim3(grid), PREP_THREADS, smem, st, p.after_sums, p);         \
+    if (p.D == 64) launch_dependent(prep_kernel<T, A, B, C, true>, dim3(grid), PREP_THREADS, smem, st, dep, p);  \
+    else launch_dependent(prep_kernel<T, A, B, C, false>, dim3(grid), PREP_THREADS, smem, st, dep, p);         \
   } while (0)
   if (w8 && w4) { if (e4m3) MPSA_PREP(true, true, true); else MPSA_PREP(true, true, false); }
   else if (w4) { if (e4m3) MPSA_PREP(false, true, true); else MPSA_PREP(false, true, false); }

@@ -683,6 +683,7 @@ col_sum_kernel(const T* x, float* part, int H, int L, int D, long long xs_b,
                long long xs_h, long long xs_l, int nchunk) {
   __shared__ float acc_s[16][128];
   __shared__ float sum_s[128];
+  grid_dependency_wait();
   grid_dependents_go();
   const int chunk = blockIdx.x, col0 = blockIdx.y * 128, bh = blockIdx.z;
   const int b = bh / H, h = bh % H;
@@ -861,9 +862,10 @@ extern "C" int mpsa_rope_quant_mx(const void* x, int in_dtype, int B, int H, int
 int mpsa::col_sums(const void* x, int in_dtype, int B, int H, int L, int D, long long xs_b, long long xs_h, long long xs_l,
                    float* part, int nchunk, cudaStream_t st) {
   const dim3 grid(nchunk * kSumCluster, (D + 127) / 128, B * H);
-  if (in_dtype == 0) col_sum_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
-  else if (in_dtype == 1) col_sum_kernel<__half><<<grid, 256, 0, st>>>((const __half*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
-  else col_sum_kernel<float><<<grid, 256, 0, st>>>((const float*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
+  const bool dep = overlaps_previous(st);
+  if (in_dtype == 0) launch_dependent(col_sum_kernel<__nv_bfloat16>, grid, 256, 0, st, dep, (const __nv_bfloat16*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
+  else if (in_dtype == 1) launch_dependent(col_sum_kernel<__half>, grid, 256, 0, st, dep, (const __half*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
+  else launch_dependent(col_sum_kernel<float>, grid, 256, 0, st, dep, (const float*)x, part, H, L, D, xs_b, xs_h, xs_l, nchunk);
   return check_launch("col_mean");
 }
 int mpsa::col_sum_chunks(int L) { return (L + kSumCluster * col_sum_rows(L) - 1) / (kSumCluster * col_sum_rows(L)); }
