@@ -1,4 +1,5 @@
-"""Build the C-ABI CUDA library in-tree: csrc/*.cu -> mpsa/libmpsa.so (sm_100a only).
+"""Build the C-ABI CUDA library in-tree: csrc/*.cu -> mpsa/libmpsa.so (sm_100a only), and the Python module in front of its short
+calls: csrc/native.cpp -> mpsa/_native.so.
 
     python mp-sparse-attn_b200/build.py [--force]
 
@@ -13,6 +14,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "mpsa", "libmpsa.so")
+NATIVE_SRC, NATIVE_OUT = os.path.join(CSRC, "native.cpp"), os.path.join(HERE, "mpsa", "_native.so")
 SOURCES = ["api.cu", "quant.cu", "prep.cu", "gemm.cu", "attn.cu", "route.cu", "attention.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=default", "--use_fast_math=false"]
@@ -30,7 +32,7 @@ def needs_build():
         return True
     t = os.path.getmtime(OUT)
     for f in os.listdir(CSRC):
-        if os.path.getmtime(os.path.join(CSRC, f)) > t:
+        if f != "native.cpp" and os.path.getmtime(os.path.join(CSRC, f)) > t:
             return True
     return os.path.getmtime(__file__) > t
 
@@ -63,5 +65,28 @@ def build_lib(force=False, verbose=False):
     return OUT
 
 
+def build_native(force=False):
+    """csrc/native.cpp -> mpsa/_native.so, the module that takes torch tensors to the library (needs torch's headers)."""
+    header = os.path.join(os.path.dirname(HERE), "include", "mpsa.h")
+    if not force and os.path.exists(NATIVE_OUT) and \
+            os.path.getmtime(NATIVE_OUT) >= max(os.path.getmtime(f) for f in (NATIVE_SRC, header, __file__)):
+        return NATIVE_OUT
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    inc = [sysconfig.get_paths()["include"], os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+           os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + i for i in inc), NATIVE_SRC, "-o", NATIVE_OUT + ".new",
+           "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on native.cpp:\n{r.stdout}")
+    os.replace(NATIVE_OUT + ".new", NATIVE_OUT)
+    return NATIVE_OUT
+
+
 if __name__ == "__main__":
+    print(build_native("--force" in sys.argv))
     print(build_lib(force="--force" in sys.argv, verbose="-v" in sys.argv))

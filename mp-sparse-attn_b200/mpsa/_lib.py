@@ -91,6 +91,35 @@ def load():
     return lib
 
 
+_native = None
+
+
+def native():
+    """The module that takes torch tensors to the library's short calls (csrc/native.cpp), built first if necessary."""
+    global _native
+    if _native is not None:
+        return _native
+    import importlib.util
+
+    import torch                                 # (the module's symbols are in torch's libraries)
+    lib = load()
+    path = os.path.join(_HERE, "_native.so")
+    if not os.path.exists(path):
+        sys.path.insert(0, os.path.dirname(_HERE))
+        try:
+            import build as _build
+            _build.build_native()
+        finally:
+            sys.path.pop(0)
+    spec = importlib.util.spec_from_file_location("mpsa._native", path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.init(*(ctypes.cast(getattr(lib, f), c_void_p).value for f in
+               ("mpsa_attention_workspace", "mpsa_attention", "mpsa_quant_pair", "mpsa_gemm_block_scaled")), torch.OutOfMemoryError)
+    _native = mod
+    return mod
+
+
 def last_error():
     buf = ctypes.create_string_buffer(512)
     load().mpsa_last_error(buf, 512)

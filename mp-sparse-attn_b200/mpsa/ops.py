@@ -3,7 +3,6 @@ arithmetic runs in the hand-written sm_100a kernels of libmpsa.so."""
 from __future__ import annotations
 
 import ctypes
-import struct
 import threading
 from dataclasses import dataclass
 from typing import Optional
@@ -224,47 +223,19 @@ def quantize_mx(x: torch.Tensor, scale: float = 1.0, *, want_fp8=True, want_fp4=
     return out
 
 
-_QUANT_PAIR_ARGS = struct.Struct("@2Q2Q2Q2q2q2q2q2q2q2i2i2f4i")     # mpsa_quant_pair_args of include/mpsa.h
-
-
 _PAIR_DTYPE = {"mxfp4": torch.uint8, "e5m2": torch.float8_e5m2, "e4m3": torch.float8_e4m3fn}
-
-
-def _empty(shape, strides, dtype, device):
-    """torch.empty at half its host time (1.3 against 2.5 us): the strides are at hand."""
-    return torch.empty_strided(shape, strides, dtype=dtype, device=device)
 
 
 def quantize_pair(q: torch.Tensor, k: torch.Tensor, sq: float, sk: float, fmt: str, tensor_layout: str = "HND"):
     """q and k quantised along the depth in the reference's output format: (codes, scales) of each.  fmt "mxfp4" (one code per
     byte, uint8), "e5m2" or "e4m3" (codes as that torch type).  One launch where the operands allow it (16 bits, aligned, depth 64 or a multiple of 128)."""
+    if fmt in _PAIR_DTYPE and tensor_layout in ("HND", "NHD"):
+        r = _lib.native().quant_pair(q, k, sq, sk, 0 if fmt == "mxfp4" else _FP8_QUANT[fmt], tensor_layout == "HND")
+        if r.__class__ is tuple:
+            return r
+        if r is not None:
+            _lib.check(r)
     _require_cuda(q, k)
-    dt = q.dtype
-    in_dtype = 0 if dt is torch.bfloat16 else 1 if dt is torch.float16 else None
-    if in_dtype is not None and k.dtype is dt and q.dim() == 4 and k.dim() == 4 and q.shape[0] == k.shape[0] and \
-            q.shape[3] == k.shape[3] and q.get_device() == k.get_device() and (q.shape[3] == 64 or q.shape[3] % 128 == 0) and \
-            sq > 0.0 and sk > 0.0 and tensor_layout in ("HND", "NHD"):
-        qs, ks = _strides16(q), _strides16(k)
-        if qs is not None and ks is not None:
-            hnd = tensor_layout == "HND"
-            B, a1, a2, D = q.shape
-            _, b1, b2, _ = k.shape
-            (Hq, Lq), (Hk, Lk) = ((a1, a2), (b1, b2)) if hnd else ((a2, a1), (b2, b1))
-            dev, nb, ct = q.device, D // 32, _PAIR_DTYPE[fmt]
-            qc, kc = _empty((B, a1, a2, D), (a1 * a2 * D, a2 * D, D, 1), ct, dev), _empty((B, b1, b2, D), (b1 * b2 * D, b2 * D, D, 1), ct, dev)
-            qsc = _empty((B, Hq, Lq, nb), (Hq * Lq * nb, Lq * nb, nb, 1), torch.uint8, dev)
-            ksc = _empty((B, Hk, Lk, nb), (Hk * Lk * nb, Lk * nb, nb, 1), torch.uint8, dev)
-            if not hnd:
-                qs, ks = (qs[0], qs[2], qs[1]), (ks[0], ks[2], ks[1])
-            cq = (Hq * Lq * D, Lq * D, D) if hnd else (Hq * Lq * D, D, Hq * D)
-            ck = (Hk * Lk * D, Lk * D, D) if hnd else (Hk * Lk * D, D, Hk * D)
-            args = _QUANT_PAIR_ARGS.pack(q.data_ptr(), k.data_ptr(), qc.data_ptr(), kc.data_ptr(), qsc.data_ptr(), ksc.data_ptr(),
-                                         qs[0], ks[0], qs[1], ks[1], qs[2], ks[2], cq[0], ck[0], cq[1], ck[1], cq[2], ck[2],
-                                         Hq, Hk, Lq, Lk, sq, sk, in_dtype, B, D, 0 if fmt == "mxfp4" else _FP8_QUANT[fmt])
-            rc = _on_device(q.get_device(), _lib.load().mpsa_quant_pair, args)
-            if rc:
-                _lib.check(rc)
-            return qc, qsc, kc, ksc
     fp4 = fmt == "mxfp4"
     out = []
     for x, s in ((q, sq), (k, sk)):
@@ -483,86 +454,40 @@ def prepare_kv(k: torch.Tensor, v: torch.Tensor, *, pv_mode: str = "fp16", fp8_e
     return kq, vt
 
 
-_ATTENTION_ARGS = struct.Struct("@3Q9q9Q2Qq2Q17i2f")       # mpsa_attention_args of include/mpsa.h
-_workspace_bytes = {}                                        # problem -> workspace size (bounded)
 _UNIFORM = {None: 0, "fp8": 1, "fp4": 2}
-
-
-def _strides16(t):
-    """Strides of a 4-D 16-bit tensor if the one-call path can read it as it is, else None."""
-    a, b, c, d = t.stride()
-    if d != 1 or (a | b | c) & 7 or t.data_ptr() & 15:
-        return None
-    return a, b, c
 
 
 def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out_dtype, pv_mode, route, tau, smooth_k,
                         nvfp4, want_flag):
     """attention_forward through one C call (mpsa_attention), or None where that entry does not take the operands.
     want_flag: keep a range flag of this call's own (quantised P.V)."""
-    dt = q.dtype
-    in_dtype = 0 if dt is torch.bfloat16 else 1 if dt is torch.float16 else None
-    qs = _strides16(q)
-    if in_dtype is None or qs is None or uniform not in _UNIFORM or out_dtype not in (torch.float32, torch.float16, torch.bfloat16) \
-            or fp8_elem not in _FP8_DESC or not sq > 0.0:
+    if uniform not in _UNIFORM or out_dtype not in (torch.float32, torch.float16, torch.bfloat16) or fp8_elem not in _FP8_DESC or not sq > 0.0:
         return None
-    B, Hq, S, D = q.shape
     index = q.get_device()
     uni = _UNIFORM[uniform]
-    skv_pad = 0
-    if kv is None:
-        if k.dtype is not dt or v.dtype is not dt or k.shape != v.shape or k.shape[0] != B or k.shape[3] != D or \
-                k.get_device() != index or v.get_device() != index:
-            return None
-        _, Hkv, Skv, _ = k.shape
-        ks, vs = _strides16(k), _strides16(v)
-        if ks is None or vs is None:
-            return None
-        kp, vp = k.data_ptr(), v.data_ptr()
-        prepared = (0,) * 9
-    else:
+    prepared = None
+    if kv is not None:
         kq, vt = kv
         codes = kq.fp8 if kq.fp8 is not None else kq.fp4
         Hkv, Skv = codes.shape[1], codes.shape[2]
         requant = isinstance(vt, QuantizedV)
         pv_mode = "requant" if requant else "fp16"
         skv_pad = (vt.vt8 if requant else vt).shape[-1]
-        if codes.get_device() != index or not _prepared_fits(kq, vt, requant, B, Hkv, Skv, D, skv_pad, uni, fp8_elem):
+        if codes.get_device() != index or not _prepared_fits(kq, vt, requant, q.shape[0], Hkv, Skv, q.shape[3], skv_pad, uni, fp8_elem):
             return None
-        ks = vs = (0, 0, 0)
-        kp = vp = 0
-        prepared = (_ptr(kq.fp8) or 0, _ptr(kq.fp8_sf) or 0, _ptr(kq.fp4) or 0, _ptr(kq.fp4_sf) or 0) + (
+        k = v = None
+        prepared = (Hkv, Skv, skv_pad, _ptr(kq.fp8) or 0, _ptr(kq.fp8_sf) or 0, _ptr(kq.fp4) or 0, _ptr(kq.fp4_sf) or 0) + (
             (0, vt.vt8.data_ptr(), vt.v8_sf.data_ptr(), vt.vt4.data_ptr(), vt.v4_sf.data_ptr()) if requant
             else (vt.data_ptr(), 0, 0, 0, 0))
-    if Hq % Hkv or (causal and Skv < S):
-        return None
     st = _state(index)
     if st.word.value:
         _raise_if_failed(q.device)
-    pv = 1 if pv_mode == "requant" else 0
-    ints = (in_dtype, _OUT_DTYPE[out_dtype], B, Hq, Hkv, S, Skv, D, skv_pad, int(causal), band, uni, int(route), pv,
-            _FP8_DESC[fp8_elem], int(smooth_k), int(nvfp4))
-    lib = _lib.load()
-    key = (ints, kp == 0, index)                   # the size depends on the number of SMs too
-    need = _workspace_bytes.get(key)
-    if need is None:
-        with torch.cuda.device(index):
-            need = lib.mpsa_attention_workspace(_ATTENTION_ARGS.pack(1, int(kp != 0), int(vp != 0), *qs, *ks, *vs, *prepared, 0, 0, 0, 0, 0,
-                                                                    *ints, sq, tau))
-        if need < 0:
-            _lib.check(need)
-        if len(_workspace_bytes) >= 1024:
-            _workspace_bytes.clear()
-        _workspace_bytes[key] = need
-    dev = q.device
-    ws = _empty((need,), (1,), torch.uint8, dev)
-    out = _empty((B, Hq, S, D), (Hq * S * D, S * D, D, 1), out_dtype, dev)
-    flag = _last.range_flag = _empty((1,), (1,), torch.int32, dev) if want_flag and pv else None
-    args = _ATTENTION_ARGS.pack(q.data_ptr(), kp, vp, *qs, *ks, *vs, *prepared, out.data_ptr(), ws.data_ptr(), need, _ptr(flag) or 0,
-                                st.status_ptr, *ints, sq, tau)
-    rc = _on_device(index, lib.mpsa_attention, args)
-    if rc:
-        _lib.check(rc)
+    pv = pv_mode == "requant"
+    flag = _last.range_flag = torch.empty(1, dtype=torch.int32, device=q.device) if want_flag and pv else None
+    out = _lib.native().attention(q, k, v, prepared, flag, st.status_ptr, _OUT_DTYPE[out_dtype], int(causal), band, uni, route, pv,
+                                  _FP8_DESC[fp8_elem], smooth_k, nvfp4, sq, tau)
+    if out.__class__ is int:
+        _lib.check(out)
     return out
 
 
@@ -986,28 +911,38 @@ def gemm_block_scaled(a: torch.Tensor, a_scale: torch.Tensor, b: torch.Tensor, b
                       alpha: float = 1.0, check: bool = False) -> torch.Tensor:
     """C[M,N] = alpha * (A.sa)(B.sb)^T.  a [M,K/epb] / b [N,K/epb] bytes (uint8 or float8), scales as 128x4
     tiles [rows/128, K/vec/4, 32,4,4] (uint8 E8M0, or E4M3 bytes for nvfp4)."""
-    _require_cuda(a, b, a_scale, b_scale)
+    if not (a.is_cuda and b.is_cuda and a_scale.is_cuda and b_scale.is_cuda):
+        _require_cuda(a, b, a_scale, b_scale)
     if mode not in _GEMM_MODE:
         raise ValueError(f"Invalid block scale type: {mode}")
     if out_dtype not in _OUT_DTYPE:
         raise ValueError(f"Unsupported dtype: {out_dtype}")
+    index = a.get_device()
+    st = _state(index)
+    if st.word.value:
+        _raise_if_failed(a.device)
+    c = _lib.native().gemm(a, a_scale, b, b_scale, M, N, K, _GEMM_MODE[mode], _FP8_DESC[a_elem], _FP8_DESC[b_elem], _OUT_DTYPE[out_dtype],
+                           alpha, st.status_ptr)
+    if c is None:
+        c = _gemm_any(a, a_scale, b, b_scale, out_dtype, M, N, K, mode, a_elem, b_elem, alpha, index, st)
+    elif c.__class__ is int:
+        _lib.check(c)
+    if check:
+        check_status(a.device)
+    return c
+
+
+def _gemm_any(a, a_scale, b, b_scale, out_dtype, M, N, K, mode, a_elem, b_elem, alpha, index, st):
+    """gemm_block_scaled on operands that native.cpp does not take as they are."""
     if a.stride(-1) != 1:
         a = a.contiguous()
     if b.stride(-1) != 1:
         b = b.contiguous()
     a_scale, b_scale = a_scale.contiguous(), b_scale.contiguous()
-    c = _empty((M, N), (N, 1), out_dtype, a.device)
-    index = a.get_device()
-    st = _state(index)
-    if st.word.value:
-        _raise_if_failed(a.device)
-    rc = _on_device(index, _lib.load().mpsa_gemm_block_scaled, a.data_ptr(), a_scale.data_ptr(), b.data_ptr(), b_scale.data_ptr(),
-                    c.data_ptr(), M, N, K, a.stride(0) * a.element_size(), b.stride(0) * b.element_size(), N, _GEMM_MODE[mode],
-                    _FP8_DESC[a_elem], _FP8_DESC[b_elem], _OUT_DTYPE[out_dtype], float(alpha), st.status_ptr)
-    if rc:
-        _lib.check(rc)
-    if check:
-        check_status(a.device)
+    c = torch.empty((M, N), dtype=out_dtype, device=a.device)
+    _lib.check(_on_device(index, _lib.load().mpsa_gemm_block_scaled, a.data_ptr(), a_scale.data_ptr(), b.data_ptr(), b_scale.data_ptr(),
+                          c.data_ptr(), M, N, K, a.stride(0) * a.element_size(), b.stride(0) * b.element_size(), N, _GEMM_MODE[mode],
+                          _FP8_DESC[a_elem], _FP8_DESC[b_elem], _OUT_DTYPE[out_dtype], float(alpha), st.status_ptr))
     return c
 
 

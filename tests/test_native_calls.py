@@ -1,0 +1,76 @@
+"""The module in front of the library's short calls (csrc/native.cpp): what it takes, what it leaves to the long way, what it refuses."""
+import pytest
+import torch
+
+
+def test_host_tensors_and_wrong_calls_are_left_alone():
+    from mpsa import _lib
+    n = _lib.native()
+    x = torch.zeros(1, 2, 128, 128, dtype=torch.bfloat16)
+    assert n.quant_pair(x, x, 1.0, 1.0, 0, True) is None
+    assert n.attention(x, x, x, None, None, 0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 1.0, 1.0) is None
+    assert n.gemm(x, x, x, x, 1, 1, 1, 0, 0, 0, 0, 1.0, 0) is None
+    for f in (n.quant_pair, n.attention, n.gemm):
+        with pytest.raises(TypeError):
+            f(x)
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+def _forms(D):
+    """(name, tensor [2, 3, 130, D], taken): views of every kind over one set of values."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x = torch.randn(2, 3, 130, D, generator=g, device="cuda", dtype=torch.bfloat16)
+    flat = torch.zeros(x.numel() + 8, device="cuda", dtype=x.dtype)
+    wide = torch.zeros(2, 3, 130, D + 8, device="cuda", dtype=x.dtype)
+    odd = torch.zeros(2, 3, 130, D + 4, device="cuda", dtype=x.dtype)
+    dense = flat[:x.numel()].view_as(x)
+    shifted = flat.clone()[1:x.numel() + 1].view_as(x)
+    forms = [("dense", dense, True), ("tokens first", x.transpose(1, 2).contiguous().transpose(1, 2), True), ("padded rows", wide[..., :D], True),
+             ("rows of an odd pitch", odd[..., :D], False), ("base off by one", shifted, False),
+             ("depth strided", torch.zeros(2, 3, 130, 2 * D, device="cuda", dtype=x.dtype)[..., ::2], False),
+             ("expanded heads", x[:, :1].expand(2, 3, 130, D), True), ("subclass", x.clone().as_subclass(_Sub), False), ("fp32", x.float(), False)]
+    for name, t, taken in forms:
+        if name not in ("expanded heads",):
+            with torch.no_grad():
+                t.copy_(x)
+        yield name, t, taken
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [64, 128])
+def test_every_form_gives_what_the_long_way_gives(D):
+    import mpsa
+    from mpsa import _lib, ops
+    for name, t, taken in _forms(D):
+        direct = _lib.native().quant_pair(t, t, 0.5, 1.0, 1, True)
+        assert (direct is not None) == taken, name
+        if name in ("rows of an odd pitch", "base off by one"):       # refused by the long way too
+            with pytest.raises(ValueError):
+                ops.quantize_pair(t, t, 0.5, 1.0, "e5m2")
+            continue
+        qc, qs, kc, ks = ops.quantize_pair(t, t, 0.5, 1.0, "e5m2")
+        for codes, scales, s in ((qc, qs, 0.5), (kc, ks, 1.0)):
+            ref = ops.quantize_mx(t, s, want_fp4=False, reference_format=True, kernel_format=False)
+            assert torch.equal(codes.view(torch.uint8), ref.fp8) and torch.equal(scales, ref.fp8_scales), name
+        out = mpsa.attention_forward(t, t, t, causal=True, out_dtype=torch.float32)
+        dense = mpsa.attention_forward(t.detach().clone().contiguous(), t.contiguous(), t.contiguous(), causal=True, out_dtype=torch.float32)
+        assert torch.equal(out, dense) if taken else float((out - dense).abs().max()) < 1e-2, name
+
+
+@pytest.mark.gpu
+def test_what_was_refused_stays_refused():
+    import mpsa
+    from mpsa import ops
+    e = torch.zeros(1, 2, 0, 128, device="cuda", dtype=torch.bfloat16)
+    x = torch.zeros(1, 2, 128, 128, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(ValueError):
+        mpsa.attention_forward(e, x, x, causal=False)
+    with pytest.raises(ValueError):
+        ops.quantize_pair(e, x, 1.0, 1.0, "mxfp4")
+    with pytest.raises(ValueError):
+        mpsa.attention_forward(x.cpu(), x, x, causal=False)
+    with pytest.raises(ValueError):
+        mpsa.attention_forward(torch.zeros(1, 3, 128, 128, device="cuda", dtype=torch.bfloat16), x, x, causal=False)
