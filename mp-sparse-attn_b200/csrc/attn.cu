@@ -618,7 +618,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  grid_dependency_wait();                           // the set-up above ran under the kernel that prepares the operands
+  // The set-up above, and what each role can do on its own, runs under the kernel that prepares the operands: they wait for it
+  // one by one.
 
   uint8_t* sK = smem + ATT_OFF_K;
   uint8_t* sV = smem + ATT_OFF_V;
@@ -630,6 +631,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     if (elect_one()) {
       tma_prefetch_desc(&tm_q8); tma_prefetch_desc(&tm_q4);
       if (PVQ) { tma_prefetch_desc(&tm_vt8); tma_prefetch_desc(&tm_vt4); } else tma_prefetch_desc(&tm_vt);
+      grid_dependency_wait();
       bool ok = true;
       int sv = 0, tv = 0;                           // ring slot; pieces requested so far (over all items)
       uint32_t v_par = 1;                           // parity of the phase that frees the slot; a fresh barrier satisfies 1
@@ -723,6 +725,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     // thread requests the K tiles: when S(t - 2) has been read its MMAs are over, so the slot of tile t - 2 takes tile t + 2.
     if (elect_one()) {
       tma_prefetch_desc(&tm_k8); tma_prefetch_desc(&tm_k4);
+      grid_dependency_wait();
       uint32_t id8[4], id4[2];
 #pragma unroll
       for (int j = 0; j < 4; ++j) id8[j] = idesc_with_sf_id(idesc_block_scaled(p.fp8_fmt, p.fp8_fmt, ATT_BM, ATT_BN, 1), j, j);
@@ -871,6 +874,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     // O += P(t).V(t) as soon as V has landed and the softmax threads have stored P (quantised P: the tile; fp16 P: 64-key
     // halves).  ROUTE: an MXFP4 tile the router leaves out gets no MMA (the commits still go out: the loader and the
     // softmax carry on).
+    grid_dependency_wait();
     if (elect_one()) {
       const uint64_t vd0 = sdesc_kmajor_sw128(smem_u32(sV));        // + slot * (VSLOT >> 4)
       const uint64_t v4d0 = sdesc_kmajor_sw64(smem_u32(sV));        // MXFP4 V^T tile (64-byte rows)
@@ -975,6 +979,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     }
   } else if (warp == 3) {
     // ------------------------------ work items, visit lists and router ----------
+    // The first item is known without asking anybody, and its list under the band rule too: it is there when the operands are (first
+    // scores 2.5 -> 1.9 us after them).
+    if (ROUTE || p.map) grid_dependency_wait();
     bool ok = true;
     int emitted = 0, reclaimed = 0;                 // slots filled, and taken back
     int next_local = 0;                             // static schedule: items taken so far
@@ -997,7 +1004,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       if (ok && it >= 0 && slots[s].redo) { redo_item = it; redo_run = rw; redo_from = s; }
     };
     // The next item into the next slot, which is free: first what has to be done again, then the schedule.  Items are
-    // numbered heaviest query tile first; they are taken from a counter in memory where the caller gives one, else in
+    // numbered heaviest query tile first; after a CTA's first they are taken from a counter in memory where the caller gives one, else in
     // snake order over the CTAs, which evens out the sum.  false: nothing left.
     auto emit = [&]() -> bool {
       int item, mode = 0, wrun = 0;
@@ -1011,9 +1018,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         wrun = run;
         run_pos = plan.start(item + 1);
       } else {
-        if (p.counter) {
+        if (p.counter && emitted > 0) {
           int n = 0;
-          if (lane == 0) n = atomicAdd(p.counter, 1);
+          if (lane == 0) n = (int)gridDim.x + atomicAdd(p.counter, 1);
           item = __shfl_sync(0xffffffffu, n, 0);
         } else {
           item = next_local * (int)gridDim.x + ((next_local & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
@@ -1145,12 +1152,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     int seq = 0;                                    // items routed
     bool exhausted = false;
     _Pragma("unroll 1") while (ok) {
+      if (!PVQ && exhausted && emitted - reclaimed < NL) break;    // (no item comes back: the end can be said at once)
       const bool want = !exhausted && emitted - seq < ahead;
       if (want ? emitted - reclaimed >= NL : (seq == emitted && reclaimed < emitted)) {
         reclaim();
         if (redo_item >= 0) exhausted = false;
       } else if (want) {
         exhausted = !emit();
+        if (!ROUTE) grid_dependency_wait();         // (before the counter and the next items; it is over by the second time)
       } else if (seq < emitted) {
         if (ROUTE) route(seq);
         ++seq;
@@ -1159,7 +1168,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
       }
     }
     if (ok && lane == 0) {
-      // every slot has been taken back: the next one says that there is nothing more
+      // the next slot, which is free, says that there is nothing more
       const int s = emitted % NL;
       slots[s].mode = -1;
       mbar_arrive(&list_full[s]);
@@ -1179,6 +1188,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
     float* mrow = reinterpret_cast<float*>(smem + ATT_OFF_MROW);
     float* mslot = reinterpret_cast<float*>(smem + ATT_OFF_MSLOT);
     uint8_t* psf_dst = sSFP + wg * 512 + lane * 16 + q * 4 + g * 2;
+    grid_dependency_wait();
     const float nvmul = NVF4 ? (p.ts_q ? *p.ts_q * *p.ts_k : p.fp4_scale) : 1.0f;   // scores of NVFP4 tiles lack the tensor scales
     // An item's epilogue is put off until this thread has done its first tile of the next item, so that neither the last
     // P.V nor the warpgroup that had the last tile is waited for.  (Not with fp16 P.V: there a P buffer of the next
