@@ -138,6 +138,48 @@ __device__ __forceinline__ int div_by(int n, int d, uint32_t magic) {
   return d == 1 ? n : (magic ? (int)__umulhi((uint32_t)n, magic) : n / d);
 }
 
+// Mean over the rows of a head, every column, rounded to T, in the order of col_sum_kernel: eight rows, 16 apart, of every 128 a thread,
+// then the threads, then the groups of 128.  mean: 128 floats, and 16 x 128 more behind them.
+template <typename T>
+__device__ __forceinline__ void own_column_mean(const T* x, long long xs_l, int L, int D, float* mean) {
+  float* const acc_s = mean + 128;
+  const int tid = threadIdx.x, c8 = tid & 15, rg = tid >> 4;
+  x += c8 * 8;
+  float total = 0.0f;
+  _Pragma("unroll 1") for (int first = 0; first < L; first += 128) {
+    uint4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int r = first + rg + 16 * k;
+      v[k] = r < L && c8 * 8 < D ? __ldg(reinterpret_cast<const uint4*>(x + (long long)r * xs_l)) : make_uint4(0, 0, 0, 0);
+    }
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const T* e = reinterpret_cast<const T*>(&v[k]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += (float)e[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc_s[rg * 128 + c8 * 8 + j] = acc[j];
+    __syncthreads();
+    if (tid < 128) {
+      float t = 0.0f;
+#pragma unroll
+      for (int g = 0; g < 16; ++g) t += acc_s[g * 128 + tid];
+      total += t;
+    }
+  }
+  if (tid < 128) {
+    float lo, hi;
+    unpack2<T>(pack2<T>(__fdiv_rn(total, (float)L), 0.0f), lo, hi);
+    mean[tid] = lo;
+  }
+}
+
 // One tile of 128 rows (depth 128 and more) or 256 rows (depth 64) of one (batch, head).  A thread owns runs of 16 elements, two
 // neighbouring lanes one 32-element block.  All loads of the CTA go out before any arithmetic, held as they arrived;
 // scale codes are gathered with shuffles and stored a row at a time, so that no thread waits for another.  (Persistent
@@ -147,7 +189,7 @@ __device__ __forceinline__ int div_by(int n, int d, uint32_t magic) {
 // 46.7 us, MXFP4 alone to one code a byte 5.7 TB/s, MXFP8 alone 6.9); a warp that meets another block - all zero, near an end
 // of the range, or whose maximum is so close below a power of two that log2 rounds up - fetches the run again after the
 // loop and takes the general code.  MXFP4 needs more registers than four CTAs an SM leave it (spills): three.
-template <typename T, bool W8, bool W4, bool E4M3, bool D64>
+template <typename T, bool W8, bool W4, bool E4M3, bool D64, bool OWN>
 __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D, float* mean) {
   constexpr bool PATTERNS = W4 && std::is_same<T, __nv_bfloat16>::value;
   constexpr int LPR = D64 ? 4 : 8;                      // 16-element runs of a row inside the tile
@@ -164,6 +206,7 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
   const int r0 = tile_l * ROWS + rl0, n_live = p.L - r0;     // run i is inside the operand iff i * RSTEP < n_live
   const T* const x0 = reinterpret_cast<const T*>(p.x) + (long long)b * p.xs_b + (long long)h * p.xs_h + (long long)r0 * p.xs_l + c;
   const long long xstep = p.xs_l * RSTEP;
+  if (OWN && p.own_sums) own_column_mean<T>(reinterpret_cast<const T*>(p.x) + (long long)b * p.xs_b + (long long)h * p.xs_h, p.xs_l, p.L, D, mean);
   uint4 raw[4][2];
   {
     const T* x = x0;
@@ -177,11 +220,11 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
       x += xstep;
     }
   }
-  const bool centred = p.part || p.mean;
+  const bool centred = p.part || p.mean || (OWN && p.own_sums);
   if (centred) {
     // "smooth K": k - mean over the sequence (ours/mxfp_attn_kernel.py:33-34), an elementwise op in the input dtype.  The
     // mean is assembled here from the partial column sums, in their order.
-    if (tid < 128 && tid < D) {
+    if (!(OWN && p.own_sums) && tid < 128 && tid < D) {
       const long long col = tile_d * 128 + tid;
       if (p.mean) {
         mean[tid] = p.mean[(long long)bh * D + col];
@@ -483,7 +526,8 @@ __device__ __forceinline__ void v_tile(const PrepV& p, int cta, int D, uint8_t* 
   }
 }
 
-template <typename T, bool W8, bool W4, bool E4M3, bool D64>
+// OWN: K's CTAs may add up the columns themselves; an instance of its own, because it costs the others 1 - 2 %
+template <typename T, bool W8, bool W4, bool E4M3, bool D64, bool OWN>
 __global__ void __launch_bounds__(PREP_THREADS, W4 ? 3 : 4) prep_kernel(const __grid_constant__ PrepCall p) {
   extern __shared__ __align__(128) uint8_t prep_smem[];
   int cta = blockIdx.x;
@@ -501,7 +545,7 @@ __global__ void __launch_bounds__(PREP_THREADS, W4 ? 3 : 4) prep_kernel(const __
   cta -= p.v.ctas;
   const int which = cta >= p.op[0].ctas;
   if (which) cta -= p.op[0].ctas;
-  quant_rows<T, W8, W4, E4M3, D64>(p.op[which], cta, p.D, reinterpret_cast<float*>(prep_smem));
+  quant_rows<T, W8, W4, E4M3, D64, OWN>(p.op[which], cta, p.D, reinterpret_cast<float*>(prep_smem));
 }
 
 template <typename T>
@@ -509,8 +553,11 @@ int launch_prep(const PrepCall& p, bool w8, bool w4, bool e4m3, int grid, size_t
   const bool dep = p.after_sums || overlaps_previous(st);
 #define MPSA_PREP(A, B, C)                                                                                                    \
   do {                                                                                                      \
-    if (p.D == 64) launch_dependent(prep_kernel<T, A, B, C, true>, dim3(grid), PREP_THREADS, smem, st, dep, p);  \
-    else launch_dependent(prep_kernel<T, A, B, C, false>, dim3(grid), PREP_THREADS, smem, st, dep, p);         \
+    if (!C && (p.op[0].own_sums || p.op[1].own_sums)) {                                                                   \
+      if (p.D == 64) launch_dependent(prep_kernel<T, A, B, false, true, true>, dim3(grid), PREP_THREADS, smem, st, dep, p);  \
+      else launch_dependent(prep_kernel<T, A, B, false, false, true>, dim3(grid), PREP_THREADS, smem, st, dep, p);         \
+    } else if (p.D == 64) launch_dependent(prep_kernel<T, A, B, C, true, false>, dim3(grid), PREP_THREADS, smem, st, dep, p);  \
+    else launch_dependent(prep_kernel<T, A, B, C, false, false>, dim3(grid), PREP_THREADS, smem, st, dep, p);         \
   } while (0)
   if (w8 && w4) { if (e4m3) MPSA_PREP(true, true, true); else MPSA_PREP(true, true, false); }
   else if (w4) { if (e4m3) MPSA_PREP(false, true, true); else MPSA_PREP(false, true, false); }
@@ -584,7 +631,7 @@ int prep_launch(PrepCall& p, int in_dtype, bool w8, bool w4, int fp8_fmt, cudaSt
     o.ctas = (int)n;
   }
   p.v.ctas = 0;
-  size_t smem = 512;
+  size_t smem = p.op[0].own_sums || p.op[1].own_sums ? 512 + 16 * 128 * 4 : 512;
   if (p.v.v) {
     const long long n = (long long)p.v.B * p.v.H * (p.v.pitch >> 7);
     ctas += n;
