@@ -45,3 +45,28 @@ def test_back_to_back_equals_one_at_a_time(S):
     for a, b, c in zip(ref, got, other):
         a, b, c = (x.view(torch.uint8) if x.dtype != torch.uint8 else x for x in (a, b, c))
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+def test_operands_made_on_another_stream():
+    """The event between the streams comes before the launch, whatever kernel the launch overlaps on its own stream."""
+    import mpsa
+    g = torch.Generator(device="cuda").manual_seed(5)
+    k, v, w = (torch.randn(1, 2, 512, 128, generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    a = torch.randn(4096, 4096, generator=g, device="cuda")
+    ref = mpsa.attention_forward(w * 3, k, v, causal=True)
+    other = torch.cuda.Stream()
+    q = torch.zeros_like(w)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        q.zero_()
+        done = torch.cuda.Event()
+        other.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(other):
+            a @ a                                       # the operand comes late
+            q.copy_(w).mul_(3)
+            done.record()
+        mpsa.attention_forward(w, k, v, causal=True)    # a launch of ours right before, on the consumer's stream
+        torch.cuda.current_stream().wait_event(done)
+        out = mpsa.attention_forward(q, k, v, causal=True)
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
