@@ -1081,7 +1081,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         mbar_arrive(&list_full[s]);                 // release: entries (__syncwarp) and slot are visible to who waits
       }
 #pragma unroll
-      for (int k = 0; k < ATT_MAX_SLOTS; ++k) if (k == s) { held[k] = mode == 0 ? item : -1; if (SPLIT) held_run[k] = wrun; }
+      for (int k = 0; k < ATT_MAX_SLOTS; ++k) if (k == s) { held[k] = mode == 0 || ROUTE ? item : -1; if (SPLIT) held_run[k] = wrun; }
       ++emitted;
       return true;
     };
@@ -1528,9 +1528,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         }
         tc_fence_before();
         mbar_arrive(o_free);
-        if (PVQ && mode == 0) {
+        // Routed, the first pass's maxima include those of tiles that were then done again in MXFP8 and may lie far above every score that
+        // counts: an item done again with them as references may be so once more, with the maxima of that pass, which are exact.
+        if (PVQ && (mode == 0 || ROUTE)) {
           const float over = m_tot - ref;           // rows of the ragged tail hold no data
-          if (m_glob < p.S && m_tot != -INFINITY && (over < ATT_WIN_LO_Q || over > ATT_WIN_HI_Q)) {
+          if (m_glob < p.S && m_tot != -INFINITY && (over < ATT_WIN_LO_Q || (mode == 0 && over > ATT_WIN_HI_Q))) {
             slots[epi_ls].redo = 1;
             if (p.range_flag) *p.range_flag = 1;
           }

@@ -82,3 +82,25 @@ def test_items_done_again_when_scores_leave_the_fixed_reference():
     ref = O.attention_mxfp(q, k2, v, causal=True, prec_map=pm.cpu(), pv_mode="requant")
     m = O.parity_metrics(out.cpu(), ref)
     assert m["cos"] >= COS_MIN and m["rel_l2"] <= REL_L2_MAX, m
+
+
+def test_promoted_tiles_whose_mxfp4_scores_lie_far_above():
+    """Queries a hundred times as large against keys with outlier channels: the MXFP4 scores of promoted tiles exceed the MXFP8 ones that
+    replace them by more octaves than a reference serves.  Every row stays finite and equals the forward over the router's own map,
+    whose references are exact; bound: P in the tile's format, both in fp32."""
+    import mpsa
+    from mpsa import ops
+    B, Hq, Hkv, S, D = 2, 20, 5, 1332, 128
+    g = torch.Generator("cuda").manual_seed(579)
+    q, k, v = (torch.randn(B, h, S, D, generator=g, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    k[..., :5] *= 20
+    q[:, :, ::3] *= 100
+    for turn in range(3):
+        k = k.roll(7 * turn, dims=2)
+        out = mpsa.attention_forward(q, k, v, causal=True, pv_mode="requant", router="online", tau=1.1, out_dtype=torch.float32, check=True)
+        assert bool(torch.isfinite(out).all())
+        qq, kq = mpsa.quantize_mx(q, ops.q_side_scale(D)), mpsa.quantize_mx(k, 1.0)
+        stat = mpsa.router_statistic(qq, kq, B, Hq, Hkv, S, S, causal=True, check=True)
+        pm = mpsa.precision_map_online(stat, S, S, causal=True, band=1, tau=1.1)
+        ref = mpsa.attention_forward(q, k, v, causal=True, pv_mode="requant", prec_map=pm, out_dtype=torch.float32, check=True)
+        assert float((out - ref).norm() / ref.norm()) < 1e-5
