@@ -30,7 +30,9 @@ __device__ __forceinline__ bool elect_one() {
   return r != 0;
 }
 
-// In a kernel launched as a dependent of the one before it: returns when that one is complete and its writes are visible.
+// In a kernel launched as a dependent of the one before it: returns when that one is complete and its writes are visible - to ordinary
+// loads below it, bulk copies included.  Not to __ldg: ld.global.nc wants its memory read-only for the whole life of the kernel, which
+// here begins while the operands may still be written.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets a kernel launched as a dependent of this one start as soon as every CTA of this one has got here (it still waits for this
 // one's end before it reads what this one writes).

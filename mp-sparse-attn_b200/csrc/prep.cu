@@ -151,7 +151,7 @@ __device__ __forceinline__ void own_column_mean(const T* x, long long xs_l, int 
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int r = first + rg + 16 * k;
-      v[k] = r < L && c8 * 8 < D ? __ldg(reinterpret_cast<const uint4*>(x + (long long)r * xs_l)) : make_uint4(0, 0, 0, 0);
+      v[k] = r < L && c8 * 8 < D ? *reinterpret_cast<const uint4*>(x + (long long)r * xs_l) : make_uint4(0, 0, 0, 0);
     }
     float acc[8];
 #pragma unroll
@@ -214,8 +214,8 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
     for (int i = 0; i < 4; ++i) {
       raw[i][0] = raw[i][1] = make_uint4(0, 0, 0, 0);
       if (i * RSTEP < n_live) {
-        raw[i][0] = __ldg(reinterpret_cast<const uint4*>(x));
-        raw[i][1] = __ldg(reinterpret_cast<const uint4*>(x) + 1);
+        raw[i][0] = reinterpret_cast<const uint4*>(x)[0];
+        raw[i][1] = reinterpret_cast<const uint4*>(x)[1];
       }
       x += xstep;
     }
@@ -374,8 +374,8 @@ __device__ __forceinline__ void quant_rows(const PrepOperand& p, int tile, int D
     const bool live = i * RSTEP < n_live;
     uint4 r[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
     if (live) {
-      r[0] = __ldg(reinterpret_cast<const uint4*>(x0 + i * xstep));
-      r[1] = __ldg(reinterpret_cast<const uint4*>(x0 + i * xstep) + 1);
+      r[0] = reinterpret_cast<const uint4*>(x0 + i * xstep)[0];
+      r[1] = reinterpret_cast<const uint4*>(x0 + i * xstep)[1];
     }
     uint32_t w[8] = {r[0].x, r[0].y, r[0].z, r[0].w, r[1].x, r[1].y, r[1].z, r[1].w};
     centre(w);
@@ -447,7 +447,7 @@ __device__ __forceinline__ void v_tile(const PrepV& p, int cta, int D, uint8_t* 
   for (int j = 0; j < 8; ++j) {
     const int i = tid + j * PREP_THREADS, key = i >> vlog, vc = i & ((1 << vlog) - 1);
     ld[j] = make_uint4(0, 0, 0, 0);
-    if (key < 128 && key0 + key < p.Skv) ld[j] = __ldg(reinterpret_cast<const uint4*>(src + (long long)(key0 + key) * p.vs_l * 2) + vc);
+    if (key < 128 && key0 + key < p.Skv) ld[j] = reinterpret_cast<const uint4*>(src + (long long)(key0 + key) * p.vs_l * 2)[vc];
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {

@@ -702,7 +702,7 @@ col_sum_kernel(const T* x, float* part, int H, int L, int D, long long xs_b,
 #pragma unroll
         for (int n = 0; n < (int)(sizeof(T) / 2); ++n) {
           v[k].q[n] = make_uint4(0, 0, 0, 0);
-          if (r + 16 * k < r_end) v[k].q[n] = __ldg(reinterpret_cast<const uint4*>(xb + (long long)(r + 16 * k) * xs_l) + n);
+          if (r + 16 * k < r_end) v[k].q[n] = reinterpret_cast<const uint4*>(xb + (long long)(r + 16 * k) * xs_l)[n];
         }
       }
 #pragma unroll
