@@ -1529,10 +1529,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         tc_fence_before();
         mbar_arrive(o_free);
         // Routed, the first pass's maxima include those of tiles that were then done again in MXFP8 and may lie far above every score that
-        // counts: an item done again with them as references may be so once more, with the maxima of that pass, which are exact.
+        // counts.  Such a maximum may be inside the window while what counts is below it: the row sum, which holds nothing else, shows it.
+        // An item done again with those maxima as references may be so once more, with the maxima of that pass, which are exact.
         if (PVQ && (mode == 0 || ROUTE)) {
           const float over = m_tot - ref;           // rows of the ragged tail hold no data
-          if (m_glob < p.S && m_tot != -INFINITY && (over < ATT_WIN_LO_Q || (mode == 0 && over > ATT_WIN_HI_Q))) {
+          if (m_glob < p.S && m_tot != -INFINITY &&
+              (over < ATT_WIN_LO_Q || (mode == 0 && (over > ATT_WIN_HI_Q || (ROUTE && l_tot < exp2_of((int)ATT_WIN_LO_Q)))))) {
             slots[epi_ls].redo = 1;
             if (p.range_flag) *p.range_flag = 1;
           }

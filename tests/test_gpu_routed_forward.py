@@ -104,3 +104,27 @@ def test_promoted_tiles_whose_mxfp4_scores_lie_far_above():
         pm = mpsa.precision_map_online(stat, S, S, causal=True, band=1, tau=1.1)
         ref = mpsa.attention_forward(q, k, v, causal=True, pv_mode="requant", prec_map=pm, out_dtype=torch.float32, check=True)
         assert float((out - ref).norm() / ref.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("S", [300, 512])
+def test_promoted_tiles_whose_mxfp4_scores_lie_far_below(S):
+    """The other side: MXFP4 scores of promoted tiles inside the range that one reference serves, MXFP8 scores that replace them and all
+    the others far below it.  Key elements next to a block's large one are zero in MXFP4 (1/16 and 5/64 of its scale) and exact in
+    MXFP8, and the queries are zero where the large one stands: every MXFP4 score is 0, the others are about -175."""
+    import mpsa
+    from mpsa import ops
+    B, Hq, Hkv, D = 1, 2, 1, 128
+    g = torch.Generator("cuda").manual_seed(S)
+    q = torch.full((B, Hq, S, D), 1.25 / ops.q_side_scale(D), device="cuda", dtype=torch.bfloat16)
+    k = -1.0 - 0.25 * torch.randint(0, 2, (B, Hkv, S, D), generator=g, device="cuda").to(torch.bfloat16)
+    q[..., ::32], k[..., ::32] = 0.0, 128.0
+    v = torch.randn(B, Hkv, S, D, generator=g, device="cuda", dtype=torch.bfloat16)
+    qq, kq = mpsa.quantize_mx(q, ops.q_side_scale(D)), mpsa.quantize_mx(k, 1.0)
+    stat = mpsa.router_statistic(qq, kq, B, Hq, Hkv, S, S, causal=True, check=True)
+    assert float(stat.abs().max()) == 0.0
+    pm = mpsa.precision_map_online(stat, S, S, causal=True, band=1, tau=1.1)
+    assert bool((pm != ops.TILE_FP4).all())
+    out = mpsa.attention_forward(q, k, v, causal=True, pv_mode="requant", router="online", tau=1.1, out_dtype=torch.float32, check=True)
+    ref = mpsa.attention_forward(q, k, v, causal=True, pv_mode="requant", prec_map=pm, out_dtype=torch.float32, check=True)
+    assert float(ref.norm(dim=-1).min()) > 0.0
+    assert float((out - ref).norm() / ref.norm()) < 1e-5
