@@ -1,8 +1,9 @@
 // The short way from torch tensors into libmpsa.so: checks, output allocation and the C call of the three entry points that programs
 // call most, in one step.  Through ctypes and struct the same took 8 - 11 us a call of the host's time, here 3: back to back, a pair of
 // quantizers over 4500 tokens 16.5 -> 11.0 us, causal attention over 128 tokens 17.0 -> 11.0.  Outputs and workspaces come from torch's allocator through its dispatcher, as
-// torch.empty does.  Operands that the one-launch paths do not take make a function return None, and the caller goes the long way;
-// an error code of the C entry is returned as an int.
+// torch.empty does, and like there the interpreter's lock is released from the first of them to the end of the C call: an allocation may
+// wait for the device, and a launch for room in its queue.  Operands that the one-launch paths do not take make a function return
+// None, and the caller goes the long way; an error code of the C entry is returned as an int.
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -41,6 +42,14 @@ bool aligned16(const at::Tensor& t) {
 int in_dtype(const at::Tensor& t) { return t.scalar_type() == at::kBFloat16 ? 0 : t.scalar_type() == at::kHalf ? 1 : -1; }
 
 at::Tensor dense(at::IntArrayRef sizes, at::ScalarType type, const at::Tensor& like) { return at::empty(sizes, like.options().dtype(type).requires_grad(false)); }
+
+// Other Python threads run while this lives.  (The caller's argument array keeps the tensors.)
+struct Unlocked {
+  PyThreadState* const state = PyEval_SaveThread();
+  Unlocked() = default;
+  Unlocked(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
 
 // The operands' device for the time of a call: the usual case costs one look.
 struct OnDevice {
@@ -134,14 +143,20 @@ PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
       if (!THPVariable_Check(a[4])) { PyErr_SetString(PyExc_TypeError, "attention: range_flag must be a tensor"); return nullptr; }
       c.range_flag = static_cast<int*>(THPVariable_Unpack(a[4]).data_ptr());
     }
-    const OnDevice device(q->device().index());
-    const long long need = workspace_fn(&c);            // (refuses empty operands)
-    if (need < 0) return PyLong_FromLongLong(need);
-    const at::Tensor ws = dense({(int64_t)need}, at::kByte, *q);
-    at::Tensor out = dense(size, kOut[c.out_dtype], *q);
-    c.out = out.data_ptr(); c.workspace = ws.data_ptr(); c.workspace_bytes = need;
-    const int rc = attention_fn(&c, c10::cuda::getCurrentCUDAStream(q->device().index()).stream());
-    return rc ? PyLong_FromLong(rc) : THPVariable_Wrap(std::move(out));
+    at::Tensor out;
+    long long rc;
+    {
+      const Unlocked unlocked;
+      const OnDevice device(q->device().index());
+      rc = workspace_fn(&c);                            // (refuses empty operands)
+      if (rc >= 0) {
+        const at::Tensor ws = dense({(int64_t)rc}, at::kByte, *q);
+        out = dense(size, kOut[c.out_dtype], *q);
+        c.out = out.data_ptr(); c.workspace = ws.data_ptr(); c.workspace_bytes = rc;
+        rc = attention_fn(&c, c10::cuda::getCurrentCUDAStream(q->device().index()).stream());
+      }
+    }
+    return rc ? PyLong_FromLongLong(rc) : THPVariable_Wrap(std::move(out));
   });
 }
 
@@ -164,22 +179,27 @@ PyObject* quant_pair(PyObject*, PyObject* const* a, Py_ssize_t n) {
         c.fp8_fmt < 0 || c.fp8_fmt > 2)
       Py_RETURN_NONE;
     c.B = (int)B; c.D = (int)D;
-    const OnDevice device(x[0]->device().index());
-    const at::ScalarType type = c.fp8_fmt == 0 ? at::kByte : c.fp8_fmt == 1 ? at::kFloat8_e5m2 : at::kFloat8_e4m3fn;
+    for (const at::Tensor* t : x)
+      if (t->size(1) > 0x7fffffff || t->size(2) > 0x7fffffff) Py_RETURN_NONE;
     at::Tensor codes[2], scales[2];
-    for (int i = 0; i < 2; ++i) {
-      const auto z = x[i]->sizes(), st = x[i]->strides();
-      const int h = hnd ? 1 : 2, l = hnd ? 2 : 1;         // where heads and length are
-      if (z[h] > 0x7fffffff || z[l] > 0x7fffffff) Py_RETURN_NONE;
-      codes[i] = dense(z, type, *x[i]);
-      scales[i] = dense({B, z[h], z[l], D / 32}, at::kByte, *x[i]);
-      const auto cs = codes[i].strides();
-      c.x[i] = x[i]->data_ptr(); c.codes[i] = codes[i].data_ptr(); c.scales[i] = scales[i].data_ptr();
-      c.H[i] = (int)z[h]; c.L[i] = (int)z[l];
-      c.x_sb[i] = st[0]; c.x_sh[i] = st[h]; c.x_sl[i] = st[l];
-      c.c_sb[i] = cs[0]; c.c_sh[i] = cs[h]; c.c_sl[i] = cs[l];
+    int rc;
+    {
+      const Unlocked unlocked;
+      const OnDevice device(x[0]->device().index());
+      const at::ScalarType type = c.fp8_fmt == 0 ? at::kByte : c.fp8_fmt == 1 ? at::kFloat8_e5m2 : at::kFloat8_e4m3fn;
+      for (int i = 0; i < 2; ++i) {
+        const auto z = x[i]->sizes(), st = x[i]->strides();
+        const int h = hnd ? 1 : 2, l = hnd ? 2 : 1;       // where heads and length are
+        codes[i] = dense(z, type, *x[i]);
+        scales[i] = dense({B, z[h], z[l], D / 32}, at::kByte, *x[i]);
+        const auto cs = codes[i].strides();
+        c.x[i] = x[i]->data_ptr(); c.codes[i] = codes[i].data_ptr(); c.scales[i] = scales[i].data_ptr();
+        c.H[i] = (int)z[h]; c.L[i] = (int)z[l];
+        c.x_sb[i] = st[0]; c.x_sh[i] = st[h]; c.x_sl[i] = st[l];
+        c.c_sb[i] = cs[0]; c.c_sh[i] = cs[h]; c.c_sl[i] = cs[l];
+      }
+      rc = quant_pair_fn(&c, c10::cuda::getCurrentCUDAStream(x[0]->device().index()).stream());
     }
-    const int rc = quant_pair_fn(&c, c10::cuda::getCurrentCUDAStream(x[0]->device().index()).stream());
     if (rc) return PyLong_FromLong(rc);
     PyObject* r = PyTuple_New(4);
     if (!r) return nullptr;
@@ -206,11 +226,16 @@ PyObject* gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (int i = 0; i < 3; ++i)
       if (w[i] <= 0 || w[i] > 0x7fffffff) Py_RETURN_NONE;
     if (w[6] < 0 || w[6] > 3) Py_RETURN_NONE;
-    const OnDevice device(x->device().index());
-    at::Tensor c = dense({(int64_t)w[0], (int64_t)w[1]}, kOut[w[6]], *x);
-    const int rc = gemm_fn(x->data_ptr(), xs->data_ptr(), y->data_ptr(), ys->data_ptr(), c.data_ptr(), (int)w[0], (int)w[1], (int)w[2],
-                           x->stride(0) * x->element_size(), y->stride(0) * y->element_size(), w[1], (int)w[3], (int)w[4], (int)w[5], (int)w[6],
-                           (float)alpha, status, c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
+    at::Tensor c;
+    int rc;
+    {
+      const Unlocked unlocked;
+      const OnDevice device(x->device().index());
+      c = dense({(int64_t)w[0], (int64_t)w[1]}, kOut[w[6]], *x);
+      rc = gemm_fn(x->data_ptr(), xs->data_ptr(), y->data_ptr(), ys->data_ptr(), c.data_ptr(), (int)w[0], (int)w[1], (int)w[2],
+                   x->stride(0) * x->element_size(), y->stride(0) * y->element_size(), w[1], (int)w[3], (int)w[4], (int)w[5], (int)w[6],
+                   (float)alpha, status, c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
+    }
     return rc ? PyLong_FromLong(rc) : THPVariable_Wrap(std::move(c));
   });
 }

@@ -74,3 +74,68 @@ def test_what_was_refused_stays_refused():
         mpsa.attention_forward(x.cpu(), x, x, causal=False)
     with pytest.raises(ValueError):
         mpsa.attention_forward(torch.zeros(1, 3, 128, 128, device="cuda", dtype=torch.bfloat16), x, x, causal=False)
+
+
+@pytest.mark.gpu
+def test_the_interpreter_is_free_during_allocation_and_launch(tmp_path):
+    """A launch into a full queue, or an allocation that has to wait for the device, must not hold every other thread up: the C entries
+    run without the interpreter's lock (here they are replaced by the call that tells)."""
+    import ctypes
+    import importlib.util
+    import shutil
+
+    from mpsa import _lib, ops
+    lib, n = _lib.load(), _lib.native()
+    path = tmp_path / "copy.so"                           # (its own function pointers)
+    shutil.copy(n.__file__, path)
+    spec = importlib.util.spec_from_file_location("copy._native", path)
+    m = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(m)
+    address = lambda f: ctypes.cast(f, ctypes.c_void_p).value
+    held = address(ctypes.pythonapi.PyGILState_Check)
+    m.init(address(lib.mpsa_attention_workspace), held, held, held, torch.OutOfMemoryError)
+    x = torch.zeros(1, 2, 128, 128, device="cuda", dtype=torch.bfloat16)
+    b = torch.zeros(128, 128, device="cuda", dtype=torch.uint8)
+    status = ops.status_word(x.device).data_ptr()
+    assert isinstance(m.attention(x, x, x, None, None, status, 0, 0, 1, 0, 0, 0, 1, 0, 0, 1.0, 1.0), torch.Tensor)
+    assert isinstance(m.quant_pair(x, x, 1.0, 1.0, 0, True), tuple)
+    assert isinstance(m.gemm(b, b, b, b, 128, 128, 128, 0, 1, 1, 0, 1.0, status), torch.Tensor)
+
+
+@pytest.mark.gpu
+def test_two_threads():
+    import threading
+
+    import mpsa
+    from mpsa import ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = [torch.randn(1, 4, n, 128, generator=g, device="cuda", dtype=torch.bfloat16) for n in (200, 640)]
+
+    def calls(t):
+        c = mpsa.quantize_mx(t.reshape(1, 1, -1, 128), want_fp4=False)
+        m, s = c.fp8.shape[2], c.fp8_sf.view(-1, 1, 32, 4, 4)
+        a = c.fp8.view(m, 128)
+        return [mpsa.attention_forward(t, t, t, causal=True), *ops.quantize_pair(t, t, 0.5, 1.0, "e5m2"),
+                ops.gemm_block_scaled(a, s, a, s, torch.float32, m, m, 128, "mxfp8")]
+
+    want = [calls(t) for t in x]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(40):
+                    got = calls(x[i])
+                    torch.cuda.current_stream().synchronize()
+                    if not all(torch.equal(p.view(torch.uint8), r.view(torch.uint8)) for p, r in zip(got, want[i])):
+                        wrong.append((i, "other results"))
+        except Exception as e:                            # noqa: BLE001 (reported by the test)
+            wrong.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:4]
