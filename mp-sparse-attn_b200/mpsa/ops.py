@@ -485,7 +485,7 @@ def _attention_one_call(q, k, v, kv, *, causal, band, uniform, sq, fp8_elem, out
     pv = pv_mode == "requant"
     flag = _last.range_flag = torch.empty(1, dtype=torch.int32, device=q.device) if want_flag and pv else None
     out = _lib.native().attention(q, k, v, prepared, flag, st.status_ptr, _OUT_DTYPE[out_dtype], int(causal), band, uni, route, pv,
-                                  _FP8_DESC[fp8_elem], smooth_k, nvfp4, sq, tau)
+                                  _FP8_DESC[fp8_elem], int(smooth_k), nvfp4, sq, tau)
     if out.__class__ is int:
         _lib.check(out)
     return out

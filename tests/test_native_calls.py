@@ -139,3 +139,15 @@ def test_two_threads():
     for t in threads:
         t.join()
     assert not wrong, wrong[:4]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flag", ["numpy", "float", "int"])
+def test_truth_values_of_any_kind(flag):
+    import numpy as np
+    import mpsa
+    x = torch.randn(1, 2, 130, 128, device="cuda", dtype=torch.bfloat16)
+    for value in (False, True):
+        given = {"numpy": np.bool_, "float": float, "int": int}[flag](value)
+        got = mpsa.attention_forward(x, x, x, causal=given, smooth_k=given)
+        assert torch.equal(got, mpsa.attention_forward(x, x, x, causal=value, smooth_k=value))
