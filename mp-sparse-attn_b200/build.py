@@ -1,5 +1,5 @@
 """Build the C-ABI CUDA library in-tree: csrc/*.cu -> mpsa/libmpsa.so (sm_100a only), and the Python module in front of its short
-calls: csrc/native.cpp -> mpsa/_native.so.
+calls: csrc/native.cpp -> mpsa/_native.<Python tag>.torch-<version>.so.
 
     python mp-sparse-attn_b200/build.py [--force]
 
@@ -14,7 +14,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "mpsa", "libmpsa.so")
-NATIVE_SRC, NATIVE_OUT = os.path.join(CSRC, "native.cpp"), os.path.join(HERE, "mpsa", "_native.so")
+NATIVE_SRC = os.path.join(CSRC, "native.cpp")
 SOURCES = ["api.cu", "quant.cu", "prep.cu", "gemm.cu", "attn.cu", "route.cu", "attention.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=default", "--use_fast_math=false"]
@@ -65,26 +65,35 @@ def build_lib(force=False, verbose=False):
     return OUT
 
 
+def native_out():
+    """Where the module for this Python and this torch is: one made for another of either is never loaded."""
+    import sysconfig
+
+    import torch
+    return os.path.join(HERE, "mpsa", f"_native.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
+
+
 def build_native(force=False):
-    """csrc/native.cpp -> mpsa/_native.so, the module that takes torch tensors to the library (needs torch's headers)."""
+    """csrc/native.cpp -> native_out(), the module that takes torch tensors to the library (needs torch's headers)."""
+    out = native_out()
     header = os.path.join(os.path.dirname(HERE), "include", "mpsa.h")
-    if not force and os.path.exists(NATIVE_OUT) and \
-            os.path.getmtime(NATIVE_OUT) >= max(os.path.getmtime(f) for f in (NATIVE_SRC, header, __file__)):
-        return NATIVE_OUT
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= max(os.path.getmtime(f) for f in (NATIVE_SRC, header, __file__)):
+        return out
     import sysconfig
 
     import torch
     base = os.path.dirname(torch.__file__)
     inc = [sysconfig.get_paths()["include"], os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
            os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
+    new = f"{out}.{os.getpid()}.new"                # (several ranks may get here at a time)
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + i for i in inc), NATIVE_SRC, "-o", NATIVE_OUT + ".new",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *("-I" + i for i in inc), NATIVE_SRC, "-o", new,
            "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on native.cpp:\n{r.stdout}")
-    os.replace(NATIVE_OUT + ".new", NATIVE_OUT)
-    return NATIVE_OUT
+    os.replace(new, out)
+    return out
 
 
 if __name__ == "__main__":

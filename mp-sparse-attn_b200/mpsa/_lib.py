@@ -94,28 +94,43 @@ def load():
 _native = None
 
 
+class _LongWay:
+    """In place of the module where it cannot be had: it takes no call, so that every one goes the long way, through ctypes."""
+
+    @staticmethod
+    def attention(*_):
+        return None
+
+    quant_pair = gemm = attention
+
+
+def _module(name, path):
+    import importlib.util
+    spec = importlib.util.spec_from_file_location(name, path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
 def native():
-    """The module that takes torch tensors to the library's short calls (csrc/native.cpp), built first if necessary."""
+    """The module that takes torch tensors to the library's short calls (csrc/native.cpp), built first if necessary; without a compiler
+    or torch's headers a stand-in, and the short calls take longer."""
     global _native
     if _native is not None:
         return _native
-    import importlib.util
-
     import torch                                 # (the module's symbols are in torch's libraries)
     lib = load()
-    path = os.path.join(_HERE, "_native.so")
-    if not os.path.exists(path):
-        sys.path.insert(0, os.path.dirname(_HERE))
-        try:
-            import build as _build
-            _build.build_native()
-        finally:
-            sys.path.pop(0)
-    spec = importlib.util.spec_from_file_location("mpsa._native", path)
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
-    mod.init(*(ctypes.cast(getattr(lib, f), c_void_p).value for f in
-               ("mpsa_attention_workspace", "mpsa_attention", "mpsa_quant_pair", "mpsa_gemm_block_scaled")), torch.OutOfMemoryError)
+    try:
+        build = _module("_mpsa_build", os.path.join(os.path.dirname(_HERE), "build.py"))
+        path = build.native_out()
+        mod = _module("mpsa._native", path if os.path.exists(path) else build.build_native())
+        mod.init(*(ctypes.cast(getattr(lib, f), c_void_p).value for f in
+                   ("mpsa_attention_workspace", "mpsa_attention", "mpsa_quant_pair", "mpsa_gemm_block_scaled")), torch.OutOfMemoryError)
+    except Exception as e:                       # noqa: BLE001 (whatever kept it from being built or loaded)
+        import warnings
+        warnings.warn(f"mpsa: the native module for short calls is not available, they go through ctypes ({type(e).__name__}: {str(e)[:500]})", RuntimeWarning,
+                      stacklevel=3)
+        mod = _LongWay
     _native = mod
     return mod
 

@@ -151,3 +151,60 @@ def test_truth_values_of_any_kind(flag):
         given = {"numpy": np.bool_, "float": float, "int": int}[flag](value)
         got = mpsa.attention_forward(x, x, x, causal=given, smooth_k=given)
         assert torch.equal(got, mpsa.attention_forward(x, x, x, causal=value, smooth_k=value))
+
+
+@pytest.fixture
+def no_module(monkeypatch, tmp_path):
+    """As on a machine without a C++ compiler and without a built module."""
+    from mpsa import _lib
+    monkeypatch.setattr(_lib, "_native", None)
+    real = _lib._module
+
+    def module(name, path):
+        mod = real(name, path)
+        if name == "_mpsa_build":
+            mod.native_out = lambda: str(tmp_path / "absent.so")
+        return mod
+    monkeypatch.setattr(_lib, "_module", module)
+    monkeypatch.setenv("CXX", str(tmp_path / "no-compiler"))
+    with pytest.warns(RuntimeWarning, match="not available"):
+        n = _lib.native()
+    assert _lib.native() is n                             # (asked for once)
+    return n
+
+
+def test_without_the_module_every_call_is_left_to_the_long_way(no_module):
+    assert [no_module.attention(1), no_module.quant_pair(2, 3), no_module.gemm()] == [None] * 3
+
+
+def test_the_module_is_that_of_this_python_and_torch():
+    import sysconfig
+
+    from mpsa import _lib
+    name = _lib.native().__file__
+    assert torch.__version__ in name and sysconfig.get_config_var("SOABI") in name
+
+
+@pytest.mark.gpu
+def test_calls_without_the_module(no_module, monkeypatch):
+    import mpsa
+    from mpsa import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(11)
+    x = torch.randn(1, 4, 300, 128, generator=g, device="cuda", dtype=torch.bfloat16)
+    c = mpsa.quantize_mx(x[:, :, :256].reshape(1, 1, -1, 128), want_fp4=False)
+    m, s = c.fp8.shape[2], c.fp8_sf.view(-1, 1, 32, 4, 4)
+    a = c.fp8.view(m, 128)
+
+    def calls():
+        kv = mpsa.prepare_kv(x, x, pv_mode="requant")
+        return [*ops.quantize_pair(x, x, 0.5, 1.0, "mxfp4"), *ops.quantize_pair(x, x, 0.5, 1.0, "e5m2"),
+                ops.gemm_block_scaled(a, s, a, s, torch.float32, m, m, 128, "mxfp8"),
+                mpsa.attention_forward(x, x, x, causal=True), mpsa.attention_forward(x, x, x, causal=False, pv_mode="requant", smooth_k=True),
+                mpsa.attention_forward(x, x, x, causal=True, pv_mode="requant", router="online", tau=1.1),
+                mpsa.attention_forward(x, x, x, causal=False, fp4_kind="nvfp4"), mpsa.attention_forward(x, None, None, causal=True, kv=kv)]
+
+    got = calls()
+    monkeypatch.undo()
+    assert _lib.native().__file__
+    for i, (p, r) in enumerate(zip(got, calls())):
+        assert torch.equal(p.view(torch.uint8), r.view(torch.uint8)), i
