@@ -61,7 +61,7 @@ long long plan(const mpsa_attention_args& a, uint8_t* ws, PrepCall& pc, AttnCall
     ac.k4 = k.fp4_packed = q4 ? cv.take(krows * 64) : nullptr;
     ac.k4_sf = k.sf4_tiled = q4 ? cv.take((long long)a.B * a.Hkv * nk * sf4) : nullptr;
     k.o8_l = 128; k.o8_h = 128ll * a.Skv; k.o8_b = k.o8_h * a.Hkv; k.p4_row = 64;
-    k.own_sums = a.smooth_k && a.Skv <= PREP_OWN_SUMS && a.fp8_fmt == 1;     // (no instances for E4M3)
+    k.own_sums = a.smooth_k && prep_own_sums((long long)a.B * a.Hkv, a.Skv, a.D) && a.fp8_fmt == 1;     // (no instances for E4M3)
     if (a.smooth_k && !k.own_sums) {
       k.nchunk = col_sum_chunks(a.Skv);
       k.part = (float*)cv.take((long long)a.B * a.Hkv * k.nchunk * a.D * 4);

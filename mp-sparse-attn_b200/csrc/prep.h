@@ -23,7 +23,7 @@ struct PrepOperand {
   float s = 1.0f;                                      // multiplied in before quantisation
   const float* part = nullptr; int nchunk = 0;         // partial column sums [B*H, nchunk, D] of the mean to subtract,
   const float* mean = nullptr;                         // or that mean itself [B*H, D],
-  bool own_sums = false;                               // or every CTA adds up its head's columns itself (at most PREP_OWN_SUMS rows, D <= 128, E5M2)
+  bool own_sums = false;                               // or every CTA adds up its head's columns itself (prep_own_sums; D <= 128, E5M2)
   uint8_t* fp8_codes = nullptr; long long o8_b = 0, o8_h = 0, o8_l = 0;
   uint8_t* fp4_unpacked = nullptr; long long o4_b = 0, o4_h = 0, o4_l = 0;
   uint8_t* fp4_packed = nullptr; long long p4_row = 0; // [B,H,L] rows of p4_row bytes
@@ -53,10 +53,17 @@ struct PrepCall {
   bool after_sums = false;                             // the kernel before this one on the stream is col_sums'
 };
 
-// Up to this many rows a CTA of K adds up the columns of its head itself, several CTAs the same, instead of waiting for a launch that
-// does it once.  2 x 8 heads, MXFP4, calls back to back: 333 tokens 17.6 -> 14.8 us, 512 tokens 18.0 -> 17.3; beyond, the launch is
-// the better way (4 x 16 heads of 512 tokens, depth 64: 24.2 -> 23.0).
-constexpr int PREP_OWN_SUMS = 512;
+// Whether the CTAs of K add up the columns of their head themselves, each the whole head (up to PREP_OWN_SUMS rows), instead of waiting
+// for a launch that does it once.  That saves the launch; it costs every CTA of K a pass over its head, in a second round of CTAs where
+// the chip does not hold all of them at once.  GPU time of a call, MXFP4 scores, depth 128, launch -> own: 16 heads of 333 rows 16.8 ->
+// 14.6 us, 64 heads of 333 (192 CTAs of K) 26.2 -> 25.1, 48 heads of 512 (192) 27.3 -> 26.9; against it 64 heads of 512 (256) 29.0 -> 31.0,
+// 128 of 512 51.3 -> 55.1, 96 of 333 (288) 30.4 -> 31.5.  Up to two tiles it pays whatever the heads (256 heads of 256 49.0 -> 45.4; depth
+// 64, where a tile has 256 rows, 64 heads of 512 23.7 -> 23.1), but for 96 heads of 333 - 384 rows of depth 64 (25.2 -> 25.9).
+constexpr int PREP_OWN_SUMS = 512, PREP_OWN_CTAS = 200;
+inline bool prep_own_sums(long long heads, int L, int D) {
+  const int rows = D == 64 ? 256 : 128, tiles = (L + rows - 1) / rows;
+  return L <= PREP_OWN_SUMS && (tiles <= 2 || heads * tiles <= PREP_OWN_CTAS);
+}
 
 PrepThresholds prep_thresholds(float s);
 bool prep_operand_ok(const PrepOperand& p, int D);     // alignment, depth and scale the kernel can take
