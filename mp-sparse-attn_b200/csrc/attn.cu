@@ -326,14 +326,16 @@ __device__ __forceinline__ void sub2(float& a, float& b, float c, float d, float
 // x = n + f with n = round(x) (adding 1.5 * 2^23 leaves n in the low mantissa bits), 2^f on [-0.5, 0.5] by a polynomial of degree 5,
 // 2^n by adding n to the exponent field.  Least largest relative error among the polynomials with value 1 at 0 (found by reweighted
 // least squares), 1.6e-7 with fp32 rounding, against the 2^-22 = 2.4e-7 that ex2.approx is specified with; zero below 2^-126 like it.
+// A NaN must not become a zero probability, by which a key would vanish from its row: its patterns, 0x7fffffff in t and in the polynomial,
+// add up to the largest finite number, which spoils the row as a NaN does.  (A NaN again, through a multiplication by 2^n, costs 2.5 %.)
 __device__ __forceinline__ void fma2(float& a, float& b, float c, float d, float e) {   // (a, b) = (a, b) * (c, d) + (e, e)
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmov.b64 z, {%4, %4};\n\t"
       "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
       : "+f"(a), "+f"(b) : "f"(c), "f"(d), "f"(e));
 }
 __device__ __forceinline__ void ex2_poly2(float& y0, float& y1, float x0, float x1) {
-  x0 = fmaxf(x0, -200.0f);
-  x1 = fmaxf(x1, -200.0f);
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-200.0f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-200.0f));
   float t0, t1, n0, n1;
   sub2(t0, t1, x0, x1, 12582912.0f);              // t = x + 1.5 * 2^23
   sub2(n0, n1, t0, t1, -12582912.0f);             // n = round(x), as a float

@@ -45,3 +45,27 @@ def test_denominators(fmt, causal, S, Skv, shift):
     err = float((lse.double() - ref).abs().max())
     assert err <= bound, (err, bound)
     assert bool(torch.isfinite(out).all())
+
+
+@pytest.mark.parametrize("pv", ["fp16", "requant"])
+def test_a_key_whose_scores_are_nan_spoils_its_rows_wherever_it_lies(pv):
+    """Scores of a key whose scale codes are NaN, at every place of a 32-key block (the exponentials of some places are formed in another
+    way): no row that sees it may come out as if the key were not there.  Rows are spoilt by not being finite or by vanishing."""
+    import mpsa
+    from mpsa import ops
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(1, 1, n, 128, generator=g, device="cuda") for n in (128, 256, 256))
+    qq, kq = mpsa.quantize_mx(q, ops.q_side_scale(128)), mpsa.quantize_mx(k, 1.0)
+    vt = mpsa.quantize_v_seq(v) if pv == "requant" else mpsa.prepare_vt(v)
+    whole = kq.fp4_sf.clone()
+
+    def call():
+        return ops.attention_forward_quantized(qq, kq, vt, 1, 1, 1, 128, 256, 128, causal=False, uniform="fp4", out_dtype=torch.float32, check=True)
+
+    usual = call().norm(dim=-1)
+    assert bool(torch.isfinite(usual).all()) and float(usual.min()) > 0.1
+    for place in range(32):
+        kq.fp4_sf.copy_(whole)
+        kq.fp4_sf[0, 0, 1, 0, place * 16:place * 16 + 4] = 255       # key 128 + place: its four blocks
+        norm = call().norm(dim=-1)
+        assert bool((~torch.isfinite(norm) | (norm < 1e-12 * usual)).all()), place
