@@ -124,11 +124,11 @@ constexpr float ATT_NO_REF = -3e38f;                  // fp16 P.V: reference of 
 // Division of the keys.  The first n_whole are done by one CTA each; the tiles of the others, laid end to end, are cut into runs
 // of run_tiles, one CTA each, so that a grid with fewer items than SMs, or with a last wave that is nearly empty, still
 // fills the chip.  An item that several runs share gets its result from attn_combine_kernel.
+static __host__ __device__ __forceinline__ int item_number(bool causal, int heads, int nq, int r, int head) { return causal ? r * heads + head : head * nq + r; }
 struct SplitPlan {
   int heads, nq, nk, causal, c1;     // c1: visible tiles of query tile 0
   int n_whole, run_tiles;
   int pad;                           // 0, or the places every item takes: a multiple of run_tiles, so that no run holds two items
-  __host__ __device__ int item_of(int r, int head) const { return causal ? r * heads + head : head * nq + r; }
   __host__ __device__ int row_of(int item) const { return causal ? item / heads : item % nq; }
   __host__ __device__ int head_of(int item) const { return causal ? item % heads : item / nq; }
   __host__ __device__ long long row_tiles(int r) const { return !causal || r == 0 ? nk : nq - 1 - r + c1; }
@@ -1516,8 +1516,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q8, const __grid_constant
         const long long row = (long long)head * p.S + m_glob;
         // a share of an item: fp32 and the log2 denominator, into its slice of the partial results
         const int part = SPLIT ? slots[epi_ls].part : -1;
-        [[maybe_unused]] const int r = nq - 1 - slots[epi_ls].qi;
-        const int item = SPLIT ? (p.causal ? r * p.Hq * p.B + head : head * nq + r) : 0;
+        const int item = SPLIT ? item_number(p.causal, p.Hq * p.B, nq, nq - 1 - slots[epi_ls].qi, head) : 0;
         const float ref = PVQ ? (mode == 1 ? m_redo + (LATE ? ATT_REF_Q : 0.0f) : ATT_REF_Q) : ref_last;
         const bool has_o = epi_part * 32 < p.D;     // this thread's 32 columns of O
         uint32_t o[32];
