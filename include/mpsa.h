@@ -219,8 +219,8 @@ int mpsa_attn_fwd_routed(const void* q8, const void* q8_sf, const void* q4, cons
                          int D, int Skv_pad, int fp8_fmt, int stages, int* range_flag, int* status, void* stream);
 
 /* A whole attention call on bf16 / fp16 inputs: quantises Q and K, prepares V and runs the fused forward - the work of
- * mxfp_attn_kernel (ours/mxfp_attn_kernel.py:19-74) in two launches, one more with smooth_k and one more where the keys of a
- * query tile are divided among CTAs (few query tiles, or a nearly empty last wave).  Strides are in elements.
+ * mxfp_attn_kernel (ours/mxfp_attn_kernel.py:19-74) in two launches, one more with smooth_k on long keys or many heads and one
+ * more where the keys of a query tile are divided among CTAs (few query tiles, or a nearly empty last wave).  Strides are in elements.
  *   q [B,Hq,S,D], k / v [B,Hkv,Skv,D], D 64 or 128.  k null: keys and values prepared earlier (k8 .. v4_sf, Skv_pad, as in
  *                 mpsa_attn_fwd, depth padded to 128) are used instead; formats that `uniform` leaves out may be null
  *   band, uniform precision rule: MXFP8 within `band` tiles of the diagonal; uniform 1: every tile MXFP8, 2: MXFP4, 0: neither

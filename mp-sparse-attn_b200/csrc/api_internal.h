@@ -34,8 +34,9 @@ bool allow_smem(F* kernel, int bytes) {
   return true;
 }
 
-// A launch that may start while the kernel before it on the stream drains (dependent: that kernel must be one of ours and
-// this one must call grid_dependency_wait() before it touches memory that the other writes or reads).
+// A launch that may start (dependent) while the kernel before it on the stream, whosever it is, still runs: once every CTA of that one has
+// ended or let its dependents go.  The kernel must call grid_dependency_wait() before it touches memory that anything before it on the
+// stream may write or read, in every CTA that does, and every launch after it has to be able to rely on that: see overlaps_previous.
 template <typename... P, typename... A>
 void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, bool dependent, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -52,8 +53,11 @@ void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t 
 }
 
 // Whether the first launch of a call may be a dependent one of whatever is before it on the stream: its CTAs then set up, and wait in
-// grid_dependency_wait(), under that kernel's tail.  Every kernel launched so waits before it touches memory, and lets its own
-// dependents go no earlier, so that what follows knows everything before it to be complete.  Not while the stream is captured: a
+// grid_dependency_wait(), under that kernel's tail.  A wait is for the one kernel before, so what follows has to know everything earlier to
+// be complete when that one is: the first kernels of a call (preparation, column sums, product) wait in every thread, and only then let
+// their dependents go.  Two later ones let them go before they wait, and wait all the same before they end: the preparation behind the
+// column sums, which starts only when those have seen the end of everything before them, and nvfp4_quant_kernel behind the preparation.
+// Not while the stream is captured: a
 // graph node with several predecessors takes ordinary edges.  Back to back: NVFP4
 // 1500 x 4096 x 4096 18.5 -> 17.2 us, routed attention over 1024 tokens 28.4 -> 27.4.
 inline bool overlaps_previous(cudaStream_t st) {

@@ -1,6 +1,7 @@
-// The whole attention call on 16-bit inputs behind one C entry: operand preparation and the forward, two launches (three with
-// smooth K), every intermediate in one workspace of the caller.  A short call is bound by the host: nine launches, as many
-// allocations and a C call for each cost 190 us where the GPU needs 40; this entry takes 8 from native.cpp (25 through ctypes, 20 of them Python).
+// The whole attention call on 16-bit inputs behind one C entry: operand preparation and the forward, two launches (one more for the
+// column sums of smooth K where prep_own_sums says so, two more for NVFP4, one more where keys are divided), every intermediate in one
+// workspace of the caller.  A short call is bound by the host: seven to nine launches, as many allocations and a C call for each cost 174 -
+// 192 us of its time where the GPU needs 14; through this entry and native.cpp a whole call takes 10.
 // Also the reference's two-operand quantizers in one launch.
 #include "../../include/mpsa.h"
 #include "api_internal.h"

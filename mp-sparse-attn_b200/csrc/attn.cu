@@ -106,7 +106,8 @@ constexpr uint32_t ENTRY_F8 = 0x8000, ENTRY_MASK = 0x4000, ENTRY_TILE = 0x3fff; 
 
 // Exponentials of a 32-key block that run on the FMA pipe (ex2_poly2).  MXFP4 tiles with quantised P.V, exponentials before the
 // block's maximum (LATE): 512 queries of 32K 179 us with 0, 173 with 2, 164 with 4, 170 with 6.  Where they wait for the maximum:
-// routed causal 8K 400 us with 0, 397 with 2, 401 with 4.  fp16 P: NVFP4 video back to back 18.5 ms with 0, 17.6 with 2, 18.3 with 4.
+// routed causal 8K 400 us with 0, 397 with 2, 401 with 4.  fp16 P, with 0 / 2 / 4 / 6, back to back under the power limit: NVFP4 video
+// 15.49 / 15.38 / 15.55 / 15.82 ms, 32 heads of 8192 884 / 877 / 883 / 896 us; in bursts 8 heads of 8192 264 / 259 / 264 / 261 us.
 constexpr int ATT_POLY_LATE = 4, ATT_POLY_EARLY = 2, ATT_POLY_F16 = 2;
 constexpr int ATT_F16_EARLY = 4;                      // fp16 P.V: exponentials of the second block that hide the vote on the reference
 constexpr int SPLIT_MIN_RUN = 8;                      // tiles of a run at least

@@ -1,6 +1,6 @@
 // The short way from torch tensors into libmpsa.so: checks, output allocation and the C call of the three entry points that programs
-// call most, in one step.  Through ctypes and struct the same took 8 - 11 us a call of the host's time, here 3: back to back, a pair of
-// quantizers over 4500 tokens 16.5 -> 11.0 us, causal attention over 128 tokens 17.0 -> 11.0.  Outputs and workspaces come from torch's allocator through its dispatcher, as
+// call most, in one step.  Up to the C call that took 8 - 11 us of the host's time through ctypes and struct, here 3: back to back, a pair
+// of quantizers over 4500 tokens 16.5 -> 11.0 us, causal attention over 128 tokens 17.0 -> 11.0.  Outputs and workspaces come from torch's allocator through its dispatcher, as
 // torch.empty does, and like there the interpreter's lock is released from the first of them to the end of the C call: an allocation may
 // wait for the device, and a launch for room in its queue.  Operands that the one-launch paths do not take make a function return
 // None, and the caller goes the long way; an error code of the C entry is returned as an int.

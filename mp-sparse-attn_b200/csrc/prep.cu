@@ -531,7 +531,9 @@ template <typename T, bool W8, bool W4, bool E4M3, bool D64, bool OWN>
 __global__ void __launch_bounds__(PREP_THREADS, W4 ? 3 : 4) prep_kernel(const __grid_constant__ PrepCall p) {
   extern __shared__ __align__(128) uint8_t prep_smem[];
   int cta = blockIdx.x;
-  if (!p.after_sums) grid_dependency_wait();            // (behind the column sums: where they are read)
+  // Behind the column sums only what reads them waits: this kernel starts once they have seen the end of everything before them, and
+  // some CTA of K waits for them in any case, so that what follows finds them complete.
+  if (!p.after_sums) grid_dependency_wait();
   grid_dependents_go();
   if (cta == 0 && threadIdx.x < 2) {
     // words the launches behind this one expect to find zero

@@ -582,6 +582,8 @@ template <typename T>
 __global__ void __launch_bounds__(kQuantThreads, sizeof(T) == 2 ? 4 : 2) nvfp4_quant_kernel(const QuantNvParams p) {
   __shared__ __align__(16) uint8_t sf[2][512];
   const int tid = threadIdx.x;
+  // (First the dependents: the one before has waited, so what the call reads is complete, and this one ends after it in any case.  For the
+  // same reason the operand, which nothing writes any more when this kernel starts, may be read by non-coherent loads.)
   grid_dependents_go();
   grid_dependency_wait();
   const T* xb = reinterpret_cast<const T*>(p.x) + (blockIdx.z / p.H) * p.xs_b + (blockIdx.z % p.H) * p.xs_h;

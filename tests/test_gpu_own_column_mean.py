@@ -1,4 +1,4 @@
-"""Smooth K in one launch (the CTAs of K add up their head's columns themselves) against the launch of its own that longer keys take:
+"""Smooth K in one launch (the CTAs of K add up their head's columns themselves) against the launch of its own that longer keys and many heads take:
 the sums are formed in the same order, so the quantised keys and the output are the same bit for bit."""
 import pytest
 import torch
