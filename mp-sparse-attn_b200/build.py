@@ -97,5 +97,8 @@ def build_native(force=False):
 
 
 if __name__ == "__main__":
-    print(build_native("--force" in sys.argv))
     print(build_lib(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    try:
+        print(build_native("--force" in sys.argv))
+    except (ImportError, OSError, RuntimeError) as e:      # (no torch, no compiler, no headers: short calls go through ctypes)
+        print(f"not built: the native module for short calls ({type(e).__name__}: {e})", file=sys.stderr)

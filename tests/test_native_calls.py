@@ -177,6 +177,25 @@ def test_without_the_module_every_call_is_left_to_the_long_way(no_module):
     assert [no_module.attention(1), no_module.quant_pair(2, 3), no_module.gemm()] == [None] * 3
 
 
+def test_build_without_the_module_still_builds_the_library(tmp_path):
+    import os
+    import shutil
+    import subprocess
+    import sys
+
+    from mpsa import _lib
+    here = os.path.dirname(os.path.dirname(_lib.lib_path()))
+    top = tmp_path / "package"
+    (top / "mpsa").mkdir(parents=True)
+    shutil.copytree(os.path.join(here, "csrc"), top / "csrc")
+    shutil.copytree(os.path.join(os.path.dirname(here), "include"), tmp_path / "include")
+    shutil.copy(os.path.join(here, "build.py"), top / "build.py")
+    lib = top / "mpsa" / "libmpsa.so"                     # up to date: nothing to compile
+    lib.write_bytes(b"")
+    r = subprocess.run([sys.executable, str(top / "build.py")], env=dict(os.environ, CXX=str(tmp_path / "no-compiler")), capture_output=True, text=True)
+    assert r.returncode == 0 and str(lib) in r.stdout and "not built" in r.stderr, (r.stdout, r.stderr)
+
+
 def test_the_module_is_that_of_this_python_and_torch():
     import sysconfig
 
